@@ -135,6 +135,29 @@ struct CantorFFT {
     }
 };
 
+// gf2x_fft_mul_buf's steps one by one on device buffers of n words: gf2e_mul
+// takes fa and fb as scratch, while the reference leaves the product's chunk
+// coefficients in FA and the transform of b in FB (untouched for a square)
+static inline int gf2e_mul_steps(const gf2e_fft_plan *plan, size_t n, const uint64_t *a,
+                                 uint64_t abits, const uint64_t *b, uint64_t bbits, uint64_t *out,
+                                 uint64_t *FA, uint64_t *FB) {
+    const size_t ca = (size_t)((abits + 31) >> 5), cb = (size_t)((bbits + 31) >> 5);
+    if (!abits || !bbits || ca + cb - 1 > n)      // gf2e_mul's own error
+        return gf2e_mul(plan, a, abits, b, bbits, out, FA, FB, nullptr);
+    const bool square = a == b && abits == bbits;
+    int st = gf2e_fft_pack(a, (size_t)((abits + 63) >> 6), FA, ca, n, nullptr);
+    if (st == GF2E_OK) st = gf2e_fft_fwd(plan, FA, nullptr);
+    if (st == GF2E_OK && !square) {
+        st = gf2e_fft_pack(b, (size_t)((bbits + 63) >> 6), FB, cb, n, nullptr);
+        if (st == GF2E_OK) st = gf2e_fft_fwd(plan, FB, nullptr);
+    }
+    if (st == GF2E_OK) st = gf2e_fft_pointwise(FA, square ? FA : FB, n, nullptr);
+    if (st == GF2E_OK) st = gf2e_fft_inv(plan, FA, nullptr);
+    if (st == GF2E_OK)
+        st = gf2e_fft_overlap_add(FA, ca + cb - 1, out, gf2e_mul_out_words(abits, bbits), nullptr);
+    return st;
+}
+
 // gf2_cantor_engine.h:207-229: host operands, host scratch FA and FB of F.n
 // words each.  The product runs on the GPU; on return out holds the
 // mul_out_words(abits, bbits) product words, FA the inverse transform (the
@@ -154,8 +177,8 @@ static inline void gf2x_fft_mul_buf(const u64 *a, u64 abits, const u64 *b, u64 b
     da.ensure(wa); db.ensure(wb); dout.ensure(ow); fa.ensure(F.n); fb.ensure(F.n);
     gf2e_or_die(gf2e_copy_to_device(da.get(), a, wa * 8, nullptr), "upload");
     gf2e_or_die(gf2e_copy_to_device(db.get(), b, wb * 8, nullptr), "upload");
-    gf2e_or_die(gf2e_mul(F.plan.get(), da.get(), abits, db.get(), bbits, dout.get(), fa.get(),
-                         fb.get(), nullptr), "gf2x_fft_mul_buf");
+    gf2e_or_die(gf2e_mul_steps(F.plan.get(), F.n, da.get(), abits, db.get(), bbits, dout.get(),
+                               fa.get(), fb.get()), "gf2x_fft_mul_buf");
     gf2e_or_die(gf2e_copy_to_host(out, dout.get(), ow * 8, nullptr), "download");
     gf2e_or_die(gf2e_copy_to_host(FA, fa.get(), F.n * 8, nullptr), "download");
     gf2e_or_die(gf2e_copy_to_host(FB, fb.get(), F.n * 8, nullptr), "download");
@@ -177,7 +200,7 @@ static inline void k_overlap_add(const u64 *F, size_t nchunks, u64 *out, size_t 
 // gf2_cantor_engine.h:207-229: device operands and scratch
 static inline void gf2x_fft_mul_buf_dev(const u64 *a, u64 abits, const u64 *b, u64 bbits,
                                         u64 *out, const CudaFFT &F, u64 *FA, u64 *FB) {
-    gf2e_or_die(gf2e_mul(F.plan, a, abits, b, bbits, out, FA, FB, nullptr), "gf2x_fft_mul");
+    gf2e_or_die(gf2e_mul_steps(F.plan, F.n, a, abits, b, bbits, out, FA, FB), "gf2x_fft_mul");
 }
 
 // gf2_cantor_engine.h:232-242: host operands, out = mul_out_words words

@@ -19,6 +19,7 @@
 // table is streamed from HBM.
 #include "gf2e_internal.cuh"
 #include "wrapmul.cuh"
+#include "slicefft_api.cuh"
 
 #include <cstdlib>
 #include <cstring>
@@ -854,7 +855,8 @@ gf2e_tune resolve_by_size(gf2e_tune c, int m) {
 int fft_plan_create_tables_cfg(int m, const u64 *tab_dev, const gf2e_tune &cfg,
                                gf2e_fft_plan **out) {
     if (m < 1 || m > 30) return invalid("FFT size exponent m=%d outside 1..30", m);
-    if (!basis_host()) return invalid("Cantor basis construction failed");
+    static const bool images_ok = basis_host() && slice_selfcheck(basis_host());
+    if (!images_ok) return invalid("Cantor basis construction failed");
     GF2E_TRY(allow_tile_smem());
     gf2e_fft_plan *p = new gf2e_fft_plan;
     p->impl.m = m;
@@ -892,11 +894,6 @@ int fft_plan_create_cfg(int m, const gf2e_tune &cfg, gf2e_fft_plan **out) {
 
 int fft_plan_create(int m, gf2e_fft_plan **out) {
     return fft_plan_create_cfg(m, tune_current(), out);
-}
-
-int fft_fwd_packed(const gf2e_fft_plan *plan, u64 *f, const u32 *src32, u64 nchunks,
-                   cudaStream_t st) {
-    return run_passes(plan->impl, true, f, src32, nchunks, st);
 }
 
 int fft_run(const gf2e_fft_plan *plan, bool forward, u64 *f, cudaStream_t st) {
@@ -945,6 +942,44 @@ int mul_fft_m(u64 abits, u64 bbits) {
     return m;
 }
 
+// Products of at most 2^24 coefficients take the bit-sliced transform
+// (slicefft.cu): up to 2^12 in one block, else in the transform buffers where
+// these are aligned for its 16-byte accesses.
+int product_batch(const gf2e_fft_plan *plan, const ProductOp &a, const ProductOp &b, int batch,
+                  u64 *fa, u64 *fb, u64 fstride, u64 *out, u64 ostride, u64 ow,
+                  cudaStream_t st) {
+    const u64 count = a.nchunks + b.nchunks - 1;
+    int m = SLICE_MIN_M;
+    while (((u64)1 << m) < count) m++;
+    // a wrapped product has more coefficients than its transform
+    m = std::min(m, std::max(plan->impl.m, SLICE_MIN_M));
+    const bool same = a.words == b.words && a.stride == b.stride && a.nchunks == b.nchunks &&
+                      a.xor0 == b.xor0;
+    const u32 *sa = reinterpret_cast<const u32 *>(a.words);
+    const u32 *sb = reinterpret_cast<const u32 *>(b.words);
+    const bool aligned = ((uintptr_t)fa | (uintptr_t)fb) % 16 == 0 && fstride % 2 == 0;
+    if (m <= SLICE_SMALL_MAX_M || (m <= SLICE_MAX_M && aligned)) {
+        const SliceOp op[2] = {{sa, 2 * a.stride, a.nchunks, (u32)a.xor0, fa},
+                               {sb, 2 * b.stride, b.nchunks, (u32)b.xor0, fb}};
+        if (m <= SLICE_SMALL_MAX_M)
+            return slice_small(m, op[0], op[1], batch, out, ostride, ow, st);
+        GF2E_TRY(slice_fwd(m, op, same ? 1 : 2, fstride, batch, st));
+        GF2E_TRY(slice_pointwise(fa, fa, same ? fa : fb, nullptr, nullptr, (u64)1 << m, fstride,
+                                 batch, st));
+        return slice_inv(m, fa, fb, fstride, batch, out, ostride, ow, st);
+    }
+    const u64 n = plan->impl.n;
+    GF2E_TRY(fft_fwd_packed_batch(plan, fa, fstride, sa, 2 * a.stride, a.nchunks, a.xor0, batch,
+                                  st));
+    if (!same)
+        GF2E_TRY(fft_fwd_packed_batch(plan, fb, fstride, sb, 2 * b.stride, b.nchunks, b.xor0,
+                                      batch, st));
+    for (int i = 0; i < batch; i++)
+        GF2E_TRY(pointwise(fa + i * fstride, (same ? fa : fb) + i * fstride, n, st));
+    GF2E_TRY(fft_run_batch(plan, false, fa, fstride, batch, st));
+    return overlap_add_batch(fa, fstride, std::min(count, n), out, ostride, ow, batch, st);
+}
+
 // full product with a plan of size >= the needed one (gf2x_fft_mul_buf)
 int mul(const gf2e_fft_plan *plan, const u64 *a, u64 abits, const u64 *b, u64 bbits,
         u64 *out, u64 *fa, u64 *fb, cudaStream_t st) {
@@ -954,16 +989,8 @@ int mul(const gf2e_fft_plan *plan, const u64 *a, u64 abits, const u64 *b, u64 bb
     if (ca + cb - 1 > n) return invalid("FFT too small: plan m=%d for %llu x %llu bits",
                                          plan->impl.m, (unsigned long long)abits,
                                          (unsigned long long)bbits);
-    GF2E_TRY(fft_fwd_packed(plan, fa, reinterpret_cast<const u32 *>(a), ca, st));
-    if (b == a && bbits == abits) {
-        GF2E_TRY(pointwise(fa, fa, n, st));
-    } else {
-        GF2E_TRY(fft_fwd_packed(plan, fb, reinterpret_cast<const u32 *>(b), cb, st));
-        GF2E_TRY(pointwise(fa, fb, n, st));
-    }
-    GF2E_TRY(fft_run(plan, false, fa, st));
-    u64 ow = ((abits + bbits + 63) >> 6) + 1;
-    return overlap_add(fa, ca + cb - 1, out, ow, st);
+    return product_batch(plan, ProductOp{a, 0, ca, 0}, ProductOp{b, 0, cb, 0}, 1, fa, fb, 0, out,
+                         0, ((abits + bbits + 63) >> 6) + 1, st);
 }
 
 // plan cache shared by the batch API and the trinomial context

@@ -40,6 +40,7 @@
 // Mbit kept 16 host cores busy on stream waits and launches while the GPU
 // idled between kernels.
 #include "gf2e_internal.cuh"
+#include "slicefft_api.cuh"
 
 #include <algorithm>
 #include <atomic>
@@ -1152,11 +1153,19 @@ private:
         for (size_t g = 0; g < p.deg.size(); g++) c = std::max(c, chunks(p, (int)g));
         return c;
     }
+    // the bit-sliced transform serves every size it has (slicefft.cu)
+    static bool sliced(const gf2e_fft_plan *plan) {
+        const int m = gf2e_fft_plan_m(plan);
+        return m >= gf2e::SLICE_MIN_M && m <= gf2e::SLICE_MAX_M;
+    }
     // forward transforms of every member of p into f (G x n)
     void fwd(gf2e_fft_plan *plan, const BPoly &p, u64 *f, u64 n) {
         const u64 nch = max_chunks(p);
         if (!nch) ckc(cudaMemsetAsync(f, 0, (size_t)G_ * n * 8, st_), "fft zero operand");
-        else ck(gf2e::fft_fwd_packed_batch(plan, f, n, reinterpret_cast<const u32 *>(p.base()),
+        else if (sliced(plan)) {
+            const gf2e::SliceOp op{reinterpret_cast<const u32 *>(p.base()), 2 * p.stride, nch, 0, f};
+            ck(gf2e::slice_fwd(gf2e_fft_plan_m(plan), &op, 1, n, G_, st_));
+        } else ck(gf2e::fft_fwd_packed_batch(plan, f, n, reinterpret_cast<const u32 *>(p.base()),
                                            2 * p.stride, nch, 0, G_, st_));
     }
     // o <- inverse of X1 Y1 + X2 Y2 (pointwise), overlap-added into a new
@@ -1164,16 +1173,29 @@ private:
     BPoly product_out(gf2e_fft_plan *plan, u64 *o, const u64 *x1, const u64 *y1, const u64 *x2,
                       const u64 *y2, u64 n, u64 need, const std::vector<long long> &dm) {
         const u64 tot = (u64)G_ * n;
-        k_pw_muladd<<<gf2e::grid_for(tot, 256), 256, 0, st_>>>(o, x1, y1, x2, y2, tot);
-        ckc(cudaGetLastError(), "k_pw_muladd");
-        ck(gf2e::fft_run_batch(plan, false, o, n, G_, st_));
         u64 so = 1;
         for (int g = 0; g < G_; g++)
             if (dm[g] >= 0) so = std::max(so, (u64)(dm[g] >> 6) + 2);
+        if (sliced(plan)) {
+            const int m = gf2e_fft_plan_m(plan);
+            Buf t = m > 16 ? alloc(tot) : Buf();
+            ck(gf2e::slice_pointwise(o, x1, y1, x2, y2, n, n, G_, st_));
+            BPoly out = make(so, false);
+            ck(gf2e::slice_inv(m, o, t ? t->p : nullptr, n, G_, out.base(), so, so, st_));
+            set_bounds(out, so, dm);
+            return out;
+        }
+        k_pw_muladd<<<gf2e::grid_for(tot, 256), 256, 0, st_>>>(o, x1, y1, x2, y2, tot);
+        ckc(cudaGetLastError(), "k_pw_muladd");
+        ck(gf2e::fft_run_batch(plan, false, o, n, G_, st_));
         BPoly out = make(so, false);
         ck(gf2e::overlap_add_batch(o, n, need, out.base(), so, so, G_, st_));
-        for (int g = 0; g < G_; g++) out.deg[g] = dm[g] < 0 ? -1 : std::min<long long>(dm[g], (long long)so * 64 - 1);
+        set_bounds(out, so, dm);
         return out;
+    }
+    void set_bounds(BPoly &out, u64 so, const std::vector<long long> &dm) const {
+        for (int g = 0; g < G_; g++)
+            out.deg[g] = dm[g] < 0 ? -1 : std::min<long long>(dm[g], (long long)so * 64 - 1);
     }
 
     // (c, d) = M (a, b); exact degrees

@@ -44,13 +44,6 @@ int frobenius_states(u64 *a, u64 *b, size_t stride, int nstates, u64 r, const u6
 int trin_set_const(u64 *states, size_t stride, int nstates, u64 r, u64 w0, cudaStream_t st);
 int trin_reduce_batch(const u64 *P, size_t pstride, size_t pw, u64 L, u64 *out, size_t ostride,
                       u64 r, const u64 *s_dev, int batch, cudaStream_t st);
-int fft_fwd_packed_batch(const gf2e_fft_plan *plan, u64 *f, u64 fstride, const u32 *src32,
-                         u64 sstride32, u64 nchunks, u64 xor0, int batch, cudaStream_t st);
-int fft_run_batch(const gf2e_fft_plan *plan, bool forward, u64 *f, u64 fstride, int batch,
-                  cudaStream_t st);
-int overlap_add_batch(const u64 *F, u64 fstride, u64 nchunks, u64 *out, u64 ostride, u64 ow,
-                      int batch, cudaStream_t st);
-int pointwise(u64 *fa, const u64 *fb, u64 n, cudaStream_t st);
 int mul_fft_m(u64 abits, u64 bbits);
 gf2e_fft_plan *cached_plan(int m);
 u64 fft_plan_n(const gf2e_fft_plan *plan);
@@ -215,7 +208,7 @@ Geometry geometry(u64 r) {
 size_t device_words(const Geometry &g, int B, int m = 1) {
     size_t w = 3 * g.stride * B + 2 * g.n * B + g.pstride * B + g.tw * B + B + g.gcap * B;
     if (m > 1) w += 2 * (size_t)m * g.stride * B + g.stride * B + (size_t)m * B;
-    if (g.wrap) w += (size_t)g.wm.per * B;
+    if (g.wrap) w = ((w + 1) & ~(size_t)1) + (size_t)g.wm.per * B;   // 16-byte aligned
     return w;
 }
 
@@ -373,26 +366,22 @@ int fill_slots(gf2e_scanner &S, cudaStream_t st) {
     return GF2E_OK;
 }
 
-// the product's last step: P = ACC * B from the inverse transform in FA
-// (overlap-add, and for wrapped products the top part put back)
-int product_tail(gf2e_scanner &S, int na, const u64 *B, cudaStream_t st) {
-    if (S.wrap)
-        return gf2e::wrap_mul_finish(S.wm, S.FA, S.n, S.ACC, S.stride, B, S.stride, S.P,
-                                     S.pstride, S.ow, na, S.WS, st);
-    return gf2e::overlap_add_batch(S.FA, S.n, 2 * S.nchunks - 1, S.P, S.pstride, S.ow, na, st);
+// P = ACC * (B + xor0) (for wrapped products the top part put back; B alone
+// there: xor0 changes no bit of the top part)
+int product(gf2e_scanner &S, int na, const u64 *B, u64 xor0, cudaStream_t st) {
+    GF2E_TRY(gf2e::product_batch(S.plan, gf2e::ProductOp{S.ACC, S.stride, S.nchunks, 0},
+                                 gf2e::ProductOp{B, S.stride, S.nchunks, xor0}, na, S.FA, S.FB,
+                                 S.n, S.P, S.pstride, S.ow, st));
+    if (!S.wrap) return GF2E_OK;
+    return gf2e::wrap_mul_finish(S.wm, S.ACC, S.stride, B, S.stride, S.P, S.pstride, S.ow, na,
+                                 S.WS, st);
 }
 
 // the launches of one degree for `na` resident s (F -> Fs squared; the
 // product then reads Fs, which becomes F)
 int degree_kernels(gf2e_scanner &S, int na, u64 *F, u64 *Fs, cudaStream_t st) {
     GF2E_TRY(gf2e::trin_square_states(F, Fs, S.stride, na, S.r, S.sdev, st));
-    GF2E_TRY(gf2e::fft_fwd_packed_batch(S.plan, S.FA, S.n, reinterpret_cast<const u32 *>(S.ACC),
-                                        2 * S.stride, S.nchunks, 0, na, st));
-    GF2E_TRY(gf2e::fft_fwd_packed_batch(S.plan, S.FB, S.n, reinterpret_cast<const u32 *>(Fs),
-                                        2 * S.stride, S.nchunks, 2, na, st));
-    GF2E_TRY(gf2e::pointwise(S.FA, S.FB, S.n * na, st));
-    GF2E_TRY(gf2e::fft_run_batch(S.plan, false, S.FA, S.n, na, st));
-    GF2E_TRY(product_tail(S, na, Fs, st));
+    GF2E_TRY(product(S, na, Fs, 2, st));
     GF2E_TRY(gf2e::trin_reduce_batch(S.P, S.pstride, S.ow, 2 * S.r - 1, S.ACC, S.stride, S.r,
                                      S.sdev, na, st));
     return GF2E_OK;
@@ -407,13 +396,7 @@ int block_kernels(gf2e_scanner &S, int na, cudaStream_t st) {
     GF2E_CHECK_LAUNCH("k_horner");
     k_horner_fold<<<na, 32, 0, st>>>(S.H, S.stride, m, S.C, S.r, S.sdev);
     GF2E_CHECK_LAUNCH("k_horner_fold");
-    GF2E_TRY(gf2e::fft_fwd_packed_batch(S.plan, S.FA, S.n, reinterpret_cast<const u32 *>(S.ACC),
-                                        2 * S.stride, S.nchunks, 0, na, st));
-    GF2E_TRY(gf2e::fft_fwd_packed_batch(S.plan, S.FB, S.n, reinterpret_cast<const u32 *>(S.C),
-                                        2 * S.stride, S.nchunks, 0, na, st));
-    GF2E_TRY(gf2e::pointwise(S.FA, S.FB, S.n * na, st));
-    GF2E_TRY(gf2e::fft_run_batch(S.plan, false, S.FA, S.n, na, st));
-    GF2E_TRY(product_tail(S, na, S.C, st));
+    GF2E_TRY(product(S, na, S.C, 0, st));
     GF2E_TRY(gf2e::trin_reduce_batch(S.P, S.pstride, S.ow, 2 * S.r - 1, S.ACC, S.stride, S.r,
                                      S.sdev, na, st));
     // h <- h^(2^m): m squarings of every residue, two per pass, back in H

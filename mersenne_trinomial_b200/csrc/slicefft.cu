@@ -1,0 +1,451 @@
+// slicefft.cu -- launches of the bit-sliced product transform
+// (slicefft.cuh): products of up to 2^24 32-bit chunk coefficients.
+//
+// A product of 2^m coefficients is seven short passes over memory a side:
+// chunk words to planes, Taylor levels above 2^16 (m > 16), the 2^16-chunk
+// conversions in shared memory 4 or 8 planes at a time (planes are
+// independent), then the butterflies in two passes over tiles of up to 512
+// slices (128 KB): levels m-1 .. low over strided rows, low-1 .. 0 over
+// consecutive slices.  Levels above an operand's own size are copies, made
+// when its conversion is stored.  Between the transforms the values stay
+// bit-sliced in the tower basis, in the order the last pass leaves them.
+#include "gf2e_internal.cuh"
+#include "slicefft.cuh"
+#include "slicefft_api.cuh"
+
+#include <algorithm>
+#include <atomic>
+
+namespace {
+
+using namespace slice;
+using gf2e::SLICE_MAX_M;
+using gf2e::SLICE_MIN_M;
+
+struct DevEx {
+    template <class F> GF2E_DEV void operator()(const F &f) const {
+        f(threadIdx.x, blockDim.x);
+        __syncthreads();
+    }
+};
+
+constexpr int IN_LOG = 7;                    // slices a block of k_slice_in / out
+constexpr int BFLY_THREADS = 512;
+constexpr int TAYLOR_THREADS = 512;
+
+// up to two operands, `batch` transforms each: blockIdx.y = operand * batch + i
+struct In {
+    const u32 *src[2];
+    u64 sstride[2], nchunks[2];
+    u32 xor0[2];
+    uint4 *f[2];
+    u64 fstride;                             // in 16-byte chunks
+    int k[2];                                // 2^k slices' coefficients converted
+    int batch;
+};
+
+__global__ void __launch_bounds__(1 << IN_LOG) k_slice_in(const In a) {
+    __shared__ u32 sm[33 << IN_LOG];
+    const int o = (int)blockIdx.y / a.batch, i = (int)blockIdx.y - o * a.batch;
+    if ((blockIdx.x << (IN_LOG + 5)) >= (1u << a.k[o])) return;
+    body_slice_in(DevEx{}, sm, a.src[o] + i * a.sstride[o], a.nchunks[o], a.xor0[o],
+                  a.f[o] + i * a.fstride, blockIdx.x << IN_LOG,
+                  a.k[o] - 5 < IN_LOG ? a.k[o] - 5 : IN_LOG);
+}
+
+// one operand's 2^k coefficients, blocks of 2^kt; blockIdx.x = block * groups
+// + plane group
+struct TaylorArgs {
+    uint4 *f;
+    u64 fstride;
+    int kt, plog, groups;
+    u32 c_src, reps, rep_stride;
+    Levels lv;
+};
+template <bool FWD>
+__global__ void __launch_bounds__(TAYLOR_THREADS, 2) k_taylor(const TaylorArgs a) {
+    extern __shared__ uint4 sm4[];
+    const u32 b = blockIdx.x / a.groups, g = blockIdx.x - b * a.groups;
+    const u32 c = g << (a.plog - 2);
+    body_taylor<FWD>(DevEx{}, reinterpret_cast<u32 *>(sm4), a.f + blockIdx.y * a.fstride,
+                     b << (a.kt - 5), a.kt, a.plog, c, a.c_src + c, a.reps, a.rep_stride, a.lv);
+}
+
+struct HiArgs {
+    const uint4 *src;
+    uint4 *dst;
+    u64 sstride, dstride;
+    u32 c_dst;
+    int groups;
+    HiGeom G;
+    Levels rows;
+};
+template <bool FWD>
+__global__ void __launch_bounds__(TAYLOR_THREADS, 2) k_taylor_hi(const HiArgs a) {
+    extern __shared__ uint4 sm4[];
+    u32 *sm = reinterpret_cast<u32 *>(sm4);
+    u32 *side = sm + ((hi_pitch(a.G) << a.G.rlog) << a.G.plog);
+    const u32 ct = blockIdx.x / a.groups, g = blockIdx.x - ct * a.groups;
+    const u32 c = g << (a.G.plog - 2);
+    body_taylor_hi<FWD>(DevEx{}, sm, side, a.src + blockIdx.y * a.sstride, c,
+                        a.dst + blockIdx.y * a.dstride, a.c_dst + c, a.G, ct, a.rows);
+}
+
+struct BflyArgs {
+    uint4 *f[2];
+    u64 fstride;
+    int m, rlog, clog, llo, collog;          // 2^collog column groups a window
+    int top[2];
+    int batch;
+};
+template <int NQ, bool FWD, bool EDGE, bool LOWP>
+__global__ void __launch_bounds__(BFLY_THREADS, 1) k_bfly(const BflyArgs a) {
+    extern __shared__ uint4 sm4[];
+    const int o = (int)blockIdx.y / a.batch, i = (int)blockIdx.y - o * a.batch;
+    const u32 win = blockIdx.x >> a.collog, col = blockIdx.x & ((1u << a.collog) - 1);
+    Tile T;
+    T.m = a.m;
+    T.rlog = a.rlog;
+    T.clog = a.clog;
+    T.llo = a.llo;
+    T.base = (win << (a.llo + a.rlog - 5)) + (col << a.clog);
+    body_bfly<NQ, FWD>(DevEx{}, sm4, a.f[o] + i * a.fstride, T, a.top[o], EDGE, LOWP);
+}
+
+// o = x1 y1 (+ x2 y2 where TWO) over 128 slices a block
+template <bool TWO>
+__global__ void __launch_bounds__(128, 2)
+k_slice_mul(uint4 *o, const uint4 *x1, const uint4 *y1, const uint4 *x2, const uint4 *y2,
+            u64 nslices, u64 fstride) {
+    extern __shared__ uint4 sm4[];
+    const u64 s0 = (u64)blockIdx.x * 128, y = blockIdx.y * fstride;
+    o += y;
+    x1 += y;
+    y1 += y;
+    if (TWO) {
+        x2 += y;
+        y2 += y;
+    }
+    const u32 n = (u32)min((u64)128, nslices - s0);
+    const u32 tid = threadIdx.x;
+    uint4 *ta = sm4, *tb = sm4 + 128 * 16, *tc = tb + 128 * 16;
+    const bool same = x1 == y1;
+    for (u32 i = tid; i < n * 16; i += 128) {
+        const u32 at = chunk_at(i >> 4, i & 15);
+        ta[at] = x1[s0 * 16 + i];
+        if (!same) tb[at] = y1[s0 * 16 + i];
+    }
+    __syncthreads();
+    mul_slices(ta, same ? ta : tb, n, tid, 128);
+    __syncthreads();
+    if (TWO) {
+        for (u32 i = tid; i < n * 16; i += 128) {
+            const u32 at = chunk_at(i >> 4, i & 15);
+            tb[at] = x2[s0 * 16 + i];
+            tc[at] = y2[s0 * 16 + i];
+        }
+        __syncthreads();
+        mul_slices(tb, tc, n, tid, 128);
+        __syncthreads();
+    }
+    for (u32 i = tid; i < n * 16; i += 128) {
+        const u32 at = chunk_at(i >> 4, i & 15);
+        uint4 v = ta[at];
+        if (TWO) {
+            const uint4 w = tb[at];
+            v.x ^= w.x; v.y ^= w.y; v.z ^= w.z; v.w ^= w.w;
+        }
+        o[s0 * 16 + i] = v;
+    }
+}
+
+__global__ void __launch_bounds__(1 << IN_LOG)
+k_slice_out(const uint4 *f, u64 fstride, u32 nsl, u32 *out, u64 ostride, u64 words) {
+    __shared__ uint4 tile[16 << IN_LOG];
+    __shared__ u32 side[(1 << IN_LOG) + 1];
+    body_slice_out(DevEx{}, tile, side, f + blockIdx.y * fstride, nsl, out + blockIdx.y * ostride,
+                   words, blockIdx.x << IN_LOG, IN_LOG);
+}
+
+struct SmallArgs {
+    const u32 *src[2];
+    u64 sstride[2], nchunks[2];
+    u32 xor0[2];
+    int m, k[2];
+    Levels lv[2], lm;
+    u32 *out;
+    u64 ostride, words;
+};
+__global__ void __launch_bounds__(512, 1) k_small_mul(const SmallArgs a) {
+    extern __shared__ uint4 sm4[];
+    const u32 ns = 1u << (a.m - 5);
+    const u64 y = blockIdx.x;
+    body_small(DevEx{}, sm4, sm4 + ns * 16, reinterpret_cast<u32 *>(sm4 + ns * 32), a.m,
+               Operand{a.src[0] + y * a.sstride[0], a.nchunks[0], a.xor0[0]},
+               Operand{a.src[1] + y * a.sstride[1], a.nchunks[1], a.xor0[1]}, a.k[0], a.k[1],
+               a.lv[0], a.lv[1], a.lm, a.out + y * a.ostride, a.words);
+}
+
+constexpr size_t SMALL_SMEM = (size_t)(1 << (SMALL_M - 5)) * 512 + 4 * ((1 << (SMALL_M - 5)) + 1);
+constexpr size_t BFLY_SMEM = (size_t)(256 << TILE_LOG);
+constexpr size_t TAYLOR_SMEM = (size_t)(4 << 11) << 3;
+constexpr int HI_TLOG = 4;
+
+HiGeom hi_geom(int rlog) {
+    HiGeom G;
+    G.rlog = rlog;
+    G.tlog = HI_TLOG;
+    G.plog = rlog >= 8 ? 2 : 3;
+    G.halo = rlog <= 5 ? 1u : 1u << (rlog - 5);
+    return G;
+}
+size_t hi_smem(const HiGeom &G) {
+    return ((size_t)(hi_pitch(G) + G.halo) << G.rlog << G.plog) * 4;
+}
+
+int allow_smem() {
+    // set once per device; two threads racing here both set the same values
+    static std::atomic<bool> done[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64 && done[dev].load(std::memory_order_acquire)) return GF2E_OK;
+    cudaError_t e = cudaSuccess;
+    auto allow = [&](const void *k, size_t n) {
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n);
+    };
+    allow((const void *)k_taylor<true>, TAYLOR_SMEM);
+    allow((const void *)k_taylor<false>, TAYLOR_SMEM);
+    size_t hs = 0;
+    for (int r = 1; r <= 8; r++) hs = std::max(hs, hi_smem(hi_geom(r)));
+    allow((const void *)k_taylor_hi<true>, hs);
+    allow((const void *)k_taylor_hi<false>, hs);
+    allow((const void *)k_small_mul, SMALL_SMEM);
+    allow((const void *)k_slice_mul<false>, 2 * 128 * 256);
+    allow((const void *)k_slice_mul<true>, 3 * 128 * 256);
+#define GF2E_SL_ALLOW(NQ, F)                                         \
+    allow((const void *)k_bfly<NQ, F, false, false>, BFLY_SMEM);     \
+    allow((const void *)k_bfly<NQ, F, true, false>, BFLY_SMEM);      \
+    allow((const void *)k_bfly<NQ, F, false, true>, BFLY_SMEM);      \
+    allow((const void *)k_bfly<NQ, F, true, true>, BFLY_SMEM);
+    GF2E_SL_ALLOW(1, true) GF2E_SL_ALLOW(1, false) GF2E_SL_ALLOW(2, true) GF2E_SL_ALLOW(2, false)
+#undef GF2E_SL_ALLOW
+    if (e != cudaSuccess) return gf2e::cuda_status(e, "sliced transform smem attribute");
+    if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
+    return GF2E_OK;
+}
+
+// a plan per size (host arithmetic only): the last pass holds the levels
+// below m - 7 (10 to 14), so that 128 tiles and more keep the SMs busy from
+// m = 17 on; the upper rows come one slice (256 bytes) wide until a tile of
+// 512 slices is full
+const Plan &plan_for(int m) {
+    static const struct All {
+        Plan p[SLICE_MAX_M + 1];
+        All() {
+            for (int m = SLICE_MIN_M; m <= SLICE_MAX_M; m++) {
+                const int low = std::min(14, std::max(10, m - 7));
+                p[m] = make_plan(m, low, m >= 22 ? TILE_LOG : 0);
+            }
+        }
+    } all;
+    return all.p[m];
+}
+
+int clog2(u64 v) {
+    int k = 0;
+    while (((u64)1 << k) < v) k++;
+    return k;
+}
+
+template <bool FWD>
+int launch_taylor(uint4 *f, u64 fstride, int batch, int m, int k, u32 c_src, cudaStream_t st) {
+    const Plan &P = plan_for(m);
+    TaylorArgs a;
+    a.f = f;
+    a.fstride = fstride;
+    a.kt = std::min(k, 16);
+    const u32 blocks = 1u << (k - a.kt);
+    const int chunks = FWD ? 8 : 16;
+    // 8 planes a block (whole 32-byte sectors) unless that leaves SMs idle
+    a.plog = blocks * (chunks / 2) * (u32)batch >= (u32)gf2e::sm_count() ? 3 : 2;
+    a.groups = chunks >> (a.plog - 2);
+    a.c_src = c_src;
+    a.reps = FWD ? 1u << (m - k) : 1u;
+    a.rep_stride = 1u << (k - 5);
+    a.lv = P.taylor[a.kt];
+    const int threads = std::max(64, std::min(TAYLOR_THREADS, 1 << (a.kt - 6 + a.plog)));
+    k_taylor<FWD><<<dim3(blocks * a.groups, batch), threads, (size_t)4 << (a.kt - 5 + a.plog), st>>>(a);
+    GF2E_CHECK_LAUNCH("k_taylor");
+    return GF2E_OK;
+}
+
+template <bool FWD>
+int launch_hi(const uint4 *src, u64 sstride, uint4 *dst, u64 dstride, u32 c_dst, int batch, int m,
+              int k, cudaStream_t st) {
+    const Plan &P = plan_for(m);
+    HiArgs a;
+    a.src = src;
+    a.dst = dst;
+    a.sstride = sstride;
+    a.dstride = dstride;
+    a.c_dst = c_dst;
+    a.G = hi_geom(k - 16);
+    a.groups = (FWD ? 8 : 16) >> (a.G.plog - 2);
+    a.rows = P.rows[k - 16];
+    k_taylor_hi<FWD><<<dim3((2048 >> HI_TLOG) * a.groups, batch), TAYLOR_THREADS, hi_smem(a.G), st>>>(a);
+    GF2E_CHECK_LAUNCH("k_taylor_hi");
+    return GF2E_OK;
+}
+
+template <int NQ, bool FWD>
+int launch_bfly(const BflyArgs &a, u32 tiles, int ny, bool edge, bool lowp, cudaStream_t st) {
+    const int tl = a.rlog + a.clog;
+    const int threads = std::max(32, std::min(BFLY_THREADS, (1 << (tl - 1)) * (4 / NQ)));
+    const size_t smem = (size_t)256 << tl;
+    const dim3 g(tiles, ny);
+    if (edge && lowp) k_bfly<NQ, FWD, true, true><<<g, threads, smem, st>>>(a);
+    else if (edge) k_bfly<NQ, FWD, true, false><<<g, threads, smem, st>>>(a);
+    else if (lowp) k_bfly<NQ, FWD, false, true><<<g, threads, smem, st>>>(a);
+    else k_bfly<NQ, FWD, false, false><<<g, threads, smem, st>>>(a);
+    GF2E_CHECK_LAUNCH("k_bfly");
+    return GF2E_OK;
+}
+
+// pass i of the butterflies (i = ntop: the low pass)
+template <bool FWD>
+int run_bfly(const Plan &P, int i, BflyArgs a, int nops, cudaStream_t st) {
+    const bool lowp = i == P.ntop;
+    a.m = P.m;
+    a.llo = lowp ? 5 : P.top[i].llo;
+    a.rlog = lowp ? P.low - 5 : P.top[i].rlog;
+    a.clog = lowp ? 0 : P.top[i].clog;
+    a.collog = a.llo - 5 - a.clog;
+    const u32 tiles = 1u << (P.m - 5 - a.rlog - a.clog);
+    const int ny = nops * a.batch;
+    // a quarter of the planes a thread while that fills idle SMs (m <= 16:
+    // every twiddle is in GF(2^16)), else half of them for one twiddle
+    if (P.m <= 16 && (u64)tiles * ny < 2 * (u64)gf2e::sm_count())
+        return launch_bfly<1, FWD>(a, tiles, ny, i == 0, lowp, st);
+    return launch_bfly<2, FWD>(a, tiles, ny, i == 0, lowp, st);
+}
+
+}  // namespace
+
+namespace gf2e {
+
+bool slice_selfcheck(const u64 *basis) {
+    for (int i = 0; i < 25; i++) {
+        u64 v = 0;
+        for (int j = 0; j < 64; j++)
+            if ((basis[i] >> j) & 1) v ^= PHI.to[j];
+        if (v != CANTOR[i]) return false;
+    }
+    return true;
+}
+
+int slice_fwd(int m, const SliceOp *ops, int nops, u64 fstride, int batch, cudaStream_t st) {
+    GF2E_TRY(allow_smem());
+    const Plan &P = plan_for(m);
+    In in;
+    in.fstride = fstride / 2;
+    in.batch = batch;
+    u32 nx = 1;
+    for (int o = 0; o < nops; o++) {
+        in.src[o] = ops[o].src;
+        in.sstride[o] = ops[o].stride;
+        in.nchunks[o] = ops[o].nchunks;
+        in.xor0[o] = ops[o].xor0;
+        in.f[o] = reinterpret_cast<uint4 *>(ops[o].f);
+        in.k[o] = std::min(m, std::max(8, clog2(ops[o].nchunks)));
+        nx = std::max(nx, 1u << std::max(0, in.k[o] - 5 - IN_LOG));
+    }
+    k_slice_in<<<dim3(nx, nops * batch), 1 << IN_LOG, 0, st>>>(in);
+    GF2E_CHECK_LAUNCH("k_slice_in");
+    BflyArgs a;
+    a.fstride = in.fstride;
+    a.batch = batch;
+    for (int o = 0; o < nops; o++) {
+        u32 c = 0;
+        if (in.k[o] > 16) {
+            GF2E_TRY(launch_hi<true>(in.f[o], in.fstride, in.f[o], in.fstride, 8, batch, m, in.k[o], st));
+            c = 8;
+        }
+        GF2E_TRY(launch_taylor<true>(in.f[o], in.fstride, batch, m, in.k[o], c, st));
+        a.f[o] = in.f[o];
+        a.top[o] = in.k[o];
+    }
+    for (int i = 0; i <= P.ntop; i++) GF2E_TRY(run_bfly<true>(P, i, a, nops, st));
+    return GF2E_OK;
+}
+
+int slice_pointwise(u64 *o, const u64 *x1, const u64 *y1, const u64 *x2, const u64 *y2, u64 n,
+                    u64 fstride, int batch, cudaStream_t st) {
+    GF2E_TRY(allow_smem());
+    const u64 ns = n / 32, fs = fstride / 2;
+    const dim3 grid((unsigned)((ns + 127) / 128), batch);
+    auto p = [](const u64 *x) { return reinterpret_cast<const uint4 *>(x); };
+    if (x2)
+        k_slice_mul<true><<<grid, 128, 3 * 128 * 256, st>>>(reinterpret_cast<uint4 *>(o), p(x1),
+                                                            p(y1), p(x2), p(y2), ns, fs);
+    else
+        k_slice_mul<false><<<grid, 128, 2 * 128 * 256, st>>>(reinterpret_cast<uint4 *>(o), p(x1),
+                                                             p(y1), nullptr, nullptr, ns,
+                                                             fs);
+    GF2E_CHECK_LAUNCH("k_slice_mul");
+    return GF2E_OK;
+}
+
+int slice_inv(int m, u64 *f, u64 *tmp, u64 fstride, int batch, u64 *out, u64 ostride, u64 ow,
+              cudaStream_t st) {
+    GF2E_TRY(allow_smem());
+    const Plan &P = plan_for(m);
+    uint4 *f4 = reinterpret_cast<uint4 *>(f);
+    const u64 fs = fstride / 2;
+    BflyArgs a;
+    a.f[0] = a.f[1] = f4;
+    a.top[0] = a.top[1] = m;
+    a.fstride = fs;
+    a.batch = batch;
+    for (int i = P.ntop; i >= 0; i--) GF2E_TRY(run_bfly<false>(P, i, a, 1, st));
+    GF2E_TRY(launch_taylor<false>(f4, fs, batch, m, m, 0, st));
+    if (m > 16) {
+        uint4 *t4 = reinterpret_cast<uint4 *>(tmp);
+        GF2E_TRY(launch_hi<false>(f4, fs, t4, fs, 0, batch, m, m, st));
+        f4 = t4;
+    }
+    const u64 words = 2 * ow;
+    const unsigned grid = (unsigned)((words + (32 << IN_LOG) - 1) >> (IN_LOG + 5));
+    k_slice_out<<<dim3(grid, batch), 1 << IN_LOG, 0, st>>>(f4, fs, 1u << (m - 5),
+                                                         reinterpret_cast<u32 *>(out),
+                                                         2 * ostride, words);
+    GF2E_CHECK_LAUNCH("k_slice_out");
+    return GF2E_OK;
+}
+
+int slice_small(int m, const SliceOp &x, const SliceOp &y, int batch, u64 *out, u64 ostride,
+                u64 ow, cudaStream_t st) {
+    GF2E_TRY(allow_smem());
+    const Plan &P = plan_for(m);
+    SmallArgs a;
+    const SliceOp *op[2] = {&x, &y};
+    for (int o = 0; o < 2; o++) {
+        a.src[o] = op[o]->src;
+        a.sstride[o] = op[o]->stride;
+        a.nchunks[o] = op[o]->nchunks;
+        a.xor0[o] = op[o]->xor0;
+        a.k[o] = std::min(m, std::max(8, clog2(op[o]->nchunks)));
+        a.lv[o] = P.taylor[a.k[o]];
+    }
+    a.m = m;
+    a.lm = P.taylor[m];
+    a.out = reinterpret_cast<u32 *>(out);
+    a.ostride = 2 * ostride;
+    a.words = 2 * ow;
+    const u32 ns = 1u << (m - 5);
+    k_small_mul<<<batch, 512, ns * 512 + 4 * (ns + 1), st>>>(a);
+    GF2E_CHECK_LAUNCH("k_small_mul");
+    return GF2E_OK;
+}
+
+}  // namespace gf2e

@@ -25,18 +25,8 @@
 #include <vector>
 
 namespace gf2e {
-int fft_fwd_packed_batch(const gf2e_fft_plan *plan, u64 *f, u64 fstride, const u32 *src32,
-                         u64 sstride32, u64 nchunks, u64 xor0, int batch, cudaStream_t st);
-int fft_run_batch(const gf2e_fft_plan *plan, bool forward, u64 *f, u64 fstride, int batch,
-                  cudaStream_t st);
-int overlap_add_batch(const u64 *F, u64 fstride, u64 nchunks, u64 *out, u64 ostride, u64 ow,
-                      int batch, cudaStream_t st);
 gf2e_fft_plan *cached_plan(int m);
 int mul_fft_m(u64 abits, u64 bbits);
-int fft_fwd_packed(const gf2e_fft_plan *plan, u64 *f, const u32 *src32, u64 nchunks,
-                   cudaStream_t st);
-int fft_run(const gf2e_fft_plan *plan, bool forward, u64 *f, cudaStream_t st);
-int pointwise(u64 *fa, const u64 *fb, u64 n, cudaStream_t st);
 }  // namespace gf2e
 
 namespace {
@@ -62,20 +52,11 @@ __global__ void k_extract_bits(const u64 *__restrict__ src, u64 sstride, u64 p, 
     }
 }
 
-// fa *= fb pointwise, batched with strides
-__global__ void k_pointwise_batch(u64 *__restrict__ fa, const u64 *__restrict__ fb, u64 n,
-                                  u64 stride) {
-    fa += (u64)blockIdx.y * stride;
-    fb += (u64)blockIdx.y * stride;
-    for (u64 k = (u64)blockIdx.x * blockDim.x + threadIdx.x; k < n;
-         k += (u64)gridDim.x * blockDim.x)
-        fa[k] = gf64_mul(fa[k], fb[k]);
-}
-
 // OA(Q)[w] = bits [D - 1 + 64 w, ...) of U (the product a_hi b_hi), and the
-// high half of R's last coefficient XORed into word 0
+// high half of R's last coefficient, which is word `rtop` of OA(R), XORed
+// into word 0
 __global__ void k_wrap_q(const u64 *__restrict__ U, u64 ustride, u64 uw, u64 shift, u64 qbits,
-                         const u64 *__restrict__ R, u64 rstride, u64 rlast,
+                         const u64 *__restrict__ P, u64 pstride, u64 rtop,
                          u64 *__restrict__ Qo, u64 qstride, u64 qw) {
     U += (u64)blockIdx.y * ustride;
     Qo += (u64)blockIdx.y * qstride;
@@ -90,7 +71,7 @@ __global__ void k_wrap_q(const u64 *__restrict__ U, u64 ustride, u64 uw, u64 shi
             v = sh ? ((lo >> sh) | (hi << (64 - sh))) : lo;
             if (qbits - b < 64) v &= (1ull << (qbits - b)) - 1;
         }
-        if (w == 0) v ^= R[(u64)blockIdx.y * rstride + rlast] >> 32;
+        if (w == 0) v ^= P[(u64)blockIdx.y * pstride + rtop];
         Qo[w] = v;
     }
 }
@@ -173,32 +154,24 @@ bool wrap_mul_plans(WrapMul &w) {
     return w.big && w.small;
 }
 
-// After the 2^mb transform product of a and b left R (2^mb coefficients per
-// batch element, stride rstride) in place: P = a b (ow words per element)
-int wrap_mul_finish(const WrapMul &w, const u64 *R, u64 rstride, const u64 *a, u64 astride,
-                    const u64 *b, u64 bstride, u64 *P, u64 pstride, u64 ow, int batch,
-                    u64 *scratch, cudaStream_t st) {
+// P holds the overlap-added 2^mb transform product R of a and b: P = a b (ow
+// words per element)
+int wrap_mul_finish(const WrapMul &w, const u64 *a, u64 astride, const u64 *b, u64 bstride,
+                    u64 *P, u64 pstride, u64 ow, int batch, u64 *scratch, cudaStream_t st) {
     const u64 S = w.per;
     u64 *Xa = scratch + w.off_xa, *Xb = scratch + w.off_xb, *FAs = scratch + w.off_fa,
         *FBs = scratch + w.off_fb, *U = scratch + w.off_u, *Q = scratch + w.off_q;
     const unsigned nb = (unsigned)batch;
-    GF2E_TRY(overlap_add_batch(R, rstride, w.n, P, pstride, ow, batch, st));
     k_extract_bits<<<dim3(grid_for(w.xw, 256, 4), nb), 256, 0, st>>>(a, astride, w.p, w.D, Xa,
                                                                         S, w.xw);
     GF2E_CHECK_LAUNCH("k_extract_bits");
     k_extract_bits<<<dim3(grid_for(w.xw, 256, 4), nb), 256, 0, st>>>(b, bstride, w.q, w.D, Xb,
                                                                         S, w.xw);
     GF2E_CHECK_LAUNCH("k_extract_bits");
-    GF2E_TRY(fft_fwd_packed_batch(w.small, FAs, S, reinterpret_cast<const u32 *>(Xa), 2 * S,
-                                  w.nsch, 0, batch, st));
-    GF2E_TRY(fft_fwd_packed_batch(w.small, FBs, S, reinterpret_cast<const u32 *>(Xb), 2 * S,
-                                  w.nsch, 0, batch, st));
-    k_pointwise_batch<<<dim3(grid_for(w.ns, 256, 4), nb), 256, 0, st>>>(FAs, FBs, w.ns, S);
-    GF2E_CHECK_LAUNCH("k_pointwise_batch");
-    GF2E_TRY(fft_run_batch(w.small, false, FAs, S, batch, st));
-    GF2E_TRY(overlap_add_batch(FAs, S, 2 * w.nsch - 1, U, S, w.uw, batch, st));
-    k_wrap_q<<<dim3(grid_for(w.qw, 256, 4), nb), 256, 0, st>>>(U, S, w.uw, w.D - 1, w.D, R,
-                                                                  rstride, w.n - 1, Q, S, w.qw);
+    GF2E_TRY(product_batch(w.small, ProductOp{Xa, S, w.nsch, 0}, ProductOp{Xb, S, w.nsch, 0},
+                           batch, FAs, FBs, S, U, S, w.uw, st));
+    k_wrap_q<<<dim3(grid_for(w.qw, 256, 4), nb), 256, 0, st>>>(U, S, w.uw, w.D - 1, w.D, P,
+                                                                  pstride, w.n / 2, Q, S, w.qw);
     GF2E_CHECK_LAUNCH("k_wrap_q");
     k_wrap_fix<<<dim3(grid_for(ow, 256, 8), nb), 256, 0, st>>>(P, pstride, ow, Q, S, w.qw,
                                                                   w.terms);
@@ -211,16 +184,10 @@ int wrap_mul_finish(const WrapMul &w, const u64 *R, u64 rstride, const u64 *a, u
 int mul_wrapped(const WrapMul &w, const u64 *a, u64 abits, const u64 *b, u64 bbits, u64 *out,
                 u64 *fa, u64 *fb, u64 *scratch, cudaStream_t st) {
     const u64 ca = (abits + 31) >> 5, cb = (bbits + 31) >> 5;
-    GF2E_TRY(fft_fwd_packed(w.big, fa, reinterpret_cast<const u32 *>(a), ca, st));
-    if (b == a && bbits == abits) {
-        GF2E_TRY(pointwise(fa, fa, w.n, st));
-    } else {
-        GF2E_TRY(fft_fwd_packed(w.big, fb, reinterpret_cast<const u32 *>(b), cb, st));
-        GF2E_TRY(pointwise(fa, fb, w.n, st));
-    }
-    GF2E_TRY(fft_run(w.big, false, fa, st));
     const u64 ow = ((abits + bbits + 63) >> 6) + 1;
-    return wrap_mul_finish(w, fa, 0, a, 0, b, 0, out, 0, ow, 1, scratch, st);
+    GF2E_TRY(product_batch(w.big, ProductOp{a, 0, ca, 0}, ProductOp{b, 0, cb, 0}, 1, fa, fb, 0,
+                           out, 0, ow, st));
+    return wrap_mul_finish(w, a, 0, b, 0, out, 0, ow, 1, scratch, st);
 }
 
 }  // namespace gf2e

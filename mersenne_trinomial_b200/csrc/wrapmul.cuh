@@ -6,6 +6,18 @@
 
 namespace gf2e {
 
+// operand of a batched product: nchunks 32-bit chunks of words + i * stride,
+// chunk 0 XORed with xor0
+struct ProductOp {
+    const u64 *words;
+    u64 stride, nchunks, xor0;
+};
+// out + i * ostride (ow words) = a_i b_i through the plan's 2^m transform
+// buffers fa and fb (fstride words apart), modulo its subspace polynomial
+// where the product has more than 2^m coefficients; both are overwritten
+int product_batch(const gf2e_fft_plan *plan, const ProductOp &a, const ProductOp &b, int batch,
+                  u64 *fa, u64 *fb, u64 fstride, u64 *out, u64 ostride, u64 ow, cudaStream_t st);
+
 struct WrapTerms {
     int n;
     u64 z[24];          // shifts of OA(Q), in 32-bit chunks
@@ -27,12 +39,10 @@ bool wrap_mul_plan(u64 abits, u64 bbits, WrapMul &w);
 // the two transform plans of a wrapped product (on the current device)
 bool wrap_mul_plans(WrapMul &w);
 
-// after the 2^mb transform product of a and b left R (2^mb coefficients per
-// batch element, stride rstride words): P = a b, ow words per element.
-// scratch holds batch * w.per words.
-int wrap_mul_finish(const WrapMul &w, const u64 *R, u64 rstride, const u64 *a, u64 astride,
-                    const u64 *b, u64 bstride, u64 *P, u64 pstride, u64 ow, int batch,
-                    u64 *scratch, cudaStream_t st);
+// P = a b, ow words per element, where P holds the 2^mb transform product of a
+// and b (product_batch).  scratch holds batch * w.per words.
+int wrap_mul_finish(const WrapMul &w, const u64 *a, u64 astride, const u64 *b, u64 bstride,
+                    u64 *P, u64 pstride, u64 ow, int batch, u64 *scratch, cudaStream_t st);
 
 // out = a b for one product ((abits + bbits + 63) / 64 + 1 words); fa and
 // fb of 2^mb words, scratch of w.per words
