@@ -942,7 +942,7 @@ int mul_fft_m(u64 abits, u64 bbits) {
     return m;
 }
 
-// Products of at most 2^24 coefficients take the bit-sliced transform
+// Products of at most 2^23 coefficients take the bit-sliced transform
 // (slicefft.cu): up to 2^12 in one block, else in the transform buffers where
 // these are aligned for its 16-byte accesses.
 int product_batch(const gf2e_fft_plan *plan, const ProductOp &a, const ProductOp &b, int batch,

@@ -1,5 +1,5 @@
 // slicefft.cu -- launches of the bit-sliced product transform
-// (slicefft.cuh): products of up to 2^24 32-bit chunk coefficients.
+// (slicefft.cuh): products of up to 2^23 32-bit chunk coefficients.
 //
 // A product of 2^m coefficients is seven short passes over memory a side:
 // chunk words to planes, Taylor levels above 2^16 (m > 16), the 2^16-chunk
@@ -27,11 +27,18 @@ struct DevEx {
         f(threadIdx.x, blockDim.x);
         __syncthreads();
     }
+    template <class F> GF2E_DEV void warps(u32 n, const F &f) const {
+        if ((threadIdx.x >> 5) < n) f(threadIdx.x >> 5);
+        __syncthreads();
+    }
+    GF2E_DEV void pair() const {             // the two blocks of a cluster
+        asm volatile("barrier.cluster.arrive.release.aligned;\n"
+                     "barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    }
 };
 
 constexpr int IN_LOG = 7;                    // slices a block of k_slice_in / out
-constexpr int BFLY_THREADS = 512;
-constexpr int TAYLOR_THREADS = 512;
+constexpr int MIN_K = 10;                    // least conversion: 2^10 coefficients
 
 // up to two operands, `batch` transforms each: blockIdx.y = operand * batch + i
 struct In {
@@ -53,22 +60,21 @@ __global__ void __launch_bounds__(1 << IN_LOG) k_slice_in(const In a) {
                   a.k[o] - 5 < IN_LOG ? a.k[o] - 5 : IN_LOG);
 }
 
-// one operand's 2^k coefficients, blocks of 2^kt; blockIdx.x = block * groups
-// + plane group
+// one operand's conversions of 2^K coefficients; blockIdx.x = block * groups
+// + plane group, a warp a plane
 struct TaylorArgs {
     uint4 *f;
     u64 fstride;
-    int kt, plog, groups;
+    int plog, groups;
     u32 c_src, reps, rep_stride;
-    Levels lv;
 };
-template <bool FWD>
-__global__ void __launch_bounds__(TAYLOR_THREADS, 2) k_taylor(const TaylorArgs a) {
+template <int K, bool FWD>
+__global__ void __launch_bounds__(256, 2) k_taylor(const TaylorArgs a) {
     extern __shared__ uint4 sm4[];
     const u32 b = blockIdx.x / a.groups, g = blockIdx.x - b * a.groups;
     const u32 c = g << (a.plog - 2);
-    body_taylor<FWD>(DevEx{}, reinterpret_cast<u32 *>(sm4), a.f + blockIdx.y * a.fstride,
-                     b << (a.kt - 5), a.kt, a.plog, c, a.c_src + c, a.reps, a.rep_stride, a.lv);
+    body_taylor<K, FWD>(DevEx{}, reinterpret_cast<u32 *>(sm4), a.f + blockIdx.y * a.fstride,
+                        b << (K - 5), a.plog, c, a.c_src + c, a.reps, a.rep_stride);
 }
 
 struct HiArgs {
@@ -77,18 +83,16 @@ struct HiArgs {
     u64 sstride, dstride;
     u32 c_dst;
     int groups;
-    HiGeom G;
-    Levels rows;
 };
-template <bool FWD>
-__global__ void __launch_bounds__(TAYLOR_THREADS, 2) k_taylor_hi(const HiArgs a) {
+template <int RLOG, bool FWD>
+__global__ void __launch_bounds__(32 << Hi<RLOG>::PLOG, RLOG >= 7 ? 2 : 1)
+k_taylor_hi(const HiArgs a) {
     extern __shared__ uint4 sm4[];
-    u32 *sm = reinterpret_cast<u32 *>(sm4);
-    u32 *side = sm + ((hi_pitch(a.G) << a.G.rlog) << a.G.plog);
     const u32 ct = blockIdx.x / a.groups, g = blockIdx.x - ct * a.groups;
-    const u32 c = g << (a.G.plog - 2);
-    body_taylor_hi<FWD>(DevEx{}, sm, side, a.src + blockIdx.y * a.sstride, c,
-                        a.dst + blockIdx.y * a.dstride, a.c_dst + c, a.G, ct, a.rows);
+    const u32 c = g << Hi<RLOG>::CL;
+    body_taylor_hi<RLOG, FWD>(DevEx{}, reinterpret_cast<u32 *>(sm4),
+                              a.src + blockIdx.y * a.sstride, c, a.dst + blockIdx.y * a.dstride,
+                              a.c_dst + c, ct);
 }
 
 struct BflyArgs {
@@ -97,19 +101,26 @@ struct BflyArgs {
     int m, rlog, clog, llo, collog;          // 2^collog column groups a window
     int top[2];
     int batch;
+    bool first, lowp;
 };
-template <int NQ, bool FWD, bool EDGE, bool LOWP>
-__global__ void __launch_bounds__(BFLY_THREADS, 1) k_bfly(const BflyArgs a) {
+// blockIdx.x = 2 * tile + half, the halves of a tile one cluster; NQ quarters
+// of a slice pair a thread (1 where the tiles leave SMs idle).  Two blocks of
+// 256 threads an SM, so that one's loads and stores pass behind the other's
+// products.
+template <int NQ, bool FWD>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NQ == 2 ? 256 : 512, NQ == 2 ? 2 : 1)
+k_bfly(const BflyArgs a) {
     extern __shared__ uint4 sm4[];
     const int o = (int)blockIdx.y / a.batch, i = (int)blockIdx.y - o * a.batch;
-    const u32 win = blockIdx.x >> a.collog, col = blockIdx.x & ((1u << a.collog) - 1);
+    const u32 half = blockIdx.x & 1, tile = blockIdx.x >> 1;
+    const u32 win = tile >> a.collog, col = tile & ((1u << a.collog) - 1);
     Tile T;
     T.m = a.m;
     T.rlog = a.rlog;
     T.clog = a.clog;
     T.llo = a.llo;
     T.base = (win << (a.llo + a.rlog - 5)) + (col << a.clog);
-    body_bfly<NQ, FWD>(DevEx{}, sm4, a.f[o] + i * a.fstride, T, a.top[o], EDGE, LOWP);
+    body_bfly<NQ, FWD>(DevEx{}, sm4, a.f[o] + i * a.fstride, T, half, a.top[o], a.first, a.lowp);
 }
 
 // o = x1 y1 (+ x2 y2 where TWO) over 128 slices a block
@@ -128,31 +139,30 @@ k_slice_mul(uint4 *o, const uint4 *x1, const uint4 *y1, const uint4 *x2, const u
     }
     const u32 n = (u32)min((u64)128, nslices - s0);
     const u32 tid = threadIdx.x;
-    uint4 *ta = sm4, *tb = sm4 + 128 * 16, *tc = tb + 128 * 16;
+    const Full ta{sm4}, tb{sm4 + 128 * 17}, tc{sm4 + 256 * 17};
     const bool same = x1 == y1;
     for (u32 i = tid; i < n * 16; i += 128) {
-        const u32 at = chunk_at(i >> 4, i & 15);
-        ta[at] = x1[s0 * 16 + i];
-        if (!same) tb[at] = y1[s0 * 16 + i];
+        copy16(&ta.chunk(i >> 4, i & 15), x1 + s0 * 16 + i);
+        if (!same) copy16(&tb.chunk(i >> 4, i & 15), y1 + s0 * 16 + i);
     }
+    copy_wait();
     __syncthreads();
     mul_slices(ta, same ? ta : tb, n, tid, 128);
     __syncthreads();
     if (TWO) {
         for (u32 i = tid; i < n * 16; i += 128) {
-            const u32 at = chunk_at(i >> 4, i & 15);
-            tb[at] = x2[s0 * 16 + i];
-            tc[at] = y2[s0 * 16 + i];
+            copy16(&tb.chunk(i >> 4, i & 15), x2 + s0 * 16 + i);
+            copy16(&tc.chunk(i >> 4, i & 15), y2 + s0 * 16 + i);
         }
+        copy_wait();
         __syncthreads();
         mul_slices(tb, tc, n, tid, 128);
         __syncthreads();
     }
     for (u32 i = tid; i < n * 16; i += 128) {
-        const u32 at = chunk_at(i >> 4, i & 15);
-        uint4 v = ta[at];
+        uint4 v = ta.chunk(i >> 4, i & 15);
         if (TWO) {
-            const uint4 w = tb[at];
+            const uint4 w = tb.chunk(i >> 4, i & 15);
             v.x ^= w.x; v.y ^= w.y; v.z ^= w.z; v.w ^= w.w;
         }
         o[s0 * 16 + i] = v;
@@ -161,10 +171,10 @@ k_slice_mul(uint4 *o, const uint4 *x1, const uint4 *y1, const uint4 *x2, const u
 
 __global__ void __launch_bounds__(1 << IN_LOG)
 k_slice_out(const uint4 *f, u64 fstride, u32 nsl, u32 *out, u64 ostride, u64 words) {
-    __shared__ uint4 tile[16 << IN_LOG];
+    __shared__ uint4 tile[17 << IN_LOG];
     __shared__ u32 side[(1 << IN_LOG) + 1];
     body_slice_out(DevEx{}, tile, side, f + blockIdx.y * fstride, nsl, out + blockIdx.y * ostride,
-                   words, blockIdx.x << IN_LOG, IN_LOG);
+                   words, blockIdx.x * ((1 << IN_LOG) - 1), IN_LOG);
 }
 
 struct SmallArgs {
@@ -180,28 +190,17 @@ __global__ void __launch_bounds__(512, 1) k_small_mul(const SmallArgs a) {
     extern __shared__ uint4 sm4[];
     const u32 ns = 1u << (a.m - 5);
     const u64 y = blockIdx.x;
-    body_small(DevEx{}, sm4, sm4 + ns * 16, reinterpret_cast<u32 *>(sm4 + ns * 32), a.m,
+    body_small(DevEx{}, sm4, sm4 + ns * 17, sm4 + ns * 34, reinterpret_cast<u32 *>(sm4 + ns * 43), a.m,
                Operand{a.src[0] + y * a.sstride[0], a.nchunks[0], a.xor0[0]},
                Operand{a.src[1] + y * a.sstride[1], a.nchunks[1], a.xor0[1]}, a.k[0], a.k[1],
                a.lv[0], a.lv[1], a.lm, a.out + y * a.ostride, a.words);
 }
 
-constexpr size_t SMALL_SMEM = (size_t)(1 << (SMALL_M - 5)) * 512 + 4 * ((1 << (SMALL_M - 5)) + 1);
-constexpr size_t BFLY_SMEM = (size_t)(256 << TILE_LOG);
-constexpr size_t TAYLOR_SMEM = (size_t)(4 << 11) << 3;
-constexpr int HI_TLOG = 4;
+constexpr size_t SLICE_BYTES = 16 * 17, HALF_BYTES = 16 * 9;
+constexpr size_t small_smem(int m) { return ((2 * SLICE_BYTES + HALF_BYTES + 4) << (m - 5)) + 4; }
+constexpr size_t BFLY_SMEM = HALF_BYTES << TILE_LOG;
 
-HiGeom hi_geom(int rlog) {
-    HiGeom G;
-    G.rlog = rlog;
-    G.tlog = HI_TLOG;
-    G.plog = rlog >= 8 ? 2 : 3;
-    G.halo = rlog <= 5 ? 1u : 1u << (rlog - 5);
-    return G;
-}
-size_t hi_smem(const HiGeom &G) {
-    return ((size_t)(hi_pitch(G) + G.halo) << G.rlog << G.plog) * 4;
-}
+size_t taylor_smem(int k, int plog) { return (size_t)(4 * ((1 << (k - 5)) + 4)) << plog; }
 
 int allow_smem() {
     // set once per device; two threads racing here both set the same values
@@ -214,21 +213,23 @@ int allow_smem() {
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n);
     };
-    allow((const void *)k_taylor<true>, TAYLOR_SMEM);
-    allow((const void *)k_taylor<false>, TAYLOR_SMEM);
-    size_t hs = 0;
-    for (int r = 1; r <= 8; r++) hs = std::max(hs, hi_smem(hi_geom(r)));
-    allow((const void *)k_taylor_hi<true>, hs);
-    allow((const void *)k_taylor_hi<false>, hs);
-    allow((const void *)k_small_mul, SMALL_SMEM);
-    allow((const void *)k_slice_mul<false>, 2 * 128 * 256);
-    allow((const void *)k_slice_mul<true>, 3 * 128 * 256);
-#define GF2E_SL_ALLOW(NQ, F)                                         \
-    allow((const void *)k_bfly<NQ, F, false, false>, BFLY_SMEM);     \
-    allow((const void *)k_bfly<NQ, F, true, false>, BFLY_SMEM);      \
-    allow((const void *)k_bfly<NQ, F, false, true>, BFLY_SMEM);      \
-    allow((const void *)k_bfly<NQ, F, true, true>, BFLY_SMEM);
-    GF2E_SL_ALLOW(1, true) GF2E_SL_ALLOW(1, false) GF2E_SL_ALLOW(2, true) GF2E_SL_ALLOW(2, false)
+#define GF2E_SL_ALLOW(K)                                             \
+    allow((const void *)k_taylor<K, true>, taylor_smem(K, 3));       \
+    allow((const void *)k_taylor<K, false>, taylor_smem(K, 3));
+    GF2E_SL_ALLOW(15) GF2E_SL_ALLOW(16)
+#undef GF2E_SL_ALLOW
+#define GF2E_SL_ALLOW(R)                                                        \
+    allow((const void *)k_taylor_hi<R, true>, 4 * Hi<R>::WORDS);    \
+    allow((const void *)k_taylor_hi<R, false>, 4 * Hi<R>::WORDS);
+    GF2E_SL_ALLOW(6) GF2E_SL_ALLOW(7)
+#undef GF2E_SL_ALLOW
+    allow((const void *)k_small_mul, small_smem(SMALL_M));
+    allow((const void *)k_slice_mul<false>, 2 * 128 * SLICE_BYTES);
+    allow((const void *)k_slice_mul<true>, 3 * 128 * SLICE_BYTES);
+#define GF2E_SL_ALLOW(NQ)                                \
+    allow((const void *)k_bfly<NQ, true>, BFLY_SMEM);    \
+    allow((const void *)k_bfly<NQ, false>, BFLY_SMEM);
+    GF2E_SL_ALLOW(1) GF2E_SL_ALLOW(2)
 #undef GF2E_SL_ALLOW
     if (e != cudaSuccess) return gf2e::cuda_status(e, "sliced transform smem attribute");
     if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
@@ -260,12 +261,11 @@ int clog2(u64 v) {
 
 template <bool FWD>
 int launch_taylor(uint4 *f, u64 fstride, int batch, int m, int k, u32 c_src, cudaStream_t st) {
-    const Plan &P = plan_for(m);
     TaylorArgs a;
     a.f = f;
     a.fstride = fstride;
-    a.kt = std::min(k, 16);
-    const u32 blocks = 1u << (k - a.kt);
+    const int kt = std::min(k, 16);
+    const u32 blocks = 1u << (k - kt);
     const int chunks = FWD ? 8 : 16;
     // 8 planes a block (whole 32-byte sectors) unless that leaves SMs idle
     a.plog = blocks * (chunks / 2) * (u32)batch >= (u32)gf2e::sm_count() ? 3 : 2;
@@ -273,41 +273,50 @@ int launch_taylor(uint4 *f, u64 fstride, int batch, int m, int k, u32 c_src, cud
     a.c_src = c_src;
     a.reps = FWD ? 1u << (m - k) : 1u;
     a.rep_stride = 1u << (k - 5);
-    a.lv = P.taylor[a.kt];
-    const int threads = std::max(64, std::min(TAYLOR_THREADS, 1 << (a.kt - 6 + a.plog)));
-    k_taylor<FWD><<<dim3(blocks * a.groups, batch), threads, (size_t)4 << (a.kt - 5 + a.plog), st>>>(a);
+    const dim3 grid(blocks * a.groups, batch);
+    const int threads = 32 << a.plog;
+    const size_t smem = taylor_smem(kt, a.plog);
+    switch (kt) {
+    case 10: k_taylor<10, FWD><<<grid, threads, smem, st>>>(a); break;
+    case 11: k_taylor<11, FWD><<<grid, threads, smem, st>>>(a); break;
+    case 12: k_taylor<12, FWD><<<grid, threads, smem, st>>>(a); break;
+    case 13: k_taylor<13, FWD><<<grid, threads, smem, st>>>(a); break;
+    case 14: k_taylor<14, FWD><<<grid, threads, smem, st>>>(a); break;
+    case 15: k_taylor<15, FWD><<<grid, threads, smem, st>>>(a); break;
+    default: k_taylor<16, FWD><<<grid, threads, smem, st>>>(a); break;
+    }
     GF2E_CHECK_LAUNCH("k_taylor");
     return GF2E_OK;
 }
 
-template <bool FWD>
-int launch_hi(const uint4 *src, u64 sstride, uint4 *dst, u64 dstride, u32 c_dst, int batch, int m,
-              int k, cudaStream_t st) {
-    const Plan &P = plan_for(m);
-    HiArgs a;
-    a.src = src;
-    a.dst = dst;
-    a.sstride = sstride;
-    a.dstride = dstride;
-    a.c_dst = c_dst;
-    a.G = hi_geom(k - 16);
-    a.groups = (FWD ? 8 : 16) >> (a.G.plog - 2);
-    a.rows = P.rows[k - 16];
-    k_taylor_hi<FWD><<<dim3((2048 >> HI_TLOG) * a.groups, batch), TAYLOR_THREADS, hi_smem(a.G), st>>>(a);
+template <int RLOG, bool FWD>
+int launch_hi_r(HiArgs a, int batch, cudaStream_t st) {
+    typedef Hi<RLOG> H;
+    a.groups = (FWD ? 8 : 16) >> H::CL;
+    k_taylor_hi<RLOG, FWD><<<dim3(H::TILES * a.groups, batch), 32 << H::PLOG, 4 * H::WORDS, st>>>(a);
     GF2E_CHECK_LAUNCH("k_taylor_hi");
     return GF2E_OK;
 }
+template <bool FWD>
+int launch_hi(const uint4 *src, u64 sstride, uint4 *dst, u64 dstride, u32 c_dst, int batch, int k,
+              cudaStream_t st) {
+    HiArgs a{src, dst, sstride, dstride, c_dst, 0};
+    switch (k - 16) {
+    case 1: return launch_hi_r<1, FWD>(a, batch, st);
+    case 2: return launch_hi_r<2, FWD>(a, batch, st);
+    case 3: return launch_hi_r<3, FWD>(a, batch, st);
+    case 4: return launch_hi_r<4, FWD>(a, batch, st);
+    case 5: return launch_hi_r<5, FWD>(a, batch, st);
+    case 6: return launch_hi_r<6, FWD>(a, batch, st);
+    default: return launch_hi_r<7, FWD>(a, batch, st);
+    }
+}
 
 template <int NQ, bool FWD>
-int launch_bfly(const BflyArgs &a, u32 tiles, int ny, bool edge, bool lowp, cudaStream_t st) {
+int launch_bfly(const BflyArgs &a, u32 tiles, int ny, cudaStream_t st) {
     const int tl = a.rlog + a.clog;
-    const int threads = std::max(32, std::min(BFLY_THREADS, (1 << (tl - 1)) * (4 / NQ)));
-    const size_t smem = (size_t)256 << tl;
-    const dim3 g(tiles, ny);
-    if (edge && lowp) k_bfly<NQ, FWD, true, true><<<g, threads, smem, st>>>(a);
-    else if (edge) k_bfly<NQ, FWD, true, false><<<g, threads, smem, st>>>(a);
-    else if (lowp) k_bfly<NQ, FWD, false, true><<<g, threads, smem, st>>>(a);
-    else k_bfly<NQ, FWD, false, false><<<g, threads, smem, st>>>(a);
+    const int threads = std::max(32, std::min(NQ == 2 ? 256 : 512, (1 << (tl - 1)) * (2 / NQ)));
+    k_bfly<NQ, FWD><<<dim3(2 * tiles, ny), threads, HALF_BYTES << tl, st>>>(a);
     GF2E_CHECK_LAUNCH("k_bfly");
     return GF2E_OK;
 }
@@ -323,11 +332,13 @@ int run_bfly(const Plan &P, int i, BflyArgs a, int nops, cudaStream_t st) {
     a.collog = a.llo - 5 - a.clog;
     const u32 tiles = 1u << (P.m - 5 - a.rlog - a.clog);
     const int ny = nops * a.batch;
-    // a quarter of the planes a thread while that fills idle SMs (m <= 16:
-    // every twiddle is in GF(2^16)), else half of them for one twiddle
-    if (P.m <= 16 && (u64)tiles * ny < 2 * (u64)gf2e::sm_count())
-        return launch_bfly<1, FWD>(a, tiles, ny, i == 0, lowp, st);
-    return launch_bfly<2, FWD>(a, tiles, ny, i == 0, lowp, st);
+    a.first = FWD && i == 0;
+    a.lowp = lowp;
+    // one quarter a thread while that fills idle SMs (m <= 16, where every
+    // twiddle is in GF(2^16))
+    if (P.m <= 16 && (u64)tiles * ny < (u64)gf2e::sm_count())
+        return launch_bfly<1, FWD>(a, tiles, ny, st);
+    return launch_bfly<2, FWD>(a, tiles, ny, st);
 }
 
 }  // namespace
@@ -357,7 +368,7 @@ int slice_fwd(int m, const SliceOp *ops, int nops, u64 fstride, int batch, cudaS
         in.nchunks[o] = ops[o].nchunks;
         in.xor0[o] = ops[o].xor0;
         in.f[o] = reinterpret_cast<uint4 *>(ops[o].f);
-        in.k[o] = std::min(m, std::max(8, clog2(ops[o].nchunks)));
+        in.k[o] = std::min(m, std::max(MIN_K, clog2(ops[o].nchunks)));
         nx = std::max(nx, 1u << std::max(0, in.k[o] - 5 - IN_LOG));
     }
     k_slice_in<<<dim3(nx, nops * batch), 1 << IN_LOG, 0, st>>>(in);
@@ -368,7 +379,7 @@ int slice_fwd(int m, const SliceOp *ops, int nops, u64 fstride, int batch, cudaS
     for (int o = 0; o < nops; o++) {
         u32 c = 0;
         if (in.k[o] > 16) {
-            GF2E_TRY(launch_hi<true>(in.f[o], in.fstride, in.f[o], in.fstride, 8, batch, m, in.k[o], st));
+            GF2E_TRY(launch_hi<true>(in.f[o], in.fstride, in.f[o], in.fstride, 8, batch, in.k[o], st));
             c = 8;
         }
         GF2E_TRY(launch_taylor<true>(in.f[o], in.fstride, batch, m, in.k[o], c, st));
@@ -386,10 +397,10 @@ int slice_pointwise(u64 *o, const u64 *x1, const u64 *y1, const u64 *x2, const u
     const dim3 grid((unsigned)((ns + 127) / 128), batch);
     auto p = [](const u64 *x) { return reinterpret_cast<const uint4 *>(x); };
     if (x2)
-        k_slice_mul<true><<<grid, 128, 3 * 128 * 256, st>>>(reinterpret_cast<uint4 *>(o), p(x1),
+        k_slice_mul<true><<<grid, 128, 3 * 128 * SLICE_BYTES, st>>>(reinterpret_cast<uint4 *>(o), p(x1),
                                                             p(y1), p(x2), p(y2), ns, fs);
     else
-        k_slice_mul<false><<<grid, 128, 2 * 128 * 256, st>>>(reinterpret_cast<uint4 *>(o), p(x1),
+        k_slice_mul<false><<<grid, 128, 2 * 128 * SLICE_BYTES, st>>>(reinterpret_cast<uint4 *>(o), p(x1),
                                                              p(y1), nullptr, nullptr, ns,
                                                              fs);
     GF2E_CHECK_LAUNCH("k_slice_mul");
@@ -411,11 +422,12 @@ int slice_inv(int m, u64 *f, u64 *tmp, u64 fstride, int batch, u64 *out, u64 ost
     GF2E_TRY(launch_taylor<false>(f4, fs, batch, m, m, 0, st));
     if (m > 16) {
         uint4 *t4 = reinterpret_cast<uint4 *>(tmp);
-        GF2E_TRY(launch_hi<false>(f4, fs, t4, fs, 0, batch, m, m, st));
+        GF2E_TRY(launch_hi<false>(f4, fs, t4, fs, 0, batch, m, st));
         f4 = t4;
     }
     const u64 words = 2 * ow;
-    const unsigned grid = (unsigned)((words + (32 << IN_LOG) - 1) >> (IN_LOG + 5));
+    const u64 per = 32 * ((1 << IN_LOG) - 1);
+    const unsigned grid = (unsigned)((words + per - 1) / per);
     k_slice_out<<<dim3(grid, batch), 1 << IN_LOG, 0, st>>>(f4, fs, 1u << (m - 5),
                                                          reinterpret_cast<u32 *>(out),
                                                          2 * ostride, words);
@@ -442,8 +454,7 @@ int slice_small(int m, const SliceOp &x, const SliceOp &y, int batch, u64 *out, 
     a.out = reinterpret_cast<u32 *>(out);
     a.ostride = 2 * ostride;
     a.words = 2 * ow;
-    const u32 ns = 1u << (m - 5);
-    k_small_mul<<<batch, 512, ns * 512 + 4 * (ns + 1), st>>>(a);
+    k_small_mul<<<batch, 512, small_smem(m), st>>>(a);
     GF2E_CHECK_LAUNCH("k_small_mul");
     return GF2E_OK;
 }

@@ -8,14 +8,14 @@
 // the ALU.  A "slice" is 32 consecutive elements held as 64 bit planes of 32
 // bits (bit e of plane p = coordinate p of element e), 256 bytes, the same
 // place in memory as the 32 elements.  GF(2^64) is taken in the tower basis
-// x_k^2 = x_k + x_0 .. x_(k-1) (the nim field: coordinate i is the product of
-// the x_k over the set bits k of i), in which the subfields GF(2^8),
-// GF(2^16), GF(2^32) are the low 8, 16, 32 coordinates.  The twiddle of
-// butterfly level L is a sum of the Cantor basis elements 1 .. m-1-L, which
-// lie in those subfields, so a multiply splits into 8 / 4 / 2 independent
-// subfield multiplies, each a Karatsuba tree of AND-XORs over planes: 61,
-// 211 and ~600 operations for 32 products, 15-38 a field product where a
-// 64 x 64 carry-less multiply by integer multiplies takes ~200.
+// x_k^2 = x_(k-1) x_k + 1 (coordinate i is the product of the x_k over the
+// set bits k of i), in which the subfields GF(2^8), GF(2^16), GF(2^32) are the
+// low 8, 16, 32 coordinates.  The twiddle of butterfly level L is a sum of the
+// Cantor basis elements 1 .. m-1-L, which lie in those subfields, so a
+// multiply splits into 8 / 4 / 2 independent subfield multiplies, each a tree
+// of three-way products down to AND-XORs over planes: 60, 204 and ~590
+// operations for 32 products, 15-37 a field product where a 64 x 64
+// carry-less multiply by integer multiplies takes ~200.
 #pragma once
 
 #include <stdint.h>
@@ -33,12 +33,56 @@ namespace slice {
 typedef uint64_t u64;
 typedef uint32_t u32;
 
+// a register of a warp: on the host the 32 lanes' values, so that the
+// warp-wide steps below also run there
+#ifdef __CUDACC__
+typedef u32 V;
+SL_HD V lane_id() { return threadIdx.x & 31; }
+SL_HD V shfl(V x, V lane) { return __shfl_sync(0xFFFFFFFFu, x, lane); }
+SL_HD V below(V a, u32 b) { return a < b ? 0xFFFFFFFFu : 0u; }      // masks
+template <class F> SL_HD V lane_load(const u32 *sm, const F &at) { return sm[at(lane_id())]; }
+template <class F> SL_HD void lane_store(u32 *sm, const F &at, V x) { sm[at(lane_id())] = x; }
+// keeps shuffles (and the registers of their results) from moving up past it
+SL_HD void warp_fence() { __syncwarp(); }
+template <class P, class F> SL_HD V lane_load_if(const u32 *sm, const P &p, const F &at) {
+    return p(lane_id()) ? sm[at(lane_id())] : 0;
+}
+template <class P, class F> SL_HD void lane_store_if(u32 *sm, const P &p, const F &at, V x) {
+    if (p(lane_id())) sm[at(lane_id())] = x;
+}
+#else
+struct V {
+    u32 l[32];
+    V(u32 x = 0) { for (u32 &v : l) v = x; }
+};
+#define SL_OP(op)                                                          \
+    inline V operator op(const V &a, const V &b) {                         \
+        V r;                                                               \
+        for (int i = 0; i < 32; i++) r.l[i] = a.l[i] op b.l[i];            \
+        return r;                                                          \
+    }
+SL_OP(^) SL_OP(&) SL_OP(|) SL_OP(+) SL_OP(-)
+#undef SL_OP
+inline V &operator^=(V &a, const V &b) { return a = a ^ b; }
+inline V operator~(const V &a) { return a ^ V(0xFFFFFFFFu); }
+inline V operator<<(const V &a, int s) { V r; for (int i = 0; i < 32; i++) r.l[i] = a.l[i] << s; return r; }
+inline V operator>>(const V &a, int s) { V r; for (int i = 0; i < 32; i++) r.l[i] = a.l[i] >> s; return r; }
+inline V lane_id() { V r; for (int i = 0; i < 32; i++) r.l[i] = i; return r; }
+inline V shfl(const V &x, const V &lane) { V r; for (int i = 0; i < 32; i++) r.l[i] = x.l[lane.l[i] & 31]; return r; }
+inline V below(const V &a, u32 b) { V r; for (int i = 0; i < 32; i++) r.l[i] = a.l[i] < b ? ~0u : 0u; return r; }
+template <class F> inline V lane_load(const u32 *sm, const F &at) { V r; for (int i = 0; i < 32; i++) r.l[i] = sm[at(i)]; return r; }
+template <class F> inline void lane_store(u32 *sm, const F &at, const V &x) { for (int i = 0; i < 32; i++) sm[at(i)] = x.l[i]; }
+inline void warp_fence() {}
+template <class P, class F> inline V lane_load_if(const u32 *sm, const P &p, const F &at) { V r; for (int i = 0; i < 32; i++) if (p(i)) r.l[i] = sm[at(i)]; return r; }
+template <class P, class F> inline void lane_store_if(u32 *sm, const P &p, const F &at, const V &x) { for (int i = 0; i < 32; i++) if (p(i)) sm[at(i)] = x.l[i]; }
+#endif
+
 // ------------------------------------------------- tower-field constants
-constexpr u64 c_delta(u64 a, int n) {            // a * v_(n-1) in GF(2^n)
+constexpr u64 c_mulx(u64 a, int n) {             // a times GF(2^n)'s own generator
     if (n == 1) return a;
     const int h = n / 2;
     const u64 lo = a & ((1ull << h) - 1), hi = a >> h;
-    return c_delta(c_delta(hi, h), h) | (c_delta(lo ^ hi, h) << h);
+    return hi | ((lo ^ c_mulx(hi, h)) << h);
 }
 constexpr u64 c_mul(u64 a, u64 b, int n) {
     if (!a || !b) return 0;
@@ -47,11 +91,11 @@ constexpr u64 c_mul(u64 a, u64 b, int n) {
     const u64 m = (1ull << h) - 1;
     const u64 p0 = c_mul(a & m, b & m, h), p1 = c_mul(a >> h, b >> h, h),
               p2 = c_mul((a & m) ^ (a >> h), (b & m) ^ (b >> h), h);
-    return (p0 ^ c_delta(p1, h)) | ((p2 ^ p0) << h);
+    return (p0 ^ p1) | ((p2 ^ p0 ^ p1 ^ c_mulx(p1, h)) << h);
 }
 // image of x under an isomorphism from GF(2)[x]/(x^64 + x^4 + x^3 + x + 1):
 // a root of the modulus in the tower field
-constexpr u64 ROOT = 0x67b6b273eb5d60f6ull;
+constexpr u64 ROOT = 0x4d12d23e481d71ddull;
 
 struct Phi {
     u64 to[64];        // to[i] = image of x^i
@@ -84,9 +128,9 @@ constexpr Phi PHI = make_phi();
 // images of the Cantor basis elements 0 .. 24 (checked against the basis in
 // the polynomial representation when a plan is made)
 constexpr u32 CANTOR[25] = {
-    0x1, 0x3, 0x6, 0xf, 0x1c, 0x30, 0x66, 0xf6, 0x1dd, 0x332, 0x604, 0xf95, 0x1c8e,
-    0x305d, 0x6638, 0xf6ee, 0x1ddf7, 0x33229, 0x6048c, 0xf95ee, 0x1c8ed9, 0x305d3c,
-    0x6638c6, 0xf6ee5d, 0x1dd773f};
+    0x1, 0x3, 0xe, 0xb, 0x62, 0xd5, 0x8c, 0xf0, 0x1450, 0x3ce3, 0xefe9, 0xb2c2, 0x2e06,
+    0x5025, 0xcf80, 0xff1, 0x110ecfb, 0x330a54a, 0xee04fec, 0xbb0ec09, 0x6236b7ac,
+    0xd56d18a7, 0x8c2888b8, 0xf0bff8be, 0x50c1afc9};
 
 // W[t] = XOR of CANTOR[j+1] over the set bits j of t, t < 2^24, by bytes of t
 struct TwTab { u32 v[768]; };
@@ -126,46 +170,73 @@ SL_HD u32 twiddle(u32 t) {
 }
 
 // ------------------------------------------------- bit-sliced field products
-template <int N> SL_HD void t_delta(const u32 *a, u32 *c) {       // c = v_(N-1) a
+// c = X a, X the generator of GF(2^N) over its half (1 for N = 1)
+template <int N> SL_HD void t_mulx(const u32 *a, u32 *c) {
     if constexpr (N == 1) {
         c[0] = a[0];
     } else {
         constexpr int H = N / 2;
-        u32 s[H], u[H];
+        u32 t[H];
+        t_mulx<H>(a + H, t);
 #pragma unroll
-        for (int i = 0; i < H; i++) s[i] = a[i] ^ a[H + i];
-        t_delta<H>(a + H, u);
-        t_delta<H>(u, c);
-        t_delta<H>(s, c + H);
+        for (int i = 0; i < H; i++) { c[H + i] = a[i] ^ t[i]; c[i] = a[H + i]; }
     }
 }
-template <int N> SL_HD void t_mul(const u32 *a, const u32 *b, u32 *c) {
-    if constexpr (N == 2) {
-        const u32 p = a[0] & b[0];
-        c[0] = p ^ (a[1] & b[1]);
-        c[1] = p ^ ((a[0] ^ a[1]) & (b[0] ^ b[1]));
+// A multiplier b prepared for products in GF(2^N).  With X^2 = t X + 1 over
+// the half field, b = b0 + b1 X acts on (a0, a1) as the matrix [b0 b1; b1 b0 +
+// t b1], equal on its second diagonal, so three half products by b0 + b1, b1
+// and b1 + b0 + t b1 make one and all else is done to b once.  The leaves are
+// GF(2^4) elements, each with the 9 sums of its bits that its 4 x 4 matrix
+// holds (3^(log2 N - 2) leaves).
+template <int N> struct Prep {
+    Prep<N / 2> p0, p1, p2;
+    SL_HD void set(const u32 *b) {
+        constexpr int H = N / 2;
+        u32 s[H], t[H];
+        t_mulx<H>(b + H, t);
+#pragma unroll
+        for (int i = 0; i < H; i++) { s[i] = b[i] ^ b[H + i]; t[i] ^= s[i]; }
+        p0.set(s);
+        p1.set(b + H);
+        p2.set(t);
+    }
+};
+template <> struct Prep<4> {
+    u32 b0, b1, b2, b3, b01, b23, e0, e1, e01;
+    SL_HD void set(const u32 *b) {
+        b0 = b[0]; b1 = b[1]; b2 = b[2]; b3 = b[3];
+        b01 = b0 ^ b1; b23 = b2 ^ b3; e0 = b0 ^ b3; e1 = b1 ^ b23; e01 = b01 ^ b2;
+    }
+};
+// c ^= a b: every AND joins an XOR, 16 three-input operations a leaf; 60 in
+// GF(2^8), 204 in GF(2^16)
+template <int N> SL_HD void t_addmul(const u32 *a, const Prep<N> &b, u32 *c) {
+    if constexpr (N == 4) {
+        c[0] ^= a[0] & b.b0; c[0] ^= a[1] & b.b1; c[0] ^= a[2] & b.b2; c[0] ^= a[3] & b.b3;
+        c[1] ^= a[0] & b.b1; c[1] ^= a[1] & b.b01; c[1] ^= a[2] & b.b3; c[1] ^= a[3] & b.b23;
+        c[2] ^= a[0] & b.b2; c[2] ^= a[1] & b.b3; c[2] ^= a[2] & b.e0; c[2] ^= a[3] & b.e1;
+        c[3] ^= a[0] & b.b3; c[3] ^= a[1] & b.b23; c[3] ^= a[2] & b.e1; c[3] ^= a[3] & b.e01;
     } else {
         constexpr int H = N / 2;
-        u32 p0[H], p1[H], sa[H], sb[H];
+        u32 p[H], s[H];
 #pragma unroll
-        for (int i = 0; i < H; i++) { sa[i] = a[i] ^ a[H + i]; sb[i] = b[i] ^ b[H + i]; }
-        t_mul<H>(a, b, p0);
-        t_mul<H>(a + H, b + H, p1);
-        t_mul<H>(sa, sb, c + H);
-        t_delta<H>(p1, c);
+        for (int i = 0; i < H; i++) { p[i] = 0; s[i] = a[i] ^ a[H + i]; }
+        t_addmul<H>(s, b.p1, p);
+        t_addmul<H>(a, b.p0, c);
+        t_addmul<H>(a + H, b.p2, c + H);
 #pragma unroll
-        for (int i = 0; i < H; i++) { c[H + i] ^= p0[i]; c[i] ^= p0[i]; }
+        for (int i = 0; i < H; i++) { c[i] ^= p[i]; c[H + i] ^= p[i]; }
     }
 }
 
 // ------------------------------------------------- linear maps on planes
 // out[p] = XOR over i < NI of bit p of M[i], in[i]; four inputs at a time
-// through their 16 XORs (NO outputs)
+// through their 16 XORs (outputs P0 .. P0 + NO - 1)
 template <bool TO, int G, int P> struct Sel {
     static constexpr u64 at(int i) { return ((TO ? PHI.to[i] : PHI.from[i]) >> P) & 1; }
     static constexpr int v = (int)(at(G) | at(G + 1) << 1 | at(G + 2) << 2 | at(G + 3) << 3);
 };
-template <bool TO, int G, int... P>
+template <bool TO, int G, int P0, int... P>
 SL_HD void lin_group(const u32 *in, u32 *out, std::integer_sequence<int, P...>) {
     u32 c[16];
     c[0] = 0;
@@ -173,138 +244,215 @@ SL_HD void lin_group(const u32 *in, u32 *out, std::integer_sequence<int, P...>) 
     for (int k = 0; k < 4; k++)
 #pragma unroll
         for (int v = 0; v < (1 << k); v++) c[(1 << k) + v] = c[v] ^ in[G + k];
-    ((out[P] ^= c[Sel<TO, G, P>::v]), ...);
+    ((out[P] ^= c[Sel<TO, G, P0 + P>::v]), ...);
 }
-template <bool TO, int NO, int... G>
+template <bool TO, int NO, int P0, int... G>
 SL_HD void lin_groups(const u32 *in, u32 *out, std::integer_sequence<int, G...>) {
-    (lin_group<TO, 4 * G>(in, out, std::make_integer_sequence<int, NO>{}), ...);
+    (lin_group<TO, 4 * G, P0>(in, out, std::make_integer_sequence<int, NO>{}), ...);
 }
-template <int NI, int NO, bool TO> SL_HD void lin_map(const u32 *in, u32 *out) {
+template <int NI, int NO, bool TO, int P0 = 0> SL_HD void lin_map(const u32 *in, u32 *out) {
 #pragma unroll
     for (int p = 0; p < NO; p++) out[p] = 0;
-    lin_groups<TO, NO>(in, out, std::make_integer_sequence<int, NI / 4>{});
+    lin_groups<TO, NO, P0>(in, out, std::make_integer_sequence<int, NI / 4>{});
 }
 
+SL_HD u32 byte_perm(u32 a, u32 b, u32 sel) {
+#ifdef __CUDACC__
+    return __byte_perm(a, b, sel);
+#else
+    const u64 v = a | (u64)b << 32;
+    u32 r = 0;
+    for (int i = 0; i < 4; i++) r |= (u32)((v >> (8 * ((sel >> (4 * i)) & 7))) & 255) << (8 * i);
+    return r;
+#endif
+}
 // 32 x 32 bit transposition in registers: bit i of x[j] <-> bit j of x[i]
 SL_HD void transpose32(u32 *x) {
 #pragma unroll
     for (int k = 0; k < 5; k++) {
         const int d = 16 >> k;
-        const u32 m = d == 16 ? 0x0000FFFFu : d == 8 ? 0x00FF00FFu : d == 4 ? 0x0F0F0F0Fu
-                    : d == 2 ? 0x33333333u : 0x55555555u;
+        const u32 m = d == 4 ? 0x0F0F0F0Fu : d == 2 ? 0x33333333u : 0x55555555u;
 #pragma unroll
         for (int j = 0; j < 32; j++) {
             if (j & d) continue;
-            const u32 t = ((x[j] >> d) ^ x[j + d]) & m;
-            x[j + d] ^= t;
-            x[j] ^= t << d;
+            const u32 a = x[j], b = x[j + d];
+            if (d == 16) {
+                x[j] = byte_perm(a, b, 0x5410);
+                x[j + d] = byte_perm(a, b, 0x7632);
+            } else if (d == 8) {
+                x[j] = byte_perm(a, b, 0x6240);
+                x[j + d] = byte_perm(a, b, 0x7351);
+            } else {
+                const u32 t = ((a >> d) ^ b) & m;
+                x[j + d] = b ^ t;
+                x[j] = a ^ (t << d);
+            }
         }
     }
 }
 
 // ------------------------------------------------- shared-memory slices
-// 16-byte chunks of a slice are XOR-swizzled by its number: any 8 slices that
-// differ in three of its four low bits put one chunk in 8 different banks,
-// which holds for the slices 8 lanes touch at every butterfly distance
-SL_HD u32 swz(u32 s) { return (s ^ (0u - ((s >> 3) & 1))) & 7; }
-SL_HD u32 chunk_at(u32 s, u32 c) { return (s << 4) + (c ^ swz(s)); }
-SL_HD u32 word_at(u32 s, u32 p) { return (chunk_at(s, p >> 2) << 2) + (p & 3); }
+// slices PITCH 16-byte chunks apart, an odd number, so that one chunk of 8
+// consecutive slices is in 8 different banks and every access of a thread is a
+// constant offset from its slice (an XOR swizzle without padding cost 24
+// address operations for 16 planes of a butterfly; the three smallest
+// butterfly distances conflict two ways here)
+template <int PITCH> struct Slab {
+    uint4 *t;
+    SL_HD uint4 &chunk(u32 s, u32 c) const { return t[s * PITCH + c]; }
+    SL_HD u32 &word(u32 s, u32 p) const { return reinterpret_cast<u32 *>(t)[s * (4 * PITCH) + p]; }
+};
+typedef Slab<17> Full;           // all 64 planes
+typedef Slab<9> Half;            // planes 0 .. 31 or 32 .. 63
 
-template <int N> SL_HD void load_planes(const uint4 *tile, u32 s, u32 c0, u32 *v) {
+// 16 bytes to shared memory, asynchronously on the device
+SL_HD void copy16(uint4 *dst, const uint4 *src) {
+#ifdef __CUDACC__
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                     (u32)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+#else
+    *dst = *src;
+#endif
+}
+SL_HD void copy_wait() {
+#ifdef __CUDACC__
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+#endif
+}
+
+// store(i, load(i)) for i < n, B loads in flight a thread before the first
+// store (global loads are not moved over shared stores otherwise: one at a
+// time, 11 of 17 us of a block of the levels above 2^16 were load latency)
+template <int B, class T, class L, class S>
+SL_HD void staged(u32 n, u32 tid, u32 nt, const L &load, const S &store) {
+    for (u32 i0 = tid; i0 < n; i0 += B * nt) {
+        T q[B];
+#pragma unroll
+        for (int k = 0; k < B; k++)
+            if (i0 + k * nt < n) q[k] = load(i0 + k * nt);
+#pragma unroll
+        for (int k = 0; k < B; k++)
+            if (i0 + k * nt < n) store(i0 + k * nt, q[k]);
+    }
+}
+
+template <int N, class S> SL_HD void load_planes(const S &tile, u32 s, u32 c0, u32 *v) {
 #pragma unroll
     for (int k = 0; k < N / 4; k++) {
-        const uint4 q = tile[chunk_at(s, c0 + k)];
+        const uint4 q = tile.chunk(s, c0 + k);
         v[4 * k] = q.x; v[4 * k + 1] = q.y; v[4 * k + 2] = q.z; v[4 * k + 3] = q.w;
     }
 }
-template <int N> SL_HD void store_planes(uint4 *tile, u32 s, u32 c0, const u32 *v) {
+template <int N, class S> SL_HD void store_planes(const S &tile, u32 s, u32 c0, const u32 *v) {
 #pragma unroll
     for (int k = 0; k < N / 4; k++) {
         uint4 q;
         q.x = v[4 * k]; q.y = v[4 * k + 1]; q.z = v[4 * k + 2]; q.w = v[4 * k + 3];
-        tile[chunk_at(s, c0 + k)] = q;
+        tile.chunk(s, c0 + k) = q;
     }
 }
 
 // ------------------------------------------------- butterflies
+// all ones where the top bit of byte b of w is set (a permute that repeats it)
+SL_HD u32 sign_byte(u32 w, int b) {
+#ifdef __CUDACC__
+    u32 r;
+    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(w), "r"((8 + b) * 0x1111));
+    return r;
+#else
+    return (u32)((int)(w << (24 - 8 * b)) >> 31);
+#endif
+}
 // masks of the N bits of w from bit `sh` (all ones where set), XORed with the
 // slice's pattern where its elements differ
 template <int N> SL_HD void masks_of(u32 w, int sh, const u32 *pat, u32 *out) {
 #pragma unroll
     for (int i = 0; i < N; i++) {
-        out[i] = (u32)((int)(w << (31 - (sh + i))) >> 31);
+        const int b = sh + i;
+        out[i] = sign_byte(w << (7 - (b & 7)), b >> 3);
         if (pat) out[i] ^= pat[i];
     }
 }
 
-// one butterfly of a group of planes [c0, c0 + N/4 chunks): FWD: u += w v,
-// v += u; inverse: v += u, u += w v.  mul(v, p): p = w v
-template <int N, bool FWD, class Mul>
-SL_HD void bfly_planes(uint4 *tile, u32 su, u32 sv, u32 c0, const Mul &mul) {
-    u32 u[N], v[N], p[N];
+// butterflies of the N planes from chunk c0: FWD: u += w v, v += u; inverse:
+// v += u, u += w v.  addmul(v, u): u += w v
+template <int N, bool FWD, class S, class Mul>
+SL_HD void bfly_planes(const S &tile, u32 su, u32 sv, u32 c0, const Mul &addmul) {
+    u32 u[N], v[N];
     load_planes<N>(tile, sv, c0, v);
     load_planes<N>(tile, su, c0, u);
     if (FWD) {
-        mul(v, p);
+        addmul(v, u);
 #pragma unroll
-        for (int i = 0; i < N; i++) { u[i] ^= p[i]; v[i] ^= u[i]; }
+        for (int i = 0; i < N; i++) v[i] ^= u[i];
+        store_planes<N>(tile, sv, c0, v);
     } else {
 #pragma unroll
         for (int i = 0; i < N; i++) v[i] ^= u[i];
-        mul(v, p);
-#pragma unroll
-        for (int i = 0; i < N; i++) u[i] ^= p[i];
+        store_planes<N>(tile, sv, c0, v);
+        addmul(v, u);
     }
-    store_planes<N>(tile, sv, c0, v);
     store_planes<N>(tile, su, c0, u);
 }
 
 // the butterfly of one slice pair over `NQ` quarters (16 planes each) from
-// quarter q0; nb = m - 1 - L bits of t decide the subfield
-template <int NQ, bool FWD>
-SL_HD void bfly_pair(uint4 *tile, u32 su, u32 sv, u32 q0, int nb, u32 w, const u32 *pat) {
+// quarter q0; nb = m - 1 - L, the number of Cantor basis elements the level's
+// twiddles are sums of, decides the subfield
+template <int NQ, bool FWD, class S>
+SL_HD void bfly_pair(const S &tile, u32 su, u32 sv, u32 q0, int nb, u32 w, const u32 *pat) {
     if (nb == 0) {                              // W[0] = 0
+#pragma unroll 1
         for (int q = 0; q < NQ; q++)
-            bfly_planes<16, FWD>(tile, su, sv, 4 * (q0 + q), [](const u32 *, u32 *p) {
-#pragma unroll
-                for (int i = 0; i < 16; i++) p[i] = 0;
-            });
+            bfly_planes<16, FWD>(tile, su, sv, 4 * (q0 + q), [](const u32 *, u32 *) {});
     } else if (nb <= 7) {
         u32 wm[8];
+        Prep<8> b;
         masks_of<8>(w, 0, pat, wm);
+        b.set(wm);
 #pragma unroll 1
-        for (int q = 0; q < 2 * NQ; q += 2)
-            bfly_planes<16, FWD>(tile, su, sv, 4 * q0 + 2 * q, [&](const u32 *v, u32 *p) {
-                t_mul<8>(v, wm, p);
-                t_mul<8>(v + 8, wm, p + 8);
+        for (int q = 0; q < NQ; q++)
+            bfly_planes<16, FWD>(tile, su, sv, 4 * (q0 + q), [&](const u32 *v, u32 *u) {
+                t_addmul<8>(v, b, u);
+                t_addmul<8>(v + 8, b, u + 8);
             });
     } else if (nb <= 15) {
         u32 wm[16];
+        Prep<16> b;
         masks_of<16>(w, 0, pat, wm);
+        b.set(wm);
 #pragma unroll 1
         for (int q = 0; q < NQ; q++)
             bfly_planes<16, FWD>(tile, su, sv, 4 * (q0 + q),
-                                 [&](const u32 *v, u32 *p) { t_mul<16>(v, wm, p); });
-    } else if constexpr (NQ >= 2) {             // m > 16: two quarters a thread
-        // w = w0 + w1 X with w1 in GF(2^8); (v0 + v1 X)(w0 + w1 X), X^2 = X + v_15
-        u32 w0[16], ws[16], w1[8];
-        masks_of<16>(w, 0, pat, w0);
-        masks_of<8>(w, 16, nullptr, w1);
-#pragma unroll
-        for (int i = 0; i < 16; i++) ws[i] = i < 8 ? w0[i] ^ w1[i] : w0[i];
+                                 [&](const u32 *v, u32 *u) { t_addmul<16>(v, b, u); });
+    } else if constexpr (NQ >= 2) {             // m > 16: two quarters at a time
+        // w = w0 + w1 X, w1 = b / t with b in GF(2^8), the high byte of w, as
+        // elements past 16 of the basis are b_i X / t + ...: the half product
+        // by w1 is one by b of (v0 + v1) / t, 1 / t = X' + t' one tower below
+        const u32 w1 = w >> 16;
+        u32 x[16];
+        Prep<16> a0, a2;
+        Prep<8> a1;
+        masks_of<16>(w ^ w1, 0, pat, x);
+        a0.set(x);
+        masks_of<16>(w ^ w1 ^ (w >> 24), 0, pat, x);          // t w1 = b
+        a2.set(x);
+        masks_of<8>(w, 24, nullptr, x);
+        a1.set(x);
 #pragma unroll 1
         for (int q = 0; q < NQ; q += 2)
-            bfly_planes<32, FWD>(tile, su, sv, 4 * (q0 + q), [&](const u32 *v, u32 *p) {
-                u32 a[16], b[16];
-                t_mul<8>(v + 16, w1, a);
-                t_mul<8>(v + 24, w1, a + 8);
-                t_delta<16>(a, p);
-                t_mul<16>(v, w0, a);
+            bfly_planes<32, FWD>(tile, su, sv, 4 * (q0 + q), [&](const u32 *v, u32 *u) {
+                u32 z[16], y[16], p[16];
 #pragma unroll
-                for (int i = 0; i < 16; i++) { p[i] ^= a[i]; b[i] = v[i] ^ v[16 + i]; }
-                t_mul<16>(b, ws, p + 16);
+                for (int i = 0; i < 16; i++) { y[i] = v[i] ^ v[16 + i]; p[i] = 0; }
+                t_mulx<8>(y, z);                          // y / t = (y1 + t' y0) + y0 X'
 #pragma unroll
-                for (int i = 0; i < 16; i++) p[16 + i] ^= a[i];
+                for (int i = 0; i < 8; i++) { z[i] ^= y[8 + i]; z[8 + i] = y[i]; }
+                t_addmul<8>(z, a1, p);
+                t_addmul<8>(z + 8, a1, p + 8);
+                t_addmul<16>(v, a0, u);
+                t_addmul<16>(v + 16, a2, u + 16);
+#pragma unroll
+                for (int i = 0; i < 16; i++) { u[i] ^= p[i]; u[16 + i] ^= p[i]; }
             });
     }
 }
@@ -319,13 +467,14 @@ SL_HD u32 tile_gslice(const Tile &T, u32 s) {
     return T.base + ((s >> T.clog) << (T.llo - 5)) + (s & ((1u << T.clog) - 1));
 }
 
-// level L >= 5 of the tile (slices hold 32 consecutive elements)
-template <int NQ, bool FWD>
-SL_HD void level_n(uint4 *tile, const Tile &T, int L, u32 tid, u32 nt) {
+// level L >= 5 of the tile (slices hold 32 consecutive elements) on its NT
+// quarters, NQ of a slice pair a thread
+template <int NT, int NQ, bool FWD, class S>
+SL_HD void level_n(const S &tile, const Tile &T, int L, u32 tid, u32 nt) {
     const int lg = L - T.llo + T.clog;
     const u32 pairs = 1u << (T.rlog + T.clog - 1);
     const int pl = T.rlog + T.clog - 1;
-    for (u32 i = tid; i < pairs * (4 / NQ); i += nt) {
+    for (u32 i = tid; i < pairs * (NT / NQ); i += nt) {
         const u32 g = i & (pairs - 1), q0 = (i >> pl) * NQ;
         const u32 su = ((g >> lg) << (lg + 1)) | (g & ((1u << lg) - 1)), sv = su | (1u << lg);
         const u32 t = tile_gslice(T, su) >> (L - 4);
@@ -335,11 +484,11 @@ SL_HD void level_n(uint4 *tile, const Tile &T, int L, u32 tid, u32 nt) {
 
 // level L <= 4 of a contiguous tile whose groups of 32 slices are transposed
 // (slice s of a group holds the elements 32 b + s)
-template <int NQ, bool FWD>
-SL_HD void level_x(uint4 *tile, const Tile &T, int L, u32 tid, u32 nt) {
+template <int NT, int NQ, bool FWD, class S>
+SL_HD void level_x(const S &tile, const Tile &T, int L, u32 tid, u32 nt) {
     const u32 pairs = 1u << (T.rlog + T.clog - 1);
     const int pl = T.rlog + T.clog - 1;
-    for (u32 i = tid; i < pairs * (4 / NQ); i += nt) {
+    for (u32 i = tid; i < pairs * (NT / NQ); i += nt) {
         const u32 g = i & (pairs - 1), q0 = (i >> pl) * NQ;
         const u32 su = ((g >> L) << (L + 1)) | (g & ((1u << L) - 1)), sv = su | (1u << L);
         const u32 G = (T.base + su) >> 5, s = su & 31;
@@ -348,44 +497,76 @@ SL_HD void level_x(uint4 *tile, const Tile &T, int L, u32 tid, u32 nt) {
     }
 }
 
-// elements of each group of 32 slices transposed (32 b + s <-> 32 s + b)
-SL_HD void transpose_groups(uint4 *tile, u32 nslices, u32 tid, u32 nt) {
-    u32 *w = reinterpret_cast<u32 *>(tile);
-    for (u32 i = tid; i < nslices * 2; i += nt) {
-        const u32 g = (i >> 6) << 5, p = i & 63;
+// elements of each group of 32 slices transposed (32 b + s <-> 32 s + b),
+// 16 NT planes
+template <int NT, class S>
+SL_HD void transpose_groups(const S &tile, u32 nslices, u32 tid, u32 nt) {
+    for (u32 i = tid; i < nslices / 2 * NT; i += nt) {
+        const u32 g = i / (16 * NT) << 5, p = i & (16 * NT - 1);
         u32 x[32];
 #pragma unroll
-        for (int s = 0; s < 32; s++) x[s] = w[word_at(g + s, p)];
+        for (int s = 0; s < 32; s++) x[s] = tile.word(g + s, p);
         transpose32(x);
 #pragma unroll
-        for (int s = 0; s < 32; s++) w[word_at(g + s, p)] = x[s];
+        for (int s = 0; s < 32; s++) tile.word(g + s, p) = x[s];
     }
 }
 
-// 32 chunk planes -> 64 tower planes, and 64 tower -> 64 polynomial planes
-SL_HD void phi_in(uint4 *tile, u32 nslices, u32 tid, u32 nt) {
+// 32 chunk planes -> tower planes 32 H .. 32 H + 31, in place
+template <int H> SL_HD void phi_in(const Half &tile, u32 nslices, u32 tid, u32 nt) {
     for (u32 s = tid; s < nslices; s += nt) {
-        u32 a[32], b[64];
+        u32 a[32], b[32];
         load_planes<32>(tile, s, 0, a);
-        lin_map<32, 64, true>(a, b);
-        store_planes<64>(tile, s, 0, b);
+        lin_map<32, 32, true, 32 * H>(a, b);
+        store_planes<32>(tile, s, 0, b);
     }
 }
-SL_HD void phi_out(uint4 *tile, u32 nslices, u32 tid, u32 nt) {
-    for (u32 s = tid; s < nslices; s += nt) {
-        u32 a[64], b[64];
-        load_planes<64>(tile, s, 0, a);
-        lin_map<64, 64, false>(a, b);
-        store_planes<64>(tile, s, 0, b);
-    }
-}
-SL_HD void mul_slices(uint4 *fa, const uint4 *fb, u32 nslices, u32 tid, u32 nt) {
+SL_HD void mul_slices(const Full &fa, const Full &fb, u32 nslices, u32 tid, u32 nt) {
     for (u32 s = tid; s < nslices; s += nt) {
         u32 a[64], b[64], c[64];
         load_planes<64>(fa, s, 0, a);
         load_planes<64>(fb, s, 0, b);
-        t_mul<64>(a, b, c);
+        Prep<64> m;
+        m.set(b);
+#pragma unroll
+        for (int i = 0; i < 64; i++) c[i] = 0;
+        t_addmul<64>(a, m, c);
         store_planes<64>(fa, s, 0, c);
+    }
+}
+
+// the same in two steps of half products, for blocks with 128 registers a
+// thread: the middle product of each slice, then the two it joins
+SL_HD void mul_mid(const Full &fa, const Full &fb, const Half &mid, u32 nslices, u32 tid, u32 nt) {
+    for (u32 s = tid; s < nslices; s += nt) {
+        u32 a[32], b[32], c[32];
+        load_planes<32>(fa, s, 0, a);
+        load_planes<32>(fa, s, 8, b);
+#pragma unroll
+        for (int i = 0; i < 32; i++) { a[i] ^= b[i]; c[i] = 0; }
+        load_planes<32>(fb, s, 8, b);
+        Prep<32> m;
+        m.set(b);
+        t_addmul<32>(a, m, c);
+        store_planes<32>(mid, s, 0, c);
+    }
+}
+SL_HD void mul_ends(const Full &fa, const Full &fb, const Half &mid, u32 nslices, u32 tid, u32 nt) {
+    for (u32 i = tid; i < 2 * nslices; i += nt) {
+        const u32 h = i >= nslices ? 1 : 0, s = i - h * nslices;
+        u32 a[32], b[32], c[32];
+        load_planes<32>(fb, s, 8, a);
+        t_mulx<32>(a, c);
+        load_planes<32>(fb, s, 0, b);
+        const u32 both = 0u - h;
+#pragma unroll
+        for (int k = 0; k < 32; k++) b[k] ^= a[k] ^ (c[k] & both);
+        Prep<32> m;
+        m.set(b);
+        load_planes<32>(fa, s, 8 * h, a);
+        load_planes<32>(mid, s, 0, c);
+        t_addmul<32>(a, m, c);
+        store_planes<32>(fa, s, 8 * h, c);
     }
 }
 
@@ -415,25 +596,23 @@ inline void add_levels(Levels &lv, int lo, int hi) {
     add_levels(lv, lo, lo + h);
 }
 
+// one level inside a word, M <= 5: shifting right by half - c takes the top
+// chunk to the lowest of the high half and the high half onto the low one
+template <int M, int A, bool FWD, class V> SL_HD V word_level(V x) {
+    constexpr int half = 1 << (M - 1), c = 1 << A;
+    constexpr u32 lowc = (1u << c) - 1, halfm = (u32)((1ull << half) - 1);
+    constexpr u32 ones = (u32)(0xFFFFFFFFull / ((1ull << (2 * half)) - 1));     // one a block
+    constexpr u32 to_a = ones * (halfm & ~lowc), to_h = (ones * lowc) << half;
+    if (!FWD) return x ^ ((x >> (half - c)) & (to_a | to_h));
+    x = x ^ ((x >> (half - c)) & to_h);
+    return x ^ ((x >> (half - c)) & to_a);
+}
 // one level on 8 words (256 coefficients), M <= 8
 template <int M, int A, bool FWD> SL_HD void reg_level(u32 *x) {
     constexpr int c = 1 << A;
     if constexpr (M <= 5) {
-        constexpr int half = 1 << (M - 1);
-        constexpr u32 lowc = (1u << c) - 1;
-        u32 lm = 0, cm = 0;                      // low halves, and their low chunks
-        for (int b = 0; b < 32; b += 2 * half) {
-            lm |= (u32)((1ull << half) - 1) << b;
-            cm |= lowc << b;
-        }
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            u32 h = (x[j] >> half) & lm, l = x[j] & lm;
-            if (FWD) h ^= (h >> (half - c)) & cm;
-            l ^= (h << c) & lm;
-            if (!FWD) h ^= (h >> (half - c)) & cm;
-            x[j] = l | (h << half);
-        }
+        for (int j = 0; j < 8; j++) x[j] = word_level<M, A, FWD>(x[j]);
     } else {
         constexpr int hw = 1 << (M - 6);         // words of a half
 #pragma unroll
@@ -478,13 +657,10 @@ template <bool FWD> SL_HD void reg_taylor8(u32 *x) {
 }
 
 // word j of plane p of a Taylor tile: at(j, p)
-struct TaylorAddr {              // [word][2^plog planes]
+struct SliceAddr {               // a Full tile of slices
+    static constexpr bool rows_first = false;
     int plog;
-    SL_HD u32 operator()(u32 j, u32 p) const { return (j << plog) + p; }
-};
-struct SliceAddr {               // a tile of slices
-    int plog;
-    SL_HD u32 operator()(u32 j, u32 p) const { return word_at(j, p); }
+    SL_HD u32 operator()(u32 j, u32 p) const { return j * 68 + p; }
 };
 
 // level (M, a), M >= 9, of 2^k coefficients (2^(k-5) words) x 2^plog planes
@@ -517,9 +693,10 @@ SL_HD void taylor_level(u32 *sm, const At &at, int k, int M, int a, u32 tid, u32
 }
 template <bool FWD, class At>
 SL_HD void taylor_regs(u32 *sm, const At &at, int k, u32 tid, u32 nt) {
-    const u32 np = 1u << at.plog, items = (1u << (k - 8)) << at.plog;
+    const u32 nr = 1u << (k - 8), items = nr << at.plog;
     for (u32 i = tid; i < items; i += nt) {
-        const u32 p = i & (np - 1), r = (i >> at.plog) << 3;
+        const u32 p = At::rows_first ? i >> (k - 8) : i & ((1u << at.plog) - 1);
+        const u32 r = (At::rows_first ? i & (nr - 1) : i >> at.plog) << 3;
         u32 x[8];
 #pragma unroll
         for (int j = 0; j < 8; j++) x[j] = sm[at(r + j, p)];
@@ -529,69 +706,151 @@ SL_HD void taylor_regs(u32 *sm, const At &at, int k, u32 tid, u32 nt) {
     }
 }
 
-// Levels of a conversion of 2^k > 2^16 coefficients above the split at 2^16:
-// rows of 2^16 coefficients, a tile of 2^tlog words (columns) of every row
-// with `halo` words to their left.  Row e with bit b set moves by 2^b
-// coefficients into row e without it; what moves past a row's end is kept
-// apart and folded once (x^65536 = y + x forward, the next row inverse).
-struct HiGeom {
-    int rlog;                    // rows 2^rlog, rlog = k - 16 (1 .. 8)
-    int tlog, plog;              // words a tile, planes
-    u32 halo;                    // words: at least 2^rlog - 1 coefficients
-};
-#ifdef __CUDACC__
-__host__
-#endif
-SL_HD u32 hi_pitch(const HiGeom &G) { return (1u << G.tlog) + G.halo; }
-SL_HD u32 hi_at(const HiGeom &G, u32 row, u32 col, u32 p) {
-    return ((row * hi_pitch(G) + col) << G.plog) + p;
-}
-SL_HD void hi_shift(u32 *sm, const HiGeom &G, int b, u32 tid, u32 nt) {
-    const u32 np = 1u << G.plog, W = hi_pitch(G);
-    const u32 items = (W << (G.rlog - 1)) << G.plog;
-    for (u32 i = tid; i < items; i += nt) {
-        const u32 p = i & (np - 1), g = i >> G.plog, rr = g / W, col = g - rr * W;
-        const u32 lo = ((rr >> b) << (b + 1)) | (rr & ((1u << b) - 1)), hi = lo | (1u << b);
-        u32 v;
-        if (b >= 5) {
-            const u32 cw = 1u << (b - 5);
-            if (col < cw) continue;
-            v = sm[hi_at(G, hi, col - cw, p)];
-        } else {
-            const int c = 1 << b;
-            v = sm[hi_at(G, hi, col, p)] << c;
-            if (col) v |= sm[hi_at(G, hi, col - 1, p)] >> (32 - c);
+// The same conversions in the registers of one warp, a plane each: word
+// r * 32 + lane of 2^k coefficients in x[r] (k >= 10).  Words half a block
+// apart are registers or lanes; a shift by less than 32 words takes the lane
+// below's word by shuffle.  (In shared memory a level costs three accesses
+// and a dozen address instructions a word: 2^16 coefficients of 32 planes of
+// two operands took 328 us at 2^23 coefficients.)
+template <int M, int A, bool FWD, int NR> SL_HD void warp_level(V (&x)[NR]) {
+    const V lane = lane_id();
+    constexpr int hw = M >= 6 ? 1 << (M - 6) : 0;          // words of a half
+    constexpr int c = 1 << A, cw = c / 32;
+    if constexpr (M <= 5) {
+#pragma unroll
+        for (int r = 0; r < NR; r++) x[r] = word_level<M, A, FWD>(x[r]);
+    } else if constexpr (hw >= 32) {
+        constexpr int hr = hw / 32;
+#pragma unroll
+        for (int b = 0; b < NR; b += 2 * hr) {
+            V *a = x + b, *h = x + b + hr;
+            if constexpr (cw >= 32) {
+                constexpr int cr = cw / 32;
+                if (FWD)
+#pragma unroll
+                    for (int j = 0; j < cr; j++) h[j] ^= h[hr - cr + j];
+#pragma unroll
+                for (int j = cr; j < hr; j++) a[j] ^= h[j - cr];
+                if (!FWD)
+#pragma unroll
+                    for (int j = 0; j < cr; j++) h[j] ^= h[hr - cr + j];
+            } else if constexpr (cw >= 1) {
+                const V from = (lane - V(cw)) & V(31), low = below(lane, cw);
+                if (FWD) h[0] ^= shfl(h[hr - 1], from) & low;
+                V prev = V(0);
+#pragma unroll
+                for (int j = 0; j < hr; j++) {
+                    const V t = shfl(h[j], from);
+                    a[j] ^= (prev & low) | (t & ~low);
+                    prev = t;
+                }
+                if (!FWD) h[0] ^= prev & low;
+            } else {
+                // the low c bits that the top chunk changes in word 0 are not
+                // among the top ones the next word takes from it
+                const V from = (lane - V(1)) & V(31), low = below(lane, 1);
+                V prev = V(0);
+                if (FWD) h[0] ^= (shfl(h[hr - 1], from) >> (32 - c)) & low;
+#pragma unroll
+                for (int j = 0; j < hr; j++) {
+                    const V t = shfl(h[j], from), p = (prev & low) | (t & ~low);
+                    a[j] ^= (h[j] << c) | (p >> (32 - c));
+                    prev = t;
+                }
+                if (!FWD) h[0] ^= (prev >> (32 - c)) & low;
+            }
         }
-        sm[hi_at(G, lo, col, p)] ^= v;
-    }
-}
-// level (M, a) of the conversion over the row index, columns from col0 on
-template <bool FWD>
-SL_HD void hi_rows(u32 *sm, const HiGeom &G, int M, int a, u32 col0, u32 tid, u32 nt) {
-    const u32 np = 1u << G.plog, n = hi_pitch(G) - col0;
-    const u32 half = 1u << (M - 1), c = 1u << a;
-    const u32 items = (n << (G.rlog - 1)) << G.plog;
-    for (u32 i = tid; i < items; i += nt) {
-        const u32 p = i & (np - 1), g = i >> G.plog, rr = g / n, col = col0 + g - rr * n;
-        const u32 j = rr & (half - 1), b = (rr >> (M - 1)) << M;
-        const u32 ih = hi_at(G, b + half + j, col, p);
-        u32 h = sm[ih];
-        const u32 top = j < c ? sm[hi_at(G, b + 2 * half - c + j, col, p)] : 0;
-        if (FWD && j < c) { h ^= top; sm[ih] = h; }
-        if (j + c < half) sm[hi_at(G, b + j + c, col, p)] ^= h;
-        if (!FWD && j < c) sm[ih] = h ^ top;
+    } else {
+        const V j = lane & V(hw - 1), lo = below(lane & V(hw), 1), hi = ~lo;
+        if constexpr (cw >= 1) {
+            const V from = (lane + V(hw - cw)) & V(31);
+            const V top = hi & below(j, cw), to_a = lo & ~below(j, cw);
+#pragma unroll
+            for (int r = 0; r < NR; r++) {
+                if (FWD) {
+                    x[r] ^= shfl(x[r], from) & top;
+                    x[r] ^= shfl(x[r], from) & to_a;
+                } else {
+                    x[r] ^= shfl(x[r], from) & (top | to_a);
+                }
+            }
+        } else {
+            const V from = (lane + V(hw)) & V(31), prev = (lane + V(hw - 1)) & V(31);
+            const V first = below(j, 1), top = hi & first, to_a = lo & ~first;
+#pragma unroll
+            for (int r = 0; r < NR; r++) {
+                const V p = shfl(x[r], prev) >> (32 - c);
+                if (FWD) x[r] ^= p & top;
+                const V h = shfl(x[r], from);
+                x[r] ^= ((h << c) & lo) ^ (p & to_a);
+                if (!FWD) x[r] ^= p & top;
+            }
+        }
     }
 }
 
+// the levels of a conversion over index bits [LO, HI) in forward or inverse
+// order (add_levels at compile time; [0, 8) of a split at 2^8 left out)
+constexpr int split_of(int m) { int h = 1; while (2 * h < m) h *= 2; return h; }
+template <bool FWD, int LO, int HI> struct Conv {
+    static constexpr int m = HI - LO, h = split_of(m);
+    template <class Op, int... I>
+    static SL_HD void own(const Op &op, std::integer_sequence<int, I...>) {
+        if (FWD) (op.template level<LO + m - I, LO + m - I - 1 - h>(), ...);
+        else (op.template level<LO + h + 1 + I, LO + I>(), ...);
+    }
+    template <class Op> static SL_HD void lower(const Op &op) {
+        if constexpr (!(LO == 0 && HI > 8 && h == 8 && Op::skip_low)) Conv<FWD, LO, LO + h>::run(op);
+    }
+    template <class Op> static SL_HD void run(const Op &op) {
+        if constexpr (m > 1) {
+            if constexpr (FWD) {
+                own(op, std::make_integer_sequence<int, m - h>{});
+                Conv<FWD, LO + h, HI>::run(op);
+                lower(op);
+            } else {
+                lower(op);
+                Conv<FWD, LO + h, HI>::run(op);
+                own(op, std::make_integer_sequence<int, m - h>{});
+            }
+        }
+    }
+};
+template <bool FWD, int NR> struct WarpLevels {
+    static constexpr bool skip_low = true;
+    V (&x)[NR];
+    template <int M, int A> SL_HD void level() const { warp_level<M, A, FWD>(x); }
+};
+
+// a Taylor tile a plane after another: word j of plane p, swizzled so that
+// 32 consecutive words, and word j of 32 consecutive groups of 8, are in
+// different banks, and the stores of 16-byte chunks of 16 slices too
+struct PlaneAddr {
+    static constexpr bool rows_first = true;
+    int plog, pitch;
+    SL_HD u32 operator()(u32 j, u32 p) const { return p * pitch + (j ^ ((j >> 5) & 7)); }
+};
+template <int K, bool FWD> SL_HD void taylor_warp(u32 *sm, const PlaneAddr &at, u32 p) {
+    constexpr int NR = 1 << (K - 10);
+    V x[NR];
+#pragma unroll
+    for (int r = 0; r < NR; r++)
+        x[r] = lane_load(sm, [&](u32 l) { return at(r * 32 + l, p); });
+    Conv<FWD, 0, K>::run(WarpLevels<FWD, NR>{x});
+#pragma unroll
+    for (int r = 0; r < NR; r++)
+        lane_store(sm, [&](u32 l) { return at(r * 32 + l, p); }, x[r]);
+}
+
 // ------------------------------------------------- host-side pass planning
+constexpr int SMALL_M = 12;      // whole products in one block up to 2^12 coefficients
 struct BflyPass { int llo, rlog, clog; };
 struct Plan {
     int m = 0;
     int low = 0;                 // the last forward pass: levels low-1 .. 0
     int ntop = 0;
     BflyPass top[3];             // forward order
-    Levels rows[9];              // rows[k-16]: conversions over k - 16 row bits
-    Levels taylor[17];           // taylor[k]: smem levels of 2^k coefficients
+    Levels taylor[SMALL_M + 1];  // taylor[k]: a small product's levels of 2^k coefficients
 };
 constexpr int TILE_LOG = 9;      // at most 512 slices a tile
 inline Plan make_plan(int m, int low, int clog) {
@@ -610,13 +869,9 @@ inline Plan make_plan(int m, int low, int clog) {
         if (c > hi - 5) c = hi - 5;
         P.top[P.ntop++] = BflyPass{hi, take, c};
     }
-    for (int k = 8; k <= 16; k++) {
+    for (int k = 8; k <= SMALL_M; k++) {
         P.taylor[k].n = 0;
         if (k > 8) add_levels(P.taylor[k], 0, k);
-    }
-    for (int k = 0; k <= 8; k++) {
-        P.rows[k].n = 0;
-        add_levels(P.rows[k], 0, k);
     }
     return P;
 }
@@ -625,18 +880,27 @@ inline Plan make_plan(int m, int low, int clog) {
 // Each body is a sequence of steps ex([&](tid, nt) {...}) with a barrier
 // after every step; `sm` is the block's shared memory.
 
-// 32-bit chunks of an operand (chunk 0 XORed with xor0, zero from nchunks)
+// 32-bit chunks of an operand of 64-bit words (chunk 0 XORed with xor0, zero from nchunks)
 // into planes 0 .. 31 of the slices [s0, s0 + 2^nlog)
 template <class Ex>
 SL_HD void body_slice_in(Ex ex, u32 *sm, const u32 *src, u64 nchunks, u32 xor0, uint4 *f, u32 s0,
                          int nlog) {
     ex([&](u32 tid, u32 nt) {
-        for (u32 i = tid; i < (32u << nlog); i += nt) {
-            const u64 k = (u64)s0 * 32 + i;
-            u32 v = k < nchunks ? src[k] : 0;
-            if (k == 0) v ^= xor0;
-            sm[(i >> 5) * 33 + (i & 31)] = v;
-        }
+        const u64 *src64 = reinterpret_cast<const u64 *>(src);
+        staged<8, u64>(
+            16u << nlog, tid, nt,
+            [&](u32 i) {
+                const u64 k = (u64)s0 * 32 + 2 * i;
+                u64 v = k < nchunks ? src64[k >> 1] : 0;
+                if (k + 1 == nchunks) v = (u32)v;
+                return v;
+            },
+            [&](u32 i, u64 v) {
+                if (i == 0 && s0 == 0) v ^= xor0;
+                u32 *w = sm + (i >> 4) * 33 + 2 * (i & 15);
+                w[0] = (u32)v;
+                w[1] = (u32)(v >> 32);
+            });
     });
     ex([&](u32 tid, u32 nt) {
         for (u32 s = tid; s < (1u << nlog); s += nt) {
@@ -658,214 +922,281 @@ SL_HD void body_slice_in(Ex ex, u32 *sm, const u32 *src, u64 nchunks, u32 xor0, 
     });
 }
 
-// Taylor conversion of the 2^k coefficients from slice s0 on, planes
+// Taylor conversion of the 2^K coefficients from slice s0 on, planes
 // [4 c0, 4 c0 + 2^plog), read at chunk offset c_src, written at chunk c0 of
 // these slices and of `reps` - 1 copies rep_stride slices apart
-template <bool FWD, class Ex>
-SL_HD void body_taylor(Ex ex, u32 *sm, uint4 *f, u32 s0, int k, int plog, u32 c0, u32 c_src,
-                       u32 reps, u32 rep_stride, const Levels &lv) {
-    const TaylorAddr at{plog};
+template <int K, bool FWD, class Ex>
+SL_HD void body_taylor(Ex ex, u32 *sm, uint4 *f, u32 s0, int plog, u32 c0, u32 c_src, u32 reps,
+                       u32 rep_stride) {
+    const PlaneAddr at{plog, (1 << (K - 5)) + 4};
     const int cl = plog - 2;                         // log2 chunks a word
-    const u32 items = 1u << (k - 5 + cl);
-    uint4 *sm4 = reinterpret_cast<uint4 *>(sm);
+    const u32 items = 1u << (K - 5 + cl);
     ex([&](u32 tid, u32 nt) {
-        for (u32 i = tid; i < items; i += nt)
-            sm4[i] = f[(u64)(s0 + (i >> cl)) * 16 + c_src + (i & ((1u << cl) - 1))];
+        staged<8, uint4>(
+            items, tid, nt,
+            [&](u32 i) {
+                return f[(u64)(s0 + (i >> cl)) * 16 + c_src + (i & ((1u << cl) - 1))];
+            },
+            [&](u32 i, const uint4 &q) {
+                const u32 j = i >> cl, c = i & ((1u << cl) - 1);
+                sm[at(j, 4 * c)] = q.x;
+                sm[at(j, 4 * c + 1)] = q.y;
+                sm[at(j, 4 * c + 2)] = q.z;
+                sm[at(j, 4 * c + 3)] = q.w;
+            });
     });
-    if (!FWD) ex([&](u32 tid, u32 nt) { taylor_regs<false>(sm, at, k, tid, nt); });
-    for (int l = 0; l < lv.n; l++) {
-        const int q = FWD ? l : lv.n - 1 - l;
-        ex([&](u32 tid, u32 nt) { taylor_level<FWD>(sm, at, k, lv.M[q], lv.a[q], tid, nt); });
-    }
-    if (FWD) ex([&](u32 tid, u32 nt) { taylor_regs<true>(sm, at, k, tid, nt); });
+    if (!FWD) ex([&](u32 tid, u32 nt) { taylor_regs<false>(sm, at, K, tid, nt); });
+    ex.warps(1u << plog, [&](u32 p) { taylor_warp<K, FWD>(sm, at, p); });
+    if (FWD) ex([&](u32 tid, u32 nt) { taylor_regs<true>(sm, at, K, tid, nt); });
     ex([&](u32 tid, u32 nt) {
         for (u32 i = tid; i < items; i += nt) {
-            const uint4 q = sm4[i];
-            for (u32 r = 0; r < reps; r++)
-                f[(u64)(s0 + r * rep_stride + (i >> cl)) * 16 + c0 + (i & ((1u << cl) - 1))] = q;
+            const u32 j = i >> cl, c = i & ((1u << cl) - 1);
+            uint4 q;
+            q.x = sm[at(j, 4 * c)];
+            q.y = sm[at(j, 4 * c + 1)];
+            q.z = sm[at(j, 4 * c + 2)];
+            q.w = sm[at(j, 4 * c + 3)];
+            for (u32 r = 0; r < reps; r++) f[(u64)(s0 + r * rep_stride + j) * 16 + c0 + c] = q;
         }
     });
 }
 
-// Taylor levels above 2^16 (HiGeom) of planes [4 c_src, ..) of `src` to
-// chunk c_dst of `dst` (not the same chunks), column tile `ct`.  `side`
-// holds the overflow of the first tile: 2^rlog rows x halo words x planes.
-template <bool FWD, class Ex>
-SL_HD void body_taylor_hi(Ex ex, u32 *sm, u32 *side, const uint4 *src, u32 c_src, uint4 *dst,
-                          u32 c_dst, const HiGeom G, u32 ct, const Levels &rows) {
-    const int cl = G.plog - 2;
-    const u32 cm = (1u << cl) - 1, T = 1u << G.tlog, W = hi_pitch(G), R = 1u << G.rlog;
-    uint4 *sm4 = reinterpret_cast<uint4 *>(sm);
-    // col < halo: the words left of the tile; `tail`: those left of column 0
-    // are the row's last words and the body is empty
+// Taylor levels above 2^16: 2^RLOG rows of 2^16 coefficients.  Row e with bit
+// b set moves by 2^b coefficients into row e without it; what moves past a
+// row's end is kept apart and folded once (x^65536 = y + x forward, the next
+// row inverse).  A warp holds one plane's rows in registers, 32 consecutive
+// words in its lanes, the first HALO of them the words to the tile's left
+// (at least 2^RLOG - 1 coefficients).
+template <int RLOG> struct Hi {
+    static constexpr int PLOG = RLOG >= 7 ? 2 : 3;         // planes a block: 4 of 128 rows
+    static constexpr int CL = PLOG - 2;                    // log2 chunks a word
+    static constexpr int R = 1 << RLOG, HALO = RLOG <= 5 ? 1 : 1 << (RLOG - 5), T = 32 - HALO;
+    static constexpr int TILES = (2048 + T - 1) / T;
+    static constexpr int PITCH = 36;             // words a row and plane
+    static SL_HD u32 at(u32 row, u32 p, u32 col) { return ((row << PLOG) + p) * PITCH + col; }
+    static constexpr int WORDS = (R << PLOG) * (PITCH + HALO);
+};
+template <bool FWD, int NR> struct RowLevels {
+    static constexpr bool skip_low = false;
+    V (&x)[NR];
+    template <int M, int A> SL_HD void level() const {
+        constexpr int half = 1 << (M - 1), c = 1 << A;
+#pragma unroll
+        for (int b = 0; b < NR; b += 2 * half) {
+            V *a = x + b, *h = x + b + half;
+            if (FWD)
+#pragma unroll
+                for (int j = 0; j < c; j++) h[j] ^= h[half - c + j];
+#pragma unroll
+            for (int j = c; j < half; j++) a[j] ^= h[j - c];
+            if (!FWD)
+#pragma unroll
+                for (int j = 0; j < c; j++) h[j] ^= h[half - c + j];
+        }
+    }
+};
+template <int B, int NR> SL_HD void hi_shift(V (&x)[NR]) {
+    const V lane = lane_id();
+    const V from = (lane - V(B >= 5 ? 1 << (B >= 5 ? B - 5 : 0) : 1)) & V(31);
+#pragma unroll
+    for (int r = 0; r < NR; r++) {
+        if (NR >= 128 && r % 16 == 0) warp_fence();
+        if (r & (1 << B)) continue;
+        const V h = x[r | (1 << B)], t = shfl(h, from);
+        if constexpr (B >= 5) x[r] ^= t;
+        else x[r] ^= (h << (1 << B)) | (t >> (32 - (1 << B)));
+    }
+}
+template <bool FWD, int RLOG, int NR, int... I>
+SL_HD void hi_shifts(V (&x)[NR], std::integer_sequence<int, I...>) {
+    (hi_shift<FWD ? RLOG - 1 - I : I>(x), ...);
+}
+
+// planes [4 c_src, ..) of `src` to chunk c_dst of `dst` (not the same
+// chunks), column tile ct; sm: Hi<RLOG>::WORDS
+template <int RLOG, bool FWD, class Ex>
+SL_HD void body_taylor_hi(Ex ex, u32 *sm, const uint4 *src, u32 c_src, uint4 *dst, u32 c_dst,
+                          u32 ct) {
+    typedef Hi<RLOG> H;
+    constexpr int R = H::R, HALO = H::HALO, T = H::T, cl = H::CL, plog = H::PLOG;
+    u32 *side = sm + (R << plog) * H::PITCH;     // overflow of the first tile
+    // `tail`: the words left of column 0 are the row's last and the body is empty
     auto load = [&](bool tail) {
         ex([&](u32 tid, u32 nt) {
-            for (u32 i = tid; i < ((R * W) << cl); i += nt) {
-                const u32 c = i & cm, g = i >> cl, row = g / W, col = g - row * W;
-                uint4 q;
-                q.x = q.y = q.z = q.w = 0;
-                const bool body = col >= G.halo;
-                if (tail ? !body : (body || ct)) {
-                    const u32 j = (ct * T + col - G.halo) & 2047;
-                    q = src[(u64)(row * 2048 + j) * 16 + c_src + c];
-                }
-                sm4[i] = q;
-            }
+staged<8, uint4>(
+                (u32)(R * 32) << cl, tid, nt,
+                [&](u32 i) {
+                    const u32 c = i & ((1u << cl) - 1), col = (i >> cl) & 31, row = i >> (cl + 5);
+                    const u32 j = ct * T + col - HALO;
+                    uint4 q;
+                    q.x = q.y = q.z = q.w = 0;
+                    if (tail ? col < HALO : (col >= HALO || ct) && (col < HALO || j < 2048))
+                        q = src[(u64)(row * 2048 + (j & 2047)) * 16 + c_src + c];
+                    return q;
+                },
+                [&](u32 i, const uint4 &q) {
+                    const u32 c = i & ((1u << cl) - 1), col = (i >> cl) & 31, row = i >> (cl + 5);
+                    sm[H::at(row, 4 * c, col)] = q.x;
+                    sm[H::at(row, 4 * c + 1, col)] = q.y;
+                    sm[H::at(row, 4 * c + 2, col)] = q.z;
+                    sm[H::at(row, 4 * c + 3, col)] = q.w;
+                });
         });
     };
-    auto shifts = [&]() {
-        for (int l = 0; l < G.rlog; l++) {
-            const int b = FWD ? G.rlog - 1 - l : l;
-            ex([&](u32 tid, u32 nt) { hi_shift(sm, G, b, tid, nt); });
-        }
-    };
-    auto inv_rows = [&]() {                       // before the shifts: the halo too
-        if (FWD) return;
-        for (int l = rows.n - 1; l >= 0; l--)
-            ex([&](u32 tid, u32 nt) { hi_rows<false>(sm, G, rows.M[l], rows.a[l], 0, tid, nt); });
-    };
-    if (ct == 0) {
-        load(true);
-        inv_rows();
-        shifts();
-        ex([&](u32 tid, u32 nt) {
-            const u32 n = (R * G.halo) << G.plog, np = 1u << G.plog;
-            for (u32 i = tid; i < n; i += nt) {
-                const u32 p = i & (np - 1), g = i >> G.plog, row = g / G.halo, q = g - row * G.halo;
-                side[i] = sm[hi_at(G, row, G.halo + q, p)];
+    for (int run = ct == 0 ? 0 : 1; run < 2; run++) {
+        const bool tail = run == 0;
+        load(tail);
+        ex.warps(1u << plog, [&](u32 p) {
+            V x[R];
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                x[r] = lane_load(sm, [&](u32 l) { return H::at(r, p, l); });
+            const auto over = [](u32 l) { return l >= (u32)H::HALO && l < 2u * H::HALO; };
+            const V left = (lane_id() - V(1)) & V(31);
+            if (!FWD) Conv<false, 0, RLOG>::run(RowLevels<false, R>{x});
+            hi_shifts<FWD, RLOG>(x, std::make_integer_sequence<int, RLOG>{});
+            if (tail) {
+#pragma unroll
+                for (int r = 0; r < R; r++)
+                    lane_store_if(side, over, [&](u32 l) { return ((r << plog) + p) * HALO + l - HALO; },
+                                  x[r]);
+                return;
             }
+            if (ct == 0) {
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    const V o = lane_load_if(side, over, [&](u32 l) {
+                        return ((r << plog) + p) * HALO + l - HALO;
+                    });
+                    if (r + 1 < R) x[r + 1] ^= o;                // y, or the next row
+                    if (FWD) x[r] ^= (o << 1) | (shfl(o, left) >> 31);      // and x
+                }
+            }
+            if (FWD) Conv<true, 0, RLOG>::run(RowLevels<true, R>{x});
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                lane_store(sm, [&](u32 l) { return H::at(r, p, l); }, x[r]);
         });
     }
-    load(false);
-    inv_rows();
-    shifts();
-    if (ct == 0) {
-        ex([&](u32 tid, u32 nt) {
-            const u32 n = (R * G.halo) << G.plog, np = 1u << G.plog;
-            for (u32 i = tid; i < n; i += nt) {
-                const u32 p = i & (np - 1), g = i >> G.plog, row = g / G.halo, q = g - row * G.halo;
-                u32 v = 0;
-                if (row) v = side[i - (G.halo << G.plog)];           // y, or the next row
-                if (FWD) {                                           // and x
-                    v ^= side[i] << 1;
-                    if (q) v ^= side[i - np] >> 31;
-                }
-                sm[hi_at(G, row, G.halo + q, p)] ^= v;
-            }
-        });
-    }
-    if (FWD)
-        for (int l = 0; l < rows.n; l++)
-            ex([&](u32 tid, u32 nt) { hi_rows<true>(sm, G, rows.M[l], rows.a[l], G.halo, tid, nt); });
     ex([&](u32 tid, u32 nt) {
-        for (u32 i = tid; i < ((R << G.tlog) << cl); i += nt) {
-            const u32 c = i & cm, g = i >> cl, row = g >> G.tlog, col = g & (T - 1);
-            dst[(u64)(row * 2048 + ct * T + col) * 16 + c_dst + c] =
-                sm4[((row * W + G.halo + col) << cl) + c];
+        for (u32 i = tid; i < ((u32)(R * 32) << cl); i += nt) {
+            const u32 c = i & ((1u << cl) - 1), col = (i >> cl) & 31, row = i >> (cl + 5);
+            const u32 j = ct * T + col - HALO;
+            if (col < HALO || j >= 2048) continue;
+            uint4 q;
+            q.x = sm[H::at(row, 4 * c, col)];
+            q.y = sm[H::at(row, 4 * c + 1, col)];
+            q.z = sm[H::at(row, 4 * c + 2, col)];
+            q.w = sm[H::at(row, 4 * c + 3, col)];
+            dst[(u64)(row * 2048 + j) * 16 + c_dst + c] = q;
         }
     });
 }
 
-// one butterfly pass over a tile; FIRST (forward): planes 0..31 are chunk
-// planes; LOWP: the pass that holds levels 4..0; LAST (inverse): back to
-// polynomial planes.  Forward levels hi-1 .. lo, inverse lo .. hi-1, those
-// at or above `top` (copies made by the Taylor step) left out.
+// one butterfly pass over half the planes of a tile (every twiddle product
+// stays inside a half).  `first` (forward): planes 0 .. 31 are chunk planes,
+// and both halves' blocks read them before either writes (ex.pair()); `lowp`:
+// the pass that holds levels 4 .. 0.  Forward levels hi-1 .. lo, inverse lo ..
+// hi-1, those at or above `top` (copies made by the Taylor step) left out.
 template <int NQ, bool FWD, class Ex>
-SL_HD void body_bfly(Ex ex, uint4 *tile, uint4 *f, const Tile T, int top, bool edge, bool lowp) {
+SL_HD void body_bfly(Ex ex, uint4 *sm, uint4 *f, const Tile T, u32 half, int top, bool first,
+                     bool lowp) {
+    const Half tile{sm};
     const u32 ns = 1u << (T.rlog + T.clog);
     const int hi = T.llo + T.rlog;
-    const bool first = FWD && edge;
     ex([&](u32 tid, u32 nt) {
-        const u32 n = ns * (first ? 8 : 16);
-        for (u32 i = tid; i < n; i += nt) {
-            const u32 s = first ? i >> 3 : i >> 4, c = first ? i & 7 : i & 15;
-            tile[chunk_at(s, c)] = f[(u64)tile_gslice(T, s) * 16 + c];
-        }
+        const u32 c0 = first ? 0 : 8 * half;
+        for (u32 i = tid; i < ns * 8; i += nt)
+            copy16(&tile.chunk(i >> 3, i & 7), f + (u64)tile_gslice(T, i >> 3) * 16 + c0 + (i & 7));
+        copy_wait();
     });
     if (FWD) {
-        if (first) ex([&](u32 tid, u32 nt) { phi_in(tile, ns, tid, nt); });
+        if (first) {
+            ex.pair();
+            ex([&](u32 tid, u32 nt) {
+                if (half) phi_in<1>(tile, ns, tid, nt);
+                else phi_in<0>(tile, ns, tid, nt);
+            });
+        }
         for (int L = (hi < top ? hi : top) - 1; L >= T.llo; L--)
-            ex([&](u32 tid, u32 nt) { level_n<NQ, true>(tile, T, L, tid, nt); });
+            ex([&](u32 tid, u32 nt) { level_n<2, NQ, true>(tile, T, L, tid, nt); });
         if (lowp) {
-            ex([&](u32 tid, u32 nt) { transpose_groups(tile, ns, tid, nt); });
+            ex([&](u32 tid, u32 nt) { transpose_groups<2>(tile, ns, tid, nt); });
             for (int L = 4; L >= 0; L--)
-                ex([&](u32 tid, u32 nt) { level_x<NQ, true>(tile, T, L, tid, nt); });
+                ex([&](u32 tid, u32 nt) { level_x<2, NQ, true>(tile, T, L, tid, nt); });
         }
     } else {
         if (lowp) {
             for (int L = 0; L <= 4; L++)
-                ex([&](u32 tid, u32 nt) { level_x<NQ, false>(tile, T, L, tid, nt); });
-            ex([&](u32 tid, u32 nt) { transpose_groups(tile, ns, tid, nt); });
+                ex([&](u32 tid, u32 nt) { level_x<2, NQ, false>(tile, T, L, tid, nt); });
+            ex([&](u32 tid, u32 nt) { transpose_groups<2>(tile, ns, tid, nt); });
         }
         for (int L = T.llo; L < hi; L++)
-            ex([&](u32 tid, u32 nt) { level_n<NQ, false>(tile, T, L, tid, nt); });
-        if (edge) ex([&](u32 tid, u32 nt) { phi_out(tile, ns, tid, nt); });
+            ex([&](u32 tid, u32 nt) { level_n<2, NQ, false>(tile, T, L, tid, nt); });
     }
     ex([&](u32 tid, u32 nt) {
-        for (u32 i = tid; i < ns * 16; i += nt)
-            f[(u64)tile_gslice(T, i >> 4) * 16 + (i & 15)] = tile[chunk_at(i >> 4, i & 15)];
+        for (u32 i = tid; i < ns * 8; i += nt)
+            f[(u64)tile_gslice(T, i >> 3) * 16 + 8 * half + (i & 7)] = tile.chunk(i >> 3, i & 7);
     });
 }
 
-// planes of slice s to its 32 output words (in chunks 0 .. 7): word e is the
-// low half of coefficient e and the high half of coefficient e - 1, the last
-// high half goes to side[s + 1]
-SL_HD void slice_words(uint4 *tile, u32 *side, u32 s) {
-    u32 lo[32], hi[32];
-    load_planes<32>(tile, s, 0, lo);
-    load_planes<32>(tile, s, 8, hi);
-    transpose32(lo);
-    transpose32(hi);
+// tower planes of slice s to its 32 output words (in chunks 0 .. 7): word e is
+// the low half of coefficient e and the high half of coefficient e - 1, the
+// last high half goes to side[s + 1]
+SL_HD void slice_words(const Full &tile, u32 *side, u32 s) {
+    u32 a[64], b[64];
+    load_planes<64>(tile, s, 0, a);
+    lin_map<64, 64, false>(a, b);
+    transpose32(b);
+    transpose32(b + 32);
 #pragma unroll
-    for (int e = 31; e > 0; e--) lo[e] ^= hi[e - 1];
-    store_planes<32>(tile, s, 0, lo);
-    side[s + 1] = hi[31];
+    for (int e = 31; e > 0; e--) b[e] ^= b[31 + e];
+    store_planes<32>(tile, s, 0, b);
+    side[s + 1] = b[63];
 }
 
-// 32-bit words 32 s0 .. of the overlap-add of the polynomial planes of a
-// transform of nsl slices (64-bit coefficients at 32-bit steps); words from
-// `words` on are not written.  side: 2^nlog + 1 words.
+// 32-bit words 32 s0 .. of the overlap-add of a transform of nsl slices in
+// tower planes (64-bit coefficients at 32-bit steps); words from `words` on
+// are not written.  The block takes 2^nlog - 1 slices and the one before them
+// for its last high half.  side: 2^nlog + 1 words.
 template <class Ex>
-SL_HD void body_slice_out(Ex ex, uint4 *tile, u32 *side, const uint4 *f, u32 nsl, u32 *out,
+SL_HD void body_slice_out(Ex ex, uint4 *sm, u32 *side, const uint4 *f, u32 nsl, u32 *out,
                           u64 words, u32 s0, int nlog) {
+    const Full tile{sm};
     const u32 n = 1u << nlog;
     ex([&](u32 tid, u32 nt) {
         for (u32 i = tid; i < n * 16; i += nt) {
-            const u32 s = i >> 4;
-            uint4 q;
-            q.x = q.y = q.z = q.w = 0;
-            if (s0 + s < nsl) q = f[(u64)(s0 + s) * 16 + (i & 15)];
-            tile[chunk_at(s, i & 15)] = q;
-        }
-        if (tid == 0) {                          // high half of the coefficient before
-            u32 v = 0;
-            if (s0 && s0 - 1 < nsl) {
-                const u32 *w = reinterpret_cast<const u32 *>(f + (u64)(s0 - 1) * 16) + 32;
-                for (int p = 0; p < 32; p++) v |= (w[p] >> 31) << p;
+            const u32 s = s0 + (i >> 4) - 1;                 // the slice before s0 first
+            if (s < nsl) {
+                copy16(&tile.chunk(i >> 4, i & 15), f + (u64)s * 16 + (i & 15));
+            } else {
+                uint4 q;
+                q.x = q.y = q.z = q.w = 0;
+                tile.chunk(i >> 4, i & 15) = q;
             }
-            side[0] = v;
         }
+        copy_wait();
     });
     ex([&](u32 tid, u32 nt) {
         for (u32 s = tid; s < n; s += nt) slice_words(tile, side, s);
     });
     ex([&](u32 tid, u32 nt) {
-        const u32 *w = reinterpret_cast<const u32 *>(tile);
-        for (u32 i = tid; i < 32 * n; i += nt) {
-            const u64 k = (u64)s0 * 32 + i;
-            if (k < words) out[k] = w[word_at(i >> 5, i & 31)] ^ ((i & 31) ? 0 : side[i >> 5]);
+        for (u32 i = 32 + tid; i < 32 * n; i += nt) {
+            const u64 k = (u64)s0 * 32 + i - 32;
+            if (k < words) out[k] = tile.word(i >> 5, i & 31) ^ ((i & 31) ? 0 : side[i >> 5]);
         }
     });
 }
 
 // a whole product of at most 2^m coefficients in one block (m <= SMALL_M)
-constexpr int SMALL_M = 12;
 struct Operand { const u32 *src; u64 nchunks; u32 xor0; };
 template <class Ex>
-SL_HD void body_small(Ex ex, uint4 *ta, uint4 *tb, u32 *side, int m, const Operand A,
+SL_HD void body_small(Ex ex, uint4 *sa, uint4 *sb, uint4 *sc, u32 *side, int m, const Operand A,
                       const Operand B, int ka, int kb, const Levels &la, const Levels &lb,
                       const Levels &lm, u32 *out, u64 words) {
     const u32 ns = 1u << (m - 5);
+    const Full ta{sa}, tb{sb};
+    const Half mid{sc};
     const Tile T{m, m - 5, 0, 5, 0};
     const SliceAddr at{5};
     // chunk words to planes 0 .. 31
@@ -873,20 +1204,20 @@ SL_HD void body_small(Ex ex, uint4 *ta, uint4 *tb, u32 *side, int m, const Opera
         for (u32 i = tid; i < 32 * ns; i += nt) {
             u32 va = i < A.nchunks ? A.src[i] : 0, vb = i < B.nchunks ? B.src[i] : 0;
             if (i == 0) { va ^= A.xor0; vb ^= B.xor0; }
-            reinterpret_cast<u32 *>(ta)[word_at(i >> 5, i & 31)] = va;
-            reinterpret_cast<u32 *>(tb)[word_at(i >> 5, i & 31)] = vb;
+            ta.word(i >> 5, i & 31) = va;
+            tb.word(i >> 5, i & 31) = vb;
         }
     });
     ex([&](u32 tid, u32 nt) {
         for (u32 i = tid; i < 2 * ns; i += nt) {
-            uint4 *t = i < ns ? ta : tb;
+            const Full &t = i < ns ? ta : tb;
             u32 x[32];
             load_planes<32>(t, i & (ns - 1), 0, x);
             transpose32(x);
             store_planes<32>(t, i & (ns - 1), 0, x);
         }
     });
-    u32 *wa = reinterpret_cast<u32 *>(ta), *wb = reinterpret_cast<u32 *>(tb);
+    u32 *wa = &ta.word(0, 0), *wb = &tb.word(0, 0);
     for (int l = 0; l < la.n || l < lb.n; l++)
         ex([&](u32 tid, u32 nt) {
             if (l < la.n) taylor_level<true>(wa, at, ka, la.M[l], la.a[l], tid, nt);
@@ -900,15 +1231,15 @@ SL_HD void body_small(Ex ex, uint4 *ta, uint4 *tb, u32 *side, int m, const Opera
     ex([&](u32 tid, u32 nt) {
         for (u32 i = tid; i < 16 * ns; i += nt) {
             const bool b = i >= 8 * ns;
-            uint4 *t = b ? tb : ta;
+            const Full &t = b ? tb : ta;
             const u32 s = (i >> 3) & (ns - 1), c = i & 7;
             const u32 from = s & ((1u << ((b ? kb : ka) - 5)) - 1);
-            t[chunk_at(s, 8 + c)] = t[chunk_at(from, c)];
+            t.chunk(s, 8 + c) = t.chunk(from, c);
         }
     });
     ex([&](u32 tid, u32 nt) {
         for (u32 i = tid; i < 2 * ns; i += nt) {
-            uint4 *t = i < ns ? ta : tb;
+            const Full &t = i < ns ? ta : tb;
             u32 a[32], b[64];
             load_planes<32>(t, i & (ns - 1), 8, a);
             lin_map<32, 64, true>(a, b);
@@ -917,25 +1248,25 @@ SL_HD void body_small(Ex ex, uint4 *ta, uint4 *tb, u32 *side, int m, const Opera
     });
     for (int L = m - 1; L >= 5; L--)
         ex([&](u32 tid, u32 nt) {
-            if (L < ka) level_n<1, true>(ta, T, L, tid, nt);
-            if (L < kb) level_n<1, true>(tb, T, L, tid, nt);
+            if (L < ka) level_n<4, 1, true>(ta, T, L, tid, nt);
+            if (L < kb) level_n<4, 1, true>(tb, T, L, tid, nt);
         });
     ex([&](u32 tid, u32 nt) {
-        transpose_groups(ta, ns, tid, nt);
-        transpose_groups(tb, ns, tid, nt);
+        transpose_groups<4>(ta, ns, tid, nt);
+        transpose_groups<4>(tb, ns, tid, nt);
     });
     for (int L = 4; L >= 0; L--)
         ex([&](u32 tid, u32 nt) {
-            level_x<1, true>(ta, T, L, tid, nt);
-            level_x<1, true>(tb, T, L, tid, nt);
+            level_x<4, 1, true>(ta, T, L, tid, nt);
+            level_x<4, 1, true>(tb, T, L, tid, nt);
         });
-    ex([&](u32 tid, u32 nt) { mul_slices(ta, tb, ns, tid, nt); });
+    ex([&](u32 tid, u32 nt) { mul_mid(ta, tb, mid, ns, tid, nt); });
+    ex([&](u32 tid, u32 nt) { mul_ends(ta, tb, mid, ns, tid, nt); });
     for (int L = 0; L <= 4; L++)
-        ex([&](u32 tid, u32 nt) { level_x<1, false>(ta, T, L, tid, nt); });
-    ex([&](u32 tid, u32 nt) { transpose_groups(ta, ns, tid, nt); });
+        ex([&](u32 tid, u32 nt) { level_x<4, 1, false>(ta, T, L, tid, nt); });
+    ex([&](u32 tid, u32 nt) { transpose_groups<4>(ta, ns, tid, nt); });
     for (int L = 5; L < m; L++)
-        ex([&](u32 tid, u32 nt) { level_n<1, false>(ta, T, L, tid, nt); });
-    ex([&](u32 tid, u32 nt) { phi_out(ta, ns, tid, nt); });
+        ex([&](u32 tid, u32 nt) { level_n<4, 1, false>(ta, T, L, tid, nt); });
     const SliceAddr at6{6};
     ex([&](u32 tid, u32 nt) { taylor_regs<false>(wa, at6, m, tid, nt); });
     for (int l = lm.n - 1; l >= 0; l--)
@@ -948,7 +1279,7 @@ SL_HD void body_small(Ex ex, uint4 *ta, uint4 *tb, u32 *side, int m, const Opera
         for (u64 k = tid; k < words; k += nt) {
             const u32 s = (u32)(k >> 5);
             u32 v = 0;
-            if (s < ns) v = wa[word_at(s, (u32)k & 31)];
+            if (s < ns) v = ta.word(s, (u32)k & 31);
             if (!(k & 31) && s <= ns) v ^= side[s];
             out[k] = v;
         }

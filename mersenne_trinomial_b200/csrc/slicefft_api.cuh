@@ -8,7 +8,7 @@
 
 namespace gf2e {
 
-constexpr int SLICE_MIN_M = 10, SLICE_MAX_M = 24;
+constexpr int SLICE_MIN_M = 10, SLICE_MAX_M = 23;
 constexpr int SLICE_SMALL_MAX_M = 12;        // whole products in one block
 
 // operand i of a batch: nchunks 32-bit chunks from src + i * stride, chunk 0

@@ -76,28 +76,24 @@ __global__ void k_wrap_q(const u64 *__restrict__ U, u64 ustride, u64 uw, u64 shi
     }
 }
 
-// P[w] ^= sum over the shifts z of OA(Q) placed at bit 32 z
-__global__ void k_wrap_fix(u64 *__restrict__ P, u64 pstride, u64 ow, const u64 *__restrict__ Q,
-                           u64 qstride, u64 qw, const gf2e::WrapTerms t) {
+// P[w] ^= sum over the shifts z of OA(Q) placed at bit 32 z: word w takes
+// words d = w - z / 2 of OA(Q), and d - 1 where z is odd (z = 1 alone).  Most
+// words lie in no shift's range; 32-bit word offsets and one range test a
+// shift took a pass at r = 136279841 from 43 us (64-bit bit offsets)
+__global__ void k_wrap_fix(u64 *__restrict__ P, u64 pstride, u32 ow, const u64 *__restrict__ Q,
+                           u64 qstride, u32 qw, const gf2e::WrapTerms t) {
     P += (u64)blockIdx.y * pstride;
     Q += (u64)blockIdx.y * qstride;
-    for (u64 w = (u64)blockIdx.x * blockDim.x + threadIdx.x; w < ow;
-         w += (u64)gridDim.x * blockDim.x) {
+    for (u32 w = blockIdx.x * blockDim.x + threadIdx.x; w < ow; w += gridDim.x * blockDim.x) {
         u64 v = 0;
         for (int k = 0; k < t.n; k++) {
-            // bit 64 w of P takes bit 64 w - 32 z of OA(Q)
-            const long long off = (long long)(64 * w) - (long long)(32 * t.z[k]);
-            if (off <= -64 || off >= (long long)(64 * qw)) continue;
-            if (off >= 0) {
-                const u64 i = (u64)off >> 6;
-                if (off & 63) {                          // a 32-bit offset
-                    v ^= Q[i] >> 32;
-                    if (i + 1 < qw) v ^= Q[i + 1] << 32;
-                } else {
-                    v ^= Q[i];
-                }
-            } else {                                     // off = -32
-                v ^= Q[0] << 32;
+            const u32 z = (u32)t.z[k], d = w - (z >> 1);
+            if (d > qw) continue;                        // below the range too
+            if (z & 1) {
+                if (d < qw) v ^= Q[d] << 32;
+                if (d) v ^= Q[d - 1] >> 32;
+            } else if (d < qw) {
+                v ^= Q[d];
             }
         }
         if (v) P[w] ^= v;
@@ -173,8 +169,8 @@ int wrap_mul_finish(const WrapMul &w, const u64 *a, u64 astride, const u64 *b, u
     k_wrap_q<<<dim3(grid_for(w.qw, 256, 4), nb), 256, 0, st>>>(U, S, w.uw, w.D - 1, w.D, P,
                                                                   pstride, w.n / 2, Q, S, w.qw);
     GF2E_CHECK_LAUNCH("k_wrap_q");
-    k_wrap_fix<<<dim3(grid_for(ow, 256, 8), nb), 256, 0, st>>>(P, pstride, ow, Q, S, w.qw,
-                                                                  w.terms);
+    k_wrap_fix<<<dim3(grid_for(ow, 256, 8), nb), 256, 0, st>>>(
+        P, pstride, (u32)ow, Q, S, (u32)w.qw, w.terms);
     GF2E_CHECK_LAUNCH("k_wrap_fix");
     return GF2E_OK;
 }

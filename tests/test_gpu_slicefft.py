@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 def _product(engine, a, ab, b, bb, shift=0):
     F = engine.CudaFFT()
-    F.init(engine.fft_m_for(ab, bb))
+    F.init(engine.engine.fft_m_for(ab, bb))
     da = engine.DeviceBuffer.from_array(a)
     db = da if b is a else engine.DeviceBuffer.from_array(b)
     ow = engine.mul_out_words(ab, bb)
