@@ -119,12 +119,13 @@ int gf2e_trin_square_batch(uint64_t *states_dev, uint64_t *scratch_dev,
                            size_t stride_words, int nstates, uint64_t r,
                            const uint64_t *s_dev, uint32_t k, void *stream);
 
-/* Squarings per pass that gf2e_trin_square_batch uses for this r, stride
- * and state count: 2, or 1 where the fused pass does not apply or does not
- * pay (r >= 2^31 - 2^16, an odd stride, states and scratch small enough to
- * stay in L2 (at most 96 MB), or GF2E_SQUARINGS_PER_PASS=1 in the
- * environment; GF2E_SQUARINGS_PER_PASS=2 uses the fused pass wherever it
- * applies).  Host only. */
+/* Squarings per pass over HBM that gf2e_trin_square_batch takes for this r,
+ * stride and state count: 2, or 1 where the fused pass does not apply (r >=
+ * 2^31 - 2^16, an odd stride), where the states and scratch are small enough to
+ * stay in L2 (at most 96 MB; passes over them, fused or not, are not over
+ * HBM), or under GF2E_SQUARINGS_PER_PASS=1 in the environment;
+ * GF2E_SQUARINGS_PER_PASS=2 uses the fused pass wherever it applies.  Host
+ * only. */
 int gf2e_trin_squarings_per_pass(uint64_t r, size_t stride_words, int nstates);
 
 /* Host-buffer form of the above, the whole of trinomial_stage2.cu `run`

@@ -30,19 +30,20 @@
 // window, XORed into the class accumulator C[c].  The unit's output is the
 // 4-way bit interleave of C[0..3] (bit 4 t + c = bit t of C[c]): cross-
 // register and in-register delta swaps, then a byte transpose by byte
-// permutes.  Lanes own units u0 + lane + 32 q, q < 6, so
+// permutes.  Lanes own units u0 + lane + 32 q, q < 4, so
 // loads and 16-byte stores are coalesced.
 //
-// Per warp tile of 192 units, one ballot lists the windows overlapping it and
-// those covering all of it.  The covering windows whose reads stay inside the
-// state are applied two at a time (both windows' 32 loads issued before
+// Per warp tile of 128 units, one ballot lists the windows overlapping it and
+// one those that cover all of it and read inside the state; the latter are
+// applied class by class, two at a time (both windows' 16 loads issued before
 // either is used) with no masks or bounds tests; the rest (windows that start
 // or end inside the tile, a few tiles per state) with per-lane bit masks and
-// bounds-tested loads.  The kernel is bound by memory latency and integer
-// issue together: measured at r = 136279841, windows one at a time with the
-// high words by shuffle ran 1.06 ms a pass (64 states), the per-tile list
-// with two loads a unit 0.72 ms, two windows at a time 0.68 ms; staging each
-// window's run in shared memory by cp.async first ran 1.5 ms (more issued
+// bounds-tested loads.  The kernel is bound by memory latency (6 of 15 cycles
+// between a warp's instructions) and the integer pipe together.  A pass of 64
+// states at r = 136279841: windows one at a time with the high words by
+// shuffle 1.06 ms, the per-tile list with two loads a unit 0.72 ms, two
+// windows at a time 0.65 ms, fast windows listed by class 0.58 ms; staging
+// each window's run in shared memory by cp.async first ran 1.5 ms (more issued
 // instructions, fewer resident warps).  Each CTA composes its state's
 // windows in warp 0 with shifts and masks (the moduli are powers of two).
 #include "gf2e_internal.cuh"
@@ -158,12 +159,12 @@ GF2E_DEV ulonglong2 interleave4(u32 c0, u32 c1, u32 c2, u32 c3) {
 }
 
 // ---- the pass: per warp tile, the overlapping windows, two at a time
-// units per lane per warp tile (384 words a tile) and resident CTAs per SM:
-// measured at r = 136279841 x 64 states, 6 units at 4 CTAs beats 8 at 3 by
-// 1.2 % and 4 at 4 by 8 % (a persistent grid of contiguous tile shares was
-// 36 % slower than any of them)
-constexpr int LANE_UNITS = 6;
-constexpr int MIN_CTAS = 4;
+// units per lane per warp tile (256 words a tile) and resident CTAs per SM.
+// A pass in us, units x CTAs an SM (64 states at r = 136279841, 64 at
+// 10001567, 256 at 999961): 6 x 4 579 / 82 / 43, 4 x 5 582 / 63 / 36, 5 x 5
+// 572 / 67 / 56, 3 x 6 594 / 63 / 34, 8 x 3 603 / 72 / 60
+constexpr int LANE_UNITS = 4;
+constexpr int MIN_CTAS = 5;
 
 // A full window over all of the tile's units, every index inside the state:
 // lane l's units u0 + l + 32 q read input words first + l + 32 q and the
@@ -246,67 +247,57 @@ GF2E_DEV int compose_windows(u64 r, u64 s, FWin *tab, u32 lane) {
     return base;
 }
 
-// One warp tile: the 32 UL units from u0 of one state.  tab[] holds the
-// state's nwin windows, `mine` is tab[lane] (lane < nwin).  One ballot lists
-// the windows overlapping the tile and another those covering all of it;
-// the covering ones whose reads stay inside the state are applied with no
-// masks or bounds tests, two of a class at a time.
+// the fast windows of one class (bits of m), two at a time
+template <int UL>
+GF2E_DEV void class_windows(const u32 *__restrict__ in32, const int *tabK, u32 m, int u0, u32 lane,
+                            u32 (&acc)[UL]) {
+    while (m) {
+        const int K1 = tabK[__ffs(m) - 1];
+        m &= m - 1;
+        const u32 f1 = (u32)(u0 + (K1 >> 5));
+        if (m) {
+            const int K2 = tabK[__ffs(m) - 1];
+            m &= m - 1;
+            full_windows2<UL>(in32, f1, (u32)K1, (u32)(u0 + (K2 >> 5)), (u32)K2, lane, acc);
+        } else {
+            full_window<UL>(in32, f1, lane, (u32)K1, acc);
+        }
+    }
+}
+
+// One warp tile: the 32 UL units from u0 of one state.  Lane k holds window
+// k of the state (`mine`, k < nwin), cls[c] the windows of class c.  One
+// ballot lists the windows overlapping the tile and another the fast ones:
+// those that cover all of it and read inside the state (the highest index is
+// u0 + floor(K/32) + 32 UL, one past the last lane's last word), which are
+// applied class by class with no masks, bounds tests or branches on the
+// class (a loop over all windows with a test and a switch each took 180
+// instructions a unit, 94 of them in the integer pipe).
 template <int UL>
 GF2E_DEV void frob4_tile(const u32 *__restrict__ in32, ulonglong2 *__restrict__ o, u32 n32,
-                         u32 nu, const FWin *tab, int nwin, const FWin &mine, u32 u0, u32 lane) {
+                         u32 nu, const FWin *tab, const int *tabK, int nwin, const FWin &mine,
+                         const u32 (&cls)[M], u32 u0, u32 lane) {
     constexpr u32 TWL = 32 * UL;
     const int B0 = (int)(u0 * UBITS), B1 = B0 + (int)(TWL * UBITS);
     const bool over = lane < (u32)nwin && mine.hi > B0 && mine.lo < B1;
     const u32 act = __ballot_sync(0xffffffffu, over);
-    const u32 full = __ballot_sync(0xffffffffu, over && mine.lo <= B0 && mine.hi >= B1);
+    const u32 fast = __ballot_sync(0xffffffffu,
+                                   over && mine.lo <= B0 && mine.hi >= B1 &&
+                                       (int)u0 + (mine.K >> 5) + (int)TWL + 1 < (int)n32);
     u32 C[M][UL];
 #pragma unroll
-    for (int c = 0; c < M; c++)
+    for (int c = 0; c < M; c++) {
 #pragma unroll
         for (int q = 0; q < UL; q++) C[c][q] = 0;
-    for (u32 m = act; m; m &= m - 1) {
-        const int k = __ffs(m) - 1;
-        const FWin w = tab[k];
-        // a full window reads without bounds tests when its highest index,
-        // u0 + floor(K/32) + 32 UL (one past the last lane's last word), is
-        // inside the state
-        const bool fast = ((full >> k) & 1) && (int)u0 + (w.K >> 5) + (int)TWL + 1 < (int)n32;
-        if (fast && (m & (m - 1))) {
-            const int k2 = __ffs(m & (m - 1)) - 1;
-            const FWin w2 = tab[k2];
-            const bool fast2 =
-                ((full >> k2) & 1) && (int)u0 + (w2.K >> 5) + (int)TWL + 1 < (int)n32;
-            if (fast2 && w2.c == w.c) {
-                const u32 f1 = (u32)((int)u0 + (w.K >> 5)), f2 = (u32)((int)u0 + (w2.K >> 5));
-                const u32 s1 = (u32)w.K & 31u, s2 = (u32)w2.K & 31u;
-                switch (w.c) {
-                    case 0: full_windows2<UL>(in32, f1, s1, f2, s2, lane, C[0]); break;
-                    case 1: full_windows2<UL>(in32, f1, s1, f2, s2, lane, C[1]); break;
-                    case 2: full_windows2<UL>(in32, f1, s1, f2, s2, lane, C[2]); break;
-                    default: full_windows2<UL>(in32, f1, s1, f2, s2, lane, C[3]); break;
-                }
-                m &= m - 1;                   // the second window is done too
-                continue;
-            }
-        }
-        const u32 first = (u32)((int)u0 + (w.K >> 5)), sh = (u32)w.K & 31u;
-        switch (w.c) {            // the class is warp-uniform (one window at a time)
-            case 0:
-                if (fast) full_window<UL>(in32, first, lane, sh, C[0]);
-                else part_window<UL>(in32, n32, u0, lane, w, C[0]);
-                break;
-            case 1:
-                if (fast) full_window<UL>(in32, first, lane, sh, C[1]);
-                else part_window<UL>(in32, n32, u0, lane, w, C[1]);
-                break;
-            case 2:
-                if (fast) full_window<UL>(in32, first, lane, sh, C[2]);
-                else part_window<UL>(in32, n32, u0, lane, w, C[2]);
-                break;
-            default:
-                if (fast) full_window<UL>(in32, first, lane, sh, C[3]);
-                else part_window<UL>(in32, n32, u0, lane, w, C[3]);
-                break;
+        class_windows<UL>(in32, tabK, fast & cls[c], (int)u0, lane, C[c]);
+    }
+    for (u32 m = act & ~fast; m; m &= m - 1) {     // windows that start or end in the tile
+        const FWin w = tab[__ffs(m) - 1];
+        switch (w.c) {
+            case 0: part_window<UL>(in32, n32, u0, lane, w, C[0]); break;
+            case 1: part_window<UL>(in32, n32, u0, lane, w, C[1]); break;
+            case 2: part_window<UL>(in32, n32, u0, lane, w, C[2]); break;
+            default: part_window<UL>(in32, n32, u0, lane, w, C[3]); break;
         }
     }
 #pragma unroll
@@ -323,12 +314,14 @@ __global__ void __launch_bounds__(256, MIN_CTAS)
 k_frob4_batch(const u64 *__restrict__ in, u64 *__restrict__ out, size_t stride, u64 r,
               const u64 *__restrict__ s_arr, u64 s_uniform) {
     __shared__ FWin tab[NCAND];
+    __shared__ int tabK[NCAND];
     __shared__ int s_nwin;
     const int st = blockIdx.y;
     const u32 lane = threadIdx.x & 31;
     if (threadIdx.x < 32) {
         const int n = compose_windows(r, s_arr ? s_arr[st] : s_uniform, tab, lane);
         if (lane == 0) s_nwin = n;
+        if (lane < (u32)n) tabK[lane] = tab[lane].K;
     }
     __syncthreads();
     const int nwin = s_nwin;
@@ -337,11 +330,15 @@ k_frob4_batch(const u64 *__restrict__ in, u64 *__restrict__ out, size_t stride, 
     const u32 *in32 = reinterpret_cast<const u32 *>(in + (size_t)st * stride);
     ulonglong2 *o = reinterpret_cast<ulonglong2 *>(out + (size_t)st * stride);
     const FWin mine = lane < (u32)nwin ? tab[lane] : FWin{0, 0, 0, 0};
+    u32 cls[M];
+#pragma unroll
+    for (int c = 0; c < M; c++)
+        cls[c] = __ballot_sync(0xffffffffu, lane < (u32)nwin && mine.c == c);
     constexpr u32 TWL = 32 * LANE_UNITS;
     const u32 ntiles = (nu + TWL - 1) / TWL;
     const u32 warps_total = (gridDim.x * blockDim.x) >> 5;
     for (u32 t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < ntiles; t += warps_total)
-        frob4_tile<LANE_UNITS>(in32, o, n32, nu, tab, nwin, mine, TWL * t, lane);
+        frob4_tile<LANE_UNITS>(in32, o, n32, nu, tab, tabK, nwin, mine, cls, TWL * t, lane);
 }
 
 }  // namespace
@@ -355,7 +352,7 @@ bool frob4_supported(u64 r, size_t stride) {
 // squarings fused per pass for the batched entry points, from
 // GF2E_SQUARINGS_PER_PASS (read at each call): 1 keeps the one-squaring
 // kernel throughout, 2 uses the fused pass wherever it applies; unset, the
-// fused pass is used where it applies and the states do not fit in L2.
+// fused pass is used where it applies and pays.
 int squarings_per_pass() {
     const char *e = getenv("GF2E_SQUARINGS_PER_PASS");
     if (!e) return 0;
@@ -367,14 +364,12 @@ int squarings_per_pass() {
 bool use_frob4(u64 r, size_t stride, int nstates) {
     const int mode = squarings_per_pass();
     if (mode == 1 || !frob4_supported(r, stride)) return false;
-    if (mode == 2) return true;
-    // the fused pass halves the HBM traffic per squaring but issues more
-    // instructions per byte: when the states and their scratch fit in L2
-    // (measured: 256 states at r ~ 10^6, 64 MB, 7 % slower fused) the
-    // one-squaring pass is kept
-    return (size_t)nstates * stride * 16 > ((size_t)96 << 20);
+    // two squarings by one fused pass or two single ones, us: 36 / 46 (256
+    // states at r = 999961), 17 / 21 (1 at 3000017, 47 K words), 21 / 21 (64 at
+    // 30011, 30 K words), 17 / 13 (16 at 4423: every CTA composes 25 windows,
+    // and most of them end inside its one tile)
+    return mode == 2 || (size_t)nstates * stride >= ((size_t)1 << 15);
 }
-
 
 int launch_frob4(const u64 *in, u64 *out, size_t stride, int nstates, u64 r, const u64 *s_dev,
                  u64 s, cudaStream_t st) {
@@ -383,11 +378,12 @@ int launch_frob4(const u64 *in, u64 *out, size_t stride, int nstates, u64 r, con
     const size_t nu = (nw + 1) / 2;
     // each warp takes four warp tiles (the window set each CTA composes then
     // serves 32 tiles) when that still gives every SM 1.5 rounds of its 4
-    // resident CTAs, else one (small states, r ~ 10^6)
+    // resident CTAs, else as many as one round of resident CTAs leaves
     const size_t twl = 32 * (size_t)LANE_UNITS;
     const size_t ntile = (nu + twl - 1) / twl;
     const bool four = (ntile + 31) / 32 * (size_t)nstates >= (size_t)6 * sm_count();
-    size_t bx = four ? (ntile + 31) / 32 : (ntile + 7) / 8;
+    const size_t round = ((size_t)MIN_CTAS * sm_count() + nstates - 1) / nstates;
+    size_t bx = four ? (ntile + 31) / 32 : std::min((ntile + 7) / 8, round);
     if (bx > 65535) bx = 65535;
     const dim3 grid((unsigned)bx, (unsigned)nstates);
     k_frob4_batch<<<grid, 256, 0, st>>>(in, out, stride, r, s_dev, s);
@@ -406,7 +402,8 @@ int trin_square_any(const u64 *in, u64 *out, size_t stride, int nstates, u64 r,
 // only single passes apply and k is odd.
 int frobenius_states(u64 *a, u64 *b, size_t stride, int nstates, u64 r, const u64 *s_dev,
                      u64 k, cudaStream_t st, u64 s_uniform) {
-    const bool fused = use_frob4(r, stride, nstates);
+    // the fused pass stores word pairs: both buffers on 16 bytes
+    const bool fused = use_frob4(r, stride, nstates) && (((uintptr_t)a | (uintptr_t)b) & 15) == 0;
     u64 n4 = fused ? k / 2 : 0, n1 = k - 2 * n4;
     if (((n4 + n1) & 1) && n4 > 0) {
         n4--;
@@ -432,5 +429,8 @@ int frobenius_states(u64 *a, u64 *b, size_t stride, int nstates, u64 r, const u6
 }  // namespace gf2e
 
 extern "C" int gf2e_trin_squarings_per_pass(uint64_t r, size_t stride_words, int nstates) {
-    return gf2e::use_frob4(r, stride_words, nstates < 1 ? 1 : nstates) ? 2 : 1;
+    // passes over HBM: states and scratch of at most 96 MB stay in L2
+    const size_t n = nstates < 1 ? 1 : nstates;
+    if (gf2e::squarings_per_pass() != 2 && n * stride_words * 16 <= ((size_t)96 << 20)) return 1;
+    return gf2e::use_frob4(r, stride_words, (int)n) ? 2 : 1;
 }

@@ -207,7 +207,8 @@ Geometry geometry(u64 r) {
 
 size_t device_words(const Geometry &g, int B, int m = 1) {
     size_t w = 3 * g.stride * B + 2 * g.n * B + g.pstride * B + g.tw * B + B + g.gcap * B;
-    if (m > 1) w += 2 * (size_t)m * g.stride * B + g.stride * B + (size_t)m * B;
+    if (m > 1)
+        w = ((w + 1) & ~(size_t)1) + 2 * (size_t)m * g.stride * B + g.stride * B + (size_t)m * B;
     if (g.wrap) w = ((w + 1) & ~(size_t)1) + (size_t)g.wm.per * B;   // 16-byte aligned
     return w;
 }
@@ -587,6 +588,7 @@ int gf2e_scanner_create_blocked(uint64_t r, int slots, int block, gf2e_scanner *
     S->G = S->sdev + B;
     if (block > 1) {
         S->H = S->G + g.gcap * B;
+        if ((S->H - S->dmem) & 1) S->H++;             // word pairs on 16 bytes
         S->HS = S->H + (size_t)block * g.stride * B;
         S->C = S->HS + (size_t)block * g.stride * B;
         S->sH = S->C + g.stride * B;

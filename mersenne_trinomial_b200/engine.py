@@ -499,7 +499,7 @@ def trin_square_batch(states, scratch, stride_words: int, nstates: int, r: int, 
 
 
 def squarings_per_pass(r: int, stride_words: int, nstates: int) -> int:
-    """Squarings one pass of trin_square_batch performs (2 where the fused
+    """Squarings one pass of trin_square_batch over HBM performs (2 where the fused
     F -> F^4 pass applies and pays, else 1)."""
     return int(lib().gf2e_trin_squarings_per_pass(r, stride_words, nstates))
 
