@@ -523,6 +523,11 @@ struct PlanImpl {
     const u64 *tab = nullptr;            // tables the passes read (d_tab or caller's)
     std::vector<Pass> fwd, inv;
     std::vector<u64> ntiles_fwd, ntiles_inv;
+    // the bit-sliced transform (slicefft.cu) for 10 <= m <= 23; the Taylor
+    // levels above 2^16 run on the words, in these passes
+    bool sliced = false;
+    std::vector<Pass> hi_fwd, hi_inv;
+    std::vector<u64> ntiles_hi;
 };
 
 // Merge runs of up to three single-level ops of one kind into register
@@ -590,6 +595,69 @@ bool use_tau_levels(int m) {
     return m >= 15;
 }
 
+// passes for the tau levels of `lv`: cascade levels (a = M - 2) grouped
+// greedily into tile passes whose rows span the index bits every level of the
+// group touches; the wider tau levels stream over HBM one at a time
+void tau_passes(const PlanImpl &P, const std::vector<std::pair<int, int>> &lv,
+                std::vector<Pass> &fwd, std::vector<Pass> &inv) {
+    const gf2e_tune &cfg = P.cfg;
+    auto choose = [&](u64 CH, u64 NS) { return choose_c(CH, NS, cfg); };
+    auto fits = [&](int lo, int hi) {
+        return hi - lo <= cfg.fft_tile_log && choose((u64)1 << lo, (u64)1 << (hi - lo)) != 0;
+    };
+    auto flush = [&](int lo, int hi, const std::vector<std::pair<int, int>> &g) {
+        if (g.empty()) return;
+        const u64 CH = (u64)1 << lo, NS = (u64)1 << (hi - lo);
+        Pass pf = make_pass(CH, NS, choose(CH, NS), P.n, cfg);
+        Pass pi = pf;
+        for (const auto &o : g) pf.ops[pf.nops++] = mkop(TAY_F, (u32)(o.second - lo), 0);
+        for (size_t k = g.size(); k-- > 0;)
+            pi.ops[pi.nops++] = mkop(TAY_I, (u32)(g[k].second - lo), 0);
+        fwd.push_back(pf);
+        inv.push_back(pi);
+    };
+    std::vector<std::pair<int, int>> grp;
+    int glo = 0, ghi = 0;
+    for (const auto &o : lv) {
+        const int M = o.first, a = o.second;
+        if (M - a != 2 || !fits(a, M)) {
+            flush(glo, ghi, grp);
+            grp.clear();
+            Pass ps;
+            memset(&ps, 0, sizeof ps);
+            ps.stream = 1;
+            ps.sM = (u32)M;
+            ps.sA = (u32)a;
+            fwd.push_back(ps);
+            inv.push_back(ps);
+            continue;
+        }
+        if (!grp.empty()) {
+            const int lo = std::min(glo, a), hi = std::max(ghi, M);
+            if ((int)grp.size() < MAXOPS && fits(lo, hi)) {
+                glo = lo;
+                ghi = hi;
+                grp.push_back(o);
+                continue;
+            }
+            flush(glo, ghi, grp);
+            grp.clear();
+        }
+        glo = a;
+        ghi = M;
+        grp.push_back(o);
+    }
+    flush(glo, ghi, grp);
+}
+
+// index bits a conversion takes as an x^2 + x cascade in one tile pass
+int cascade_bits_for(const PlanImpl &P) {
+    int bits = 0;
+    for (int k = 2; k <= P.cfg.fft_tile_log; k++)
+        if (choose_c((u64)1 << std::max(0, P.m - k), (u64)1 << k, P.cfg)) bits = k;
+    return std::max(2, std::min(bits, 10));
+}
+
 void build_passes(PlanImpl &P) {
     const int m = P.m;
     const u64 n = P.n;
@@ -612,62 +680,9 @@ void build_passes(PlanImpl &P) {
     std::vector<Pass> fwd, inv;
     const bool tau = use_tau_levels(m);
     if (tau) {
-        // cascade levels (a = M - 2) grouped greedily into tile passes whose
-        // rows span the index bits every level of the group touches; the
-        // wider tau levels stream over HBM one at a time
-        int cascade_bits = 0;
-        for (int k = 2; k <= cfg.fft_tile_log; k++)
-            if (choose((u64)1 << std::max(0, m - k), (u64)1 << k)) cascade_bits = k;
-        cascade_bits = std::min(cascade_bits, 10);
         std::vector<std::pair<int, int>> lv;
-        tau_levels(0, m, std::max(cascade_bits, 2), lv);
-        auto fits = [&](int lo, int hi) {
-            return hi - lo <= cfg.fft_tile_log &&
-                   choose((u64)1 << lo, (u64)1 << (hi - lo)) != 0;
-        };
-        auto flush = [&](int lo, int hi, const std::vector<std::pair<int, int>> &g) {
-            if (g.empty()) return;
-            const u64 CH = (u64)1 << lo, NS = (u64)1 << (hi - lo);
-            Pass pf = mk(CH, NS, choose(CH, NS));
-            Pass pi = pf;
-            for (const auto &o : g) pf.ops[pf.nops++] = mkop(TAY_F, (u32)(o.second - lo), 0);
-            for (size_t k = g.size(); k-- > 0;)
-                pi.ops[pi.nops++] = mkop(TAY_I, (u32)(g[k].second - lo), 0);
-            fwd.push_back(pf);
-            inv.push_back(pi);
-        };
-        std::vector<std::pair<int, int>> grp;
-        int glo = 0, ghi = 0;
-        for (const auto &o : lv) {
-            const int M = o.first, a = o.second;
-            if (M - a != 2 || !fits(a, M)) {
-                flush(glo, ghi, grp);
-                grp.clear();
-                Pass ps;
-                memset(&ps, 0, sizeof ps);
-                ps.stream = 1;
-                ps.sM = (u32)M;
-                ps.sA = (u32)a;
-                fwd.push_back(ps);
-                inv.push_back(ps);
-                continue;
-            }
-            if (!grp.empty()) {
-                const int lo = std::min(glo, a), hi = std::max(ghi, M);
-                if ((int)grp.size() < MAXOPS && fits(lo, hi)) {
-                    glo = lo;
-                    ghi = hi;
-                    grp.push_back(o);
-                    continue;
-                }
-                flush(glo, ghi, grp);
-                grp.clear();
-            }
-            glo = a;
-            ghi = M;
-            grp.push_back(o);
-        }
-        flush(glo, ghi, grp);
+        tau_levels(0, m, cascade_bits_for(P), lv);
+        tau_passes(P, lv, fwd, inv);
     }
     // Taylor depths 0..L0-1, grouped levels
     for (int L = 0; !tau && L < L0 && L <= m - 2; L++) {
@@ -742,14 +757,25 @@ void build_passes(PlanImpl &P) {
     P.inv = inv_all;
     for (auto &p : P.fwd) merge_stages(p, cfg);
     for (auto &p : P.inv) merge_stages(p, cfg);
+    P.sliced = m >= gf2e::SLICE_MIN_M && m <= gf2e::SLICE_MAX_M && !getenv("GF2E_FFT_TAYLOR");
+    if (P.sliced && m > 16) {
+        std::vector<std::pair<int, int>> lv, hi;
+        tau_levels(0, m, cascade_bits_for(P), lv);
+        for (const auto &o : lv)
+            if (o.first > 16) hi.push_back(o);
+        tau_passes(P, hi, P.hi_fwd, P.hi_inv);
+        std::reverse(P.hi_inv.begin(), P.hi_inv.end());
+        for (auto *v : {&P.hi_fwd, &P.hi_inv})
+            for (auto &p : *v) merge_stages(p, cfg);
+        for (auto &p : P.hi_fwd) P.ntiles_hi.push_back(pass_tiles(p, n));
+    }
     for (auto &p : P.fwd) P.ntiles_fwd.push_back(pass_tiles(p, n));
     for (auto &p : P.inv) P.ntiles_inv.push_back(pass_tiles(p, n));
 }
 
-int run_passes(const PlanImpl &P, bool forward, u64 *f, const u32 *src32, u64 nchunks,
-               cudaStream_t st, int batch = 1, Batch bt = Batch{0, 0, 0}) {
-    const auto &ps = forward ? P.fwd : P.inv;
-    const auto &nt = forward ? P.ntiles_fwd : P.ntiles_inv;
+int run_list(const PlanImpl &P, const std::vector<Pass> &ps, const std::vector<u64> &nt,
+             bool forward, u64 *f, const u32 *src32, u64 nchunks, cudaStream_t st, int batch,
+             Batch bt) {
     if (src32 && !ps.empty() && ps[0].stream) {
         // the first pass streams: pack the operands first
         dim3 grid((unsigned)gf2e::grid_for(P.n, 256, 8), (unsigned)batch);
@@ -795,6 +821,26 @@ int run_passes(const PlanImpl &P, bool forward, u64 *f, const u32 *src32, u64 nc
         }
 #undef GF2E_FFT_LAUNCH
         GF2E_CHECK_LAUNCH("k_fft_pass");
+    }
+    return GF2E_OK;
+}
+
+int run_passes(const PlanImpl &P, bool forward, u64 *f, const u32 *src32, u64 nchunks,
+               cudaStream_t st, int batch = 1, Batch bt = Batch{0, 0, 0}) {
+    return run_list(P, forward ? P.fwd : P.inv, forward ? P.ntiles_fwd : P.ntiles_inv, forward, f,
+                    src32, nchunks, st, batch, bt);
+}
+
+// one transform in place: bit-sliced where the plan and the buffer (16-byte
+// accesses) allow it
+int run_transform(const PlanImpl &P, bool forward, u64 *f, cudaStream_t st) {
+    if (!P.sliced || ((uintptr_t)f & 15)) return run_passes(P, forward, f, nullptr, 0, st);
+    if (forward && !P.hi_fwd.empty())
+        GF2E_TRY(run_list(P, P.hi_fwd, P.ntiles_hi, true, f, nullptr, 0, st, 1, Batch{0, 0, 0}));
+    GF2E_TRY(gf2e::slice_transform(P.m, forward, f, st));
+    if (!forward && !P.hi_inv.empty()) {
+        std::vector<u64> nt(P.ntiles_hi.rbegin(), P.ntiles_hi.rend());
+        return run_list(P, P.hi_inv, nt, false, f, nullptr, 0, st, 1, Batch{0, 0, 0});
     }
     return GF2E_OK;
 }
@@ -897,7 +943,7 @@ int fft_plan_create(int m, gf2e_fft_plan **out) {
 }
 
 int fft_run(const gf2e_fft_plan *plan, bool forward, u64 *f, cudaStream_t st) {
-    return run_passes(plan->impl, forward, f, nullptr, 0, st);
+    return run_transform(plan->impl, forward, f, st);
 }
 
 // `batch` transforms in one launch per pass: transform y at f + y*fstride,
@@ -1040,8 +1086,10 @@ int gf2e_fft_plan_m(const gf2e_fft_plan *plan) { return plan ? plan->impl.m : -1
 
 int gf2e_fft_plan_passes(const gf2e_fft_plan *plan, int *fwd, int *inv) {
     if (!plan) return gf2e::invalid("null plan");
-    if (fwd) *fwd = (int)plan->impl.fwd.size();
-    if (inv) *inv = (int)plan->impl.inv.size();
+    const PlanImpl &P = plan->impl;
+    const int sliced = P.sliced ? gf2e::slice_transform_passes(P.m) + (int)P.hi_fwd.size() : 0;
+    if (fwd) *fwd = sliced ? sliced : (int)P.fwd.size();
+    if (inv) *inv = sliced ? sliced : (int)P.inv.size();
     return GF2E_OK;
 }
 

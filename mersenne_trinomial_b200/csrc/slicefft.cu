@@ -177,6 +177,45 @@ k_slice_out(const uint4 *f, u64 fstride, u32 nsl, u32 *out, u64 ostride, u64 wor
                    words, blockIdx.x * ((1 << IN_LOG) - 1), IN_LOG);
 }
 
+// 128 slices of natural words <-> tower planes, in place.  GROUPED: slice s of
+// 32 takes the elements 32 b + s (the order of the last forward pass), else
+// its own 32.
+template <bool IN, bool GROUPED>
+__global__ void __launch_bounds__(128, 2) k_slice_words(uint4 *f, u32 ns) {
+    extern __shared__ uint4 sm4[];
+    const Full src{sm4}, dst{sm4 + 128 * 17};
+    f += (u64)blockIdx.x * 128 * 16;
+    const u32 n = min(128u, ns), s = threadIdx.x, g = s & ~31u;
+    for (u32 i = s; i < n * 16; i += 128) copy16(&src.chunk(i >> 4, i & 15), f + i);
+    copy_wait();
+    __syncthreads();
+    if (s < n) {
+        u32 a[64], b[64];
+        if (IN && GROUPED) {
+#pragma unroll
+            for (int e = 0; e < 32; e++) {
+                a[2 * e] = src.word(g + e, 2 * (s & 31));
+                a[2 * e + 1] = src.word(g + e, 2 * (s & 31) + 1);
+            }
+        } else {
+            load_planes<64>(src, s, 0, a);
+        }
+        if (IN) words_to_planes(a, b);
+        else planes_to_words(a, b);
+        if (!IN && GROUPED) {
+#pragma unroll
+            for (int e = 0; e < 32; e++) {
+                dst.word(g + e, 2 * (s & 31)) = b[2 * e];
+                dst.word(g + e, 2 * (s & 31) + 1) = b[2 * e + 1];
+            }
+        } else {
+            store_planes<64>(dst, s, 0, b);
+        }
+    }
+    __syncthreads();
+    for (u32 i = s; i < n * 16; i += 128) f[i] = dst.chunk(i >> 4, i & 15);
+}
+
 struct SmallArgs {
     const u32 *src[2];
     u64 sstride[2], nchunks[2];
@@ -224,6 +263,10 @@ int allow_smem() {
     GF2E_SL_ALLOW(6) GF2E_SL_ALLOW(7)
 #undef GF2E_SL_ALLOW
     allow((const void *)k_small_mul, small_smem(SMALL_M));
+    allow((const void *)k_slice_words<true, true>, 2 * 128 * SLICE_BYTES);
+    allow((const void *)k_slice_words<true, false>, 2 * 128 * SLICE_BYTES);
+    allow((const void *)k_slice_words<false, true>, 2 * 128 * SLICE_BYTES);
+    allow((const void *)k_slice_words<false, false>, 2 * 128 * SLICE_BYTES);
     allow((const void *)k_slice_mul<false>, 2 * 128 * SLICE_BYTES);
     allow((const void *)k_slice_mul<true>, 3 * 128 * SLICE_BYTES);
 #define GF2E_SL_ALLOW(NQ)                                \
@@ -259,14 +302,15 @@ int clog2(u64 v) {
     return k;
 }
 
+// `chunks`: of a slice, 8 (the 32 chunk planes of an operand) or 16
 template <bool FWD>
-int launch_taylor(uint4 *f, u64 fstride, int batch, int m, int k, u32 c_src, cudaStream_t st) {
+int launch_taylor(uint4 *f, u64 fstride, int batch, int m, int k, int chunks, u32 c_src,
+                  cudaStream_t st) {
     TaylorArgs a;
     a.f = f;
     a.fstride = fstride;
     const int kt = std::min(k, 16);
     const u32 blocks = 1u << (k - kt);
-    const int chunks = FWD ? 8 : 16;
     // 8 planes a block (whole 32-byte sectors) unless that leaves SMs idle
     a.plog = blocks * (chunks / 2) * (u32)batch >= (u32)gf2e::sm_count() ? 3 : 2;
     a.groups = chunks >> (a.plog - 2);
@@ -323,7 +367,7 @@ int launch_bfly(const BflyArgs &a, u32 tiles, int ny, cudaStream_t st) {
 
 // pass i of the butterflies (i = ntop: the low pass)
 template <bool FWD>
-int run_bfly(const Plan &P, int i, BflyArgs a, int nops, cudaStream_t st) {
+int run_bfly(const Plan &P, int i, BflyArgs a, int nops, bool first, cudaStream_t st) {
     const bool lowp = i == P.ntop;
     a.m = P.m;
     a.llo = lowp ? 5 : P.top[i].llo;
@@ -332,7 +376,7 @@ int run_bfly(const Plan &P, int i, BflyArgs a, int nops, cudaStream_t st) {
     a.collog = a.llo - 5 - a.clog;
     const u32 tiles = 1u << (P.m - 5 - a.rlog - a.clog);
     const int ny = nops * a.batch;
-    a.first = FWD && i == 0;
+    a.first = first && i == 0;
     a.lowp = lowp;
     // one quarter a thread while that fills idle SMs (m <= 16, where every
     // twiddle is in GF(2^16))
@@ -382,11 +426,11 @@ int slice_fwd(int m, const SliceOp *ops, int nops, u64 fstride, int batch, cudaS
             GF2E_TRY(launch_hi<true>(in.f[o], in.fstride, in.f[o], in.fstride, 8, batch, in.k[o], st));
             c = 8;
         }
-        GF2E_TRY(launch_taylor<true>(in.f[o], in.fstride, batch, m, in.k[o], c, st));
+        GF2E_TRY(launch_taylor<true>(in.f[o], in.fstride, batch, m, in.k[o], 8, c, st));
         a.f[o] = in.f[o];
         a.top[o] = in.k[o];
     }
-    for (int i = 0; i <= P.ntop; i++) GF2E_TRY(run_bfly<true>(P, i, a, nops, st));
+    for (int i = 0; i <= P.ntop; i++) GF2E_TRY(run_bfly<true>(P, i, a, nops, true, st));
     return GF2E_OK;
 }
 
@@ -418,8 +462,8 @@ int slice_inv(int m, u64 *f, u64 *tmp, u64 fstride, int batch, u64 *out, u64 ost
     a.top[0] = a.top[1] = m;
     a.fstride = fs;
     a.batch = batch;
-    for (int i = P.ntop; i >= 0; i--) GF2E_TRY(run_bfly<false>(P, i, a, 1, st));
-    GF2E_TRY(launch_taylor<false>(f4, fs, batch, m, m, 0, st));
+    for (int i = P.ntop; i >= 0; i--) GF2E_TRY(run_bfly<false>(P, i, a, 1, false, st));
+    GF2E_TRY(launch_taylor<false>(f4, fs, batch, m, m, 16, 0, st));
     if (m > 16) {
         uint4 *t4 = reinterpret_cast<uint4 *>(tmp);
         GF2E_TRY(launch_hi<false>(f4, fs, t4, fs, 0, batch, m, st));
@@ -434,6 +478,37 @@ int slice_inv(int m, u64 *f, u64 *tmp, u64 fstride, int batch, u64 *out, u64 ost
     GF2E_CHECK_LAUNCH("k_slice_out");
     return GF2E_OK;
 }
+
+int slice_transform(int m, bool forward, u64 *f, cudaStream_t st) {
+    GF2E_TRY(allow_smem());
+    const Plan &P = plan_for(m);
+    uint4 *f4 = reinterpret_cast<uint4 *>(f);
+    const u32 ns = 1u << (m - 5);
+    const u32 grid = (ns + 127) / 128;
+    const size_t smem = 2 * 128 * SLICE_BYTES;
+    BflyArgs a;
+    a.f[0] = a.f[1] = f4;
+    a.top[0] = a.top[1] = m;
+    a.fstride = 0;
+    a.batch = 1;
+    if (forward) {
+        k_slice_words<true, false><<<grid, 128, smem, st>>>(f4, ns);
+        GF2E_CHECK_LAUNCH("k_slice_words");
+        GF2E_TRY(launch_taylor<true>(f4, 0, 1, m, m, 16, 0, st));
+        for (int i = 0; i <= P.ntop; i++) GF2E_TRY(run_bfly<true>(P, i, a, 1, false, st));
+        k_slice_words<false, true><<<grid, 128, smem, st>>>(f4, ns);
+    } else {
+        k_slice_words<true, true><<<grid, 128, smem, st>>>(f4, ns);
+        GF2E_CHECK_LAUNCH("k_slice_words");
+        for (int i = P.ntop; i >= 0; i--) GF2E_TRY(run_bfly<false>(P, i, a, 1, false, st));
+        GF2E_TRY(launch_taylor<false>(f4, 0, 1, m, m, 16, 0, st));
+        k_slice_words<false, false><<<grid, 128, smem, st>>>(f4, ns);
+    }
+    GF2E_CHECK_LAUNCH("k_slice_words");
+    return GF2E_OK;
+}
+
+int slice_transform_passes(int m) { return plan_for(m).ntop + 4; }
 
 int slice_small(int m, const SliceOp &x, const SliceOp &y, int batch, u64 *out, u64 ostride,
                 u64 ow, cudaStream_t st) {

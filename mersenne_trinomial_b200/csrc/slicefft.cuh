@@ -842,6 +842,25 @@ template <int K, bool FWD> SL_HD void taylor_warp(u32 *sm, const PlaneAddr &at, 
         lane_store(sm, [&](u32 l) { return at(r * 32 + l, p); }, x[r]);
 }
 
+// 32 elements (words lo, hi of each in order) to planes of the tower basis, and
+// back
+SL_HD void words_to_planes(const u32 *w, u32 *planes) {
+    u32 a[64];
+#pragma unroll
+    for (int e = 0; e < 32; e++) { a[e] = w[2 * e]; a[32 + e] = w[2 * e + 1]; }
+    transpose32(a);
+    transpose32(a + 32);
+    lin_map<64, 64, true>(a, planes);
+}
+SL_HD void planes_to_words(const u32 *planes, u32 *w) {
+    u32 a[64];
+    lin_map<64, 64, false>(planes, a);
+    transpose32(a);
+    transpose32(a + 32);
+#pragma unroll
+    for (int e = 0; e < 32; e++) { w[2 * e] = a[e]; w[2 * e + 1] = a[32 + e]; }
+}
+
 // ------------------------------------------------- host-side pass planning
 constexpr int SMALL_M = 12;      // whole products in one block up to 2^12 coefficients
 struct BflyPass { int llo, rlog, clog; };

@@ -32,6 +32,11 @@ int slice_inv(int m, u64 *f, u64 *tmp, u64 fstride, int batch, u64 *out, u64 ost
 // out = x y, whole products of at most 2^m coefficients (m <= 12)
 int slice_small(int m, const SliceOp &x, const SliceOp &y, int batch, u64 *out, u64 ostride,
                 u64 ow, cudaStream_t st);
+// the transform itself in place on 2^m words (16-byte aligned) in natural
+// order, but for the Taylor levels above 2^16, which the caller runs on the
+// words before (forward) or after it
+int slice_transform(int m, bool forward, u64 *f, cudaStream_t st);
+int slice_transform_passes(int m);
 // the tower images of the Cantor basis agree with the basis itself
 bool slice_selfcheck(const u64 *basis);
 
