@@ -523,7 +523,7 @@ struct PlanImpl {
     const u64 *tab = nullptr;            // tables the passes read (d_tab or caller's)
     std::vector<Pass> fwd, inv;
     std::vector<u64> ntiles_fwd, ntiles_inv;
-    // the bit-sliced transform (slicefft.cu) for 10 <= m <= 23; the Taylor
+    // the bit-sliced transform (slicefft.cu) for 11 <= m <= 24; the Taylor
     // levels above 2^16 run on the words, in these passes
     bool sliced = false;
     std::vector<Pass> hi_fwd, hi_inv;
@@ -757,7 +757,9 @@ void build_passes(PlanImpl &P) {
     P.inv = inv_all;
     for (auto &p : P.fwd) merge_stages(p, cfg);
     for (auto &p : P.inv) merge_stages(p, cfg);
-    P.sliced = m >= gf2e::SLICE_MIN_M && m <= gf2e::SLICE_MAX_M && !getenv("GF2E_FFT_TAYLOR");
+    // (one forward and one inverse transform, words / sliced: 59 / 64 us at m =
+    // 10, 76 / 73 at 11, 133 / 72 at 12, 469 / 222 at 20)
+    P.sliced = m >= 11 && m <= gf2e::SLICE_MAX_M && !getenv("GF2E_FFT_TAYLOR");
     if (P.sliced && m > 16) {
         std::vector<std::pair<int, int>> lv, hi;
         tau_levels(0, m, cascade_bits_for(P), lv);
@@ -989,8 +991,8 @@ int mul_fft_m(u64 abits, u64 bbits) {
 }
 
 // Products of at most 2^23 coefficients take the bit-sliced transform
-// (slicefft.cu): up to 2^12 in one block, else in the transform buffers where
-// these are aligned for its 16-byte accesses.
+// (slicefft.cu): up to 2^14 in one cluster of blocks, else in the transform
+// buffers where these are aligned for its 16-byte accesses.
 int product_batch(const gf2e_fft_plan *plan, const ProductOp &a, const ProductOp &b, int batch,
                   u64 *fa, u64 *fb, u64 fstride, u64 *out, u64 ostride, u64 ow,
                   cudaStream_t st) {
@@ -1004,7 +1006,7 @@ int product_batch(const gf2e_fft_plan *plan, const ProductOp &a, const ProductOp
     const u32 *sa = reinterpret_cast<const u32 *>(a.words);
     const u32 *sb = reinterpret_cast<const u32 *>(b.words);
     const bool aligned = ((uintptr_t)fa | (uintptr_t)fb) % 16 == 0 && fstride % 2 == 0;
-    if (m <= SLICE_SMALL_MAX_M || (m <= SLICE_MAX_M && aligned)) {
+    if (m <= SLICE_SMALL_MAX_M || (m <= SLICE_PRODUCT_MAX_M && aligned)) {
         const SliceOp op[2] = {{sa, 2 * a.stride, a.nchunks, (u32)a.xor0, fa},
                                {sb, 2 * b.stride, b.nchunks, (u32)b.xor0, fb}};
         if (m <= SLICE_SMALL_MAX_M)

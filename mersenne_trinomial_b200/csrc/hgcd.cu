@@ -1156,7 +1156,7 @@ private:
     // the bit-sliced transform serves every size it has (slicefft.cu)
     static bool sliced(const gf2e_fft_plan *plan) {
         const int m = gf2e_fft_plan_m(plan);
-        return m >= gf2e::SLICE_MIN_M && m <= gf2e::SLICE_MAX_M;
+        return m >= gf2e::SLICE_MIN_M && m <= gf2e::SLICE_PRODUCT_MAX_M;
     }
     // forward transforms of every member of p into f (G x n)
     void fwd(gf2e_fft_plan *plan, const BPoly &p, u64 *f, u64 n) {

@@ -13,6 +13,8 @@
 #include "slicefft.cuh"
 #include "slicefft_api.cuh"
 
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <atomic>
 
@@ -217,26 +219,43 @@ __global__ void __launch_bounds__(128, 2) k_slice_words(uint4 *f, u32 ns) {
 }
 
 struct SmallArgs {
-    const u32 *src[2];
-    u64 sstride[2], nchunks[2];
-    u32 xor0[2];
-    int m, k[2];
-    Levels lv[2], lm;
+    Operand op[2];
+    u64 sstride[2];
+    int m;
     u32 *out;
     u64 ostride, words;
 };
-__global__ void __launch_bounds__(512, 1) k_small_mul(const SmallArgs a) {
+struct ClusterEx {
+    uint4 *sm;
+    GF2E_DEV u32 rank() const { return blockIdx.x & 7; }
+    GF2E_DEV uint4 *mem(u32 r) const {
+        return r == rank() ? sm : cooperative_groups::this_cluster().map_shared_rank(sm, r);
+    }
+    template <class F> GF2E_DEV void block(const F &f) const {
+        f(rank(), threadIdx.x, blockDim.x);
+        __syncthreads();
+    }
+    template <class F> GF2E_DEV void warps(const F &f) const {
+        f(rank(), threadIdx.x >> 5, blockDim.x >> 5);
+        __syncthreads();
+    }
+    template <class F> GF2E_DEV void cluster(const F &f) const {
+        f(rank(), threadIdx.x, blockDim.x);
+        cooperative_groups::this_cluster().sync();
+    }
+};
+// blockIdx.x = 8 * product + rank
+__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256, 2) k_small_mul(const SmallArgs a) {
     extern __shared__ uint4 sm4[];
-    const u32 ns = 1u << (a.m - 5);
-    const u64 y = blockIdx.x;
-    body_small(DevEx{}, sm4, sm4 + ns * 17, sm4 + ns * 34, reinterpret_cast<u32 *>(sm4 + ns * 43), a.m,
-               Operand{a.src[0] + y * a.sstride[0], a.nchunks[0], a.xor0[0]},
-               Operand{a.src[1] + y * a.sstride[1], a.nchunks[1], a.xor0[1]}, a.k[0], a.k[1],
-               a.lv[0], a.lv[1], a.lm, a.out + y * a.ostride, a.words);
+    const u64 y = blockIdx.x >> 3;
+    Operand A = a.op[0], B = a.op[1];
+    A.src += y * a.sstride[0];
+    B.src += y * a.sstride[1];
+    body_small(ClusterEx{sm4}, a.m, A, B, a.out + y * a.ostride, a.words);
 }
 
 constexpr size_t SLICE_BYTES = 16 * 17, HALF_BYTES = 16 * 9;
-constexpr size_t small_smem(int m) { return ((2 * SLICE_BYTES + HALF_BYTES + 4) << (m - 5)) + 4; }
+constexpr size_t small_smem(int m) { return 16 * (size_t)small_chunks(m); }
 constexpr size_t BFLY_SMEM = HALF_BYTES << TILE_LOG;
 
 size_t taylor_smem(int k, int plog) { return (size_t)(4 * ((1 << (k - 5)) + 4)) << plog; }
@@ -262,7 +281,7 @@ int allow_smem() {
     allow((const void *)k_taylor_hi<R, false>, 4 * Hi<R>::WORDS);
     GF2E_SL_ALLOW(6) GF2E_SL_ALLOW(7)
 #undef GF2E_SL_ALLOW
-    allow((const void *)k_small_mul, small_smem(SMALL_M));
+    allow((const void *)k_small_mul, small_smem(gf2e::SLICE_SMALL_MAX_M));
     allow((const void *)k_slice_words<true, true>, 2 * 128 * SLICE_BYTES);
     allow((const void *)k_slice_words<true, false>, 2 * 128 * SLICE_BYTES);
     allow((const void *)k_slice_words<false, true>, 2 * 128 * SLICE_BYTES);
@@ -513,23 +532,19 @@ int slice_transform_passes(int m) { return plan_for(m).ntop + 4; }
 int slice_small(int m, const SliceOp &x, const SliceOp &y, int batch, u64 *out, u64 ostride,
                 u64 ow, cudaStream_t st) {
     GF2E_TRY(allow_smem());
-    const Plan &P = plan_for(m);
     SmallArgs a;
     const SliceOp *op[2] = {&x, &y};
     for (int o = 0; o < 2; o++) {
-        a.src[o] = op[o]->src;
+        a.op[o] = Operand{op[o]->src, op[o]->nchunks, op[o]->xor0,
+                          std::min(m, std::max(MIN_K, clog2(op[o]->nchunks)))};
         a.sstride[o] = op[o]->stride;
-        a.nchunks[o] = op[o]->nchunks;
-        a.xor0[o] = op[o]->xor0;
-        a.k[o] = std::min(m, std::max(8, clog2(op[o]->nchunks)));
-        a.lv[o] = P.taylor[a.k[o]];
     }
     a.m = m;
-    a.lm = P.taylor[m];
     a.out = reinterpret_cast<u32 *>(out);
     a.ostride = 2 * ostride;
     a.words = 2 * ow;
-    k_small_mul<<<batch, 512, small_smem(m), st>>>(a);
+    // 128 threads up to m = 12 (64 slice pairs a level): four blocks an SM
+    k_small_mul<<<8 * batch, m <= 12 ? 128 : 256, small_smem(m), st>>>(a);
     GF2E_CHECK_LAUNCH("k_small_mul");
     return GF2E_OK;
 }

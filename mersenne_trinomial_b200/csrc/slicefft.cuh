@@ -229,6 +229,29 @@ template <int N> SL_HD void t_addmul(const u32 *a, const Prep<N> &b, u32 *c) {
     }
 }
 
+// the same for a multiplier used once: its sums are made on the way down, so
+// that few of them are held at a time
+template <int N> SL_HD void t_addmul_once(const u32 *a, const u32 *b, u32 *c) {
+    if constexpr (N == 4) {
+        Prep<4> w;
+        w.set(b);
+        t_addmul<4>(a, w, c);
+    } else {
+        constexpr int H = N / 2;
+        u32 p[H], s[H], t[H];
+#pragma unroll
+        for (int i = 0; i < H; i++) { p[i] = 0; s[i] = a[i] ^ a[H + i]; }
+        t_addmul_once<H>(s, b + H, p);
+#pragma unroll
+        for (int i = 0; i < H; i++) { c[i] ^= p[i]; c[H + i] ^= p[i]; s[i] = b[i] ^ b[H + i]; }
+        t_addmul_once<H>(a, s, c);
+        t_mulx<H>(b + H, t);
+#pragma unroll
+        for (int i = 0; i < H; i++) t[i] ^= s[i];
+        t_addmul_once<H>(a + H, t, c + H);
+    }
+}
+
 // ------------------------------------------------- linear maps on planes
 // out[p] = XOR over i < NI of bit p of M[i], in[i]; four inputs at a time
 // through their 16 XORs (outputs P0 .. P0 + NO - 1)
@@ -304,6 +327,7 @@ template <int PITCH> struct Slab {
 };
 typedef Slab<17> Full;           // all 64 planes
 typedef Slab<9> Half;            // planes 0 .. 31 or 32 .. 63
+typedef Slab<5> Quarter;         // 16 planes
 
 // 16 bytes to shared memory, asynchronously on the device
 SL_HD void copy16(uint4 *dst, const uint4 *src) {
@@ -521,52 +545,25 @@ template <int H> SL_HD void phi_in(const Half &tile, u32 nslices, u32 tid, u32 n
         store_planes<32>(tile, s, 0, b);
     }
 }
+template <class S> SL_HD void phi_quarter(const S &dst, u32 s, u32 q, const u32 *a) {
+    u32 b[16];
+    switch (q) {
+    case 0: lin_map<32, 16, true, 0>(a, b); break;
+    case 1: lin_map<32, 16, true, 16>(a, b); break;
+    case 2: lin_map<32, 16, true, 32>(a, b); break;
+    default: lin_map<32, 16, true, 48>(a, b); break;
+    }
+    store_planes<16>(dst, s, 0, b);
+}
 SL_HD void mul_slices(const Full &fa, const Full &fb, u32 nslices, u32 tid, u32 nt) {
     for (u32 s = tid; s < nslices; s += nt) {
         u32 a[64], b[64], c[64];
         load_planes<64>(fa, s, 0, a);
         load_planes<64>(fb, s, 0, b);
-        Prep<64> m;
-        m.set(b);
 #pragma unroll
         for (int i = 0; i < 64; i++) c[i] = 0;
-        t_addmul<64>(a, m, c);
+        t_addmul_once<64>(a, b, c);
         store_planes<64>(fa, s, 0, c);
-    }
-}
-
-// the same in two steps of half products, for blocks with 128 registers a
-// thread: the middle product of each slice, then the two it joins
-SL_HD void mul_mid(const Full &fa, const Full &fb, const Half &mid, u32 nslices, u32 tid, u32 nt) {
-    for (u32 s = tid; s < nslices; s += nt) {
-        u32 a[32], b[32], c[32];
-        load_planes<32>(fa, s, 0, a);
-        load_planes<32>(fa, s, 8, b);
-#pragma unroll
-        for (int i = 0; i < 32; i++) { a[i] ^= b[i]; c[i] = 0; }
-        load_planes<32>(fb, s, 8, b);
-        Prep<32> m;
-        m.set(b);
-        t_addmul<32>(a, m, c);
-        store_planes<32>(mid, s, 0, c);
-    }
-}
-SL_HD void mul_ends(const Full &fa, const Full &fb, const Half &mid, u32 nslices, u32 tid, u32 nt) {
-    for (u32 i = tid; i < 2 * nslices; i += nt) {
-        const u32 h = i >= nslices ? 1 : 0, s = i - h * nslices;
-        u32 a[32], b[32], c[32];
-        load_planes<32>(fb, s, 8, a);
-        t_mulx<32>(a, c);
-        load_planes<32>(fb, s, 0, b);
-        const u32 both = 0u - h;
-#pragma unroll
-        for (int k = 0; k < 32; k++) b[k] ^= a[k] ^ (c[k] & both);
-        Prep<32> m;
-        m.set(b);
-        load_planes<32>(fa, s, 8 * h, a);
-        load_planes<32>(mid, s, 0, c);
-        t_addmul<32>(a, m, c);
-        store_planes<32>(fa, s, 8 * h, c);
     }
 }
 
@@ -574,28 +571,11 @@ SL_HD void mul_ends(const Full &fa, const Full &fb, const Half &mid, u32 nslices
 // Conversion of 2^k coefficients (index bits [0, k), k <= 16) by levels at
 // x^(2^h) + x: level (M, a) acts on blocks of 2^M coefficients in chunks of
 // 2^a (forward: Hi[0..c) ^= Top, then A[c..) ^= Hi; the inverse in reverse).
-// Levels with chunks of 256 coefficients and more, and those of a conversion
-// split at 2^8 (M > 8), work on whole words in shared memory; the 8-bit
-// conversions of each 256 consecutive coefficients run in 8 registers.
-constexpr int MAX_LV = 32;
-struct Levels {
-    int n;
-    signed char M[MAX_LV], a[MAX_LV];
-};
-inline void add_levels(Levels &lv, int lo, int hi) {
-    const int m = hi - lo;
-    if (m <= 1) return;
-    int h = 1;
-    while (2 * h < m) h *= 2;
-    for (int M = m; M > h; M--) {
-        lv.M[lv.n] = (signed char)(lo + M);
-        lv.a[lv.n++] = (signed char)(lo + M - 1 - h);
-    }
-    add_levels(lv, lo + h, hi);
-    if (hi > 8 && lo == 0 && h == 8) return;     // [0, 8) in registers
-    add_levels(lv, lo, lo + h);
-}
-
+// A conversion of m bits, h the largest power of two below m, is the levels
+// (M, M - 1 - h), M = m .. h + 1, and the conversions of the upper m - h and
+// the lower h bits.  The 8-bit conversions of each 256 consecutive
+// coefficients run in 8 registers of a thread, the levels above them in the
+// registers of a warp.
 // one level inside a word, M <= 5: shifting right by half - c takes the top
 // chunk to the lowest of the high half and the high half onto the low one
 template <int M, int A, bool FWD, class V> SL_HD V word_level(V x) {
@@ -656,41 +636,7 @@ template <bool FWD> SL_HD void reg_taylor8(u32 *x) {
     }
 }
 
-// word j of plane p of a Taylor tile: at(j, p)
-struct SliceAddr {               // a Full tile of slices
-    static constexpr bool rows_first = false;
-    int plog;
-    SL_HD u32 operator()(u32 j, u32 p) const { return j * 68 + p; }
-};
-
-// level (M, a), M >= 9, of 2^k coefficients (2^(k-5) words) x 2^plog planes
-template <bool FWD, class At>
-SL_HD void taylor_level(u32 *sm, const At &at, int k, int M, int a, u32 tid, u32 nt) {
-    const int hl = M - 6;                            // log2 words of a half
-    const u32 hw = 1u << hl, np = 1u << at.plog;
-    const u32 items = (1u << (k - 6)) << at.plog;
-    for (u32 i = tid; i < items; i += nt) {
-        const u32 p = i & (np - 1), g = i >> at.plog;
-        const u32 j = g & (hw - 1), b = (g >> hl) << (hl + 1);
-        const u32 ih = at(b + hw + j, p);
-        u32 h = sm[ih];
-        if (a >= 5) {
-            const u32 cw = 1u << (a - 5);
-            const u32 top = j < cw ? sm[at(b + hw + hw - cw + j, p)] : 0;
-            if (FWD && j < cw) { h ^= top; sm[ih] = h; }
-            if (j + cw < hw) sm[at(b + j + cw, p)] ^= h;
-            if (!FWD && j < cw) sm[ih] = h ^ top;
-        } else {
-            // the top bits read from word j-1 are not the low bits word 0 changes
-            const int c = 1 << a;
-            const u32 prev = j ? sm[at(b + hw + j - 1, p)] : 0;
-            const u32 top = j ? 0 : sm[at(b + 2 * hw - 1, p)] >> (32 - c);
-            if (FWD && j == 0) { h ^= top; sm[ih] = h; }
-            sm[at(b + j, p)] ^= (h << c) | (j ? prev >> (32 - c) : 0);
-            if (!FWD && j == 0) sm[ih] = h ^ top;
-        }
-    }
-}
+// the 8-bit conversions of 2^k coefficients; word j of plane p is at(j, p)
 template <bool FWD, class At>
 SL_HD void taylor_regs(u32 *sm, const At &at, int k, u32 tid, u32 nt) {
     const u32 nr = 1u << (k - 8), items = nr << at.plog;
@@ -790,7 +736,7 @@ template <int M, int A, bool FWD, int NR> SL_HD void warp_level(V (&x)[NR]) {
 }
 
 // the levels of a conversion over index bits [LO, HI) in forward or inverse
-// order (add_levels at compile time; [0, 8) of a split at 2^8 left out)
+// order ([0, 8) of a split at 2^8 left out where Op::skip_low)
 constexpr int split_of(int m) { int h = 1; while (2 * h < m) h *= 2; return h; }
 template <bool FWD, int LO, int HI> struct Conv {
     static constexpr int m = HI - LO, h = split_of(m);
@@ -830,7 +776,7 @@ struct PlaneAddr {
     int plog, pitch;
     SL_HD u32 operator()(u32 j, u32 p) const { return p * pitch + (j ^ ((j >> 5) & 7)); }
 };
-template <int K, bool FWD> SL_HD void taylor_warp(u32 *sm, const PlaneAddr &at, u32 p) {
+template <int K, bool FWD, class At> SL_HD void taylor_warp(u32 *sm, const At &at, u32 p) {
     constexpr int NR = 1 << (K - 10);
     V x[NR];
 #pragma unroll
@@ -862,14 +808,12 @@ SL_HD void planes_to_words(const u32 *planes, u32 *w) {
 }
 
 // ------------------------------------------------- host-side pass planning
-constexpr int SMALL_M = 12;      // whole products in one block up to 2^12 coefficients
 struct BflyPass { int llo, rlog, clog; };
 struct Plan {
     int m = 0;
     int low = 0;                 // the last forward pass: levels low-1 .. 0
     int ntop = 0;
     BflyPass top[3];             // forward order
-    Levels taylor[SMALL_M + 1];  // taylor[k]: a small product's levels of 2^k coefficients
 };
 constexpr int TILE_LOG = 9;      // at most 512 slices a tile
 inline Plan make_plan(int m, int low, int clog) {
@@ -887,10 +831,6 @@ inline Plan make_plan(int m, int low, int clog) {
         if (c > TILE_LOG - take) c = TILE_LOG - take;
         if (c > hi - 5) c = hi - 5;
         P.top[P.ntop++] = BflyPass{hi, take, c};
-    }
-    for (int k = 8; k <= SMALL_M; k++) {
-        P.taylor[k].n = 0;
-        if (k > 8) add_levels(P.taylor[k], 0, k);
     }
     return P;
 }
@@ -1207,101 +1147,168 @@ SL_HD void body_slice_out(Ex ex, uint4 *sm, u32 *side, const uint4 *f, u32 nsl, 
     });
 }
 
-// a whole product of at most 2^m coefficients in one block (m <= SMALL_M)
-struct Operand { const u32 *src; u64 nchunks; u32 xor0; };
+// Whole products of at most 2^m coefficients, 10 <= m <= 14, by a cluster of
+// 8 blocks: block 4 o + q takes quarter q (16 planes) of operand o up to its
+// transform (every twiddle is in GF(2^16) there, so quarters stay apart), the
+// products are shared out by slices, blocks 0 .. 3 run the inverse of their
+// quarters, and the slices are shared out again for the words.  ex.mem(r) is
+// the shared memory of block r; ex.block(f) and ex.cluster(f) run f(rank, tid,
+// threads) on every block, with a barrier of the block or the cluster after.
+// (One block for a whole product took 72 us at m = 12, its levels bound by
+// one SM; as separate launches 79 us at m = 13.)
+struct Operand { const u32 *src; u64 nchunks; u32 xor0; int k; };
+struct RowAddr {                 // word j of plane p of slices PITCH words apart
+    static constexpr bool rows_first = false;
+    int plog, pitch;
+    SL_HD u32 operator()(u32 j, u32 p) const { return j * pitch + p; }
+};
+// 16-byte chunks a block: 32 planes, 16 planes, 2^(m-8) + 1 words
+#ifdef __CUDACC__
+__host__
+#endif
+SL_HD constexpr u32 small_chunks(int m) { return (14u << (m - 5)) + 20; }
+template <bool FWD, class At> SL_HD void taylor_warp_k(u32 *sm, const At &at, int k, u32 p) {
+    switch (k) {
+    case 10: taylor_warp<10, FWD>(sm, at, p); break;
+    case 11: taylor_warp<11, FWD>(sm, at, p); break;
+    case 12: taylor_warp<12, FWD>(sm, at, p); break;
+    case 13: taylor_warp<13, FWD>(sm, at, p); break;
+    default: taylor_warp<14, FWD>(sm, at, p); break;
+    }
+}
 template <class Ex>
-SL_HD void body_small(Ex ex, uint4 *sa, uint4 *sb, uint4 *sc, u32 *side, int m, const Operand A,
-                      const Operand B, int ka, int kb, const Levels &la, const Levels &lb,
-                      const Levels &lm, u32 *out, u64 words) {
-    const u32 ns = 1u << (m - 5);
-    const Full ta{sa}, tb{sb};
-    const Half mid{sc};
+SL_HD void body_small(Ex ex, int m, const Operand &A, const Operand &B, u32 *out, u64 words) {
+    const u32 ns = 1u << (m - 5), nb = ns / 8;
     const Tile T{m, m - 5, 0, 5, 0};
-    const SliceAddr at{5};
-    // chunk words to planes 0 .. 31
-    ex([&](u32 tid, u32 nt) {
-        for (u32 i = tid; i < 32 * ns; i += nt) {
-            u32 va = i < A.nchunks ? A.src[i] : 0, vb = i < B.nchunks ? B.src[i] : 0;
-            if (i == 0) { va ^= A.xor0; vb ^= B.xor0; }
-            ta.word(i >> 5, i & 31) = va;
-            tb.word(i >> 5, i & 31) = vb;
-        }
+    const auto half = [&](u32 r) { return Half{ex.mem(r)}; };
+    const auto quarter = [&](u32 r) { return Quarter{ex.mem(r) + 9 * ns}; };
+    const auto side = [&](u32 r) { return reinterpret_cast<u32 *>(ex.mem(r) + 14 * ns); };
+    const auto op = [&](u32 r) -> const Operand & { return r < 4 ? A : B; };
+    const RowAddr at_half{5, 36}, at_quarter{4, 20};
+    // chunk words, their planes, the conversion (all 32 planes in every block)
+    ex.block([&](u32 r, u32 tid, u32 nt) {
+        const Operand &o = op(r);
+        const Half h = half(r);
+        for (u32 i = tid; i < (1u << o.k); i += nt)
+            h.word(i >> 5, i & 31) = (i < o.nchunks ? o.src[i] : 0) ^ (i == 0 ? o.xor0 : 0);
     });
-    ex([&](u32 tid, u32 nt) {
-        for (u32 i = tid; i < 2 * ns; i += nt) {
-            const Full &t = i < ns ? ta : tb;
+    ex.block([&](u32 r, u32 tid, u32 nt) {
+        const Half h = half(r);
+        for (u32 i = tid; i < (1u << (op(r).k - 5)); i += nt) {
             u32 x[32];
-            load_planes<32>(t, i & (ns - 1), 0, x);
+            load_planes<32>(h, i, 0, x);
             transpose32(x);
-            store_planes<32>(t, i & (ns - 1), 0, x);
+            store_planes<32>(h, i, 0, x);
         }
     });
-    u32 *wa = &ta.word(0, 0), *wb = &tb.word(0, 0);
-    for (int l = 0; l < la.n || l < lb.n; l++)
-        ex([&](u32 tid, u32 nt) {
-            if (l < la.n) taylor_level<true>(wa, at, ka, la.M[l], la.a[l], tid, nt);
-            if (l < lb.n) taylor_level<true>(wb, at, kb, lb.M[l], lb.a[l], tid, nt);
-        });
-    ex([&](u32 tid, u32 nt) {
-        taylor_regs<true>(wa, at, ka, tid, nt);
-        taylor_regs<true>(wb, at, kb, tid, nt);
+    ex.warps([&](u32 r, u32 w, u32 nw) {
+        for (u32 p = w; p < 32; p += nw) taylor_warp_k<true>(&half(r).word(0, 0), at_half, op(r).k, p);
     });
-    // copies of the converted slices (through planes 32 .. 63), tower planes
-    ex([&](u32 tid, u32 nt) {
-        for (u32 i = tid; i < 16 * ns; i += nt) {
-            const bool b = i >= 8 * ns;
-            const Full &t = b ? tb : ta;
-            const u32 s = (i >> 3) & (ns - 1), c = i & 7;
-            const u32 from = s & ((1u << ((b ? kb : ka) - 5)) - 1);
-            t.chunk(s, 8 + c) = t.chunk(from, c);
-        }
+    ex.block([&](u32 r, u32 tid, u32 nt) {
+        taylor_regs<true>(&half(r).word(0, 0), at_half, op(r).k, tid, nt);
     });
-    ex([&](u32 tid, u32 nt) {
-        for (u32 i = tid; i < 2 * ns; i += nt) {
-            const Full &t = i < ns ? ta : tb;
-            u32 a[32], b[64];
-            load_planes<32>(t, i & (ns - 1), 8, a);
-            lin_map<32, 64, true>(a, b);
-            store_planes<64>(t, i & (ns - 1), 0, b);
+    // tower planes of the quarter, copies included
+    ex.block([&](u32 r, u32 tid, u32 nt) {
+        for (u32 i = tid; i < ns; i += nt) {
+            u32 a[32];
+            load_planes<32>(half(r), i & ((1u << (op(r).k - 5)) - 1), 0, a);
+            phi_quarter(quarter(r), i, r & 3, a);
         }
     });
     for (int L = m - 1; L >= 5; L--)
-        ex([&](u32 tid, u32 nt) {
-            if (L < ka) level_n<4, 1, true>(ta, T, L, tid, nt);
-            if (L < kb) level_n<4, 1, true>(tb, T, L, tid, nt);
+        ex.block([&](u32 r, u32 tid, u32 nt) {
+            if (L < op(r).k) level_n<1, 1, true>(quarter(r), T, L, tid, nt);
         });
-    ex([&](u32 tid, u32 nt) {
-        transpose_groups<4>(ta, ns, tid, nt);
-        transpose_groups<4>(tb, ns, tid, nt);
-    });
-    for (int L = 4; L >= 0; L--)
-        ex([&](u32 tid, u32 nt) {
-            level_x<4, 1, true>(ta, T, L, tid, nt);
-            level_x<4, 1, true>(tb, T, L, tid, nt);
-        });
-    ex([&](u32 tid, u32 nt) { mul_mid(ta, tb, mid, ns, tid, nt); });
-    ex([&](u32 tid, u32 nt) { mul_ends(ta, tb, mid, ns, tid, nt); });
-    for (int L = 0; L <= 4; L++)
-        ex([&](u32 tid, u32 nt) { level_x<4, 1, false>(ta, T, L, tid, nt); });
-    ex([&](u32 tid, u32 nt) { transpose_groups<4>(ta, ns, tid, nt); });
-    for (int L = 5; L < m; L++)
-        ex([&](u32 tid, u32 nt) { level_n<4, 1, false>(ta, T, L, tid, nt); });
-    const SliceAddr at6{6};
-    ex([&](u32 tid, u32 nt) { taylor_regs<false>(wa, at6, m, tid, nt); });
-    for (int l = lm.n - 1; l >= 0; l--)
-        ex([&](u32 tid, u32 nt) { taylor_level<false>(wa, at6, m, lm.M[l], lm.a[l], tid, nt); });
-    ex([&](u32 tid, u32 nt) {
-        if (tid == 0) side[0] = 0;
-        for (u32 s = tid; s < ns; s += nt) slice_words(ta, side, s);
-    });
-    ex([&](u32 tid, u32 nt) {
-        for (u64 k = tid; k < words; k += nt) {
-            const u32 s = (u32)(k >> 5);
-            u32 v = 0;
-            if (s < ns) v = ta.word(s, (u32)k & 31);
-            if (!(k & 31) && s <= ns) v ^= side[s];
-            out[k] = v;
+    ex.block([&](u32 r, u32 tid, u32 nt) { transpose_groups<1>(quarter(r), ns, tid, nt); });
+    for (int L = 4; L >= 1; L--)
+        ex.block([&](u32 r, u32 tid, u32 nt) { level_x<1, 1, true>(quarter(r), T, L, tid, nt); });
+    ex.cluster([&](u32 r, u32 tid, u32 nt) { level_x<1, 1, true>(quarter(r), T, 0, tid, nt); });
+    // products of slices r nb .. r nb + nb - 1: the middle half product, then
+    // the two it joins
+    ex.block([&](u32 r, u32 tid, u32 nt) {
+        for (u32 i = tid; i < nb; i += nt) {
+            const u32 s = r * nb + i;
+            u32 a[32], b[32], c[32];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                load_planes<16>(quarter(h), s, 0, a + 16 * h);
+                load_planes<16>(quarter(2 + h), s, 0, b + 16 * h);
+            }
+#pragma unroll
+            for (int k = 0; k < 32; k++) { a[k] ^= b[k]; c[k] = 0; }
+#pragma unroll
+            for (int h = 0; h < 2; h++) load_planes<16>(quarter(6 + h), s, 0, b + 16 * h);
+            t_addmul_once<32>(a, b, c);
+            store_planes<32>(half(r), i, 0, c);
         }
+    });
+    ex.cluster([&](u32 r, u32 tid, u32 nt) {
+        for (u32 i = tid; i < 2 * nb; i += nt) {
+            const u32 h = i >= nb ? 1 : 0, j = i - h * nb, s = r * nb + j, both = 0u - h;
+            u32 a[32], b[32], c[32];
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                load_planes<16>(quarter(6 + k), s, 0, a + 16 * k);
+                load_planes<16>(quarter(4 + k), s, 0, b + 16 * k);
+            }
+            t_mulx<32>(a, c);
+#pragma unroll
+            for (int k = 0; k < 32; k++) b[k] ^= a[k] ^ (c[k] & both);
+#pragma unroll
+            for (int k = 0; k < 2; k++) load_planes<16>(quarter(2 * h + k), s, 0, a + 16 * k);
+            load_planes<32>(half(r), j, 0, c);
+            t_addmul_once<32>(a, b, c);
+#pragma unroll
+            for (int k = 0; k < 2; k++) store_planes<16>(quarter(2 * h + k), s, 0, c + 16 * k);
+        }
+    });
+    for (int L = 0; L <= 4; L++)
+        ex.block([&](u32 r, u32 tid, u32 nt) {
+            if (r < 4) level_x<1, 1, false>(quarter(r), T, L, tid, nt);
+        });
+    ex.block([&](u32 r, u32 tid, u32 nt) {
+        if (r < 4) transpose_groups<1>(quarter(r), ns, tid, nt);
+    });
+    for (int L = 5; L < m; L++)
+        ex.block([&](u32 r, u32 tid, u32 nt) {
+            if (r < 4) level_n<1, 1, false>(quarter(r), T, L, tid, nt);
+        });
+    ex.block([&](u32 r, u32 tid, u32 nt) {
+        if (r < 4) taylor_regs<false>(&quarter(r).word(0, 0), at_quarter, m, tid, nt);
+    });
+    ex.warps([&](u32 r, u32 w, u32 nw) {
+        if (r < 4)
+            for (u32 p = w; p < 16; p += nw)
+                taylor_warp_k<false>(&quarter(r).word(0, 0), at_quarter, m, p);
+    });
+    ex.cluster([](u32, u32, u32) {});
+    // words of slices r nb .. (and the last high half of the slice before)
+    ex.cluster([&](u32 r, u32 tid, u32 nt) {
+        for (u32 i = tid; i <= nb; i += nt) {
+            const u32 s = r * nb + i - 1;
+            u32 a[64], b[64];
+            if (s >= ns) {                       // before slice 0
+                side(r)[0] = 0;
+                continue;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++) load_planes<16>(quarter(q), s, 0, a + 16 * q);
+            lin_map<64, 64, false>(a, b);
+            transpose32(b);
+            transpose32(b + 32);
+#pragma unroll
+            for (int e = 31; e > 0; e--) b[e] ^= b[31 + e];
+            if (i) store_planes<32>(half(r), i - 1, 0, b);
+            side(r)[i] = b[63];
+        }
+    });
+    ex.block([&](u32 r, u32 tid, u32 nt) {
+        const u64 k0 = (u64)r * nb * 32;
+        for (u32 i = tid; i < 32 * nb; i += nt)
+            if (k0 + i < words) out[k0 + i] = half(r).word(i >> 5, i & 31) ^ ((i & 31) ? 0 : side(r)[i >> 5]);
+        if (r == 7)
+            for (u64 k = (u64)ns * 32 + tid; k < words; k += nt)
+                out[k] = k == (u64)ns * 32 ? side(r)[nb] : 0;
     });
 }
 

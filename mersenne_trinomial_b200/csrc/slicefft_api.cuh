@@ -8,8 +8,11 @@
 
 namespace gf2e {
 
-constexpr int SLICE_MIN_M = 10, SLICE_MAX_M = 23;
-constexpr int SLICE_SMALL_MAX_M = 12;        // whole products in one block
+constexpr int SLICE_MIN_M = 10, SLICE_MAX_M = 24;
+// products keep 2^(m-16) <= 128 rows of the Taylor levels above 2^16 in a
+// warp's registers
+constexpr int SLICE_PRODUCT_MAX_M = 23;
+constexpr int SLICE_SMALL_MAX_M = 14;        // whole products in one cluster of blocks
 
 // operand i of a batch: nchunks 32-bit chunks from src + i * stride, chunk 0
 // XORed with xor0; its transform goes to f + i * fstride words
@@ -29,7 +32,7 @@ int slice_pointwise(u64 *o, const u64 *x1, const u64 *y1, const u64 *x2, const u
 // its coefficients into out + i * ostride, ow words each
 int slice_inv(int m, u64 *f, u64 *tmp, u64 fstride, int batch, u64 *out, u64 ostride, u64 ow,
               cudaStream_t st);
-// out = x y, whole products of at most 2^m coefficients (m <= 12)
+// out = x y, whole products of at most 2^m coefficients (10 <= m <= 14)
 int slice_small(int m, const SliceOp &x, const SliceOp &y, int batch, u64 *out, u64 ostride,
                 u64 ow, cudaStream_t st);
 // the transform itself in place on 2^m words (16-byte aligned) in natural
