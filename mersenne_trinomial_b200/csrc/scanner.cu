@@ -94,8 +94,9 @@ struct gf2e_scanner {
 };
 
 // operands of at least this many bits take the half-gcd (hgcd.cu) at
-// interval ends; smaller ones the quadratic batched gcd (gcd.cu)
-constexpr u64 GCD_LARGE_BITS = 1ull << 19;
+// interval ends; smaller ones the quadratic batched gcd (gcd.cu): 24 gcds take
+// 23 / 21 ms at 130000 bits, 34 / 43 ms at 200000, one 18 / 20 and 27 / 42
+constexpr u64 GCD_LARGE_BITS = 150000;
 // device words one member of a lockstep half-gcd batch draws from the gcd
 // pool, per operand word (its high-water mark: 1.52 GB at r = 136279841)
 constexpr size_t HGCD_WORDS_PER_WORD = 90;
