@@ -34,83 +34,82 @@ GF2E_DEV long long warp_degree(const u64 *X, long long top) {
     return -1;
 }
 
-// one Lehmer round on exact 64-bit windows of A and B taken at bit `lo`
-// (deg A = da >= deg B): whole quotients while every bit they depend on is
-// exact (a row's window bits are exact above its matrix degree), the
-// half-gcd stop (deg B < m) is not reached and the 2x2 matrix stays within
-// degree 31; mode 1 (no quotient fits) is the single shift-XOR A ^= B << k.
+// One Lehmer round on 64-bit windows of A and B taken at bit `lo` (deg A = da
+// >= deg B = db >= m): division steps one degree at a time, on windows kept
+// left-aligned at the degree each is known to.  With f = (window, row) of the
+// vector with its leading coefficient at bit 63 and g the other, s_f and s_g
+// the places each has been shifted up: where g's top bit is set, and f is the
+// longer (s_g > s_f), they swap; then g += f clears the bit, and g moves up one
+// place.  The rows move with their windows, so the entries are the rows shifted
+// down by s_f and s_g at the end, of degree at most s_g and s_f.  Every bit
+// decided on is exact: a window shifted by s has 64 - s exact bits, and there
+// are at most 62 steps.  A swap needs s_g <= 31 (entries of 32 bits) and deg g
+// >= m (the half-gcd's stop: deg a' >= m).
+//
+// Each step is a dozen integer operations without a branch; the lanes of a
+// warp hold the columns of the matrix by parity and run the windows side by
+// side.  (Whole quotients, each a loop over its own degrees with a degree
+// search and the role swap after it, took 3258 cycles a round on one thread.)
 struct Lehmer {
-    u32 mt[4];
+    u32 ef, eg;         // this lane's column of the rows of a' and b'
     long long k;
-    int mode;
+    int mode;           // 1: a gap of more than 31 degrees, A ^= B << k alone
 };
 GF2E_DEV Lehmer lehmer_round(u64 wa, u64 wb, long long da, long long db, long long lo,
-                             long long m) {
+                             long long m, int lane) {
     Lehmer L;
-    u32 ma0 = 1, ma1 = 0, mb0 = 0, mb1 = 1;
-    int dga = (int)(da - lo), dgb = deg64(wb), dma = 0, dmb = 0, steps = 0;
-    const bool exact = (lo == 0);
-    const int dstop = (int)max(-1LL, m - lo);          // window degree of x^m
-    // the windows left-aligned (leading coefficient at bit 63): the division
-    // below then tests one bit and shifts, with no degree search per step
-    u64 A = wa << (63 - dga);
-    u64 B = dgb >= 0 ? wb << (63 - dgb) : 0;
-    for (int it = 0; it < 64; it++) {
-        if (dgb < 0 || dgb < dstop) break;              // b = 0 / half-gcd stop
-        const int dq = dga - dgb;
-        const int ndm = max(dma, dmb + dq);
-        if (ndm > 31) break;                            // matrix degree bound
-        if (!exact && dgb < ndm) break;                 // quotient not exact
-        // a <- a mod b, row a += q row b: at each of the dq + 1 degrees from
-        // the top, XOR in b (and x^(dq-j) row b) when a's leading bit is set,
-        // then move one degree down.  Afterwards bit 63 of A is degree dgb.
-        // At the top degree the bit is a's leading coefficient, always set.
-        u32 s0 = mb0 << dq, s1 = mb1 << dq;
-        A ^= B;
-        ma0 ^= s0;
-        ma1 ^= s1;
-#pragma unroll 1
-        for (int j = 1; j <= dq; j++) {
-            A <<= 1;
-            s0 >>= 1;
-            s1 >>= 1;
-            const u64 msk = (u64)((long long)A >> 63);
-            A ^= B & msk;
-            ma0 ^= s0 & (u32)msk;
-            ma1 ^= s1 & (u32)msk;
+    L.k = da - db;
+    L.mode = L.k > 31 ? 1 : 0;
+    L.ef = L.eg = 0;
+    if (L.mode) return L;
+    const int dga = (int)(da - lo);
+    const int lim = m > lo ? min(31, dga - (int)(m - lo)) : 31;
+    u64 A = wa << (63 - dga), B = wb << (63 - dga);
+    int N = 0;                                          // s_f - s_g
+    int t = 0;                                          // s_f + s_g
+    u64 p, q;
+    {
+        u32 p1 = (lane & 1) ^ 1, q1 = lane & 1;
+        if (lim == 31) {
+            // s_g <= t <= 31 and rows of 32 bits: no test
+#pragma unroll
+            for (int i = 0; i < 31; i++) {
+                const int bh = (int)(B >> 32), c = bh >> 31, sw = (bh & N) >> 31;
+                const u64 c64 = ((u64)(u32)c << 32) | (u32)c, s64 = ((u64)(u32)sw << 32) | (u32)sw;
+                const u64 a = A;
+                const u32 x = p1;
+                A = (a & ~s64) | (B & s64);
+                p1 = (x & ~(u32)sw) | (q1 & (u32)sw);
+                B = (B ^ (a & c64)) << 1;
+                q1 = (q1 ^ (x & (u32)c)) << 1;
+                N = (N ^ sw) - 1 - sw;
+            }
+            t = 31;
         }
-        const int c = A ? __clzll(A) : 64;
-        const u64 Bn = A ? A << c : 0;
-        const int dr = A ? dgb - c : -1;
-        A = B;                                          // (a, b) <- (b, a mod b)
-        B = Bn;
-        dga = dgb;
-        dgb = dr;
-        u32 y = ma0; ma0 = mb0; mb0 = y;
-        y = ma1; ma1 = mb1; mb1 = y;
-        dma = dmb;
-        dmb = ndm;
-        steps++;
+        p = p1;
+        q = q1;
     }
-    if (steps == 0) {
-        L.mode = 1;
-        L.k = da - db;
-        L.mt[0] = L.mt[1] = L.mt[2] = L.mt[3] = 0;
-    } else {
-        L.mode = 0;
-        L.k = 0;
-        L.mt[0] = ma0; L.mt[1] = ma1; L.mt[2] = mb0; L.mt[3] = mb1;
+    int R = 2 * lim - t;                                // R + N < 0: s_g > lim
+#pragma unroll 4
+    for (; t < 62; t++) {
+        const int bh = (int)(B >> 32);
+        if ((bh & N & (R + N)) < 0) break;              // a swap that is not allowed
+        const int c = bh >> 31, sw = (bh & N) >> 31;
+        const u64 c64 = ((u64)(u32)c << 32) | (u32)c, s64 = ((u64)(u32)sw << 32) | (u32)sw;
+        const u64 a = A, x = p;
+        A = (a & ~s64) | (B & s64);
+        p = (x & ~s64) | (q & s64);
+        B = (B ^ (a & c64)) << 1;
+        q = (q ^ (x & c64)) << 1;
+        N = (N ^ sw) - 1 - sw;
+        R--;
     }
+    const int sf = (t + N) >> 1;
+    L.ef = (u32)(p >> sf);
+    L.eg = (u32)(q >> (t - sf));
     return L;
 }
 
-// lo and hi parts of x (64 bits) times a 32-bit polynomial
-GF2E_DEV u64 mul64x32_lo(u64 x, const Masked &m) {
-    return clmul_masked(mask32((u32)x), m) ^ (clmul_masked(mask32((u32)(x >> 32)), m) << 32);
-}
-GF2E_DEV u64 mul64x32_hi(u64 x, const Masked &m) {
-    return clmul_masked(mask32((u32)(x >> 32)), m) >> 32;
-}
 // x * m_a and x * m_b as 96 bits each (lo: bits 0..63, hi: bits 64..95) by
 // 16-entry tables T[v] = v * m (v a nibble, entries of up to 35 bits), one
 // pass over x's nibbles for both: lookups, shifts and XORs, no multiplies
@@ -138,15 +137,6 @@ GF2E_DEV u64 shl_word(const u64 *X, long long w, long long k) {
     u64 h = (w >= ks) ? X[w - ks] : 0, l = (w >= ks + 1) ? X[w - ks - 1] : 0;
     return kb ? ((h << kb) | (l >> (64 - kb))) : h;
 }
-// word w of one new vector / row: mode 0: m0*X + m1*Y; mode 1 (row a): X ^ (Y << k)
-GF2E_DEV u64 new_word(int mode, const u64 *X, const u64 *Y, long long w, const Masked &m0,
-                      const Masked &m1, long long k, bool is_a) {
-    if (mode == 1) return is_a ? (X[w] ^ shl_word(Y, w, k)) : Y[w];
-    u64 v = mul64x32_lo(X[w], m0) ^ mul64x32_lo(Y[w], m1);
-    if (w >= 1) v ^= mul64x32_hi(X[w - 1], m0) ^ mul64x32_hi(Y[w - 1], m1);
-    return v;
-}
-
 // what the rounds ended with (thread 0's counters)
 struct LehmerEnd {
     int parity = 0;              // which copy of the rows holds the result
@@ -161,10 +151,10 @@ struct LehmerEnd {
 // Lehmer rounds, pipelined: while warps 1..15 apply round r's matrix to the
 // vectors A, B and to the accumulated rows (one output word per item, the
 // carry from word w-1 recomputed, so no barrier inside the round), warp 0
-// computes the three top words of the new A and B itself, reads their
-// degrees and 64-bit windows off them and runs round r+1's Euclid steps on
-// thread 0.  One barrier per round; when the new windows are not within
-// those three words (a large drop in degree), warp 0 scans the new vectors
+// computes the six top 32-bit chunks of the new A and B itself, reads their
+// degrees and 64-bit windows off them and runs round r+1's division steps.
+// One barrier per round; when the new windows are not within
+// those chunks (a large drop in degree), warp 0 scans the new vectors
 // after the barrier instead.  Round state is double-buffered by parity.
 // Shared memory: V[4][W] (two buffers of A, B), R[2][4][mw].
 // The caller has put a and b (zeros above) into V[0 .. W), V[W .. 2 W) and, with
@@ -180,7 +170,7 @@ GF2E_DEV LehmerEnd lehmer_cta(u64 *V, u64 W, u64 *R, u64 mw, long long da0, long
     const int tid = threadIdx.x;
     const long long max_rounds = 2 * (max(da0, db0) + 2) + 16;
 
-    // thread 0: publish round q's state from degrees/roles and windows
+    // warp 0: publish round q's state from degrees/roles and windows
     auto publish = [&](int q, int va, int vb, int ra, long long da, long long db, u64 wa, u64 wb,
                        long long md, long long round) {
         if (da < db) {
@@ -189,25 +179,30 @@ GF2E_DEV LehmerEnd lehmer_cta(u64 *V, u64 W, u64 *R, u64 mw, long long da0, long
             long long t = da; da = db; db = t;
             u64 u = wa; wa = wb; wb = u;
         }
-        s_va[q] = va; s_vb[q] = vb; s_ra[q] = ra;
-        s_top[q] = da >> 6;
-        s_md[q] = md;
-        if (db < m || round > max_rounds) {
-            s_done[q] = 1;
+        const bool done = db < m || round > max_rounds;
+        if (tid == 0) {
+            s_va[q] = va; s_vb[q] = vb; s_ra[q] = ra;
+            s_top[q] = da >> 6;
+            s_md[q] = md;
+            s_done[q] = done;
             if (round > max_rounds) E.status = GF2E_ERR_TIMEOUT;
             E.rounds = round;
-            return;
         }
-        s_done[q] = 0;
+        if (done) return;
         const long long lo = da >= 63 ? da - 63 : 0;
         const long long c0 = clock64();
-        Lehmer L = lehmer_round(wa, wb, da, db, lo, m);
+        const Lehmer L = lehmer_round(wa, wb, da, db, lo, m, tid);
         E.cyc_serial += clock64() - c0;
-        s_mode[q] = L.mode;
-        s_k[q] = L.k;
-        for (int i = 0; i < 4; i++) s_m[q][i] = L.mt[i];
+        if (tid < 2) {
+            s_m[q][tid] = L.ef;
+            s_m[q][2 + tid] = L.eg;
+        }
+        if (tid == 0) {
+            s_mode[q] = L.mode;
+            s_k[q] = L.k;
+        }
     };
-    // thread 0: degrees and windows of vectors va, vb read from shared memory
+    // warp 0: degrees and windows of vectors va, vb read from shared memory
     auto publish_from_vectors = [&](int q, int va, int vb, int ra, long long da, long long db,
                                     long long md, long long round) {
         const long long dhi = max(da, db);
@@ -215,7 +210,7 @@ GF2E_DEV LehmerEnd lehmer_cta(u64 *V, u64 W, u64 *R, u64 mw, long long da0, long
         publish(q, va, vb, ra, da, db, win_at(V + (u64)va * W, (long long)W, lo),
                 win_at(V + (u64)vb * W, (long long)W, lo), md, round);
     };
-    if (tid == 0) publish_from_vectors(0, 0, 1, 0, da0, db0, 0, 0);
+    if (tid < 32) publish_from_vectors(0, 0, 1, 0, da0, db0, 0, 0);
     __syncthreads();
 
     for (long long round = 0;; round++) {
@@ -239,8 +234,6 @@ GF2E_DEV LehmerEnd lehmer_cta(u64 *V, u64 W, u64 *R, u64 mw, long long da0, long
         u64 *A2 = V + (u64)spare[0] * W, *B2 = V + (u64)spare[1] * W;
         const u64 *RA = R + (u64)(p * 4 + 2 * ra) * mw, *RB = R + (u64)(p * 4 + 2 * (ra ^ 1)) * mw;
         u64 *N = R + (u64)q * 4 * mw;
-        const Masked m0 = mask32(s_m[p][0]), m1 = mask32(s_m[p][1]), m2 = mask32(s_m[p][2]),
-                     m3 = mask32(s_m[p][3]);
         const long long md_next =
             ROWS ? min((long long)mw - 2, md + (mode == 1 ? (k >> 6) + 1 : 1)) : 0;
         const int warp = tid >> 5;
@@ -306,48 +299,63 @@ GF2E_DEV LehmerEnd lehmer_cta(u64 *V, u64 W, u64 *R, u64 mw, long long da0, long
                 B2[w] = 0;
             }
         } else if (warp == 0) {
-            // warp 0: the three top words of the new A (lanes 0-2) and B (3-5)
-            // in one pass (each lane with its own matrix row), then their
+            // warp 0: the six top 32-bit chunks of the new A and B, then their
             // degrees and the next windows by ballot and shuffle
-            const int lane = tid;
-            const bool vb = lane >= 3;
-            const long long w = top - (lane % 3);
-            u64 val = 0;
-            if (lane < 6 && w >= 0)
-                val = new_word(mode, A, B, w, vb ? m2 : m0, vb ? m3 : m1, k, !vb);
-            const unsigned nz = __ballot_sync(0xffffffffu, lane < 6 && val != 0);
-            const int fa = __ffs(nz & 7u) - 1, fb = __ffs((nz >> 3) & 7u) - 1;
-            const u64 ta = __shfl_sync(0xffffffffu, val, fa < 0 ? 0 : fa);
-            const u64 tb = __shfl_sync(0xffffffffu, val, fb < 0 ? 3 : 3 + fb);
-            const long long dn0 = fa < 0 ? -1 : (top - fa) * 64 + 63 - __clzll(ta);
-            const long long dn1 = fb < 0 ? -1 : (top - fb) * 64 + 63 - __clzll(tb);
+            const int lane = tid, r = lane >> 4, c = lane & 7;
+            const long long g0 = 2 * top + 1;                 // chunk c is number g0 - c
+            u32 ch = 0;
+            if (mode != 1) {
+                // lane (row r, vector, c < 7) multiplies one chunk of A or B by
+                // its entry; the rows' sums, and the high half of the chunk below
+                const u32 *X = reinterpret_cast<const u32 *>((lane & 8) ? B : A);
+                const u32 x = c < 7 && g0 - c >= 0 ? X[g0 - c] : 0;
+                u64 P = clmul32(x, s_m[p][2 * r + ((lane >> 3) & 1)]);
+                P ^= __shfl_xor_sync(0xffffffffu, P, 8);
+                const u32 up = __shfl_down_sync(0xffffffffu, (u32)(P >> 32), 1);
+                ch = c < 6 ? (u32)P ^ up : 0;
+            } else {
+                const long long w = top - (c >> 1);
+                u64 v = 0;
+                if (c < 6 && w >= 0) v = r ? B[w] : A[w] ^ shl_word(B, w, k);
+                ch = (u32)((c & 1) ? v : v >> 32);
+            }
+            const unsigned nz = __ballot_sync(0xffffffffu, ch != 0);
+            const int fa = __ffs(nz & 63u) - 1, fb = __ffs((nz >> 16) & 63u) - 1;
+            const u32 ta = __shfl_sync(0xffffffffu, ch, fa < 0 ? 0 : fa);
+            const u32 tb = __shfl_sync(0xffffffffu, ch, fb < 0 ? 16 : 16 + fb);
+            const long long dn0 = fa < 0 ? -1 : (g0 - fa) * 32 + 31 - __clz(ta);
+            const long long dn1 = fb < 0 ? -1 : (g0 - fb) * 32 + 31 - __clz(tb);
             bool slow = dn0 < 0 || dn1 < 0;
-            long long lo = 0;
+            const long long dhi = max(dn0, dn1), lo = dhi >= 63 ? dhi - 63 : 0;
+            slow = slow || (lo >> 5) < g0 - 5;
+            // the windows' lowest chunk is chunk i0, the two above it i0 - 1, i0 - 2
+            const int i0 = slow ? 2 : (int)(g0 - (lo >> 5));
+            const int i1 = max(i0 - 1, 0), i2 = max(i0 - 2, 0);
+            u32 x[2][3];
+#pragma unroll
+            for (int v = 0; v < 2; v++) {
+                x[v][0] = __shfl_sync(0xffffffffu, ch, 16 * v + i0);
+                x[v][1] = __shfl_sync(0xffffffffu, ch, 16 * v + i1);
+                x[v][2] = __shfl_sync(0xffffffffu, ch, 16 * v + i2);
+                if (i0 < 1) x[v][1] = 0;
+                if (i0 < 2) x[v][2] = 0;
+            }
             if (!slow) {
-                const long long dhi = max(dn0, dn1);
-                lo = dhi >= 63 ? dhi - 63 : 0;
-                slow = (lo >> 6) < top - 2;
+                const unsigned sb = (unsigned)(lo & 31);
+                u64 win[2];
+#pragma unroll
+                for (int v = 0; v < 2; v++)
+                    win[v] = ((u64)__funnelshift_r(x[v][1], x[v][2], sb) << 32) |
+                             __funnelshift_r(x[v][0], x[v][1], sb);
+                publish(q, spare[0], spare[1], 0, dn0, dn1, win[0], win[1], md_next, round + 1);
             }
-            // the windows' low words are words lo/64 (lane top - lo/64) and
-            // lo/64 + 1 (one lane lower) of the new vectors
-            const int ia = slow ? 0 : (int)(top - (lo >> 6));
-            const int ib = ia >= 1 ? ia - 1 : 0;
-            const u64 x0a = __shfl_sync(0xffffffffu, val, ia), x1a = __shfl_sync(0xffffffffu, val, ib);
-            const u64 x0b = __shfl_sync(0xffffffffu, val, 3 + ia), x1b = __shfl_sync(0xffffffffu, val, 3 + ib);
-            if (lane == 0) {
-                if (!slow) {
-                    const unsigned sb = (unsigned)(lo & 63);
-                    publish(q, spare[0], spare[1], 0, dn0, dn1, funnel64(x0a, ia >= 1 ? x1a : 0, sb),
-                            funnel64(x0b, ia >= 1 ? x1b : 0, sb), md_next, round + 1);
-                }
-                s_slow = slow;
-            }
+            if (lane == 0) s_slow = slow;
         }
         __syncthreads();
         if (s_slow) {                                  // degrees from the full new vectors
             if (tid < 32) {
                 const long long d0 = warp_degree(A2, top), d1 = warp_degree(B2, top);
-                if (tid == 0) publish_from_vectors(q, spare[0], spare[1], 0, d0, d1, md_next, round + 1);
+                publish_from_vectors(q, spare[0], spare[1], 0, d0, d1, md_next, round + 1);
             }
             __syncthreads();
         }
