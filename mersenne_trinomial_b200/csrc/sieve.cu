@@ -178,22 +178,25 @@ size_t region_want(int dmin, int dmax) {
 }
 
 // ---- small field GF(2^d), d <= 31, modulus q (bit d set)
-GF2E_DEV u32 sf_mul(u32 a, u32 b, u32 q, int d) {
-    u64 t = clmul32(a, b);
-    for (int bit = 2 * d - 2; bit >= d; bit--)
-        if ((t >> bit) & 1) t ^= (u64)q << (bit - d);
+// t mod q, a fold at a time by q's low terms (a bit-serial reduction made the
+// start values of the table chains 20 to 35 us of latency a degree)
+GF2E_DEV u32 sf_reduce(u64 t, u32 q, int d) {
+    const u32 low = q ^ (1u << d);
+    for (u64 h = t >> d; h; h = t >> d) {
+        t &= (1u << d) - 1;
+        for (u32 l = low; l; l &= l - 1) t ^= h << (__ffs(l) - 1);
+    }
     return (u32)t;
 }
 GF2E_DEV u32 sf_mulx(u32 a, u32 q, int d) {
-    u32 t = a << 1;
+    const u32 t = a << 1;
     return ((t >> d) & 1) ? (t ^ q) : t;
 }
-GF2E_DEV u32 sf_powx(u64 e, u32 q, int d) {     // x^e
-    u32 r = 1, b = 2;
-    while (e) {
-        if (e & 1) r = sf_mul(r, b, q, d);
-        b = sf_mul(b, b, q, d);
-        e >>= 1;
+GF2E_DEV u32 sf_powx(u32 e, u32 q, int d) {     // x^e by squaring and times x
+    u32 r = 1;
+    for (int bit = 31 - __clz(e); bit >= 0; bit--) {
+        r = sf_reduce(spread32(r), q, d);
+        if ((e >> bit) & 1) r = sf_mulx(r, q, d);
     }
     return r;
 }
@@ -250,35 +253,97 @@ GF2E_DEV bool progression(u64 j, u64 v, int d, u64 M, u64 &first, u64 &n) {
     return true;
 }
 
-__global__ void k_tables(u32 *__restrict__ A, u32 *__restrict__ L, int d, u32 q, u64 M) {
-    u64 nchunk = (M + 31) >> 5;
-    for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x; t < nchunk;
-         t += (u64)gridDim.x * blockDim.x) {
-        u64 i0 = t << 5;
-        u32 v = sf_powx(i0, q, d);
-        for (int e = 0; e < 32; e++) {
-            u64 i = i0 + e;
-            if (i >= M) break;
-            A[i] = v;
-            L[v] = (u32)i;
-            v = sf_mulx(v, q, d);
-        }
+// the same in 32 bits, for d <= 31 (a 64-bit division is five 32-bit ones)
+GF2E_DEV u32 gcd_inv32(u32 a, u32 m, u32 *inv) {
+    int t = 0, nt = 1;
+    u32 r = m, nr = a % m;
+    while (nr) {
+        const u32 q = r / nr;
+        const int tmp = t - (int)q * nt;
+        t = nt;
+        nt = tmp;
+        const u32 rr = r - q * nr;
+        r = nr;
+        nr = rr;
     }
+    *inv = t < 0 ? (u32)t + m : (u32)t;
+    return r;
+}
+GF2E_DEV bool progression32(u32 j, u32 v, int d, u32 M, u32 &first, u32 &n) {
+    u32 inv;
+    const u32 gg = gcd_inv32(j, M, &inv);
+    u32 s0;
+    if (gg == 1) {
+        n = M;
+        s0 = (u32)mod_mersenne((u64)inv * v, d, M);
+    } else {
+        if (v % gg) return false;
+        n = M / gg;
+        u32 inv2;
+        gcd_inv32(j / gg, n, &inv2);              // coprime after dividing out gg
+        s0 = (u32)((u64)inv2 * (v / gg) % n);
+    }
+    first = s0 ? s0 : n;
+    return true;
 }
 
 struct DegreeArgs {
     int d;
     u32 q;
+    u32 *A, *L;                           // tables of 2^d entries
+    u32 blk0[2], nblk[2];                 // this degree's blocks of k_tables, k_classes
     u64 M, rmod, smax;
+    u64 seq;                              // bit 0 of x^0 .. x^(2d-2)
     int nsub;
     u64 subq[6];
     u64 strip;                            // strip width (entries of best[] per CTA)
     ListCaps caps;
 };
+// degrees sieved by one launch of each kernel: all up to GROUP_D but the
+// largest (whose tables need the whole region), whose launches are latency
+// (a degree alone took 35 us at d <= 20); larger ones one at a time, so that
+// their tables stay in L2 from one kernel to the next
+constexpr int GROUP_D = 20, GROUP_MAX = GROUP_D - 1;
+struct Group {
+    int n;
+    DegreeArgs a[GROUP_MAX];
+};
+GF2E_DEV const DegreeArgs &degree_of(const Group &G, int k) {
+    int i = 0;
+    while (i + 1 < G.n && blockIdx.x >= G.a[i + 1].blk0[k]) i++;
+    return G.a[i];
+}
+
+__global__ void k_tables(const __grid_constant__ Group G) {
+    const DegreeArgs &a = degree_of(G, 0);
+    const int d = a.d;
+    const u32 q = a.q, M = (u32)a.M, nchunk = (M + 31) >> 5;
+    u32 *__restrict__ A = a.A, *__restrict__ L = a.L;
+    for (u32 t = (blockIdx.x - a.blk0[0]) * blockDim.x + threadIdx.x; t < nchunk;
+         t += a.nblk[0] * blockDim.x) {
+        const u32 i0 = t << 5;
+        u32 v = sf_powx(i0, q, d);
+        for (u32 e = 0; e < 32; e++) {
+            const u32 i = i0 + e;
+            if (i >= M) break;
+            A[i] = v;
+            L[v] = i;
+            v = sf_mulx(v, q, d);
+        }
+    }
+}
 
 // j is the least element of its cyclotomic coset {j 2^i mod M}
 GF2E_DEV bool coset_least(u64 j, int d, u64 M) {
     u64 jj = j;
+    for (int i = 1; i < d; i++) {
+        jj = ((jj << 1) | (jj >> (d - 1))) & M;
+        if (jj < j) return false;
+    }
+    return true;
+}
+GF2E_DEV bool coset_least32(u32 j, int d, u32 M) {
+    u32 jj = j;
     for (int i = 1; i < d; i++) {
         jj = ((jj << 1) | (jj >> (d - 1))) & M;
         if (jj < j) return false;
@@ -293,10 +358,11 @@ GF2E_DEV bool coset_least(u64 j, int d, u64 M) {
 // with one active lane per warp.  work(i, false) pads the final partial
 // batch; every lane of the warp calls work together.
 template <typename Pred, typename Work>
-GF2E_DEV void for_each_selected(u64 begin, u64 end, u64 *wq, Pred &&pred, Work &&work) {
+GF2E_DEV void for_each_selected(u64 begin, u64 end, u64 *wq, u32 block, u32 blocks, Pred &&pred,
+                                Work &&work) {
     const int lane = threadIdx.x & 31;
-    const u64 gw = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const u64 nw = ((u64)gridDim.x * blockDim.x) >> 5;
+    const u64 gw = ((u64)block * blockDim.x + threadIdx.x) >> 5;
+    const u64 nw = ((u64)blocks * blockDim.x) >> 5;
     int qn = 0;
     for (u64 base = begin + gw * 32; base < end; base += nw * 32) {
         const u64 i = base + lane;
@@ -319,7 +385,8 @@ GF2E_DEV void for_each_selected(u64 begin, u64 end, u64 *wq, Pred &&pred, Work &
 // every coset leader j in [1, M) (about 1 in d of the j)
 template <typename Work>
 GF2E_DEV void for_each_leader(u64 M, int d, u64 *wq, Work &&work) {
-    for_each_selected(1, M, wq, [&](u64 j) { return coset_least(j, d, M); }, work);
+    for_each_selected(1, M, wq, blockIdx.x, gridDim.x,
+                      [&](u64 j) { return coset_least(j, d, M); }, work);
 }
 
 GF2E_DEV void add_stats(unsigned long long my_classes, unsigned long long my_marks, int d,
@@ -369,40 +436,57 @@ GF2E_DEV void class_flush(ClassQueue &q, int qn, Work &&work) {
     work(v ? q.j[lane] : 0, v ? q.first[lane] : 0, v ? q.n[lane] : 1, v);
 }
 
+// Minimal polynomial of beta = x^j, j a coset leader of degree d: the
+// connection polynomial of s_k = bit 0 of beta^k, k < 2d (Berlekamp-Massey;
+// any nonzero functional of an irreducible recurrence has it).  s_0 .. s_(d-1)
+// come from the table, the rest from u = beta^d: bit 0 of beta^k u is the
+// parity of beta^k and w, w_i = bit 0 of x^i u, the parity of u and `seq` from
+// place i on.  (Elimination on beta^0 .. beta^d keeps d pivots in local
+// memory.)  0 if something is inconsistent.
+GF2E_DEV u32 minimal_poly(const u32 *__restrict__ A, u32 j, int d, u32 M, u64 seq) {
+    const u32 u = A[mod_mersenne((u64)j * d, d, M)];
+    u32 w = 0;
+    for (int i = 0; i < d; i++) w |= (u32)(__popc(u & (u32)(seq >> i)) & 1) << i;
+    u64 s = 0;
+    u32 idx = 0;
+    for (int k = 0; k < d; k++) {
+        const u32 v = A[idx];
+        s |= (u64)(v & 1) << k | (u64)(__popc(v & w) & 1) << (d + k);
+        idx += j;
+        if (idx >= M) idx -= M;
+    }
+    u32 C = 1, B = 1, R = 0;
+    int len = 0, gap = 1;
+    for (int n = 0; n < 2 * d; n++) {
+        R = R << 1 | (u32)((s >> n) & 1);               // bit i is s_(n-i)
+        const bool off = __popc(C & R) & 1, grow = off && 2 * len <= n;
+        const u32 T = C;
+        if (off) C ^= B << gap;
+        if (grow) { len = n + 1 - len; B = T; }
+        gap = grow ? 1 : gap + 1;
+    }
+    const u32 mask = __brev(C) >> (31 - d);
+    return len == d && (mask >> d) == 1 && (mask & 1) ? mask : 0;
+}
+
 __global__ void __launch_bounds__(256)
-k_classes(const u32 *__restrict__ A, const u32 *__restrict__ L, const DegreeArgs a,
-          unsigned long long *__restrict__ best, Prog *__restrict__ strip, Prog *__restrict__ heavy,
-          Counters *__restrict__ cnt) {
+k_classes(const __grid_constant__ Group G, unsigned long long *__restrict__ best,
+          Prog *__restrict__ strip, Prog *__restrict__ heavy, Counters *__restrict__ cnt) {
     __shared__ u64 wq_all[8][64];
     __shared__ ClassQueue cq_all[8];
+    const DegreeArgs &a = degree_of(G, 1);
     const int d = a.d;
-    const u64 M = a.M;
+    const u32 M = (u32)a.M, rmod = (u32)a.rmod;
+    const u32 *__restrict__ A = a.A, *__restrict__ L = a.L;
     unsigned long long my_classes = 0, my_marks = 0;
     ClassQueue &cq = cq_all[threadIdx.x >> 5];
     int cqn = 0;
-    // minimal polynomial of beta = x^j (first linear dependency among
-    // beta^0..beta^d over GF(2)) and the marks of its progression
+    // the marks of a class's progression
     auto mark = [&](u64 j, u64 first, u64 n, bool valid) {
         if (!valid) return;
         const u64 count = (a.smax - first) / n + 1;
-        u32 prow[DMAX + 1], ptag[DMAX + 1];
-        int pbit[DMAX + 1];
-        int np = 0;
-        u32 mask = 0;
-        u64 idx = 0;
-        for (int k = 0; k <= d; k++) {
-            u32 row = A[idx], tag = 1u << k;
-            for (int p = 0; p < np; p++)
-                if ((row >> pbit[p]) & 1) { row ^= prow[p]; tag ^= ptag[p]; }
-            if (row == 0) { mask = tag; break; }
-            pbit[np] = 31 - __clz(row);
-            prow[np] = row;
-            ptag[np] = tag;
-            np++;
-            idx += j;
-            if (idx >= M) idx -= M;
-        }
-        if (!((mask >> d) & 1) || !(mask & 1)) {        // cannot happen
+        const u32 mask = minimal_poly(A, (u32)j, d, M, a.seq);
+        if (!mask) {                                    // cannot happen
             atomicAdd(&cnt->bad, 1ull);
             return;
         }
@@ -428,19 +512,22 @@ k_classes(const u32 *__restrict__ A, const u32 *__restrict__ L, const DegreeArgs
             }
         }
     };
-    for_each_leader(M, d, wq_all[threadIdx.x >> 5], [&](u64 j, bool valid) {
-        bool ok = valid;
-        for (int k = 0; k < a.nsub && ok; k++)
-            if (j % a.subq[k] == 0) ok = false;
-        u64 first = 0, n = 1;
-        if (ok) {
-            my_classes++;
-            const u64 u = mod_mersenne(j * a.rmod, d, M);
-            if (u == 0) ok = false;
-            else ok = progression(j, L[A[u] ^ 1u], d, M, first, n) && first <= a.smax;
-        }
-        class_push(cq, cqn, ok, j, first, n, mark);
-    });
+    for_each_selected(
+        1, M, wq_all[threadIdx.x >> 5], blockIdx.x - a.blk0[1], a.nblk[1],
+        [&](u64 j) { return coset_least32((u32)j, d, M); },
+        [&](u64 j, bool valid) {
+            bool ok = valid;
+            for (int k = 0; k < a.nsub && ok; k++)
+                if ((u32)j % (u32)a.subq[k] == 0) ok = false;
+            u32 first = 0, n = 1;
+            if (ok) {
+                my_classes++;
+                const u32 u = (u32)mod_mersenne(j * rmod, d, M);
+                if (u == 0) ok = false;
+                else ok = progression32((u32)j, L[A[u] ^ 1u], d, M, first, n) && first <= a.smax;
+            }
+            class_push(cq, cqn, ok, j, first, n, mark);
+        });
     class_flush(cq, cqn, mark);
     add_stats(my_classes, my_marks, d, cnt);
 }
@@ -708,7 +795,8 @@ k_wide_match(const E *__restrict__ L, const ulonglong2 *__restrict__ list, u64 c
         if (valid) wide_mark(j, first, n, a, best, heavy, cnt, my_marks);
     };
     for_each_selected(
-        0, nl, wq_all[threadIdx.x >> 5], [&](u64 i) { return list[i].y - a.lo < a.len; },
+        0, nl, wq_all[threadIdx.x >> 5], blockIdx.x, gridDim.x,
+        [&](u64 i) { return list[i].y - a.lo < a.len; },
         [&](u64 i, bool valid) {
             u64 j = 0, first = 0, n = 1;
             bool ok = valid;
@@ -897,6 +985,12 @@ int gf2e_sieve_run(uint64_t r, int dmin, int dmax, uint64_t smax, uint64_t *best
             a.q = (u32)cached_primitive(d);
             a.rmod = rmod;
             a.smax = smax;
+            a.seq = 0;
+            for (u64 v = 1, i = 0; i + 1 < 2 * (u64)d; i++) {
+                a.seq |= (v & 1) << i;
+                v <<= 1;
+                if ((v >> d) & 1) v ^= a.q;
+            }
             a.strip = strip_w;
             a.caps = caps;
             a.nsub = np;
@@ -953,12 +1047,29 @@ int gf2e_sieve_run(uint64_t r, int dmin, int dmax, uint64_t smax, uint64_t *best
     if (!args.empty()) {
         u32 *A = (u32 *)reg;
         u32 *L = (u32 *)(reg + dense_table_bytes(std::min(dmax, wfrom - 1)));
-        for (const DegreeArgs &a : args) {
-            u64 nchunk = (a.M + 31) >> 5;
-            k_tables<<<gf2e::grid_for(nchunk, 256, 16), 256, 0, st>>>(A, L, a.d, a.q, a.M);
+        for (size_t at = 0; at < args.size();) {
+            // the tables of a group side by side: those below the largest
+            // degree fit where its own go
+            Group G;
+            G.n = 0;
+            u64 off = 0;
+            u32 blocks[2] = {0, 0};
+            do {
+                DegreeArgs &a = G.a[G.n++];
+                a = args[at++];
+                a.A = A + off;
+                a.L = L + off;
+                off += (u64)1 << a.d;
+                const u64 work[2] = {(a.M + 31) >> 5, a.M};
+                for (int k = 0; k < 2; k++) {
+                    a.blk0[k] = blocks[k];
+                    a.nblk[k] = (u32)gf2e::grid_for(work[k], 256, 16);
+                    blocks[k] += a.nblk[k];
+                }
+            } while (at + 1 < args.size() && args[at].d <= GROUP_D && G.n < GROUP_MAX);
+            k_tables<<<blocks[0], 256, 0, st>>>(G);
             GF2E_CHECK_LAUNCH("k_tables");
-            k_classes<<<gf2e::grid_for(a.M, 256, 16), 256, 0, st>>>(A, L, a, best, strip, heavy,
-                                                                    cnt);
+            k_classes<<<blocks[1], 256, 0, st>>>(G, best, strip, heavy, cnt);
             GF2E_CHECK_LAUNCH("k_classes");
         }
     }
