@@ -319,17 +319,29 @@ __global__ void k_tables(const __grid_constant__ Group G) {
     const int d = a.d;
     const u32 q = a.q, M = (u32)a.M, nchunk = (M + 31) >> 5;
     u32 *__restrict__ A = a.A, *__restrict__ L = a.L;
-    for (u32 t = (blockIdx.x - a.blk0[0]) * blockDim.x + threadIdx.x; t < nchunk;
-         t += a.nblk[0] * blockDim.x) {
-        const u32 i0 = t << 5;
-        u32 v = sf_powx(i0, q, d);
+    // a warp's 32 chains of 32 elements pass through shared memory, so that A is
+    // stored a line at a time (a lane storing its own chain touched 32 lines a
+    // store: 345 us at d = 24)
+    __shared__ u32 s_chain[8][32][33];
+    u32 (*chain)[33] = s_chain[threadIdx.x >> 5];
+    const u32 lane = threadIdx.x & 31;
+    for (u32 t0 = (blockIdx.x - a.blk0[0]) * blockDim.x + (threadIdx.x & ~31u); t0 < nchunk;
+         t0 += a.nblk[0] * blockDim.x) {
+        const u32 i0 = (t0 + lane) << 5;
+        u32 v = i0 < M ? sf_powx(i0, q, d) : 1;
+#pragma unroll 8
         for (u32 e = 0; e < 32; e++) {
-            const u32 i = i0 + e;
-            if (i >= M) break;
-            A[i] = v;
-            L[v] = i;
+            chain[lane][e] = v;
+            if (i0 + e < M) L[v] = i0 + e;
             v = sf_mulx(v, q, d);
         }
+        __syncwarp();
+#pragma unroll 8
+        for (u32 e = 0; e < 32; e++) {
+            const u32 i = ((t0 + e) << 5) + lane;
+            if (i < M) A[i] = chain[e][lane];
+        }
+        __syncwarp();
     }
 }
 
@@ -532,33 +544,128 @@ k_classes(const __grid_constant__ Group G, unsigned long long *__restrict__ best
     add_stats(my_classes, my_marks, d, cnt);
 }
 
-// heavy progressions: block-strided over records, threads over marks
-__global__ void k_heavy(const Prog *__restrict__ heavy, const Counters *__restrict__ cnt,
-                        u64 smax, unsigned long long *__restrict__ best, u64 hcap) {
+// heavy progressions in [lo, hi], a window of best[] that stays in L2 (the
+// marks are random: over all of a 545 MB best[] at once each read and wrote a
+// DRAM sector of its own, 1.42 ms for 33 M marks): a warp a record, lanes over
+// marks, or a lane a record where a window holds at most one or two of them
+constexpr u64 HEAVY_WINDOW = 1ull << 23;       // entries (64 MB)
+__global__ void __launch_bounds__(256)
+k_heavy(const Prog *__restrict__ heavy, const Counters *__restrict__ cnt, u64 lo, u64 hi,
+        unsigned long long *__restrict__ best, u64 hcap) {
     u64 nh = cnt->nheavy;
     if (nh > hcap) nh = hcap;
-    for (u64 rec = blockIdx.x; rec < nh; rec += gridDim.x) {
-        Prog p = heavy[rec];
-        for (u64 s = p.s0 + (u64)threadIdx.x * p.n; s <= smax; s += (u64)blockDim.x * p.n)
-            atomicMin(&best[s], (unsigned long long)p.key);
+    const int lane = threadIdx.x & 31;
+    const u64 nw = ((u64)gridDim.x * blockDim.x) >> 5;
+    auto start = [&](const Prog &p) {
+        if (p.s0 >= lo) return p.s0;
+        const u64 num = lo - p.s0 + p.n - 1;
+        const u64 k = num >> 32 ? num / p.n : (u32)num / (u32)p.n;
+        return p.s0 + k * p.n;
+    };
+    // neighbours in the list are of one degree and go to different warps: the
+    // short periods have hundreds of times the marks of the long ones
+    for (u64 base = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5; base < nh;
+         base += nw * 32) {
+        const u64 rec = base + lane * nw;
+        const bool have = rec < nh;
+        const Prog p = have ? heavy[rec] : Prog{~0ull, 1, 0};
+        u64 s = have ? start(p) : ~0ull;
+        const bool few = p.n * 4 > hi - lo;
+        if (few)
+            for (; s <= hi; s += p.n) atomicMin(&best[s], (unsigned long long)p.key);
+        for (unsigned m = __ballot_sync(0xffffffffu, have && !few); m; m &= m - 1) {
+            const int k = __ffs(m) - 1;
+            const u64 n = __shfl_sync(0xffffffffu, p.n, k), key = __shfl_sync(0xffffffffu, p.key, k);
+            for (u64 t = __shfl_sync(0xffffffffu, s, k) + lane * n; t <= hi; t += 32 * n)
+                atomicMin(&best[t], (unsigned long long)key);
+        }
     }
 }
 
-// short-period progressions, one STRIP-wide slice of best[] per CTA
+// Short-period progressions are marked in shared memory by their rank among
+// the list's keys where there are at most RANKED of them (at d <= 24 some
+// 1500): 32-bit minima there are one native operation, 64-bit ones a
+// compare-and-swap loop.  k_rank writes the list again, in key order, behind
+// its first RANKED records.
+constexpr u64 RANKED = 8192;
+static_assert(2 * RANKED <= SCAP, "room for the ordered list");
+__global__ void __launch_bounds__(256) k_rank(Prog *__restrict__ strip,
+                                              const Counters *__restrict__ cnt, u64 scap) {
+    __shared__ u64 keys[1024];
+    const u64 ns = cnt->nstrip;
+    if (ns > scap || ns > RANKED) return;
+    const u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool have = i < ns;
+    const Prog p = have ? strip[i] : Prog{0, 0, 0};
+    u64 rank = 0;
+    for (u64 base = 0; base < ns; base += 1024) {
+        const u64 n = min((u64)1024, ns - base);
+        __syncthreads();
+        for (u64 k = threadIdx.x; k < n; k += blockDim.x) keys[k] = strip[base + k].key;
+        __syncthreads();
+        for (u64 k = 0; k < n; k++) rank += keys[k] < p.key;
+    }
+    if (have) strip[RANKED + rank] = p;
+}
+
+// one STRIP-wide slice of best[] per CTA
 __global__ void __launch_bounds__(512)
 k_strip(const Prog *__restrict__ strip, const Counters *__restrict__ cnt, u64 smax,
         unsigned long long *__restrict__ best, const u64 STRIP, u64 scap) {
     extern __shared__ unsigned long long sb[];
     u64 ns = cnt->nstrip;
-    if (ns > scap) ns = scap;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const u64 nstrips = (smax + 1 + STRIP - 1) / STRIP;
+    if (ns <= scap && ns <= RANKED && smax < (1ull << 31)) {
+        u32 *rk = reinterpret_cast<u32 *>(sb);
+        const Prog *__restrict__ order = strip + RANKED;
+        const u32 W = (u32)STRIP;
+        for (u64 sid = blockIdx.x; sid < nstrips; sid += gridDim.x) {
+            const u32 lo = (u32)(sid * STRIP), len = min(W, (u32)smax - lo + 1);
+            for (u32 i = threadIdx.x; i < W; i += blockDim.x) rk[i] = ~0u;
+            __syncthreads();
+            // 32 progressions a warp: those with many marks one after the
+            // other, lanes over marks, the others a lane each
+            for (u32 base = warp; base < ns; base += nwarps * 32) {
+                const u32 pi = base + lane * nwarps;      // short periods apart
+                u32 n = 1, at = ~0u;                      // first mark, from lo
+                if (pi < ns) {
+                    const Prog p = order[pi];
+                    const u32 s0 = (u32)p.s0;
+                    n = (u32)p.n;
+                    const u32 past = s0 >= lo ? 0 : (lo - s0) % n;
+                    at = s0 >= lo ? s0 - lo : past ? n - past : 0;
+                }
+                const bool few = pi < ns && n * 16 > W;
+                if (few)
+                    for (; at < len; at += n) atomicMin(&rk[at], pi);
+                for (unsigned m = __ballot_sync(0xffffffffu, pi < ns && !few); m; m &= m - 1) {
+                    const int k = __ffs(m) - 1;
+                    const u32 pn = __shfl_sync(0xffffffffu, n, k), pr = base + k * nwarps;
+                    const u32 first = __shfl_sync(0xffffffffu, at, k);
+                    if (first >= len) continue;
+                    for (u32 t = first + lane * pn; t < len; t += 32 * pn) atomicMin(&rk[t], pr);
+                }
+            }
+            __syncthreads();
+            for (u32 i = threadIdx.x; i < len; i += blockDim.x) {
+                const u32 v = rk[i];
+                if (v != ~0u) {
+                    const unsigned long long key = order[v].key;
+                    if (key < best[(u64)lo + i]) best[(u64)lo + i] = key;
+                }
+            }
+            __syncthreads();
+        }
+        return;
+    }
+    if (ns > scap) ns = scap;
     for (u64 sid = blockIdx.x; sid < nstrips; sid += gridDim.x) {
         const u64 lo = sid * STRIP;
         const u64 hi = (lo + STRIP - 1 < smax) ? lo + STRIP - 1 : smax;   // inclusive
         for (u64 i = threadIdx.x; i < STRIP; i += blockDim.x) sb[i] = ~0ull;
         __syncthreads();
         // warps take progressions, lanes take marks
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
         for (u64 pi = warp; pi < ns; pi += nwarps) {
             Prog p = strip[pi];
             if (p.s0 > hi) continue;
@@ -1108,8 +1215,14 @@ int gf2e_sieve_run(uint64_t r, int dmin, int dmax, uint64_t smax, uint64_t *best
         }
         GF2E_CHECK_LAUNCH("k_wide_classes");
     }
-    k_heavy<<<gf2e::sm_count() * 16, 256, 0, st>>>(heavy, cnt, smax, best, caps.heavy);
-    GF2E_CHECK_LAUNCH("k_heavy");
+    const u64 window = std::max(HEAVY_WINDOW, smax / 32 + 1);
+    for (u64 lo = 0; lo <= smax; lo += window) {
+        k_heavy<<<gf2e::sm_count() * 8, 256, 0, st>>>(
+            heavy, cnt, lo, std::min(smax, lo + window - 1), best, caps.heavy);
+        GF2E_CHECK_LAUNCH("k_heavy");
+    }
+    k_rank<<<(unsigned)(RANKED / 256), 256, 0, st>>>(strip, cnt, caps.strip);
+    GF2E_CHECK_LAUNCH("k_rank");
     u64 nstrips = (smax + strip_w) / strip_w;
     k_strip<<<gf2e::grid_for(nstrips * 512, 512, 2), 512, strip_w * sizeof(u64), st>>>(
         strip, cnt, smax, best, strip_w, caps.strip);
