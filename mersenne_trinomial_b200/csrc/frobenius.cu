@@ -42,7 +42,9 @@
 // between a warp's instructions) and the integer pipe together.  A pass of 64
 // states at r = 136279841: windows one at a time with the high words by
 // shuffle 1.06 ms, the per-tile list with two loads a unit 0.72 ms, two
-// windows at a time 0.65 ms, fast windows listed by class 0.58 ms; staging
+// windows at a time 0.65 ms, fast windows listed by class 0.58 ms (1 state 29
+// us, 256 states at 999961 46 us; the windows that end inside a tile without
+// branches, their loads together, 15 and 27); staging
 // each window's run in shared memory by cp.async first ran 1.5 ms (more issued
 // instructions, fewer resident warps).  Each CTA composes its state's
 // windows in warp 0 with shifts and masks (the moduli are powers of two).
@@ -166,18 +168,25 @@ GF2E_DEV ulonglong2 interleave4(u32 c0, u32 c1, u32 c2, u32 c3) {
 constexpr int LANE_UNITS = 4;
 constexpr int MIN_CTAS = 5;
 
+// A word of a state: by a read-only load, or by a plain one in a chained pass
+// (read-only loads are for data that nobody writes while a CTA lives).
+template <bool RO>
+GF2E_DEV u32 state_word(const u32 *p) {
+    return RO ? __ldg(p) : *p;
+}
+
 // A full window over all of the tile's units, every index inside the state:
 // lane l's units u0 + l + 32 q read input words first + l + 32 q and the
 // word after it (the high word of the funnel shift) with two plain loads.
-template <int UL>
-GF2E_DEV void full_window(const u32 *__restrict__ in32, u32 first, u32 lane, u32 sh,
+template <int UL, bool RO>
+GF2E_DEV void full_window(const u32 *in32, u32 first, u32 lane, u32 sh,
                           u32 (&acc)[UL]) {
-    const u32 *__restrict__ p = in32 + (first + lane);
+    const u32 *p = in32 + (first + lane);
     u32 lo[UL], hi[UL];
 #pragma unroll
     for (int q = 0; q < UL; q++) {
-        lo[q] = __ldg(p + 32 * q);
-        hi[q] = __ldg(p + 32 * q + 1);
+        lo[q] = state_word<RO>(p + 32 * q);
+        hi[q] = state_word<RO>(p + 32 * q + 1);
     }
 #pragma unroll
     for (int q = 0; q < UL; q++) acc[q] ^= __funnelshift_r(lo[q], hi[q], sh);
@@ -185,18 +194,18 @@ GF2E_DEV void full_window(const u32 *__restrict__ in32, u32 first, u32 lane, u32
 
 // Two full windows of one class, every load of both issued before use, so
 // their memory latencies overlap.
-template <int UL>
-GF2E_DEV void full_windows2(const u32 *__restrict__ in32, u32 first1, u32 sh1, u32 first2, u32 sh2,
+template <int UL, bool RO>
+GF2E_DEV void full_windows2(const u32 *in32, u32 first1, u32 sh1, u32 first2, u32 sh2,
                          u32 lane, u32 (&acc)[UL]) {
-    const u32 *__restrict__ p1 = in32 + (first1 + lane);
-    const u32 *__restrict__ p2 = in32 + (first2 + lane);
+    const u32 *p1 = in32 + (first1 + lane);
+    const u32 *p2 = in32 + (first2 + lane);
     u32 l1[UL], h1[UL], l2[UL], h2[UL];
 #pragma unroll
     for (int q = 0; q < UL; q++) {
-        l1[q] = __ldg(p1 + 32 * q);
-        h1[q] = __ldg(p1 + 32 * q + 1);
-        l2[q] = __ldg(p2 + 32 * q);
-        h2[q] = __ldg(p2 + 32 * q + 1);
+        l1[q] = state_word<RO>(p1 + 32 * q);
+        h1[q] = state_word<RO>(p1 + 32 * q + 1);
+        l2[q] = state_word<RO>(p2 + 32 * q);
+        h2[q] = state_word<RO>(p2 + 32 * q + 1);
     }
 #pragma unroll
     for (int q = 0; q < UL; q++)
@@ -204,24 +213,27 @@ GF2E_DEV void full_windows2(const u32 *__restrict__ in32, u32 first1, u32 sh1, u
 }
 
 // Any other overlapping window: per unit the bits t whose output position
-// 128 u + c + 4 t lies in [lo, hi), loads bounds-tested.
-template <int UL>
-GF2E_DEV void part_window(const u32 *__restrict__ in32, u32 n32, u32 u0, u32 lane, FWin w,
+// 128 u + c + 4 t lies in [lo, hi), loads bounds-tested.  Positions are below
+// 2^31 (r < 2^31 - 2^16 and a tile ends less than 2^15 bits past r), and
+// lo, hi - 1 and j0 are all c mod 4, so the shifts are exact.  No branches:
+// the loads of all units are issued together.
+template <int UL, bool RO>
+GF2E_DEV void part_window(const u32 *in32, u32 n32, u32 u0, u32 lane, const FWin &w,
                         u32 (&acc)[UL]) {
+    u32 lo[UL], hi[UL];
 #pragma unroll
     for (int q = 0; q < UL; q++) {
-        const int64_t u = (int64_t)u0 + lane + 32 * q;
-        const int64_t j0 = u * UBITS + w.c;
-        const int64_t tlo = w.lo > j0 ? (w.lo - j0) / M : 0;
-        int64_t thi = w.hi > j0 ? (w.hi - 1 - j0) / M + 1 : 0;
-        if (thi > 32) thi = 32;
-        if (tlo >= thi) continue;
-        const u32 mask = (thi == 32 ? 0xffffffffu : ((1u << thi) - 1u)) & ~((1u << tlo) - 1u);
-        const int64_t P = 32 * u + w.K;
-        const int64_t i = P >> 5;
-        const u32 lo = (i >= 0 && i < (int64_t)n32) ? __ldg(in32 + i) : 0u;
-        const u32 hi = (i + 1 >= 0 && i + 1 < (int64_t)n32) ? __ldg(in32 + i + 1) : 0u;
-        acc[q] ^= __funnelshift_r(lo, hi, (u32)P & 31u) & mask;
+        const u32 i = u0 + lane + 32 * q + (u32)(w.K >> 5);     // negative: above any n32
+        lo[q] = i < n32 ? state_word<RO>(in32 + i) : 0u;
+        hi[q] = i + 1 < n32 ? state_word<RO>(in32 + i + 1) : 0u;
+    }
+#pragma unroll
+    for (int q = 0; q < UL; q++) {
+        const int j0 = (int)((u0 + lane + 32 * q) * UBITS) + w.c;
+        const int tlo = max((w.lo - j0) >> KL, 0);
+        const int thi = min(((w.hi - 1 - j0) >> KL) + 1, 32);
+        const u32 mask = tlo < thi ? (0xffffffffu >> (32 - (thi - tlo))) << tlo : 0u;
+        acc[q] ^= __funnelshift_r(lo[q], hi[q], (u32)w.K & 31u) & mask;
     }
 }
 
@@ -248,8 +260,8 @@ GF2E_DEV int compose_windows(u64 r, u64 s, FWin *tab, u32 lane) {
 }
 
 // the fast windows of one class (bits of m), two at a time
-template <int UL>
-GF2E_DEV void class_windows(const u32 *__restrict__ in32, const int *tabK, u32 m, int u0, u32 lane,
+template <int UL, bool RO>
+GF2E_DEV void class_windows(const u32 *in32, const int *tabK, u32 m, int u0, u32 lane,
                             u32 (&acc)[UL]) {
     while (m) {
         const int K1 = tabK[__ffs(m) - 1];
@@ -258,9 +270,9 @@ GF2E_DEV void class_windows(const u32 *__restrict__ in32, const int *tabK, u32 m
         if (m) {
             const int K2 = tabK[__ffs(m) - 1];
             m &= m - 1;
-            full_windows2<UL>(in32, f1, (u32)K1, (u32)(u0 + (K2 >> 5)), (u32)K2, lane, acc);
+            full_windows2<UL, RO>(in32, f1, (u32)K1, (u32)(u0 + (K2 >> 5)), (u32)K2, lane, acc);
         } else {
-            full_window<UL>(in32, f1, lane, (u32)K1, acc);
+            full_window<UL, RO>(in32, f1, lane, (u32)K1, acc);
         }
     }
 }
@@ -273,8 +285,8 @@ GF2E_DEV void class_windows(const u32 *__restrict__ in32, const int *tabK, u32 m
 // applied class by class with no masks, bounds tests or branches on the
 // class (a loop over all windows with a test and a switch each took 180
 // instructions a unit, 94 of them in the integer pipe).
-template <int UL>
-GF2E_DEV void frob4_tile(const u32 *__restrict__ in32, ulonglong2 *__restrict__ o, u32 n32,
+template <int UL, bool RO>
+GF2E_DEV void frob4_tile(const u32 *in32, ulonglong2 *o, u32 n32,
                          u32 nu, const FWin *tab, const int *tabK, int nwin, const FWin &mine,
                          const u32 (&cls)[M], u32 u0, u32 lane) {
     constexpr u32 TWL = 32 * UL;
@@ -289,15 +301,15 @@ GF2E_DEV void frob4_tile(const u32 *__restrict__ in32, ulonglong2 *__restrict__ 
     for (int c = 0; c < M; c++) {
 #pragma unroll
         for (int q = 0; q < UL; q++) C[c][q] = 0;
-        class_windows<UL>(in32, tabK, fast & cls[c], (int)u0, lane, C[c]);
+        class_windows<UL, RO>(in32, tabK, fast & cls[c], (int)u0, lane, C[c]);
     }
     for (u32 m = act & ~fast; m; m &= m - 1) {     // windows that start or end in the tile
         const FWin w = tab[__ffs(m) - 1];
         switch (w.c) {
-            case 0: part_window<UL>(in32, n32, u0, lane, w, C[0]); break;
-            case 1: part_window<UL>(in32, n32, u0, lane, w, C[1]); break;
-            case 2: part_window<UL>(in32, n32, u0, lane, w, C[2]); break;
-            default: part_window<UL>(in32, n32, u0, lane, w, C[3]); break;
+            case 0: part_window<UL, RO>(in32, n32, u0, lane, w, C[0]); break;
+            case 1: part_window<UL, RO>(in32, n32, u0, lane, w, C[1]); break;
+            case 2: part_window<UL, RO>(in32, n32, u0, lane, w, C[2]); break;
+            default: part_window<UL, RO>(in32, n32, u0, lane, w, C[3]); break;
         }
     }
 #pragma unroll
@@ -310,20 +322,27 @@ GF2E_DEV void frob4_tile(const u32 *__restrict__ in32, ulonglong2 *__restrict__ 
 // Batched F -> F^4 mod T (r < 2^31 - 2^16, even stride): blockIdx.y = state;
 // warp 0 composes the state's windows for the CTA, the warps stride over
 // its tiles.
+// RO: every word read was written before this kernel's first CTA started (not a
+// chained pass)
+template <bool RO>
 __global__ void __launch_bounds__(256, MIN_CTAS)
-k_frob4_batch(const u64 *__restrict__ in, u64 *__restrict__ out, size_t stride, u64 r,
+k_frob4_batch(const u64 *in, u64 *out, size_t stride, u64 r,
               const u64 *__restrict__ s_arr, u64 s_uniform) {
     __shared__ FWin tab[NCAND];
     __shared__ int tabK[NCAND];
     __shared__ int s_nwin;
     const int st = blockIdx.y;
     const u32 lane = threadIdx.x & 31;
+    cudaTriggerProgrammaticLaunchCompletion();
     if (threadIdx.x < 32) {
         const int n = compose_windows(r, s_arr ? s_arr[st] : s_uniform, tab, lane);
         if (lane == 0) s_nwin = n;
         if (lane < (u32)n) tabK[lane] = tab[lane].K;
     }
     __syncthreads();
+    // everything above reads only r and s; from here on the states, which the
+    // previous pass of the same call may still have been writing
+    if (!RO) cudaGridDependencySynchronize();
     const int nwin = s_nwin;
     const u32 nw = (u32)((r + 63) >> 6);
     const u32 n32 = 2 * nw, nu = (nw + 1) >> 1;
@@ -338,7 +357,7 @@ k_frob4_batch(const u64 *__restrict__ in, u64 *__restrict__ out, size_t stride, 
     const u32 ntiles = (nu + TWL - 1) / TWL;
     const u32 warps_total = (gridDim.x * blockDim.x) >> 5;
     for (u32 t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < ntiles; t += warps_total)
-        frob4_tile<LANE_UNITS>(in32, o, n32, nu, tab, tabK, nwin, mine, cls, TWL * t, lane);
+        frob4_tile<LANE_UNITS, RO>(in32, o, n32, nu, tab, tabK, nwin, mine, cls, TWL * t, lane);
 }
 
 }  // namespace
@@ -360,65 +379,85 @@ int squarings_per_pass() {
     return v == 1 || v == 2 ? v : 0;
 }
 
-// fused pass for this batch: applies (r, stride) and pays (not in L2), or forced
-bool use_frob4(u64 r, size_t stride, int nstates) {
-    const int mode = squarings_per_pass();
-    if (mode == 1 || !frob4_supported(r, stride)) return false;
-    // two squarings by one fused pass or two single ones, us: 36 / 46 (256
-    // states at r = 999961), 17 / 21 (1 at 3000017, 47 K words), 21 / 21 (64 at
-    // 30011, 30 K words), 17 / 13 (16 at 4423: every CTA composes 25 windows,
-    // and most of them end inside its one tile)
-    return mode == 2 || (size_t)nstates * stride >= ((size_t)1 << 15);
+// fused pass for this batch: applies (r, stride), and not switched off.  Two
+// squarings by one fused pass or two single ones, us: 607 / 797 (64 states at
+// r = 136279841), 14 / 28 (1), 25 / 47 (256 at 999961), 7 / 17 (24 at 99767),
+// 6 / 13 (16 at 4423)
+bool use_frob4(u64 r, size_t stride) {
+    return squarings_per_pass() != 1 && frob4_supported(r, stride);
 }
 
+// `chained`: the launch before this one on `st` was a pass of the same call,
+// so this one's CTAs may start (and compose their windows) while its last
+// ones drain; the kernel waits for it before it touches the states.  A pass
+// without / with, us: 8.6 / 6.8 (32 states at r = 100003), 12.7 / 10.9 (64 at
+// 999961), 27.9 / 25.5 (256), 14.8 / 13.9 (1 at 136279841).  Batches of many
+// rounds gain nothing and keep read-only loads (582 us, plain 588, 64 states).
 int launch_frob4(const u64 *in, u64 *out, size_t stride, int nstates, u64 r, const u64 *s_dev,
-                 u64 s, cudaStream_t st) {
+                 u64 s, cudaStream_t st, bool chained) {
     if (!frob4_supported(r, stride)) return invalid("launch_frob4: needs r < 2^31, even stride");
     const size_t nw = (size_t)((r + 63) >> 6);
     const size_t nu = (nw + 1) / 2;
-    // each warp takes four warp tiles (the window set each CTA composes then
-    // serves 32 tiles) when that still gives every SM 1.5 rounds of its 4
-    // resident CTAs, else as many as one round of resident CTAs leaves
+    // Warp tiles a warp (the window set each CTA composes serves 8 times as
+    // many): four when that leaves 16 rounds of the resident CTAs, three when
+    // it leaves one, else as many as one round leaves.  A pass in us by tiles
+    // a warp 1 / 2 / 3 / 4 / 6 / 8: 64 states at r = 136279841 690 / 626 / 607
+    // / 602 / 634 / 652, 3 of them 39 / 38 / 38 / 45 / 40 / 43, 16 at 30000001
+    // 45 / 44 / 43 / 48 / 48 / 51, 4 at 10001567 (0.9 rounds of one tile) 11 /
+    // 13 / 17 / 19 / 27 / 33
     const size_t twl = 32 * (size_t)LANE_UNITS;
     const size_t ntile = (nu + twl - 1) / twl;
-    const bool four = (ntile + 31) / 32 * (size_t)nstates >= (size_t)6 * sm_count();
-    const size_t round = ((size_t)MIN_CTAS * sm_count() + nstates - 1) / nstates;
-    size_t bx = four ? (ntile + 31) / 32 : std::min((ntile + 7) / 8, round);
+    const size_t slots = (size_t)MIN_CTAS * sm_count();
+    auto ctas = [&](size_t t) { return (ntile + 8 * t - 1) / (8 * t); };
+    const bool deep = ctas(4) * nstates >= 16 * slots;
+    size_t bx = deep              ? ctas(4)
+                : ctas(3) * nstates >= slots    ? ctas(3)
+                                                : std::min(ctas(1), (slots + nstates - 1) / nstates);
     if (bx > 65535) bx = 65535;
-    const dim3 grid((unsigned)bx, (unsigned)nstates);
-    k_frob4_batch<<<grid, 256, 0, st>>>(in, out, stride, r, s_dev, s);
-    GF2E_CHECK_LAUNCH("k_frob4_batch");
-    return GF2E_OK;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)bx, (unsigned)nstates);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = chained && !deep ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, cfg.numAttrs ? k_frob4_batch<false> : k_frob4_batch<true>,
+                                             in, out, stride, r, s_dev, s);
+    return e == cudaSuccess ? GF2E_OK : cuda_status(e, "k_frob4_batch");
 }
 
 int trin_square_any(const u64 *in, u64 *out, size_t stride, int nstates, u64 r,
                     const u64 *s_dev, u64 s, cudaStream_t st);
 
 // k squarings of every state (s_dev[i] for state i, s_uniform for all when
-// s_dev is null), alternating between a
-// and b, the result left in a.  Squarings go two per pass where the fused
-// kernel applies; the passes are made even in number (one fused pass turned
-// into two single ones when needed), so no copy is needed unless k = 1 or
-// only single passes apply and k is odd.
+// s_dev is null), alternating between a and b.  Squarings go two per pass
+// where the fused kernel applies.  With `where` null the result is left in a:
+// the passes are made even in number (one fused pass turned into two single
+// ones when needed), so no copy is needed unless k = 1 or only single passes
+// apply and k is odd.  Otherwise *where is the buffer that holds it.
 int frobenius_states(u64 *a, u64 *b, size_t stride, int nstates, u64 r, const u64 *s_dev,
-                     u64 k, cudaStream_t st, u64 s_uniform) {
+                     u64 k, cudaStream_t st, u64 s_uniform, u64 **where) {
     // the fused pass stores word pairs: both buffers on 16 bytes
-    const bool fused = use_frob4(r, stride, nstates) && (((uintptr_t)a | (uintptr_t)b) & 15) == 0;
+    const bool fused = use_frob4(r, stride) && (((uintptr_t)a | (uintptr_t)b) & 15) == 0;
     u64 n4 = fused ? k / 2 : 0, n1 = k - 2 * n4;
-    if (((n4 + n1) & 1) && n4 > 0) {
+    if (!where && ((n4 + n1) & 1) && n4 > 0) {
         n4--;
         n1 += 2;
     }
     u64 *x = a, *y = b;
     for (u64 i = 0; i < n4; i++) {
-        GF2E_TRY(launch_frob4(x, y, stride, nstates, r, s_dev, s_uniform, st));
+        GF2E_TRY(launch_frob4(x, y, stride, nstates, r, s_dev, s_uniform, st, i > 0));
         std::swap(x, y);
     }
     for (u64 i = 0; i < n1; i++) {
         GF2E_TRY(trin_square_any(x, y, stride, nstates, r, s_dev, s_uniform, st));
         std::swap(x, y);
     }
-    if (x != a) {
+    if (where) {
+        *where = x;
+    } else if (x != a) {
         cudaError_t e = cudaMemcpyAsync(a, x, (size_t)nstates * stride * 8,
                                         cudaMemcpyDeviceToDevice, st);
         if (e != cudaSuccess) return cuda_status(e, "frobenius copy-back");
@@ -432,5 +471,5 @@ extern "C" int gf2e_trin_squarings_per_pass(uint64_t r, size_t stride_words, int
     // passes over HBM: states and scratch of at most 96 MB stay in L2
     const size_t n = nstates < 1 ? 1 : nstates;
     if (gf2e::squarings_per_pass() != 2 && n * stride_words * 16 <= ((size_t)96 << 20)) return 1;
-    return gf2e::use_frob4(r, stride_words, (int)n) ? 2 : 1;
+    return gf2e::use_frob4(r, stride_words) ? 2 : 1;
 }

@@ -40,7 +40,7 @@ namespace gf2e {
 int trin_square_states(const u64 *in, u64 *out, size_t stride, int nstates, u64 r,
                        const u64 *s_dev, cudaStream_t st);
 int frobenius_states(u64 *a, u64 *b, size_t stride, int nstates, u64 r, const u64 *s_dev,
-                     u64 k, cudaStream_t st, u64 s_uniform);
+                     u64 k, cudaStream_t st, u64 s_uniform = 0, u64 **where = nullptr);
 int trin_set_const(u64 *states, size_t stride, int nstates, u64 r, u64 w0, cudaStream_t st);
 int trin_reduce_batch(const u64 *P, size_t pstride, size_t pw, u64 L, u64 *out, size_t ostride,
                       u64 r, const u64 *s_dev, int batch, cudaStream_t st);

@@ -16,7 +16,7 @@ int mul(const gf2e_fft_plan *plan, const u64 *a, u64 abits, const u64 *b, u64 bb
 int mul_fft_m(u64 abits, u64 bbits);
 gf2e_fft_plan *cached_plan(int m);
 int frobenius_states(u64 *a, u64 *b, size_t stride, int nstates, u64 r, const u64 *s_dev,
-                     u64 k, cudaStream_t st, u64 s_uniform);
+                     u64 k, cudaStream_t st, u64 s_uniform = 0, u64 **where = nullptr);
 }  // namespace gf2e
 
 namespace {

@@ -334,7 +334,7 @@ int launch_square(const u64 *in, u64 *out, size_t stride, int nstates, u64 r,
 
 namespace gf2e {
 int frobenius_states(u64 *a, u64 *b, size_t stride, int nstates, u64 r, const u64 *s_dev,
-                     u64 k, cudaStream_t st, u64 s_uniform = 0);
+                     u64 k, cudaStream_t st, u64 s_uniform = 0, u64 **where = nullptr);
 int trin_reduce(const u64 *P, size_t pw, u64 L, u64 *out, u64 r, u64 s, cudaStream_t st) {
     const size_t nw = (size_t)((r + 63) >> 6);
     int threads = 256;
