@@ -491,52 +491,65 @@ int gf2e_trin_frobenius_host(uint64_t r, const uint64_t *s_host, int nstates, ui
     e = cudaMemcpyAsync(sdev, s_host, (size_t)nstates * 8, cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return gf2e::cuda_status(e, "frobenius s upload");
     GF2E_TRY(gf2e::trin_set_const(states, stride, nstates, r, 2, st));
-    // Large batches go in groups, one after another on `st`, each group's
-    // readback on a copy stream while the next group squares, so only the
-    // last group's copy adds to the time.  Group sizes shrink towards the
-    // end (..., 64, 16, 4 states; the first group takes the rest): a
-    // group's readback (17 MB a state at r = 136279841) takes well under
-    // the squaring time of a group a quarter its size for any k worth
-    // batching, the large first group keeps most launches wide, and the
-    // exposed last copy is 4 states.
-    const bool split = nstates >= 8 && (size_t)nstates * nw * 8 >= ((size_t)256 << 20);
-    if (!split) {
-        GF2E_TRY(gf2e_trin_square_batch(states, scratch, stride, nstates, r, sdev, k, stream));
-        e = cudaMemcpy2DAsync(out_host, out_stride_words * 8, states, stride * 8, nw * 8,
-                              (size_t)nstates, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        return gf2e::cuda_status(e, "frobenius readback");
-    }
-    int groups[32], ngroups = 0, left = nstates;
-    for (int sz = 4; left > sz && ngroups < 31; sz *= 4) {
-        groups[ngroups++] = sz;
-        left -= sz;
-    }
-    groups[ngroups++] = left;
-    std::reverse(groups, groups + ngroups);
-    if (!W.copy_st || W.copy_dev != dev) {
-        W.release_stream();
-        e = cudaStreamCreateWithFlags(&W.copy_st, cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&W.ev_done, cudaEventDisableTiming);
-        if (e != cudaSuccess) {
+    // Batches of 48 MB and more go in groups, one after another on `st`, each
+    // group's readback on a copy stream while the next ones square.  A state's
+    // readback (PCIe) takes as long as about 70 squarings of it.  Up to k = 128
+    // (and for fewer than 16 states) neither hides all of the other, and groups
+    // are equal: a sixteenth of the
+    // batch, 32 MB at least (a pass over 17 / 34 / 51 / 119 MB takes 14 / 21 /
+    // 35 / 75 us).  For larger k sizes shrink towards the end (..., 64, 16, 4
+    // states; the first group takes the rest): the large first group keeps
+    // launches wide and a group's readback takes less than the squaring of the
+    // next, so only the last group's adds to the time.  7 states at r =
+    // 136279841, k = 65: 4.73 ms as one group, 2.95 in groups of two.
+    const size_t bytes = (size_t)nstates * nw * 8;
+    const bool split = nstates >= 2 && bytes >= ((size_t)48 << 20);
+    const size_t share = std::max((size_t)32 << 20, bytes / 16);
+    const int equal = (int)std::min((share + nw * 8 - 1) / (nw * 8), (size_t)nstates);
+    // the size of the next group when `left` states remain
+    auto group = [&](int left) {
+        if (!split) return left;
+        if (k <= 128 || nstates < 16) return std::min(equal, left);
+        for (int sz = 4; left > sz; sz *= 4) left -= sz;
+        return left;
+    };
+    cudaStream_t copy_st = st;
+    if (split) {
+        if (!W.copy_st || W.copy_dev != dev) {
             W.release_stream();
-            return gf2e::cuda_status(e, "frobenius copy stream");
+            e = cudaStreamCreateWithFlags(&W.copy_st, cudaStreamNonBlocking);
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&W.ev_done, cudaEventDisableTiming);
+            if (e != cudaSuccess) {
+                W.release_stream();
+                return gf2e::cuda_status(e, "frobenius copy stream");
+            }
+            W.copy_dev = dev;
         }
-        W.copy_dev = dev;
+        copy_st = W.copy_st;
     }
-    cudaStream_t copy_st = W.copy_st;
-    cudaEvent_t ev_done = W.ev_done;
-    for (int gi = 0, g0 = 0; gi < ngroups; g0 += groups[gi], gi++) {
-        const int ng = groups[gi];
-        GF2E_TRY(gf2e_trin_square_batch(states + stride * g0, scratch + stride * g0, stride, ng,
-                                        r, sdev + g0, k, stream));
-        e = cudaEventRecord(ev_done, st);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(copy_st, ev_done, 0);
-        if (e == cudaSuccess)
-            e = cudaMemcpy2DAsync(out_host + (size_t)g0 * out_stride_words, out_stride_words * 8,
-                                  states + stride * g0, stride * 8, nw * 8, (size_t)ng,
-                                  cudaMemcpyDeviceToHost, copy_st);
+    // a readback to pageable memory blocks this thread, so the next group's
+    // squarings are launched before it
+    u64 *done = nullptr, *next = nullptr;
+    auto square = [&](int g0, int ng) {
+        return gf2e::frobenius_states(states + stride * g0, scratch + stride * g0, stride, ng, r,
+                                      sdev + g0, k, st, 0, &next);
+    };
+    int g0 = 0, ng = group(nstates);
+    GF2E_TRY(square(0, ng));
+    while (ng > 0) {
+        const int g1 = g0 + ng, n1 = g1 < nstates ? group(nstates - g1) : 0;
+        done = next;
+        if (split) {
+            e = cudaEventRecord(W.ev_done, st);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(copy_st, W.ev_done, 0);
+            if (e != cudaSuccess) return gf2e::cuda_status(e, "frobenius group event");
+        }
+        if (n1) GF2E_TRY(square(g1, n1));
+        e = cudaMemcpy2DAsync(out_host + (size_t)g0 * out_stride_words, out_stride_words * 8, done,
+                              stride * 8, nw * 8, (size_t)ng, cudaMemcpyDeviceToHost, copy_st);
         if (e != cudaSuccess) return gf2e::cuda_status(e, "frobenius group readback");
+        g0 = g1;
+        ng = n1;
     }
     e = cudaStreamSynchronize(copy_st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
