@@ -398,23 +398,24 @@ template <int N> SL_HD void masks_of(u32 w, int sh, const u32 *pat, u32 *out) {
     }
 }
 
-// butterflies of the N planes from chunk c0: FWD: u += w v, v += u; inverse:
-// v += u, u += w v.  addmul(v, u): u += w v
-template <int N, bool FWD, class S, class Mul>
-SL_HD void bfly_planes(const S &tile, u32 su, u32 sv, u32 c0, const Mul &addmul) {
+// butterflies of the N planes from chunk c0: DIR 1 (forward): u += w v, v += u;
+// 0 (inverse): v += u, u += w v; 2: by `fwd`, all ones forward, else zero (one
+// copy of the code for both).  addmul(v, u): u += w v
+template <int N, int DIR, class S, class Mul>
+SL_HD void bfly_planes(const S &tile, u32 su, u32 sv, u32 c0, u32 fwd, const Mul &addmul) {
     u32 u[N], v[N];
     load_planes<N>(tile, sv, c0, v);
     load_planes<N>(tile, su, c0, u);
-    if (FWD) {
-        addmul(v, u);
+    if (DIR != 1) {
 #pragma unroll
-        for (int i = 0; i < N; i++) v[i] ^= u[i];
-        store_planes<N>(tile, sv, c0, v);
-    } else {
+        for (int i = 0; i < N; i++) v[i] ^= DIR ? u[i] & ~fwd : u[i];
+        if (DIR == 0) store_planes<N>(tile, sv, c0, v);
+    }
+    addmul(v, u);
+    if (DIR != 0) {
 #pragma unroll
-        for (int i = 0; i < N; i++) v[i] ^= u[i];
+        for (int i = 0; i < N; i++) v[i] ^= DIR == 2 ? u[i] & fwd : u[i];
         store_planes<N>(tile, sv, c0, v);
-        addmul(v, u);
     }
     store_planes<N>(tile, su, c0, u);
 }
@@ -422,12 +423,13 @@ SL_HD void bfly_planes(const S &tile, u32 su, u32 sv, u32 c0, const Mul &addmul)
 // the butterfly of one slice pair over `NQ` quarters (16 planes each) from
 // quarter q0; nb = m - 1 - L, the number of Cantor basis elements the level's
 // twiddles are sums of, decides the subfield
-template <int NQ, bool FWD, class S>
-SL_HD void bfly_pair(const S &tile, u32 su, u32 sv, u32 q0, int nb, u32 w, const u32 *pat) {
+template <int NQ, int DIR, class S>
+SL_HD void bfly_pair(const S &tile, u32 su, u32 sv, u32 q0, int nb, u32 w, const u32 *pat,
+                     u32 fwd) {
     if (nb == 0) {                              // W[0] = 0
 #pragma unroll 1
         for (int q = 0; q < NQ; q++)
-            bfly_planes<16, FWD>(tile, su, sv, 4 * (q0 + q), [](const u32 *, u32 *) {});
+            bfly_planes<16, DIR>(tile, su, sv, 4 * (q0 + q), fwd, [](const u32 *, u32 *) {});
     } else if (nb <= 7) {
         u32 wm[8];
         Prep<8> b;
@@ -435,7 +437,7 @@ SL_HD void bfly_pair(const S &tile, u32 su, u32 sv, u32 q0, int nb, u32 w, const
         b.set(wm);
 #pragma unroll 1
         for (int q = 0; q < NQ; q++)
-            bfly_planes<16, FWD>(tile, su, sv, 4 * (q0 + q), [&](const u32 *v, u32 *u) {
+            bfly_planes<16, DIR>(tile, su, sv, 4 * (q0 + q), fwd, [&](const u32 *v, u32 *u) {
                 t_addmul<8>(v, b, u);
                 t_addmul<8>(v + 8, b, u + 8);
             });
@@ -446,7 +448,7 @@ SL_HD void bfly_pair(const S &tile, u32 su, u32 sv, u32 q0, int nb, u32 w, const
         b.set(wm);
 #pragma unroll 1
         for (int q = 0; q < NQ; q++)
-            bfly_planes<16, FWD>(tile, su, sv, 4 * (q0 + q),
+            bfly_planes<16, DIR>(tile, su, sv, 4 * (q0 + q), fwd,
                                  [&](const u32 *v, u32 *u) { t_addmul<16>(v, b, u); });
     } else if constexpr (NQ >= 2) {             // m > 16: two quarters at a time
         // w = w0 + w1 X, w1 = b / t with b in GF(2^8), the high byte of w, as
@@ -464,7 +466,7 @@ SL_HD void bfly_pair(const S &tile, u32 su, u32 sv, u32 q0, int nb, u32 w, const
         a1.set(x);
 #pragma unroll 1
         for (int q = 0; q < NQ; q += 2)
-            bfly_planes<32, FWD>(tile, su, sv, 4 * (q0 + q), [&](const u32 *v, u32 *u) {
+            bfly_planes<32, DIR>(tile, su, sv, 4 * (q0 + q), fwd, [&](const u32 *v, u32 *u) {
                 u32 z[16], y[16], p[16];
 #pragma unroll
                 for (int i = 0; i < 16; i++) { y[i] = v[i] ^ v[16 + i]; p[i] = 0; }
@@ -493,8 +495,8 @@ SL_HD u32 tile_gslice(const Tile &T, u32 s) {
 
 // level L >= 5 of the tile (slices hold 32 consecutive elements) on its NT
 // quarters, NQ of a slice pair a thread
-template <int NT, int NQ, bool FWD, class S>
-SL_HD void level_n(const S &tile, const Tile &T, int L, u32 tid, u32 nt) {
+template <int NT, int NQ, int DIR, class S>
+SL_HD void level_n(const S &tile, const Tile &T, int L, u32 tid, u32 nt, u32 fwd = 0) {
     const int lg = L - T.llo + T.clog;
     const u32 pairs = 1u << (T.rlog + T.clog - 1);
     const int pl = T.rlog + T.clog - 1;
@@ -502,14 +504,14 @@ SL_HD void level_n(const S &tile, const Tile &T, int L, u32 tid, u32 nt) {
         const u32 g = i & (pairs - 1), q0 = (i >> pl) * NQ;
         const u32 su = ((g >> lg) << (lg + 1)) | (g & ((1u << lg) - 1)), sv = su | (1u << lg);
         const u32 t = tile_gslice(T, su) >> (L - 4);
-        bfly_pair<NQ, FWD>(tile, su, sv, q0, T.m - 1 - L, twiddle(t), nullptr);
+        bfly_pair<NQ, DIR>(tile, su, sv, q0, T.m - 1 - L, twiddle(t), nullptr, fwd);
     }
 }
 
 // level L <= 4 of a contiguous tile whose groups of 32 slices are transposed
 // (slice s of a group holds the elements 32 b + s)
-template <int NT, int NQ, bool FWD, class S>
-SL_HD void level_x(const S &tile, const Tile &T, int L, u32 tid, u32 nt) {
+template <int NT, int NQ, int DIR, class S>
+SL_HD void level_x(const S &tile, const Tile &T, int L, u32 tid, u32 nt, u32 fwd = 0) {
     const u32 pairs = 1u << (T.rlog + T.clog - 1);
     const int pl = T.rlog + T.clog - 1;
     for (u32 i = tid; i < pairs * (NT / NQ); i += nt) {
@@ -517,7 +519,7 @@ SL_HD void level_x(const S &tile, const Tile &T, int L, u32 tid, u32 nt) {
         const u32 su = ((g >> L) << (L + 1)) | (g & ((1u << L) - 1)), sv = su | (1u << L);
         const u32 G = (T.base + su) >> 5, s = su & 31;
         const u32 t = (G << (9 - L)) | (s >> (L + 1));
-        bfly_pair<NQ, FWD>(tile, su, sv, q0, T.m - 1 - L, twiddle(t), PATTAB.v[L]);
+        bfly_pair<NQ, DIR>(tile, su, sv, q0, T.m - 1 - L, twiddle(t), PATTAB.v[L], fwd);
     }
 }
 
@@ -1155,18 +1157,39 @@ SL_HD void body_slice_out(Ex ex, uint4 *sm, u32 *side, const uint4 *f, u32 nsl, 
 // the shared memory of block r; ex.block(f) and ex.cluster(f) run f(rank, tid,
 // threads) on every block, with a barrier of the block or the cluster after.
 // (One block for a whole product took 72 us at m = 12, its levels bound by
-// one SM; as separate launches 79 us at m = 13.)
+// one SM; as separate launches 79 us at m = 13.)  Each line of code runs a few
+// times a block, and fetching it takes longer than running it (half of the
+// stalls), so both directions of the levels share one copy, as the three
+// products of a slice do, and the map back from tower planes is by table: @@
 struct Operand { const u32 *src; u64 nchunks; u32 xor0; int k; };
 struct RowAddr {                 // word j of plane p of slices PITCH words apart
     static constexpr bool rows_first = false;
     int plog, pitch;
     SL_HD u32 operator()(u32 j, u32 p) const { return j * pitch + p; }
 };
-// 16-byte chunks a block: 32 planes, 16 planes, 2^(m-8) + 1 words
+// the map from tower planes by the 16 nibbles of a coefficient (entry v of
+// nibble k at 16 k + v: the 16 entries fill the 32 banks once)
+struct FromTable { u64 v[256]; };
+constexpr FromTable make_from_table() {
+    FromTable t{};
+    for (int k = 0; k < 16; k++)
+        for (int v = 0; v < 16; v++) {
+            u64 x = 0;
+            for (int b = 0; b < 4; b++)
+                if (v >> b & 1) x ^= PHI.from[4 * k + b];
+            t.v[16 * k + v] = x;
+        }
+    return t;
+}
+#ifdef __CUDACC__
+__device__
+#endif
+static const FromTable FROM4 = make_from_table();
+// 16-byte chunks a block: 32 planes, 16 planes
 #ifdef __CUDACC__
 __host__
 #endif
-SL_HD constexpr u32 small_chunks(int m) { return (14u << (m - 5)) + 20; }
+SL_HD constexpr u32 small_chunks(int m) { return 14u << (m - 5); }
 template <bool FWD, class At> SL_HD void taylor_warp_k(u32 *sm, const At &at, int k, u32 p) {
     switch (k) {
     case 10: taylor_warp<10, FWD>(sm, at, p); break;
@@ -1182,7 +1205,10 @@ SL_HD void body_small(Ex ex, int m, const Operand &A, const Operand &B, u32 *out
     const Tile T{m, m - 5, 0, 5, 0};
     const auto half = [&](u32 r) { return Half{ex.mem(r)}; };
     const auto quarter = [&](u32 r) { return Quarter{ex.mem(r) + 9 * ns}; };
-    const auto side = [&](u32 r) { return reinterpret_cast<u32 *>(ex.mem(r) + 14 * ns); };
+    // in the space of the 32 planes, once those are used: the middle products,
+    // later the words of nb + 1 slices, and the table at its end
+    const auto words_of = [&](u32 r) { return Full{ex.mem(r)}; };
+    const auto table = [&](u32 r) { return reinterpret_cast<u64 *>(ex.mem(r) + 9 * ns - 128); };
     const auto op = [&](u32 r) -> const Operand & { return r < 4 ? A : B; };
     const RowAddr at_half{5, 36}, at_quarter{4, 20};
     // chunk words, their planes, the conversion (all 32 planes in every block)
@@ -1215,64 +1241,60 @@ SL_HD void body_small(Ex ex, int m, const Operand &A, const Operand &B, u32 *out
             phi_quarter(quarter(r), i, r & 3, a);
         }
     });
-    for (int L = m - 1; L >= 5; L--)
-        ex.block([&](u32 r, u32 tid, u32 nt) {
-            if (L < op(r).k) level_n<1, 1, true>(quarter(r), T, L, tid, nt);
-        });
-    ex.block([&](u32 r, u32 tid, u32 nt) { transpose_groups<1>(quarter(r), ns, tid, nt); });
-    for (int L = 4; L >= 1; L--)
-        ex.block([&](u32 r, u32 tid, u32 nt) { level_x<1, 1, true>(quarter(r), T, L, tid, nt); });
-    ex.cluster([&](u32 r, u32 tid, u32 nt) { level_x<1, 1, true>(quarter(r), T, 0, tid, nt); });
-    // products of slices r nb .. r nb + nb - 1: the middle half product, then
-    // the two it joins
-    ex.block([&](u32 r, u32 tid, u32 nt) {
-        for (u32 i = tid; i < nb; i += nt) {
-            const u32 s = r * nb + i;
-            u32 a[32], b[32], c[32];
+#pragma unroll 1
+    for (int pass = 0; pass < 2; pass++) {       // forward, inverse
+        // levels m - 1 .. 5, the transposition, levels 4 .. 0, or back
+#pragma unroll 1
+        for (int i = 0; i <= m; i++)
+            ex.block([&](u32 r, u32 tid, u32 nt) {
+                const int j = pass ? m - i : i, L = j < m - 5 ? m - 1 - j : m - j;
+                const u32 fwd = pass ? 0u : ~0u;
+                if (pass ? r >= 4 : j < m - 5 && L >= op(r).k) return;
+                if (j < m - 5) level_n<1, 1, 2>(quarter(r), T, L, tid, nt, fwd);
+                else if (j > m - 5) level_x<1, 1, 2>(quarter(r), T, L, tid, nt, fwd);
+                else transpose_groups<1>(quarter(r), ns, tid, nt);
+            });
+        if (pass) break;
+        ex.cluster([](u32, u32, u32) {});
+        // products of slices r nb .. r nb + nb - 1: the middle half product,
+        // then the two it joins
+#pragma unroll 1
+        for (u32 join = 0; join < 2; join++)
+            ex.block([&](u32 r, u32 tid, u32 nt) {
+                if (!join)
+                    for (u32 i = tid; i < 256; i += nt) table(r)[i] = FROM4.v[i];
+                for (u32 i = tid; i < (nb << join); i += nt) {
+                    const u32 h = i >= nb ? 1 : 0, j = i - h * nb, s = r * nb + j;
+                    u32 a[32], b[32], c[32];
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                load_planes<16>(quarter(h), s, 0, a + 16 * h);
-                load_planes<16>(quarter(2 + h), s, 0, b + 16 * h);
-            }
+                    for (int k = 0; k < 2; k++) load_planes<16>(quarter(6 + k), s, 0, a + 16 * k);
+                    t_mulx<32>(a, c);
 #pragma unroll
-            for (int k = 0; k < 32; k++) { a[k] ^= b[k]; c[k] = 0; }
+                    for (int k = 0; k < 2; k++) load_planes<16>(quarter(4 + k), s, 0, b + 16 * k);
 #pragma unroll
-            for (int h = 0; h < 2; h++) load_planes<16>(quarter(6 + h), s, 0, b + 16 * h);
-            t_addmul_once<32>(a, b, c);
-            store_planes<32>(half(r), i, 0, c);
-        }
-    });
-    ex.cluster([&](u32 r, u32 tid, u32 nt) {
-        for (u32 i = tid; i < 2 * nb; i += nt) {
-            const u32 h = i >= nb ? 1 : 0, j = i - h * nb, s = r * nb + j, both = 0u - h;
-            u32 a[32], b[32], c[32];
+                    for (int k = 0; k < 32; k++)
+                        b[k] = a[k] ^ (b[k] & (0u - join)) ^ (c[k] & (0u - h));
 #pragma unroll
-            for (int k = 0; k < 2; k++) {
-                load_planes<16>(quarter(6 + k), s, 0, a + 16 * k);
-                load_planes<16>(quarter(4 + k), s, 0, b + 16 * k);
-            }
-            t_mulx<32>(a, c);
+                    for (int k = 0; k < 2; k++) load_planes<16>(quarter(2 * h + k), s, 0, a + 16 * k);
+                    if (join) {
+                        load_planes<32>(half(r), j, 0, c);
+                    } else {
 #pragma unroll
-            for (int k = 0; k < 32; k++) b[k] ^= a[k] ^ (c[k] & both);
+                        for (int k = 0; k < 2; k++) load_planes<16>(quarter(2 + k), s, 0, c + 16 * k);
 #pragma unroll
-            for (int k = 0; k < 2; k++) load_planes<16>(quarter(2 * h + k), s, 0, a + 16 * k);
-            load_planes<32>(half(r), j, 0, c);
-            t_addmul_once<32>(a, b, c);
+                        for (int k = 0; k < 32; k++) { a[k] ^= c[k]; c[k] = 0; }
+                    }
+                    t_addmul_once<32>(a, b, c);
+                    if (join) {
 #pragma unroll
-            for (int k = 0; k < 2; k++) store_planes<16>(quarter(2 * h + k), s, 0, c + 16 * k);
-        }
-    });
-    for (int L = 0; L <= 4; L++)
-        ex.block([&](u32 r, u32 tid, u32 nt) {
-            if (r < 4) level_x<1, 1, false>(quarter(r), T, L, tid, nt);
-        });
-    ex.block([&](u32 r, u32 tid, u32 nt) {
-        if (r < 4) transpose_groups<1>(quarter(r), ns, tid, nt);
-    });
-    for (int L = 5; L < m; L++)
-        ex.block([&](u32 r, u32 tid, u32 nt) {
-            if (r < 4) level_n<1, 1, false>(quarter(r), T, L, tid, nt);
-        });
+                        for (int k = 0; k < 2; k++) store_planes<16>(quarter(2 * h + k), s, 0, c + 16 * k);
+                    } else {
+                        store_planes<32>(half(r), j, 0, c);
+                    }
+                }
+            });
+        ex.cluster([](u32, u32, u32) {});
+    }
     ex.block([&](u32 r, u32 tid, u32 nt) {
         if (r < 4) taylor_regs<false>(&quarter(r).word(0, 0), at_quarter, m, tid, nt);
     });
@@ -1282,33 +1304,44 @@ SL_HD void body_small(Ex ex, int m, const Operand &A, const Operand &B, u32 *out
                 taylor_warp_k<false>(&quarter(r).word(0, 0), at_quarter, m, p);
     });
     ex.cluster([](u32, u32, u32) {});
-    // words of slices r nb .. (and the last high half of the slice before)
+    // words of slices r nb .. and of the one before them: coefficients of 64
+    // tower bits, the map, and the overlap-add of their halves
     ex.cluster([&](u32 r, u32 tid, u32 nt) {
-        for (u32 i = tid; i <= nb; i += nt) {
-            const u32 s = r * nb + i - 1;
-            u32 a[64], b[64];
-            if (s >= ns) {                       // before slice 0
-                side(r)[0] = 0;
-                continue;
+        for (u32 i = tid; i < 2 * (nb + 1); i += nt) {
+            const u32 h = i & 1, j = i >> 1, s = r * nb + j - 1;
+            u32 a[32];
+#pragma unroll
+            for (int k = 0; k < 32; k++) a[k] = 0;
+            if (s < ns) {                        // else before slice 0
+#pragma unroll
+                for (int k = 0; k < 2; k++) load_planes<16>(quarter(2 * h + k), s, 0, a + 16 * k);
+                transpose32(a);
             }
-#pragma unroll
-            for (int q = 0; q < 4; q++) load_planes<16>(quarter(q), s, 0, a + 16 * q);
-            lin_map<64, 64, false>(a, b);
-            transpose32(b);
-            transpose32(b + 32);
-#pragma unroll
-            for (int e = 31; e > 0; e--) b[e] ^= b[31 + e];
-            if (i) store_planes<32>(half(r), i - 1, 0, b);
-            side(r)[i] = b[63];
+            store_planes<32>(words_of(r), j, 8 * h, a);
         }
     });
     ex.block([&](u32 r, u32 tid, u32 nt) {
+        const Full w = words_of(r);
+        const u64 *t = table(r);
+        for (u32 i = tid; i < 32 * (nb + 1); i += nt) {
+            u32 &lo = w.word(i >> 5, i & 31), &hi = w.word(i >> 5, 32 + (i & 31));
+            u64 x = 0;
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+                x ^= t[16 * k + (lo >> (4 * k) & 15)] ^ t[128 + 16 * k + (hi >> (4 * k) & 15)];
+            lo = (u32)x;
+            hi = (u32)(x >> 32);
+        }
+    });
+    ex.block([&](u32 r, u32 tid, u32 nt) {
+        const Full w = words_of(r);
         const u64 k0 = (u64)r * nb * 32;
         for (u32 i = tid; i < 32 * nb; i += nt)
-            if (k0 + i < words) out[k0 + i] = half(r).word(i >> 5, i & 31) ^ ((i & 31) ? 0 : side(r)[i >> 5]);
+            if (k0 + i < words)
+                out[k0 + i] = w.word((i + 32) >> 5, i & 31) ^ w.word((i + 31) >> 5, 32 + ((i + 31) & 31));
         if (r == 7)
             for (u64 k = (u64)ns * 32 + tid; k < words; k += nt)
-                out[k] = k == (u64)ns * 32 ? side(r)[nb] : 0;
+                out[k] = k == (u64)ns * 32 ? w.word(nb, 63) : 0;
     });
 }
 
