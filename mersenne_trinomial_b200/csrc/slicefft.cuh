@@ -426,11 +426,11 @@ SL_HD void bfly_planes(const S &tile, u32 su, u32 sv, u32 c0, u32 fwd, const Mul
 template <int NQ, int DIR, class S>
 SL_HD void bfly_pair(const S &tile, u32 su, u32 sv, u32 q0, int nb, u32 w, const u32 *pat,
                      u32 fwd) {
-    if (nb == 0) {                              // W[0] = 0
+    if (DIR != 2 && nb == 0) {                  // W[0] = 0
 #pragma unroll 1
         for (int q = 0; q < NQ; q++)
             bfly_planes<16, DIR>(tile, su, sv, 4 * (q0 + q), fwd, [](const u32 *, u32 *) {});
-    } else if (nb <= 7) {
+    } else if (DIR != 2 && nb <= 7) {
         u32 wm[8];
         Prep<8> b;
         masks_of<8>(w, 0, pat, wm);
@@ -493,6 +493,17 @@ SL_HD u32 tile_gslice(const Tile &T, u32 s) {
     return T.base + ((s >> T.clog) << (T.llo - 5)) + (s & ((1u << T.clog) - 1));
 }
 
+// the same for twiddles in GF(2^8) and 8 planes from chunk c0
+template <int DIR, class S>
+SL_HD void bfly_pair8(const S &tile, u32 su, u32 sv, u32 c0, u32 w, const u32 *pat, u32 fwd) {
+    u32 wm[8];
+    Prep<8> b;
+    masks_of<8>(w, 0, pat, wm);
+    b.set(wm);
+    bfly_planes<8, DIR>(tile, su, sv, c0, fwd,
+                        [&](const u32 *v, u32 *u) { t_addmul<8>(v, b, u); });
+}
+
 // level L >= 5 of the tile (slices hold 32 consecutive elements) on its NT
 // quarters, NQ of a slice pair a thread
 template <int NT, int NQ, int DIR, class S>
@@ -500,6 +511,15 @@ SL_HD void level_n(const S &tile, const Tile &T, int L, u32 tid, u32 nt, u32 fwd
     const int lg = L - T.llo + T.clog;
     const u32 pairs = 1u << (T.rlog + T.clog - 1);
     const int pl = T.rlog + T.clog - 1;
+    if (DIR == 2 && T.m - 1 - L <= 7) {          // few slices: 8 planes a thread
+        for (u32 i = tid; i < 2 * NT * pairs; i += nt) {
+            const u32 g = i & (pairs - 1);
+            const u32 su = ((g >> lg) << (lg + 1)) | (g & ((1u << lg) - 1));
+            bfly_pair8<DIR>(tile, su, su | (1u << lg), 2 * (i >> pl),
+                            twiddle(tile_gslice(T, su) >> (L - 4)), nullptr, fwd);
+        }
+        return;
+    }
     for (u32 i = tid; i < pairs * (NT / NQ); i += nt) {
         const u32 g = i & (pairs - 1), q0 = (i >> pl) * NQ;
         const u32 su = ((g >> lg) << (lg + 1)) | (g & ((1u << lg) - 1)), sv = su | (1u << lg);
@@ -514,11 +534,23 @@ template <int NT, int NQ, int DIR, class S>
 SL_HD void level_x(const S &tile, const Tile &T, int L, u32 tid, u32 nt, u32 fwd = 0) {
     const u32 pairs = 1u << (T.rlog + T.clog - 1);
     const int pl = T.rlog + T.clog - 1;
-    for (u32 i = tid; i < pairs * (NT / NQ); i += nt) {
-        const u32 g = i & (pairs - 1), q0 = (i >> pl) * NQ;
-        const u32 su = ((g >> L) << (L + 1)) | (g & ((1u << L) - 1)), sv = su | (1u << L);
+    const auto pair_of = [&](u32 g, u32 &su, u32 &t) {
+        su = ((g >> L) << (L + 1)) | (g & ((1u << L) - 1));
         const u32 G = (T.base + su) >> 5, s = su & 31;
-        const u32 t = (G << (9 - L)) | (s >> (L + 1));
+        t = (G << (9 - L)) | (s >> (L + 1));
+    };
+    u32 su, t;
+    if (DIR == 2 && T.m - 1 - L <= 7) {
+        for (u32 i = tid; i < 2 * NT * pairs; i += nt) {
+            pair_of(i & (pairs - 1), su, t);
+            bfly_pair8<DIR>(tile, su, su | (1u << L), 2 * (i >> pl), twiddle(t), PATTAB.v[L], fwd);
+        }
+        return;
+    }
+    for (u32 i = tid; i < pairs * (NT / NQ); i += nt) {
+        const u32 q0 = (i >> pl) * NQ;
+        pair_of(i & (pairs - 1), su, t);
+        const u32 sv = su | (1u << L);
         bfly_pair<NQ, DIR>(tile, su, sv, q0, T.m - 1 - L, twiddle(t), PATTAB.v[L], fwd);
     }
 }
@@ -1158,9 +1190,12 @@ SL_HD void body_slice_out(Ex ex, uint4 *sm, u32 *side, const uint4 *f, u32 nsl, 
 // threads) on every block, with a barrier of the block or the cluster after.
 // (One block for a whole product took 72 us at m = 12, its levels bound by
 // one SM; as separate launches 79 us at m = 13.)  Each line of code runs a few
-// times a block, and fetching it takes longer than running it (half of the
-// stalls), so both directions of the levels share one copy, as the three
-// products of a slice do, and the map back from tower planes is by table: @@
+// times a block, and on a cold start half of the stalls are instruction
+// fetches, so both directions of the levels share one copy, as the three
+// products of a slice do, and the map back from tower planes is by table
+// (70001 x 51203 bits: 43.0 to 38.9 us).  The four blocks of an operand convert
+// 8 of its 32 planes each, and the three half products of a slice run side by
+// side (38.9 to 34.8 us).
 struct Operand { const u32 *src; u64 nchunks; u32 xor0; int k; };
 struct RowAddr {                 // word j of plane p of slices PITCH words apart
     static constexpr bool rows_first = false;
@@ -1210,13 +1245,15 @@ SL_HD void body_small(Ex ex, int m, const Operand &A, const Operand &B, u32 *out
     const auto words_of = [&](u32 r) { return Full{ex.mem(r)}; };
     const auto table = [&](u32 r) { return reinterpret_cast<u64 *>(ex.mem(r) + 9 * ns - 128); };
     const auto op = [&](u32 r) -> const Operand & { return r < 4 ? A : B; };
-    const RowAddr at_half{5, 36}, at_quarter{4, 20};
-    // chunk words, their planes, the conversion (all 32 planes in every block)
+    const RowAddr at_half{3, 36}, at_quarter{4, 20};
+    // chunk words, their planes, the conversion of 8 planes a block
     ex.block([&](u32 r, u32 tid, u32 nt) {
         const Operand &o = op(r);
         const Half h = half(r);
-        for (u32 i = tid; i < (1u << o.k); i += nt)
-            h.word(i >> 5, i & 31) = (i < o.nchunks ? o.src[i] : 0) ^ (i == 0 ? o.xor0 : 0);
+        staged<16, u32>(
+            1u << o.k, tid, nt,
+            [&](u32 i) { return (i < o.nchunks ? o.src[i] : 0) ^ (i == 0 ? o.xor0 : 0); },
+            [&](u32 i, u32 v) { h.word(i >> 5, i & 31) = v; });
     });
     ex.block([&](u32 r, u32 tid, u32 nt) {
         const Half h = half(r);
@@ -1228,16 +1265,20 @@ SL_HD void body_small(Ex ex, int m, const Operand &A, const Operand &B, u32 *out
         }
     });
     ex.warps([&](u32 r, u32 w, u32 nw) {
-        for (u32 p = w; p < 32; p += nw) taylor_warp_k<true>(&half(r).word(0, 0), at_half, op(r).k, p);
+        for (u32 p = w; p < 8; p += nw)
+            taylor_warp_k<true>(&half(r).word(0, 8 * (r & 3)), at_half, op(r).k, p);
     });
     ex.block([&](u32 r, u32 tid, u32 nt) {
-        taylor_regs<true>(&half(r).word(0, 0), at_half, op(r).k, tid, nt);
+        taylor_regs<true>(&half(r).word(0, 8 * (r & 3)), at_half, op(r).k, tid, nt);
     });
+    ex.cluster([](u32, u32, u32) {});
     // tower planes of the quarter, copies included
     ex.block([&](u32 r, u32 tid, u32 nt) {
         for (u32 i = tid; i < ns; i += nt) {
             u32 a[32];
-            load_planes<32>(half(r), i & ((1u << (op(r).k - 5)) - 1), 0, a);
+#pragma unroll
+            for (u32 b = 0; b < 4; b++)
+                load_planes<8>(half((r & 4) + b), i & ((1u << (op(r).k - 5)) - 1), 2 * b, a + 8 * b);
             phi_quarter(quarter(r), i, r & 3, a);
         }
     });
@@ -1256,43 +1297,41 @@ SL_HD void body_small(Ex ex, int m, const Operand &A, const Operand &B, u32 *out
             });
         if (pass) break;
         ex.cluster([](u32, u32, u32) {});
-        // products of slices r nb .. r nb + nb - 1: the middle half product,
-        // then the two it joins
-#pragma unroll 1
-        for (u32 join = 0; join < 2; join++)
-            ex.block([&](u32 r, u32 tid, u32 nt) {
-                if (!join)
-                    for (u32 i = tid; i < 256; i += nt) table(r)[i] = FROM4.v[i];
-                for (u32 i = tid; i < (nb << join); i += nt) {
-                    const u32 h = i >= nb ? 1 : 0, j = i - h * nb, s = r * nb + j;
-                    u32 a[32], b[32], c[32];
+        // products of slices r nb .. r nb + nb - 1: (a0 + a1) b1, a0 (b0 + b1)
+        // and a1 (b0 + b1 + X b1), then the first added to the other two
+        ex.block([&](u32 r, u32 tid, u32 nt) {
+            for (u32 i = tid; i < 256; i += nt) table(r)[i] = FROM4.v[i];
+            for (u32 i = tid; i < 3 * nb; i += nt) {
+                const u32 join = i >= nb ? 1 : 0, h = i >= 2 * nb ? 1 : 0;
+                const u32 s = r * nb + i - (join + h) * nb;
+                u32 a[32], b[32], c[32];
 #pragma unroll
-                    for (int k = 0; k < 2; k++) load_planes<16>(quarter(6 + k), s, 0, a + 16 * k);
-                    t_mulx<32>(a, c);
+                for (int k = 0; k < 2; k++) load_planes<16>(quarter(6 + k), s, 0, a + 16 * k);
+                t_mulx<32>(a, c);
 #pragma unroll
-                    for (int k = 0; k < 2; k++) load_planes<16>(quarter(4 + k), s, 0, b + 16 * k);
+                for (int k = 0; k < 2; k++) load_planes<16>(quarter(4 + k), s, 0, b + 16 * k);
 #pragma unroll
-                    for (int k = 0; k < 32; k++)
-                        b[k] = a[k] ^ (b[k] & (0u - join)) ^ (c[k] & (0u - h));
+                for (int k = 0; k < 32; k++)
+                    b[k] = a[k] ^ (b[k] & (0u - join)) ^ (c[k] & (0u - h));
 #pragma unroll
-                    for (int k = 0; k < 2; k++) load_planes<16>(quarter(2 * h + k), s, 0, a + 16 * k);
-                    if (join) {
-                        load_planes<32>(half(r), j, 0, c);
-                    } else {
+                for (int k = 0; k < 2; k++) load_planes<16>(quarter(2 * h + k), s, 0, a + 16 * k);
 #pragma unroll
-                        for (int k = 0; k < 2; k++) load_planes<16>(quarter(2 + k), s, 0, c + 16 * k);
+                for (int k = 0; k < 2; k++) load_planes<16>(quarter(2 + k), s, 0, c + 16 * k);
 #pragma unroll
-                        for (int k = 0; k < 32; k++) { a[k] ^= c[k]; c[k] = 0; }
-                    }
-                    t_addmul_once<32>(a, b, c);
-                    if (join) {
-#pragma unroll
-                        for (int k = 0; k < 2; k++) store_planes<16>(quarter(2 * h + k), s, 0, c + 16 * k);
-                    } else {
-                        store_planes<32>(half(r), j, 0, c);
-                    }
-                }
-            });
+                for (int k = 0; k < 32; k++) { a[k] ^= c[k] & (join - 1u); c[k] = 0; }
+                t_addmul_once<32>(a, b, c);
+                store_planes<32>(half(r), i, 0, c);
+            }
+        });
+        ex.block([&](u32 r, u32 tid, u32 nt) {
+            for (u32 i = tid; i < 16 * nb; i += nt) {
+                const u32 h = (i >> 3) & 1, j = i >> 4, c = i & 7;
+                uint4 x = half(r).chunk(j, c);
+                const uint4 y = half(r).chunk((1 + h) * nb + j, c);
+                x.x ^= y.x; x.y ^= y.y; x.z ^= y.z; x.w ^= y.w;
+                quarter(2 * h + (c >> 2)).chunk(r * nb + j, c & 3) = x;
+            }
+        });
         ex.cluster([](u32, u32, u32) {});
     }
     ex.block([&](u32 r, u32 tid, u32 nt) {
