@@ -1195,7 +1195,9 @@ SL_HD void body_slice_out(Ex ex, uint4 *sm, u32 *side, const uint4 *f, u32 nsl, 
 // products of a slice do, and the map back from tower planes is by table
 // (70001 x 51203 bits: 43.0 to 38.9 us).  The four blocks of an operand convert
 // 8 of its 32 planes each, and the three half products of a slice run side by
-// side (38.9 to 34.8 us).
+// side (38.9 to 34.8 us).  What a block needs of the others is copied first,
+// from another block each, instead of read where it is used by all from one (a
+// product of 200001 x 200000 bits: 143 K cycles to 121 K).
 struct Operand { const u32 *src; u64 nchunks; u32 xor0; int k; };
 struct RowAddr {                 // word j of plane p of slices PITCH words apart
     static constexpr bool rows_first = false;
@@ -1248,11 +1250,12 @@ SL_HD void body_small(Ex ex, int m, const Operand &A, const Operand &B, u32 *out
     const RowAddr at_half{3, 36}, at_quarter{4, 20};
     // chunk words, their planes, the conversion of 8 planes a block
     ex.block([&](u32 r, u32 tid, u32 nt) {
-        const Operand &o = op(r);
+        const u32 *src = op(r).src;
+        const u32 nch = (u32)op(r).nchunks, xor0 = op(r).xor0;
         const Half h = half(r);
         staged<16, u32>(
-            1u << o.k, tid, nt,
-            [&](u32 i) { return (i < o.nchunks ? o.src[i] : 0) ^ (i == 0 ? o.xor0 : 0); },
+            1u << op(r).k, tid, nt,
+            [&](u32 i) { return (i < nch ? src[i] : 0) ^ (i == 0 ? xor0 : 0); },
             [&](u32 i, u32 v) { h.word(i >> 5, i & 31) = v; });
     });
     ex.block([&](u32 r, u32 tid, u32 nt) {
@@ -1272,13 +1275,27 @@ SL_HD void body_small(Ex ex, int m, const Operand &A, const Operand &B, u32 *out
         taylor_regs<true>(&half(r).word(0, 8 * (r & 3)), at_half, op(r).k, tid, nt);
     });
     ex.cluster([](u32, u32, u32) {});
+    // the planes of the other three blocks, each block beginning with another
+    // one's (all reading one block's at a time took 11 K cycles at m = 14)
+    ex.block([&](u32 r, u32 tid, u32 nt) {
+        const int kl = op(r).k - 4;
+        const auto from = [&](u32 i) { return (r + 1 + (i >> kl)) & 3; };
+        staged<8, uint4>(
+            3u << kl, tid, nt,
+            [&](u32 i) {
+                const u32 j = (i & ((1u << kl) - 1)) >> 1;
+                return half((r & 4) + from(i)).chunk(j, 2 * from(i) + (i & 1));
+            },
+            [&](u32 i, const uint4 &q) {
+                const u32 j = (i & ((1u << kl) - 1)) >> 1;
+                half(r).chunk(j, 2 * from(i) + (i & 1)) = q;
+            });
+    });
     // tower planes of the quarter, copies included
     ex.block([&](u32 r, u32 tid, u32 nt) {
         for (u32 i = tid; i < ns; i += nt) {
             u32 a[32];
-#pragma unroll
-            for (u32 b = 0; b < 4; b++)
-                load_planes<8>(half((r & 4) + b), i & ((1u << (op(r).k - 5)) - 1), 2 * b, a + 8 * b);
+            load_planes<32>(half(r), i & ((1u << (op(r).k - 5)) - 1), 0, a);
             phi_quarter(quarter(r), i, r & 3, a);
         }
     });
@@ -1297,26 +1314,40 @@ SL_HD void body_small(Ex ex, int m, const Operand &A, const Operand &B, u32 *out
             });
         if (pass) break;
         ex.cluster([](u32, u32, u32) {});
-        // products of slices r nb .. r nb + nb - 1: (a0 + a1) b1, a0 (b0 + b1)
-        // and a1 (b0 + b1 + X b1), then the first added to the other two
+        // slices r nb .. r nb + nb - 1 of all quarters, after the space of 3 nb
+        // products, each block beginning with another quarter
+        const auto own = [&](u32 r, u32 q) { return Quarter{ex.mem(r) + (27 + 5 * q) * nb}; };
+        const u32 nbl = (u32)(m - 8);
         ex.block([&](u32 r, u32 tid, u32 nt) {
-            for (u32 i = tid; i < 256; i += nt) table(r)[i] = FROM4.v[i];
+            staged<8, uint4>(
+                32 * nb, tid, nt,
+                [&](u32 i) {
+                    return quarter((r + (i >> (nbl + 2))) & 7)
+                        .chunk(r * nb + ((i >> 2) & (nb - 1)), i & 3);
+                },
+                [&](u32 i, const uint4 &q) {
+                    own(r, (r + (i >> (nbl + 2))) & 7).chunk((i >> 2) & (nb - 1), i & 3) = q;
+                });
+        });
+        // their products (a0 + a1) b1, a0 (b0 + b1) and a1 (b0 + b1 + X b1),
+        // then the first added to the other two
+        ex.block([&](u32 r, u32 tid, u32 nt) {
             for (u32 i = tid; i < 3 * nb; i += nt) {
                 const u32 join = i >= nb ? 1 : 0, h = i >= 2 * nb ? 1 : 0;
-                const u32 s = r * nb + i - (join + h) * nb;
+                const u32 s = i - (join + h) * nb;
                 u32 a[32], b[32], c[32];
 #pragma unroll
-                for (int k = 0; k < 2; k++) load_planes<16>(quarter(6 + k), s, 0, a + 16 * k);
+                for (int k = 0; k < 2; k++) load_planes<16>(own(r, 6 + k), s, 0, a + 16 * k);
                 t_mulx<32>(a, c);
 #pragma unroll
-                for (int k = 0; k < 2; k++) load_planes<16>(quarter(4 + k), s, 0, b + 16 * k);
+                for (int k = 0; k < 2; k++) load_planes<16>(own(r, 4 + k), s, 0, b + 16 * k);
 #pragma unroll
                 for (int k = 0; k < 32; k++)
                     b[k] = a[k] ^ (b[k] & (0u - join)) ^ (c[k] & (0u - h));
 #pragma unroll
-                for (int k = 0; k < 2; k++) load_planes<16>(quarter(2 * h + k), s, 0, a + 16 * k);
+                for (int k = 0; k < 2; k++) load_planes<16>(own(r, 2 * h + k), s, 0, a + 16 * k);
 #pragma unroll
-                for (int k = 0; k < 2; k++) load_planes<16>(quarter(2 + k), s, 0, c + 16 * k);
+                for (int k = 0; k < 2; k++) load_planes<16>(own(r, 2 + k), s, 0, c + 16 * k);
 #pragma unroll
                 for (int k = 0; k < 32; k++) { a[k] ^= c[k] & (join - 1u); c[k] = 0; }
                 t_addmul_once<32>(a, b, c);
@@ -1324,6 +1355,7 @@ SL_HD void body_small(Ex ex, int m, const Operand &A, const Operand &B, u32 *out
             }
         });
         ex.block([&](u32 r, u32 tid, u32 nt) {
+            for (u32 i = tid; i < 256; i += nt) table(r)[i] = FROM4.v[i];
             for (u32 i = tid; i < 16 * nb; i += nt) {
                 const u32 h = (i >> 3) & 1, j = i >> 4, c = i & 7;
                 uint4 x = half(r).chunk(j, c);
