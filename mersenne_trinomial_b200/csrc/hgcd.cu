@@ -56,10 +56,6 @@
 namespace gf2e {
 int mul_fft_m(u64 abits, u64 bbits);
 gf2e_fft_plan *cached_plan(int m);
-int fft_fwd_packed(const gf2e_fft_plan *plan, u64 *f, const u32 *src32, u64 nchunks,
-                   cudaStream_t st);
-int fft_run(const gf2e_fft_plan *plan, bool forward, u64 *f, cudaStream_t st);
-int overlap_add(const u64 *F, u64 nchunks, u64 *out, u64 ow, cudaStream_t st);
 int fft_fwd_packed_batch(const gf2e_fft_plan *plan, u64 *f, u64 fstride, const u32 *src32,
                          u64 sstride32, u64 nchunks, u64 xor0, int batch, cudaStream_t st);
 int fft_run_batch(const gf2e_fft_plan *plan, bool forward, u64 *f, u64 fstride, int batch,

@@ -33,17 +33,18 @@
 //               L2-resident up to d = 23: 2 x 32 MB, 2 x 8 GB at d = 31).
 //   k_classes   one thread per j: coset/subfield filters, Zech lookup,
 //               progression; the minimal polynomial only for classes that
-//               mark some s <= smax, by GF(2) elimination on the powers
-//               beta^0..beta^d (O(d^2) word ops instead of O(d^2) field
-//               multiplies; the minimal polynomial is unique so the mask is
-//               identical).  Progressions are routed by length:
+//               mark some s <= smax, by Berlekamp-Massey on one bit of
+//               the powers beta^0..beta^(2d-1) (the minimal polynomial is
+//               unique, so the mask is identical).  Progressions are routed by length:
 //                 n < strip width    -> strip list (applied in shared memory)
 //                 <= INLINE marks    -> marked at once with atomicMin
 //                 otherwise          -> heavy list (grid-stride atomicMin)
-//   k_heavy     all heavy progressions of all degrees, one launch.
+//   k_heavy     all heavy progressions of all degrees, in windows of best[]
+//               that stay in L2.
 //   k_strip     each CTA owns a strip-wide slice of best[], applies every
-//               short-period progression with shared-memory atomics and
-//               writes the slice back once (last writer, so plain min).
+//               short-period progression with shared-memory minima of the
+//               progressions' 32-bit ranks (k_rank) and writes the slice back
+//               once (last writer, so plain min).
 // All degrees are enqueued on one stream with no host round trip; the only
 // synchronisation is the final overflow/status read.  A progression that
 // finds the strip or heavy list full is marked inline by its class thread

@@ -1,6 +1,5 @@
-"""Fused squaring passes (csrc/frobenius.cu) below the L2 size: batches at both
-sides of the 2^15-word rule, and states on 8 bytes only, which keep the
-one-squaring kernel, against the oracle."""
+"""Fused squaring passes (csrc/frobenius.cu) below the L2 size, and states on 8
+bytes only, which keep the one-squaring kernel, against the oracle."""
 import numpy as np
 import pytest
 
@@ -9,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("shift", [0, 8])
 @pytest.mark.parametrize("r,n", [(30011, 64), (30011, 70), (99767, 24), (999961, 3), (2100001, 1)])
-def test_batches_around_the_rule(engine, oracle, r, n, shift):
+def test_small_batches(engine, oracle, r, n, shift):
     rng = np.random.default_rng(r + n)
     nw = (r + 63) // 64
     stride = nw + (nw & 1)
