@@ -1197,7 +1197,8 @@ SL_HD void body_slice_out(Ex ex, uint4 *sm, u32 *side, const uint4 *f, u32 nsl, 
 // 8 of its 32 planes each, and the three half products of a slice run side by
 // side (38.9 to 34.8 us).  What a block needs of the others is copied first,
 // from another block each, instead of read where it is used by all from one (a
-// product of 200001 x 200000 bits: 143 K cycles to 121 K).
+// product of 200001 x 200000 bits: 143 K cycles to 121 K); 32.8 us with the
+// words' loads unconditional.
 struct Operand { const u32 *src; u64 nchunks; u32 xor0; int k; };
 struct RowAddr {                 // word j of plane p of slices PITCH words apart
     static constexpr bool rows_first = false;
