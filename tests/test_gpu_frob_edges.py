@@ -30,6 +30,24 @@ def test_small_states(engine, oracle, r):
         assert (got[i, :nw] == oracle.trin_square_k(st[i, :nw].copy(), r, si, 13)).all(), si
 
 
+# single squarings: a word a thread up to 2^15 words, warp tiles above
+@pytest.mark.parametrize("r", [5, 65, 129, 4423, 44687, 2097151, 2097153])
+def test_single_squarings(engine, oracle, r):
+    half = (r - 1) // 2
+    nw = (r + 63) // 64
+    stride = nw + (nw & 1)
+    for s in sorted({1, 2, min(64, half), max(1, half // 3), max(1, half - 1), half}):
+        st = np.zeros((1, stride), dtype=np.uint64)
+        st[0, :nw] = np.random.default_rng(r + s).integers(0, 1 << 64, size=nw, dtype=np.uint64)
+        if r % 64:
+            st[0, nw - 1] &= np.uint64((1 << (r % 64)) - 1)
+        a, b = engine.DeviceBuffer.from_array(st.reshape(-1)), engine.DeviceBuffer(st.nbytes)
+        engine.trin_square_batch(a, b, stride, 1, r,
+                                 engine.DeviceBuffer.from_array(np.array([s], dtype=np.uint64)), 1)
+        want = oracle.trin_square_k(st[0, :nw].copy(), r, s, 1)
+        assert (a.to_numpy(stride)[:nw] == want).all(), s
+
+
 # whole batches in one group (below 48 MB), equal groups with a remainder,
 # groups of one state, and shrinking groups (k > 128, 16 states and more);
 # ends in either buffer (k odd, k/2 even and odd)
