@@ -163,7 +163,7 @@ template <bool ROWS>
 GF2E_DEV LehmerEnd lehmer_cta(u64 *V, u64 W, u64 *R, u64 mw, long long da0, long long db0,
                               long long m) {
     LehmerEnd E;
-    __shared__ int s_va[2], s_vb[2], s_ra[2], s_mode[2], s_done[2], s_slow;
+    __shared__ int s_va[2], s_vb[2], s_ra[2], s_mode[2], s_done[2], s_slow[2];
     __shared__ long long s_k[2], s_top[2], s_md[2];
     __shared__ u32 s_m[2][4];
     __shared__ u64 s_tab[(BASE_THREADS / 32 / 4) * 3][64];   // per apply warp: v * m_e
@@ -349,10 +349,12 @@ GF2E_DEV LehmerEnd lehmer_cta(u64 *V, u64 W, u64 *R, u64 mw, long long da0, long
                              __funnelshift_r(x[v][0], x[v][1], sb);
                 publish(q, spare[0], spare[1], 0, dn0, dn1, win[0], win[1], md_next, round + 1);
             }
-            if (lane == 0) s_slow = slow;
+            if (lane == 0) s_slow[p] = slow;
         }
         __syncthreads();
-        if (s_slow) {                                  // degrees from the full new vectors
+        // of its own parity too: warp 0 may be deciding the next round before
+        // another warp has read this
+        if (s_slow[p]) {                                // degrees from the full new vectors
             if (tid < 32) {
                 const long long d0 = warp_degree(A2, top), d1 = warp_degree(B2, top);
                 publish_from_vectors(q, spare[0], spare[1], 0, d0, d1, md_next, round + 1);
