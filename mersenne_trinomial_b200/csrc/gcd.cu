@@ -13,10 +13,12 @@
 // full operands, (A', B') = M (A, B), with carry-less 64x32 multiplies
 // (masked integer products), about 32 degrees per round per operand.  A
 // degree gap wider than the matrix allows is a single shift-XOR round.  The
-// Operands of up to 6399 words run in shared memory with the half-gcd's
-// pipelined rounds (lehmer.cuh); longer ones from global memory, as above.  The
 // loop is bounded by deg A + deg B + 8 rounds (each round lowers the sum by
 // at least one); exceeding it returns GF2E_ERR_TIMEOUT instead of looping.
+//
+// That is the kernel for operands in global memory.  Operands of up to 6399
+// words run in shared memory with the half-gcd's pipelined rounds
+// (lehmer.cuh), bounded in the same way.
 #include "gf2e_internal.cuh"
 #include "lehmer.cuh"
 

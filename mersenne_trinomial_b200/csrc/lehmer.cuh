@@ -140,13 +140,14 @@ GF2E_DEV u64 shl_word(const u64 *X, long long w, long long k) {
 // what the rounds ended with (thread 0's counters)
 struct LehmerEnd {
     int parity = 0;              // which copy of the rows holds the result
-    int va = 0, ra = 0;          // vector of a', row of a'
+    int va = 0, ra = 0;          // vector of a' (of the gcd without ROWS), row of a'
     int status = GF2E_OK;
     long long rounds = 0, cyc_serial = 0;
 };
 
 // (a', b') = M (a, b) with deg a' >= m > deg b'; with ROWS the matrix M in four
-// arrays of mw words (row-major M00 M01 M10 M11).  m = 0 runs to b' = 0.
+// arrays of mw words (row-major M00 M01 M10 M11).  Without, m = 0: the gcd, at
+// b' = 0 or b' = 1.
 //
 // Lehmer rounds, pipelined: while warps 1..15 apply round r's matrix to the
 // vectors A, B and to the accumulated rows (one output word per item, the
@@ -179,9 +180,13 @@ GF2E_DEV LehmerEnd lehmer_cta(u64 *V, u64 W, u64 *R, u64 mw, long long da0, long
             long long t = da; da = db; db = t;
             u64 u = wa; wa = wb; wb = u;
         }
-        const bool done = db < m || round > max_rounds;
+        // a gcd with 1 is 1: beside a long a each round would clear one
+        // coefficient of it (a unit against 409000 bits: 200000 rounds)
+        const bool unit = !ROWS && db == 0;
+        const bool done = unit || db < m || round > max_rounds;
         if (tid == 0) {
-            s_va[q] = va; s_vb[q] = vb; s_ra[q] = ra;
+            s_va[q] = unit ? vb : va;
+            s_vb[q] = vb; s_ra[q] = ra;
             s_top[q] = da >> 6;
             s_md[q] = md;
             s_done[q] = done;

@@ -1,0 +1,35 @@
+"""Quadratic gcds (csrc/gcd.cu) of long operands with 1, in shared memory and,
+from 6400 words on, in global memory, alone and beside ordinary pairs."""
+import time
+
+import numpy as np
+import pytest
+
+from mersenne_trinomial_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def _poly(bits, seed):
+    w = W.random_bits(bits, seed)
+    w[(bits - 1) >> 6] |= np.uint64(1 << ((bits - 1) & 63))
+    return w
+
+
+@pytest.mark.parametrize("bits", [409_000, 420_000])
+def test_long_operand_with_one(engine, oracle, bits):
+    one = np.array([1], dtype=np.uint64)
+    a, x, y = _poly(bits, 1), _poly(700, 2), _poly(650, 3)
+    buf = engine.DeviceBuffer.from_array
+    pairs = [(buf(a), bits, buf(one), 1), (buf(one), 1, buf(a), bits), (buf(x), 700, buf(y), 650)]
+    engine.engine.gcd_batch(pairs, g_cap_words=16)             # the kernel is loaded
+    t0 = time.perf_counter()
+    degs, gs = engine.engine.gcd_batch(pairs, g_cap_words=16)
+    # a round for each coefficient is 0.2 s and more, the small gcd 0.1 ms
+    assert time.perf_counter() - t0 < 0.05
+    assert degs[0] == degs[1] == 0
+    for g in gs[:2]:
+        assert g[0] == 1 and not g[1:].any()
+    d, w = oracle.poly_gcd(x, y)
+    w = np.asarray(w, dtype=np.uint64)
+    assert int(degs[2]) == d and (gs[2][: w.size] == w).all()

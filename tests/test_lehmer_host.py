@@ -106,3 +106,18 @@ def test_matrix_in_any_warp_order(lib, first, last):
         row = parity * 4 + 2 * ra
         e = [_value(R[(row + k) * mw:(row + k + 1) * mw]) for k in range(2)]
         assert _mul(e[0], a) ^ _mul(e[1], b) == v, (ab, bb)
+
+
+# a gcd with 1, or that comes down to 1, ends there: no round for each
+# coefficient of the other operand
+@pytest.mark.parametrize("bits", [1, 64, 65, 3000])
+def test_unit_operand_takes_no_rounds(lib, bits):
+    a = _poly(bits, bits)
+    for x, y in ((a, 1), (1, a)):
+        st, g, *_, rounds = _run(lib, x, y, _order(0, 15))
+        assert (st, g) == (0, 1)
+        assert rounds == 0
+    a = _mul(_poly(2000, 9), 0b10) ^ 1              # a = 1 mod x
+    st, g, *_, rounds = _run(lib, a, 0b10, _order(0, 15))
+    assert (st, g) == (0, 1)
+    assert rounds <= 2 * 2000
