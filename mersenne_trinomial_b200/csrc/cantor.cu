@@ -528,8 +528,11 @@ struct PlanImpl {
     const u64 *tab = nullptr;            // tables the passes read (d_tab or caller's)
     std::vector<Pass> fwd, inv;
     std::vector<u64> ntiles_fwd, ntiles_inv;
-    // the bit-sliced transform (slicefft.cu) for 11 <= m <= 24; the Taylor
-    // levels above 2^16 run on the words, in these passes
+    // the bit-sliced forms (slicefft.cu) may be taken; not under
+    // GF2E_FFT_TAYLOR, which chooses among word passes
+    bool slices = true;
+    // the bit-sliced transform for 11 <= m <= 24; the Taylor levels above 2^16
+    // run on the words, in these passes
     bool sliced = false;
     std::vector<Pass> hi_fwd, hi_inv;
     std::vector<u64> ntiles_hi;
@@ -764,7 +767,8 @@ void build_passes(PlanImpl &P) {
     for (auto &p : P.inv) merge_stages(p, cfg);
     // (one forward and one inverse transform, words / sliced: 59 / 64 us at m =
     // 10, 76 / 73 at 11, 133 / 72 at 12, 469 / 222 at 20)
-    P.sliced = m >= 11 && m <= gf2e::SLICE_MAX_M && !getenv("GF2E_FFT_TAYLOR");
+    P.slices = !getenv("GF2E_FFT_TAYLOR");
+    P.sliced = P.slices && m >= 11 && m <= gf2e::SLICE_MAX_M;
     if (P.sliced && m > 16) {
         std::vector<std::pair<int, int>> lv, hi;
         tau_levels(0, m, cascade_bits_for(P), lv);
@@ -968,6 +972,11 @@ int fft_run_batch(const gf2e_fft_plan *plan, bool forward, u64 *f, u64 fstride, 
 
 u64 fft_plan_n(const gf2e_fft_plan *plan) { return plan->impl.n; }
 
+// products of this plan's own size may run bit-sliced
+bool fft_plan_slices(const gf2e_fft_plan *plan) {
+    return plan->impl.slices && plan->impl.m >= SLICE_MIN_M && plan->impl.m <= SLICE_PRODUCT_MAX_M;
+}
+
 int pointwise(u64 *fa, const u64 *fb, u64 n, cudaStream_t st) {
     k_pointwise<<<grid_for(n, 256), 256, 0, st>>>(fa, fb, n);
     GF2E_CHECK_LAUNCH("k_pointwise");
@@ -997,7 +1006,8 @@ int mul_fft_m(u64 abits, u64 bbits) {
 
 // Products of at most 2^23 coefficients take the bit-sliced transform
 // (slicefft.cu): up to 2^14 in one cluster of blocks, else in the transform
-// buffers where these are aligned for its 16-byte accesses.
+// buffers where these are aligned for its 16-byte accesses.  A plan made under
+// GF2E_FFT_TAYLOR keeps its word passes.
 int product_batch(const gf2e_fft_plan *plan, const ProductOp &a, const ProductOp &b, int batch,
                   u64 *fa, u64 *fb, u64 fstride, u64 *out, u64 ostride, u64 ow,
                   cudaStream_t st) {
@@ -1011,7 +1021,7 @@ int product_batch(const gf2e_fft_plan *plan, const ProductOp &a, const ProductOp
     const u32 *sa = reinterpret_cast<const u32 *>(a.words);
     const u32 *sb = reinterpret_cast<const u32 *>(b.words);
     const bool aligned = ((uintptr_t)fa | (uintptr_t)fb) % 16 == 0 && fstride % 2 == 0;
-    if (m <= SLICE_SMALL_MAX_M || (m <= SLICE_PRODUCT_MAX_M && aligned)) {
+    if (plan->impl.slices && (m <= SLICE_SMALL_MAX_M || (m <= SLICE_PRODUCT_MAX_M && aligned))) {
         const SliceOp op[2] = {{sa, 2 * a.stride, a.nchunks, (u32)a.xor0, fa},
                                {sb, 2 * b.stride, b.nchunks, (u32)b.xor0, fb}};
         if (m <= SLICE_SMALL_MAX_M)

@@ -63,6 +63,7 @@ int fft_run_batch(const gf2e_fft_plan *plan, bool forward, u64 *f, u64 fstride, 
 int overlap_add_batch(const u64 *F, u64 fstride, u64 nchunks, u64 *out, u64 ostride, u64 ow,
                       int batch, cudaStream_t st);
 u64 fft_plan_n(const gf2e_fft_plan *plan);
+bool fft_plan_slices(const gf2e_fft_plan *plan);
 }  // namespace gf2e
 
 namespace {
@@ -821,16 +822,11 @@ private:
         for (size_t g = 0; g < p.deg.size(); g++) c = std::max(c, chunks(p, (int)g));
         return c;
     }
-    // the bit-sliced transform serves every size it has (slicefft.cu)
-    static bool sliced(const gf2e_fft_plan *plan) {
-        const int m = gf2e_fft_plan_m(plan);
-        return m >= gf2e::SLICE_MIN_M && m <= gf2e::SLICE_PRODUCT_MAX_M;
-    }
     // forward transforms of every member of p into f (G x n)
     void fwd(gf2e_fft_plan *plan, const BPoly &p, u64 *f, u64 n) {
         const u64 nch = max_chunks(p);
         if (!nch) ckc(cudaMemsetAsync(f, 0, (size_t)G_ * n * 8, st_), "fft zero operand");
-        else if (sliced(plan)) {
+        else if (gf2e::fft_plan_slices(plan)) {
             const gf2e::SliceOp op{reinterpret_cast<const u32 *>(p.base()), 2 * p.stride, nch, 0, f};
             ck(gf2e::slice_fwd(gf2e_fft_plan_m(plan), &op, 1, n, G_, st_));
         } else ck(gf2e::fft_fwd_packed_batch(plan, f, n, reinterpret_cast<const u32 *>(p.base()),
@@ -844,7 +840,7 @@ private:
         u64 so = 1;
         for (int g = 0; g < G_; g++)
             if (dm[g] >= 0) so = std::max(so, (u64)(dm[g] >> 6) + 2);
-        if (sliced(plan)) {
+        if (gf2e::fft_plan_slices(plan)) {
             const int m = gf2e_fft_plan_m(plan);
             Buf t = m > 16 ? alloc(tot) : Buf();
             ck(gf2e::slice_pointwise(o, x1, y1, x2, y2, n, n, G_, st_));
