@@ -508,8 +508,12 @@ int gf2e_tune_get(gf2e_tune *t);              /* current (env applied) */
 int gf2e_tune_set(const gf2e_tune *t);        /* validated; INVALID if out of range */
 
 /* FFT autotune at size 2^m: candidates over tile size, column floor and
- * stage depths.  best_ms = fwd + inv time of the winner.  report (may be
- * NULL) receives one line per candidate: "tile cmin tlv blv ms ok". */
+ * stage depths of the word passes, the ones that have these knobs: transforms
+ * and products that run bit-sliced (16-byte buffers, 2^11 to 2^24 points;
+ * products of up to 2^23) are the same under every tuning, but for the Taylor
+ * levels above 2^16 of a single transform.  best_ms = fwd + inv time of the
+ * winner's word passes.  report (may be NULL) receives one line per candidate:
+ * "tile cmin tlv blv ms ok". */
 int gf2e_fft_autotune(int m, int reps, gf2e_tune *best, double *best_ms,
                       char *report, size_t report_cap);
 

@@ -957,6 +957,11 @@ int fft_run(const gf2e_fft_plan *plan, bool forward, u64 *f, cudaStream_t st) {
     return run_transform(plan->impl, forward, f, st);
 }
 
+// one transform by the word passes, which the tuning knobs act on
+int fft_run_words(const gf2e_fft_plan *plan, bool forward, u64 *f, cudaStream_t st) {
+    return run_passes(plan->impl, forward, f, nullptr, 0, st);
+}
+
 // `batch` transforms in one launch per pass: transform y at f + y*fstride,
 // packed from src32 + y*sstride32 (chunk 0 XORed with xor0)
 int fft_fwd_packed_batch(const gf2e_fft_plan *plan, u64 *f, u64 fstride, const u32 *src32,

@@ -8,7 +8,9 @@
 // same contract holds here, over this engine's knobs:
 //   FFT   tile size (2^11..2^13 elements of shared memory per pass), the
 //         least contiguous column count of a tile row, and the number of
-//         Taylor / butterfly levels fused per register stage;
+//         Taylor / butterfly levels fused per register stage.  They act on
+//         the word passes (cantor.cu), which are what is checked and timed;
+//         the bit-sliced transforms and products have no knobs;
 //   sieve the strip width of k_strip (entries of best[] per CTA);
 //   scan  the gcd interval schedule (L0 doubling to Lmax), from a cost
 //         model over measured per-degree and per-gcd costs, and the block
@@ -24,7 +26,7 @@
 
 namespace gf2e {
 int fft_plan_create_cfg(int m, const gf2e_tune &cfg, gf2e_fft_plan **out);
-int fft_run(const gf2e_fft_plan *plan, bool forward, u64 *f, cudaStream_t st);
+int fft_run_words(const gf2e_fft_plan *plan, bool forward, u64 *f, cudaStream_t st);
 }  // namespace gf2e
 
 namespace {
@@ -215,7 +217,7 @@ int gf2e_fft_autotune(int m, int reps, gf2e_tune *best, double *best_ms, char *r
         gf2e_fft_plan *p = nullptr;
         GF2E_TRY(gf2e::fft_plan_create_cfg(m, builtin_default(), &p));
         cudaError_t e = cudaMemcpyAsync(d_ref, d_in, n * 8, cudaMemcpyDeviceToDevice, se.st);
-        int st = (e == cudaSuccess) ? gf2e::fft_run(p, true, d_ref, se.st)
+        int st = (e == cudaSuccess) ? gf2e::fft_run_words(p, true, d_ref, se.st)
                                     : gf2e::cuda_status(e, "autotune copy");
         if (st == GF2E_OK) st = gf2e::cuda_status(cudaStreamSynchronize(se.st), "autotune ref");
         gf2e_fft_plan_destroy(p);
@@ -239,19 +241,19 @@ int gf2e_fft_autotune(int m, int reps, gf2e_tune *best, double *best_ms, char *r
                     unsigned long long dfw = 1, dinv = 1;
                     float ms = 0;
                     cudaError_t e = cudaMemcpyAsync(d_w, d_in, n * 8, cudaMemcpyDeviceToDevice, se.st);
-                    int st = (e == cudaSuccess) ? gf2e::fft_run(p, true, d_w, se.st)
+                    int st = (e == cudaSuccess) ? gf2e::fft_run_words(p, true, d_w, se.st)
                                                 : gf2e::cuda_status(e, "autotune copy");
                     if (st == GF2E_OK) st = count_diff(d_w, d_ref, n, d_cnt, se.st, &dfw);
-                    if (st == GF2E_OK) st = gf2e::fft_run(p, false, d_w, se.st);
+                    if (st == GF2E_OK) st = gf2e::fft_run_words(p, false, d_w, se.st);
                     if (st == GF2E_OK) st = count_diff(d_w, d_in, n, d_cnt, se.st, &dinv);
                     // timing: one warm-up fwd+inv, then reps of fwd+inv
                     if (st == GF2E_OK && dfw == 0 && dinv == 0) {
-                        st = gf2e::fft_run(p, true, d_w, se.st);
-                        if (st == GF2E_OK) st = gf2e::fft_run(p, false, d_w, se.st);
+                        st = gf2e::fft_run_words(p, true, d_w, se.st);
+                        if (st == GF2E_OK) st = gf2e::fft_run_words(p, false, d_w, se.st);
                         if (st == GF2E_OK) cudaEventRecord(se.a, se.st);
                         for (int r = 0; r < reps && st == GF2E_OK; r++) {
-                            st = gf2e::fft_run(p, true, d_w, se.st);
-                            if (st == GF2E_OK) st = gf2e::fft_run(p, false, d_w, se.st);
+                            st = gf2e::fft_run_words(p, true, d_w, se.st);
+                            if (st == GF2E_OK) st = gf2e::fft_run_words(p, false, d_w, se.st);
                         }
                         if (st == GF2E_OK) {
                             cudaEventRecord(se.b, se.st);
