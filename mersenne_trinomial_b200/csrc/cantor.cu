@@ -418,7 +418,11 @@ __global__ void k_pack_batch(const u32 *__restrict__ src32, u64 sstride32, u64 n
     }
 }
 
-__global__ void k_pointwise(u64 *__restrict__ fa, const u64 *__restrict__ fb, u64 n) {
+// blockIdx.y selects the pair at y * stride
+__global__ void k_pointwise(u64 *__restrict__ fa, const u64 *__restrict__ fb, u64 n,
+                            u64 stride = 0) {
+    fa += blockIdx.y * stride;
+    fb += blockIdx.y * stride;
     for (u64 k = (u64)blockIdx.x * blockDim.x + threadIdx.x; k < n;
          k += (u64)gridDim.x * blockDim.x)
         fa[k] = gf64_mul(fa[k], fb[k]);
@@ -988,6 +992,13 @@ int pointwise(u64 *fa, const u64 *fb, u64 n, cudaStream_t st) {
     return GF2E_OK;
 }
 
+int pointwise_batch(u64 *fa, const u64 *fb, u64 n, u64 fstride, int batch, cudaStream_t st) {
+    const int per = std::max(1, grid_for(n, 256) / batch);
+    k_pointwise<<<dim3(per, batch), 256, 0, st>>>(fa, fb, n, fstride);
+    GF2E_CHECK_LAUNCH("k_pointwise batch");
+    return GF2E_OK;
+}
+
 int overlap_add(const u64 *F, u64 nchunks, u64 *out, u64 ow, cudaStream_t st) {
     k_overlap_add<<<grid_for(ow, 256), 256, 0, st>>>(F, nchunks, out, ow);
     GF2E_CHECK_LAUNCH("k_overlap_add");
@@ -1009,9 +1020,25 @@ int mul_fft_m(u64 abits, u64 bbits) {
     return m;
 }
 
+// Products by the word passes where these are shorter than the cluster
+// product, whose transform has 2^10 coefficients at least: it takes 24 us for
+// up to half as many products as there are SMs (8 blocks each, 4 an SM), and
+// again for each further such wave.  2^3 coefficients and fewer are below one
+// wave in words, 2^4 .. 2^7 below two, 2^8 below three, 2^9 below four.  64
+// degrees of a scan in us, words / cluster: m = 3, 32 s 1904 / 2232; m = 4, 64 s
+// 2362 / 2241; m = 5, 64 s 2754 / 2333, 96 s 2755 / 3805; m = 7, 64 s 3611 /
+// 2362, 96 s 3669 / 3757, 512 s 6857 / 12647; m = 8, 128 s 4137 / 3805, 192 s
+// 4530 / 5376; m = 9, 192 s 5905 / 5286, 256 s 5925 / 6794, 2048 s 44182 /
+// 48972; m = 10, 512 s 13380 / 12887.  One product of 32 bits 16 / 25, a square
+// 13 / 25.
+bool words_shorter(int m, int batch) {
+    const int waves = m <= 3 ? 0 : m <= 7 ? 1 : m - 6;
+    return m < SLICE_MIN_M && batch > waves * (sm_count() / 2);
+}
+
 // Products of at most 2^23 coefficients take the bit-sliced transform
-// (slicefft.cu): up to 2^14 in one cluster of blocks, else in the transform
-// buffers where these are aligned for its 16-byte accesses.  A plan made under
+// (slicefft.cu): up to 2^14 in one cluster of blocks (but see above), else in
+// the transform buffers where these are aligned for its 16-byte accesses.  A plan made under
 // GF2E_FFT_TAYLOR keeps its word passes.
 int product_batch(const gf2e_fft_plan *plan, const ProductOp &a, const ProductOp &b, int batch,
                   u64 *fa, u64 *fb, u64 fstride, u64 *out, u64 ostride, u64 ow,
@@ -1026,7 +1053,8 @@ int product_batch(const gf2e_fft_plan *plan, const ProductOp &a, const ProductOp
     const u32 *sa = reinterpret_cast<const u32 *>(a.words);
     const u32 *sb = reinterpret_cast<const u32 *>(b.words);
     const bool aligned = ((uintptr_t)fa | (uintptr_t)fb) % 16 == 0 && fstride % 2 == 0;
-    if (plan->impl.slices && (m <= SLICE_SMALL_MAX_M || (m <= SLICE_PRODUCT_MAX_M && aligned))) {
+    if (plan->impl.slices && !words_shorter(plan->impl.m, batch) &&
+        (m <= SLICE_SMALL_MAX_M || (m <= SLICE_PRODUCT_MAX_M && aligned))) {
         const SliceOp op[2] = {{sa, 2 * a.stride, a.nchunks, (u32)a.xor0, fa},
                                {sb, 2 * b.stride, b.nchunks, (u32)b.xor0, fb}};
         if (m <= SLICE_SMALL_MAX_M)
@@ -1042,8 +1070,7 @@ int product_batch(const gf2e_fft_plan *plan, const ProductOp &a, const ProductOp
     if (!same)
         GF2E_TRY(fft_fwd_packed_batch(plan, fb, fstride, sb, 2 * b.stride, b.nchunks, b.xor0,
                                       batch, st));
-    for (int i = 0; i < batch; i++)
-        GF2E_TRY(pointwise(fa + i * fstride, (same ? fa : fb) + i * fstride, n, st));
+    GF2E_TRY(pointwise_batch(fa, same ? fa : fb, n, fstride, batch, st));
     GF2E_TRY(fft_run_batch(plan, false, fa, fstride, batch, st));
     return overlap_add_batch(fa, fstride, std::min(count, n), out, ostride, ow, batch, st);
 }
