@@ -358,6 +358,11 @@ int run_gcd_smem(const gf2e_gcd_job *jobs, int njobs, int64_t *deg_host, void *w
 
 }  // namespace
 
+namespace gf2e {
+// operands of this many bits run in shared memory
+bool gcd_in_shared(u64 bits) { return ((bits + 63) >> 6) + 1 <= SMEM_WORDS; }
+}  // namespace gf2e
+
 extern "C" {
 
 int gf2e_gcd_workspace_size(const gf2e_gcd_job *jobs, int njobs, size_t *bytes) {
@@ -381,9 +386,9 @@ int gf2e_gcd_batch(const gf2e_gcd_job *jobs, int njobs, int64_t *deg_host, void 
     if (njobs > 65535) return gf2e::invalid("gf2e_gcd_batch: at most 65535 jobs");
     cudaStream_t st = (cudaStream_t)stream;
     u64 most = 0;
-    for (int i = 0; i < njobs; i++)
-        most = std::max<u64>(most, (std::max(jobs[i].abits, jobs[i].bbits) + 63) >> 6);
-    if (most + 1 <= SMEM_WORDS) return run_gcd_smem(jobs, njobs, deg_host, workspace, most + 1, st);
+    for (int i = 0; i < njobs; i++) most = std::max<u64>(most, std::max(jobs[i].abits, jobs[i].bbits));
+    if (gf2e::gcd_in_shared(most))
+        return run_gcd_smem(jobs, njobs, deg_host, workspace, ((most + 63) >> 6) + 1, st);
     static_assert(sizeof(GcdSmem) <= sizeof(GcdDev), "job array in the same workspace");
     std::vector<GcdDev> host(njobs);
     char *ws = (char *)workspace;

@@ -47,6 +47,7 @@ int trin_reduce_batch(const u64 *P, size_t pstride, size_t pw, u64 L, u64 *out, 
 int mul_fft_m(u64 abits, u64 bbits);
 gf2e_fft_plan *cached_plan(int m);
 u64 fft_plan_n(const gf2e_fft_plan *plan);
+bool gcd_in_shared(u64 bits);
 }  // namespace gf2e
 
 struct gf2e_scanner {
@@ -95,8 +96,17 @@ struct gf2e_scanner {
 
 // operands of at least this many bits take the half-gcd (hgcd.cu) at
 // interval ends; smaller ones the quadratic batched gcd (gcd.cu): 24 gcds take
-// 23 / 21 ms at 130000 bits, 34 / 43 ms at 200000, one 18 / 20 and 27 / 42
+// 23 / 21 ms at 130000 bits, 34 / 43 ms at 200000, one 18 / 20 and 27 / 42.
+// Half-gcds run GCD_PART at a time, quadratic ones an SM each, so many at once
+// take the quadratic gcd (up to 409000 bits, where it runs in shared memory)
+// while its waves of bits / 200000 parts are fewer than the half-gcd's parts.
+// Half-gcd / quadratic, ms: 160000 bits 64 gcds 32 / 29, 65 52 / 29, 148 92 / 29,
+// 592 285 / 114; 200000 bits 64 47 / 42, 148 103 / 50, 592 351 / 166; 300000 65
+// 99 / 87, 150 166 / 173, 592 574 / 348; 400000 65 127 / 154, 148 215 / 149, 150
+// 217 / 295, 592 741 / 591.
 constexpr u64 GCD_LARGE_BITS = 150000;
+constexpr size_t GCD_PART = 64;
+constexpr u64 GCD_PART_BITS = 200000;
 // device words one member of a lockstep half-gcd batch draws from the gcd
 // pool, per operand word (its high-water mark: 1.52 GB at r = 136279841)
 constexpr size_t HGCD_WORDS_PER_WORD = 90;
@@ -204,6 +214,18 @@ Geometry geometry(u64 r) {
     g.pstride = g.ow + (g.ow & 1);
     g.gcap = std::min<size_t>(g.tw, 4096);
     return g;
+}
+
+// `due` interval gcds go to the quadratic kernel, see GCD_LARGE_BITS
+bool quadratic_gcds(u64 r, size_t due) {
+    if (r < GCD_LARGE_BITS) return true;
+    if (due <= GCD_PART || !gf2e::gcd_in_shared(r + 1)) return false;
+    const u64 sm = (u64)gf2e::sm_count();
+    return (due + sm - 1) / sm * r < (due + GCD_PART - 1) / GCD_PART * GCD_PART_BITS;
+}
+// whether a scanner of `slots` ever has that many
+bool keeps_quadratic_workspace(u64 r, size_t slots) {
+    return r < GCD_LARGE_BITS || (slots > GCD_PART && gf2e::gcd_in_shared(r + 1));
 }
 
 size_t device_words(const Geometry &g, int B, int m = 1) {
@@ -455,7 +477,7 @@ int degree_step(gf2e_scanner &S, cudaStream_t st) {
                                  S.G + S.gcap * q, S.gcap};
     }
     const auto t_gcd = std::chrono::steady_clock::now();
-    if (S.r >= GCD_LARGE_BITS) {
+    if (!quadratic_gcds(S.r, due.size())) {
         const int par = std::max(1, std::min((int)due.size(), S.gcd_parallel));
         GF2E_TRY(gf2e_gcd_large(S.jobs.data(), (int)due.size(), S.degs.data(), par, nullptr, st));
     } else {
@@ -536,14 +558,16 @@ int gf2e_scanner_footprint_blocked(uint64_t r, int slots, int block, size_t *byt
         return gf2e::invalid("scanner: block size must be 1 or even in 2..62");
     Geometry g = geometry(r);
     size_t words = device_words(g, slots, block);
-    // gcd workspace: job table + 4 buffers per job (quadratic gcd), or room
+    // gcd workspace: job table + 4 buffers per job (quadratic gcd), and room
     // for 16 members of a half-gcd batch (a batch sizes itself from the
     // memory free when it starts, so more slots only make it run in parts)
-    size_t gw = ((size_t)slots * 96 + 255) + (size_t)slots * 4 * (g.tw + 1) * 8;
+    size_t gw = 0;
+    if (keeps_quadratic_workspace(r, (size_t)slots))
+        gw = ((size_t)slots * 96 + 255) + (size_t)slots * 4 * (g.tw + 1) * 8;
     if (r >= GCD_LARGE_BITS) {
         int par = 16;
         if (const char *env = getenv("GF2E_SCAN_GCD_PARALLEL")) par = std::max(1, atoi(env));
-        gw = (size_t)std::min(par, slots) * HGCD_WORDS_PER_WORD * (g.tw + 1) * 8;
+        gw += (size_t)std::min(par, slots) * HGCD_WORDS_PER_WORD * (g.tw + 1) * 8;
     }
     *bytes = words * 8 + gw;
     return GF2E_OK;
@@ -598,8 +622,9 @@ int gf2e_scanner_create_blocked(uint64_t r, int slots, int block, gf2e_scanner *
     if (S->wrap) S->WS = S->dmem + (device_words(g, slots, block) - (size_t)g.wm.per * B);
     std::vector<gf2e_gcd_job> tmp(B, gf2e_gcd_job{S->ACC, r, S->T, r + 1, S->G, g.gcap});
     int st = GF2E_OK;
-    if (r < GCD_LARGE_BITS) st = gf2e_gcd_workspace_size(tmp.data(), B, &S->gws_bytes);
-    if (st == GF2E_OK && r < GCD_LARGE_BITS) {
+    const bool gws = keeps_quadratic_workspace(r, (size_t)B);
+    if (gws) st = gf2e_gcd_workspace_size(tmp.data(), B, &S->gws_bytes);
+    if (st == GF2E_OK && gws) {
         e = cudaMalloc(&S->gws, S->gws_bytes);
         if (e != cudaSuccess) st = gf2e::cuda_status(e, "scanner gcd workspace");
     }
