@@ -1036,9 +1036,21 @@ bool words_shorter(int m, int batch) {
     return m < SLICE_MIN_M && batch > waves * (sm_count() / 2);
 }
 
+// The word passes read a before they write fb and write `out` from fa alone, so
+// a single product's fb may hold a or the output, and a square leaves it alone
+// (fb may be fa).  The sliced ones read both operands in one launch and pass
+// the inverse through fb: such a product keeps its word passes.
+bool shares_fb(const ProductOp &a, const u64 *fa, const u64 *fb, u64 n, const u64 *out, u64 ow) {
+    auto meets = [&](const u64 *p, u64 words) {
+        return (uintptr_t)p < (uintptr_t)(fb + n) && (uintptr_t)fb < (uintptr_t)(p + words);
+    };
+    return meets(a.words, (a.nchunks + 1) / 2) || meets(fa, n) || meets(out, ow);
+}
+
 // Products of at most 2^23 coefficients take the bit-sliced transform
 // (slicefft.cu): up to 2^14 in one cluster of blocks (but see above), else in
-// the transform buffers where these are aligned for its 16-byte accesses.  A plan made under
+// the transform buffers where these are aligned for its 16-byte accesses and
+// apart from each other and the operands.  A plan made under
 // GF2E_FFT_TAYLOR keeps its word passes.
 int product_batch(const gf2e_fft_plan *plan, const ProductOp &a, const ProductOp &b, int batch,
                   u64 *fa, u64 *fb, u64 fstride, u64 *out, u64 ostride, u64 ow,
@@ -1052,9 +1064,10 @@ int product_batch(const gf2e_fft_plan *plan, const ProductOp &a, const ProductOp
                       a.xor0 == b.xor0;
     const u32 *sa = reinterpret_cast<const u32 *>(a.words);
     const u32 *sb = reinterpret_cast<const u32 *>(b.words);
-    const bool aligned = ((uintptr_t)fa | (uintptr_t)fb) % 16 == 0 && fstride % 2 == 0;
+    const bool buffers = ((uintptr_t)fa | (uintptr_t)fb) % 16 == 0 && fstride % 2 == 0 &&
+                         (batch > 1 || !shares_fb(a, fa, fb, (u64)1 << m, out, ow));
     if (plan->impl.slices && !words_shorter(plan->impl.m, batch) &&
-        (m <= SLICE_SMALL_MAX_M || (m <= SLICE_PRODUCT_MAX_M && aligned))) {
+        (m <= SLICE_SMALL_MAX_M || (m <= SLICE_PRODUCT_MAX_M && buffers))) {
         const SliceOp op[2] = {{sa, 2 * a.stride, a.nchunks, (u32)a.xor0, fa},
                                {sb, 2 * b.stride, b.nchunks, (u32)b.xor0, fb}};
         if (m <= SLICE_SMALL_MAX_M)
