@@ -24,6 +24,8 @@
 
 #include <algorithm>
 #include <atomic>
+#include <iterator>
+#include <utility>
 #include <vector>
 
 namespace {
@@ -326,6 +328,28 @@ int allow_gcd_smem() {
     return GF2E_OK;
 }
 
+// Whether a result's place meets an operand's.  The kernel above writes each
+// result while other jobs may still be loading, where k_gcd_batch works on
+// copies made before any result is written.
+bool results_meet_operands(const gf2e_gcd_job *jobs, int njobs) {
+    std::vector<std::pair<uintptr_t, uintptr_t>> op;
+    for (int i = 0; i < njobs; i++) {
+        const gf2e_gcd_job &j = jobs[i];
+        op.push_back({(uintptr_t)j.a_dev, (uintptr_t)(j.a_dev + ((j.abits + 63) >> 6))});
+        op.push_back({(uintptr_t)j.b_dev, (uintptr_t)(j.b_dev + ((j.bbits + 63) >> 6))});
+    }
+    std::sort(op.begin(), op.end());
+    for (size_t i = 1; i < op.size(); i++)                  // the furthest end so far
+        op[i].second = std::max(op[i].second, op[i - 1].second);
+    for (int i = 0; i < njobs; i++) {
+        if (!jobs[i].g_dev || !jobs[i].g_cap_words) continue;
+        const uintptr_t g0 = (uintptr_t)jobs[i].g_dev, g1 = (uintptr_t)(jobs[i].g_dev + jobs[i].g_cap_words);
+        auto it = std::lower_bound(op.begin(), op.end(), std::make_pair(g1, (uintptr_t)0));
+        if (it != op.begin() && std::prev(it)->second > g0) return true;
+    }
+    return false;
+}
+
 int run_gcd_smem(const gf2e_gcd_job *jobs, int njobs, int64_t *deg_host, void *ws, u64 W,
                  cudaStream_t st) {
     GF2E_TRY(allow_gcd_smem());
@@ -387,7 +411,7 @@ int gf2e_gcd_batch(const gf2e_gcd_job *jobs, int njobs, int64_t *deg_host, void 
     cudaStream_t st = (cudaStream_t)stream;
     u64 most = 0;
     for (int i = 0; i < njobs; i++) most = std::max<u64>(most, std::max(jobs[i].abits, jobs[i].bbits));
-    if (gf2e::gcd_in_shared(most))
+    if (gf2e::gcd_in_shared(most) && !results_meet_operands(jobs, njobs))
         return run_gcd_smem(jobs, njobs, deg_host, workspace, ((most + 63) >> 6) + 1, st);
     static_assert(sizeof(GcdSmem) <= sizeof(GcdDev), "job array in the same workspace");
     std::vector<GcdDev> host(njobs);
