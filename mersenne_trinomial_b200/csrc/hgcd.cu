@@ -832,20 +832,25 @@ private:
         } else ck(gf2e::fft_fwd_packed_batch(plan, f, n, reinterpret_cast<const u32 *>(p.base()),
                                            2 * p.stride, nch, 0, G_, st_));
     }
+    // transforms whose sliced inverse passes through a second buffer
+    static bool inverse_tmp(const gf2e_fft_plan *plan) {
+        return gf2e::fft_plan_slices(plan) && gf2e_fft_plan_m(plan) > 16;
+    }
     // o <- inverse of X1 Y1 + X2 Y2 (pointwise), overlap-added into a new
-    // batched polynomial of degree bounds dm
-    BPoly product_out(gf2e_fft_plan *plan, u64 *o, const u64 *x1, const u64 *y1, const u64 *x2,
-                      const u64 *y2, u64 n, u64 need, const std::vector<long long> &dm) {
+    // batched polynomial of degree bounds dm.  tmp (inverse_tmp): as large as
+    // o, not o; it may be an operand, which is lost
+    BPoly product_out(gf2e_fft_plan *plan, u64 *o, u64 *tmp, const u64 *x1, const u64 *y1,
+                      const u64 *x2, const u64 *y2, u64 n, u64 need,
+                      const std::vector<long long> &dm) {
         const u64 tot = (u64)G_ * n;
         u64 so = 1;
         for (int g = 0; g < G_; g++)
             if (dm[g] >= 0) so = std::max(so, (u64)(dm[g] >> 6) + 2);
         if (gf2e::fft_plan_slices(plan)) {
             const int m = gf2e_fft_plan_m(plan);
-            Buf t = m > 16 ? alloc(tot) : Buf();
             ck(gf2e::slice_pointwise(o, x1, y1, x2, y2, n, n, G_, st_));
             BPoly out = make(so, false);
-            ck(gf2e::slice_inv(m, o, t ? t->p : nullptr, n, G_, out.base(), so, so, st_));
+            ck(gf2e::slice_inv(m, o, tmp, n, G_, out.base(), so, so, st_));
             set_bounds(out, so, dm);
             return out;
         }
@@ -921,8 +926,8 @@ private:
             Buf F0 = alloc(G_ * n), F1 = alloc(G_ * n);
             fwd(plan, M.e[2 * row], F0->p, n);
             fwd(plan, M.e[2 * row + 1], F1->p, n);
-            (row ? d : c) = product_out(plan, F0->p, F0->p, Fa->p, F1->p, Fb->p, n, need,
-                                        sum_bound(M.e[2 * row], a, M.e[2 * row + 1], b));
+            (row ? d : c) = product_out(plan, F0->p, F1->p, F0->p, Fa->p, F1->p, Fb->p, n,
+                                        need, sum_bound(M.e[2 * row], a, M.e[2 * row + 1], b));
         }
         stats.fft_mul2 += 2;
     }
@@ -952,19 +957,22 @@ private:
             gf2e_fft_plan *plan = gf2e::cached_plan(fft_m(need));
             if (!plan) throw Fail{GF2E_ERR_CUDA};
             const u64 n = gf2e::fft_plan_n(plan);
-            Buf F2[4], F1[4];
+            // one row of M2 at a time: seven transforms, eight with the sliced
+            // inverse's second buffer
+            Buf F1[4], F2[2];
             for (int i = 0; i < 4; i++) {
-                F2[i] = alloc(G_ * n);
-                fwd(plan, M2.e[i], F2[i]->p, n);
                 F1[i] = alloc(G_ * n);
                 fwd(plan, M1.e[i], F1[i]->p, n);
             }
-            Buf O = alloc(G_ * n);
-            for (int i = 0; i < 2; i++)
+            for (int k = 0; k < 2; k++) F2[k] = alloc(G_ * n);
+            Buf O = alloc(G_ * n), T = inverse_tmp(plan) ? alloc(G_ * n) : Buf();
+            for (int i = 0; i < 2; i++) {
+                for (int k = 0; k < 2; k++) fwd(plan, M2.e[2 * i + k], F2[k]->p, n);
                 for (int j = 0; j < 2; j++)
-                    r.e[2 * i + j] = product_out(plan, O->p, F2[2 * i]->p, F1[j]->p, F2[2 * i + 1]->p,
-                                                 F1[2 + j]->p, n, need,
+                    r.e[2 * i + j] = product_out(plan, O->p, T ? T->p : nullptr, F2[0]->p, F1[j]->p,
+                                                 F2[1]->p, F1[2 + j]->p, n, need,
                                                  sum_bound(M2.e[2 * i], M1.e[j], M2.e[2 * i + 1], M1.e[2 + j]));
+            }
             stats.fft_mul2 += 4;
         } else {
             PairB P[4];
@@ -1256,8 +1264,8 @@ cudaMemPool_t hgcd_pool() {
 
 // members in flight: the caller's cap, GMAX, and what device memory holds
 // (per member about 40 operand-sized buffers and 12 transforms of the
-// largest matrix product: 1.52 GB measured at r = 136279841), counting as
-// free what the gcd pool holds from earlier gcds but does not use
+// largest matrix product: 1.49 GB, 1.43 measured, for 8 at r = 136279841),
+// counting as free what the gcd pool holds from earlier gcds but does not use
 int batch_size(cudaMemPool_t pool, const gf2e_gcd_job *jobs, int njobs, int max_parallel) {
     u64 bits = 1;
     for (int i = 0; i < njobs; i++) bits = std::max(bits, std::max(jobs[i].abits, jobs[i].bbits));

@@ -108,7 +108,8 @@ constexpr u64 GCD_LARGE_BITS = 150000;
 constexpr size_t GCD_PART = 64;
 constexpr u64 GCD_PART_BITS = 200000;
 // device words one member of a lockstep half-gcd batch draws from the gcd
-// pool, per operand word (its high-water mark: 1.52 GB at r = 136279841)
+// pool, per operand word (high-water marks: 84 for 8 at r = 136279841, 1.43 GB
+// each, 86 for 16 at 50000183, 84 for 64 at 1600183)
 constexpr size_t HGCD_WORDS_PER_WORD = 90;
 
 namespace gf2e {
