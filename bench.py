@@ -246,14 +246,7 @@ def main():
     states = torch.empty(stride * n, dtype=torch.int64, device="cuda")
     scratch = torch.empty_like(states)
     s_dev = torch.from_numpy(s_host.view(np.int64)).cuda()
-    per_pass = M.engine.squarings_per_pass(r, stride, n)
-    # passes of the squaring kernel per step (an odd pass count gets one
-    # fused pass split in two, as gf2e_trin_square_batch does)
-    n4 = k // 2 if per_pass == 2 else 0
-    n1 = k - 2 * n4
-    if (n4 + n1) % 2 and n4 > 0:
-        n4, n1 = n4 - 1, n1 + 2
-    copy_back = (n4 + n1) % 2
+    n4, n1, copy_back = squaring_passes(M, r, stride, n, k)
     launches_per_step = 1 + n4 + n1 + copy_back
     ev = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
           for _ in range(args.steps)]
@@ -364,6 +357,20 @@ def main():
     return 0
 
 
+def squaring_passes(M, r, stride, n, k):
+    """The passes trin_square_batch takes for k squarings of n states (on 16
+    bytes): two-squaring ones, single ones, and whether a copy follows.  An odd
+    number of passes gets one of the first split in two."""
+    # the library answers for passes over HBM; below that size too, the fused
+    # pass runs wherever it applies, which more states show
+    over_hbm = max(n, (96 << 20) // (16 * stride) + 1)
+    n4 = k // 2 if M.engine.squarings_per_pass(r, stride, over_hbm) == 2 else 0
+    n1 = k - 2 * n4
+    if (n4 + n1) % 2 and n4 > 0:
+        n4, n1 = n4 - 1, n1 + 2
+    return n4, n1, (n4 + n1) % 2
+
+
 def _ev_time(torch, fn, reps=3, flush=None):
     ts = []
     for _ in range(reps):
@@ -468,48 +475,28 @@ def run_extras(torch, M, W, sq_rate=None):
     bytes3 = sum(48 * (1 << M.engine.fft_m_for(ab, bb)) + (ab + bb) // 4 for ab, bb in c3["sizes"])
     peak = measured_peaks()[0]
 
-    def pass_bytes():
-        # bytes the tile passes must move: each forward/inverse pass reads and
-        # writes the n points once (two forwards and one inverse per product),
-        # plus the 48 n of packing, pointwise product and overlap-add
-        tot = 0
-        for ab, bb in c3["sizes"]:
-            m = M.engine.fft_m_for(ab, bb)
-            F = M.CudaFFT()
-            F.init(m)
-            f, i = F.passes()
-            F.fini()
-            tot += 16 * (1 << m) * (2 * f + i) + 48 * (1 << m) + (ab + bb) // 4
-        return tot
-    pb3 = pass_bytes()
     out["mul_config3"] = {"products_per_s": 64 / (ms / 1e3), "ms": ms,
                           "algorithmic_GBps": bytes3 / (ms / 1e3) / 1e9,
                           "frac_of_measured_hbm": bytes3 / (ms / 1e3) / 1e9 / peak,
-                          "pass_GBps": pb3 / (ms / 1e3) / 1e9,
-                          "pass_frac_of_measured_hbm": pb3 / (ms / 1e3) / 1e9 / peak,
-                          "operand_bits": tot_bits, "tuning": "built-in default"}
-    # autotune the transform at the largest config-3 size (2^23 points), then
-    # the same 64 products under the chosen settings
+                          "operand_bits": tot_bits}
+    # autotune the word passes at the largest config-3 size (2^23 points); the
+    # products above run bit-sliced, which has no knobs, so they are the same
+    # under any choice, and the default is put back
     from mersenne_trinomial_b200 import autotune as A
+    saved = A.tune_get()
     dflt = A.resolve_by_size(A.tune_default(), 23)
     t0 = time.perf_counter()
     tuned = A.fft_autotune(23, reps=2)
     tune_s = time.perf_counter() - t0
-    ms_t = _ev_time(torch, lambda: M.mul_batch_dev(jobs, workspace=wsb), 3, flush)
+    A.tune_set(**saved)
     dflt_row = [c for c in tuned["candidates"]
                 if all(c[k] == dflt[k] for k in ("fft_tile_log", "fft_cmin", "fft_taylor_lv",
                                                   "fft_bfly_lv"))]
-    pb3t = pass_bytes()
-    out["mul_config3_tuned"] = {
-        "products_per_s": 64 / (ms_t / 1e3), "ms": ms_t,
-        "algorithmic_GBps": bytes3 / (ms_t / 1e3) / 1e9,
-        "frac_of_measured_hbm": bytes3 / (ms_t / 1e3) / 1e9 / peak,
-        "pass_GBps": pb3t / (ms_t / 1e3) / 1e9,
-        "pass_frac_of_measured_hbm": pb3t / (ms_t / 1e3) / 1e9 / peak,
+    out["fft_autotune_m23"] = {
         "tuning": {k: v for k, v in tuned["best"].items() if k.startswith("fft_")},
         "autotune_s": tune_s, "candidates_verified": len(tuned["candidates"]),
-        "fwd_inv_ms_m23": {"tuned": tuned["best_fwd_inv_ms"],
-                           "default": dflt_row[0]["ms"] if dflt_row else None}}
+        "word_passes_fwd_inv_ms": {"tuned": tuned["best_fwd_inv_ms"],
+                                   "default": dflt_row[0]["ms"] if dflt_row else None}}
     del bufs, jobs, wsb
     out["deep_scan_r136279841"] = deep_scan_sample(torch, M)
     # blocked DDF: block size from the measured modmul (per-degree sample) and
