@@ -5,6 +5,7 @@ import pytest
 import torch
 
 import bench
+from kernel_names import kernel_counts, launched
 
 pytestmark = pytest.mark.gpu
 
@@ -19,12 +20,6 @@ def test_counted_passes_are_the_launched_ones(engine, r, n, k):
     s = torch.from_numpy(np.arange(1, n + 1)).cuda()
     engine.trin_square_batch(a, b, stride, n, r, s, k)
     torch.cuda.synchronize()
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
-        engine.trin_square_batch(a, b, stride, n, r, s, k)
-        torch.cuda.synchronize()
-    count = {"k_frob4_batch": 0, "k_square_batch": 0, "Memcpy DtoD": 0}
-    for e in p.key_averages():
-        for name in count:
-            if name in e.key:
-                count[name] += e.count
-    assert tuple(count.values()) == bench.squaring_passes(engine, r, stride, n, k)
+    names = kernel_counts(lambda: engine.trin_square_batch(a, b, stride, n, r, s, k))
+    got = tuple(launched(names, x) for x in ("k_frob4_batch", "k_square_batch", "Memcpy DtoD"))
+    assert got == bench.squaring_passes(engine, r, stride, n, k)

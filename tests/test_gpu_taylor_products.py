@@ -16,9 +16,9 @@ pytestmark = pytest.mark.gpu
 
 SCRIPT = r"""
 import sys
-sys.path.insert(0, %(root)r)
+sys.path[:0] = [%(root)r, %(root)r + "/tests"]
 import numpy as np
-import torch
+from kernel_names import kernel_counts, launched
 import mersenne_trinomial_b200 as M
 from mersenne_trinomial_b200 import engine as E
 from mersenne_trinomial_b200 import workloads as W
@@ -41,12 +41,6 @@ for ab, bb in %(sizes)r:
     n = min(words.size, 2 * ow) // 2 * 2
     assert (words[:n].view(np.uint64) == got[: n // 2]).all(), ("coefficients", ab, bb)
     F.fini()
-def kernels(f):
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
-        f()
-        torch.cuda.synchronize()
-    return {e.key for e in p.key_averages()}
-torch.zeros(1, device="cuda")
 pairs, plain = [], []
 for k in (1, 2):
     bits = 150000 + k
@@ -54,9 +48,9 @@ for k in (1, 2):
     plain.append((a, b))
     pairs.append((M.DeviceBuffer.from_array(a), bits, M.DeviceBuffer.from_array(b), bits - 7))
 got = []
-names = kernels(lambda: got.append(E.gcd_large(pairs, g_cap_words=8, max_parallel=2)))
-assert any("k_hgcd_base" in k for k in names), names
-assert not any("k_bfly" in k or "k_slice" in k for k in names), names
+names = kernel_counts(lambda: got.append(E.gcd_large(pairs, g_cap_words=8, max_parallel=2)))
+assert launched(names, "k_hgcd_base"), names
+assert not launched(names, "k_bfly") and not launched(names, "k_slice"), names
 for (a, b), d in zip(plain, got[0][0]):
     assert int(d) == O.poly_gcd(a, b)[0]
 print("ok")
