@@ -38,8 +38,9 @@
 // applied class by class, two at a time (both windows' 16 loads issued before
 // either is used) with no masks or bounds tests; the rest (windows that start
 // or end inside the tile, a few tiles per state) with per-lane bit masks and
-// bounds-tested loads.  The kernel is bound by memory latency (6 of 15 cycles
-// between a warp's instructions) and the integer pipe together.  A pass of 64
+// bounds-tested loads.  The kernel is bound by memory latency: 7 of 17 cycles
+// between a warp's instructions wait for loads, the integer pipe is 48 % busy
+// and 53 % of the issue slots are used (8 states).  A pass of 64
 // states at r = 136279841: windows one at a time with the high words by
 // shuffle 1.06 ms, the per-tile list with two loads a unit 0.72 ms, two
 // windows at a time 0.65 ms, fast windows listed by class 0.58 ms (1 state 29

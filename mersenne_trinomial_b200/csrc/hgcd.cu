@@ -4,7 +4,7 @@
 // NTL's GF2X GCD (gf2_gcd_ntl.cpp:32-42; a half-gcd over gf2x products,
 // ~62 s per gcd on 6 CPU cores) or its hybrid HGCD with GPU multiplies
 // (gf2_gcd_ntl.cpp:360-452, GpuMulHook gf2_gcd.h:155-190).  The quadratic
-// GPU gcd (gcd.cu) is fine to ~10^6 bits; this file is the r-bit path.
+// GPU gcd (gcd.cu) is fine to ~10^5 bits; this file is the r-bit path.
 //
 // Algorithm (the classical polynomial half-gcd; every matrix is unimodular
 // over GF(2), so the gcd is preserved whatever the degrees do, and the
@@ -438,7 +438,8 @@ struct Tunables {
 
 // A lockstep batch fills the GPU with every product, so the FFT's lower
 // work pays from smaller sizes than for one gcd, whose small products leave
-// most SMs idle either way (measured, 64 gcds of 16 Mbit at once: 6.3 s
+// most SMs idle either way (measured with the word passes, 64 gcds of 16 Mbit
+// at once, which take 3.6 s from 2^16 with the sliced ones: 6.3 s
 // with the FFT from 2^15 bits, 6.5 s from 2^16, 7.5 s from 2^17, 8.3 s from
 // 2^18, 11.7 s from 2^19, 17.2 s from 2^20).
 Tunables tunables(bool lockstep = false) {
