@@ -8,7 +8,7 @@
 // the ALU.  A "slice" is 32 consecutive elements held as 64 bit planes of 32
 // bits (bit e of plane p = coordinate p of element e), 256 bytes, the same
 // place in memory as the 32 elements.  GF(2^64) is taken in the tower basis
-// x_k^2 = x_(k-1) x_k + 1 (coordinate i is the product of the x_k over the
+// x_k^2 = x_(k-1) x_k + 1 (Wiedemann's tower; coordinate i is the product of the x_k over the
 // set bits k of i), in which the subfields GF(2^8), GF(2^16), GF(2^32) are the
 // low 8, 16, 32 coordinates.  The twiddle of butterfly level L is a sum of the
 // Cantor basis elements 1 .. m-1-L, which lie in those subfields, so a

@@ -23,10 +23,13 @@ def test_long_operand_with_one(engine, oracle, bits):
     buf = engine.DeviceBuffer.from_array
     pairs = [(buf(a), bits, buf(one), 1), (buf(one), 1, buf(a), bits), (buf(x), 700, buf(y), 650)]
     engine.engine.gcd_batch(pairs, g_cap_words=16)             # the kernel is loaded
-    t0 = time.perf_counter()
-    degs, gs = engine.engine.gcd_batch(pairs, g_cap_words=16)
+    best = 1e9
+    for _ in range(5):
+        t0 = time.perf_counter()
+        degs, gs = engine.engine.gcd_batch(pairs, g_cap_words=16)
+        best = min(best, time.perf_counter() - t0)
     # a round for each coefficient is 0.2 s and more, the small gcd 0.1 ms
-    assert time.perf_counter() - t0 < 0.05
+    assert best < 0.05
     assert degs[0] == degs[1] == 0
     for g in gs[:2]:
         assert g[0] == 1 and not g[1:].any()
