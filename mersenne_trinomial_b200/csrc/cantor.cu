@@ -941,8 +941,7 @@ int fft_plan_create_cfg(int m, const gf2e_tune &cfg, gf2e_fft_plan **out) {
     twiddle_byte_tables(tab.data());
     u64 *d_tab = nullptr;
     cudaError_t e = cudaMalloc(&d_tab, tab.size() * sizeof(u64));
-    if (e == cudaSuccess)
-        e = cudaMemcpy(d_tab, tab.data(), tab.size() * sizeof(u64), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = upload_and_wait(d_tab, tab.data(), tab.size() * sizeof(u64));
     if (e != cudaSuccess) {
         cudaFree(d_tab);
         return cuda_status(e, "fft plan twiddle tables");

@@ -39,6 +39,15 @@ inline int invalid(const char *fmt, ...) {
 int grid_for(size_t work, int threads, int ctas_per_sm = 8);
 int sm_count();
 
+// host memory to the device, there when the call returns: cudaMemcpy from
+// pageable memory may return with the last of the copy under way, on a stream
+// that others (the library's and most callers' are non-blocking ones) do not
+// wait for
+inline cudaError_t upload_and_wait(void *dst, const void *src, size_t bytes) {
+    const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+    return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
 // process-wide tuning in force (defaults, then environment overrides)
 gf2e_tune tune_current();
 

@@ -60,7 +60,7 @@ int setup_device(int dev) {
         return gf2e::invalid("twiddle table size mismatch");
     u64 host_tab[TAB_WORDS];
     gf2e::twiddle_byte_tables(host_tab);
-    e = cudaMemcpyToSymbol(g_noalloc_twiddles, host_tab, sizeof host_tab);
+    e = gf2e::upload_and_wait(d.twiddles, host_tab, sizeof host_tab);
     if (e != cudaSuccess) return gf2e::cuda_status(e, "noalloc twiddle upload");
     // plans go into a local table first: a failure part way destroys the
     // ones already made, and the next call starts the set-up afresh

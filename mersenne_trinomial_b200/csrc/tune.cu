@@ -209,7 +209,7 @@ int gf2e_fft_autotune(int m, int reps, gf2e_tune *best, double *best_ms, char *r
         std::vector<u64> h(n);
         u64 s = 0xfeedfaceull;
         for (auto &w : h) w = splitmix(s);
-        cudaError_t e = cudaMemcpy(d_in, h.data(), n * 8, cudaMemcpyHostToDevice);
+        cudaError_t e = gf2e::upload_and_wait(d_in, h.data(), n * 8);
         if (e != cudaSuccess) return gf2e::cuda_status(e, "autotune input");
     }
     // reference forward transform under the built-in default tuning
