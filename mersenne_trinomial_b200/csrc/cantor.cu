@@ -7,8 +7,9 @@
 //
 // Products of up to 2^23 coefficients and single transforms of 2^11 .. 2^24
 // run bit-sliced in a tower basis (slicefft.cu); what follows is the word form,
-// for the other sizes, buffers on 8 bytes only, and plans with the levels of
-// the reference (GF2E_FFT_TAYLOR).
+// for the other sizes, large batches of short products, buffers on 8 bytes only
+// or shared with an operand, and plans with the levels of the reference
+// (GF2E_FFT_TAYLOR).
 //
 // B200 mapping.  Every Taylor level and butterfly level acts on "rows" of a
 // strided 2-D view of the array, so a run of consecutive levels fits in one
